@@ -86,7 +86,8 @@ class CompileOpts(ctypes.Structure):
     """``kcg_compile_opts``."""
     _fields_ = [("kernel", ctypes.c_int32), ("num_stages", ctypes.c_int32),
                 ("num_sms", ctypes.c_int32), ("force", ctypes.c_int32), ("b_trans", ctypes.c_int32),
-                ("serpentine", ctypes.c_int32), ("reserved", ctypes.c_int32 * 2)]
+                ("serpentine", ctypes.c_int32), ("edge_tiles", ctypes.c_int32),
+                ("reserved", ctypes.c_int32 * 1)]
 
 
 class Epilogue(ctypes.Structure):

@@ -247,6 +247,7 @@ struct Resolved {
   int btrans = 0;
   int serpentine = 0;
   int out_f32 = 0;  // DATATYPE_C = float32 with 16-bit A and B
+  int edge = 0;     // tiles may hang over the edges of the problem
 };
 
 // The reference's KernelArgMatmul.check() (Operators/matmul.py:180-194) for the
@@ -289,6 +290,9 @@ int simt_smem_bytes(const Cfg& c) {
   return 4 * (ab > cc ? ab : cc);
 }
 
+// Tiles (or K blocks) of `b` that cover `n`; the last one may hang over.
+int blocks_of(int n, int b) { return b > 0 ? (n + b - 1) / b : n; }
+
 int resolve(const Cfg& c, const kcg_compile_opts* opts, Resolved* r) {
   const int dt = c[KCG_CFG_DATATYPE_A];
   if (!dtype_str(dt)) return fail(KCG_E_BAD_CONFIG, "unsupported DATATYPE_A %d (2 float16, 4 float32, 62 bfloat16)", dt);
@@ -303,7 +307,8 @@ int resolve(const Cfg& c, const kcg_compile_opts* opts, Resolved* r) {
   if (bm <= 0 || bn <= 0 || bk <= 0 || M <= 0 || N <= 0 || K <= 0)
     return fail(KCG_E_BAD_CONFIG, "sizes must be positive");
   // problem-size check of KernelArgMatmul.check()
-  if (M % bm || N % bn || K % bk)
+  r->edge = (opts && opts->edge_tiles) ? 1 : 0;
+  if (!r->edge && (M % bm || N % bn || K % bk))
     return fail(KCG_E_BAD_CONFIG, "M,N,K = %d,%d,%d not divisible by BLOCK_SIZE_M,N,K = %d,%d,%d", M, N, K, bm, bn, bk);
   r->num_sms = (opts && opts->num_sms > 0) ? opts->num_sms : 148;
   int want = opts ? opts->kernel : KCG_KERNEL_AUTO;
@@ -320,6 +325,15 @@ int resolve(const Cfg& c, const kcg_compile_opts* opts, Resolved* r) {
     want = (kcg::tc_config_error(dt, bm, bn, bk, st, 1) == 0) ? KCG_KERNEL_TCGEN05 : KCG_KERNEL_SIMT;
   }
   r->kernel = want;
+  if (r->edge) {
+    // Tiles that hang over an edge: TMA reads zeros past it and clips the stores; direct stores and the fused
+    // epilogue work in whole blocks of 32 (fp32) or 64 columns, which therefore must not straddle the edge.
+    if (!(want == KCG_KERNEL_TCGEN05 || want == KCG_KERNEL_TCGEN05_PAIR || want == KCG_KERNEL_TCGEN05_CLUSTERK))
+      return fail(KCG_E_BAD_CONFIG, "tiles over the edge need a tcgen05 kernel (KERNEL_VARIANT 2, 4 or 5)");
+    const int nstep = dt == KCG_DTYPE_FLOAT32 ? 32 : 64;
+    if (N % nstep || (K * (dt == KCG_DTYPE_FLOAT32 ? 4 : 2)) % 16)
+      return fail(KCG_E_BAD_CONFIG, "tiles over the edge need N a multiple of %d and rows of 16-byte units", nstep);
+  }
   if (r->out_f32 && !(want == KCG_KERNEL_TCGEN05 || want == KCG_KERNEL_TCGEN05_PAIR))
     return fail(KCG_E_BAD_CONFIG, "a float32 C with 16-bit A and B needs a single-pass tcgen05 kernel (KERNEL_VARIANT 2 or 4)");
   r->btrans = (opts && opts->b_trans) ? 1 : 0;
@@ -330,8 +344,11 @@ int resolve(const Cfg& c, const kcg_compile_opts* opts, Resolved* r) {
   if (r->serpentine && c[KCG_CFG_BLOCK_MAPPING] < 2)
     return fail(KCG_E_BAD_CONFIG, "the serpentine raster needs BLOCK_MAPPING >= 2 (rows per group)");
   if (r->btrans) {
-    const bool single_pass16 = (want == KCG_KERNEL_TCGEN05 || want == KCG_KERNEL_TCGEN05_PAIR) && dt != KCG_DTYPE_FLOAT32;
-    if (!single_pass16)
+    // (the cluster split-K kernel takes it under the extended rules only: a plain config of it stays rejected)
+    const bool tc16 = (want == KCG_KERNEL_TCGEN05 || want == KCG_KERNEL_TCGEN05_PAIR ||
+                       (want == KCG_KERNEL_TCGEN05_CLUSTERK && r->edge)) &&
+                      dt != KCG_DTYPE_FLOAT32;
+    if (!tc16)
       return fail(KCG_E_BAD_CONFIG, "a B stored N x K (b_trans) needs a single-pass tcgen05 kernel with fp16 / bf16 data");
     if (K % 8) return fail(KCG_E_BAD_CONFIG, "K must be a multiple of 8 for the TMA row stride of an N x K stored B");
   }
@@ -343,7 +360,7 @@ int resolve(const Cfg& c, const kcg_compile_opts* opts, Resolved* r) {
     if (e) return fail(KCG_E_BAD_CONFIG, "tile %dx%dx%d / %d stages not buildable by the tcgen05 kernel (rule %d)", bm, bn, bk, r->stages, e);
     if (N % 8) return fail(KCG_E_BAD_CONFIG, "N must be a multiple of 8 for TMA row strides");
     const int splitk = c[KCG_CFG_LOCAL_SPLIT_U] > 0 ? c[KCG_CFG_LOCAL_SPLIT_U] : 1;
-    if (splitk > K / bk) return fail(KCG_E_BAD_CONFIG, "LOCAL_SPLIT_U %d exceeds the %d K blocks", splitk, K / bk);
+    if (splitk > blocks_of(K, bk)) return fail(KCG_E_BAD_CONFIG, "LOCAL_SPLIT_U %d exceeds the %d K blocks", splitk, blocks_of(K, bk));
   } else if (want == KCG_KERNEL_TCGEN05_PAIR) {
     // CTA pairs: each CTA holds BM/2 rows of the tile and BN/2 columns of B
     const int f32 = (dt == KCG_DTYPE_FLOAT32) ? 1 : 0;
@@ -352,7 +369,7 @@ int resolve(const Cfg& c, const kcg_compile_opts* opts, Resolved* r) {
     if ((bm / 256) * bn > (f32 ? 256 : 512))
       return fail(KCG_E_BAD_CONFIG, "accumulators of the tile exceed the TMEM columns available");
     const int splitk = c[KCG_CFG_LOCAL_SPLIT_U] > 0 ? c[KCG_CFG_LOCAL_SPLIT_U] : 1;
-    if (splitk > K / bk) return fail(KCG_E_BAD_CONFIG, "LOCAL_SPLIT_U %d exceeds the %d K blocks", splitk, K / bk);
+    if (splitk > blocks_of(K, bk)) return fail(KCG_E_BAD_CONFIG, "LOCAL_SPLIT_U %d exceeds the %d K blocks", splitk, blocks_of(K, bk));
     auto ok = [&](int st) { return bn % 2 == 0 && kcg::tc_config_error(dt, bm / 2, bn / 2, bk, st, f32) == 0; };
     int st = (opts && opts->num_stages > 0) ? opts->num_stages : 2;
     if (!(opts && opts->num_stages > 0) && c[KCG_CFG_SHARED_PREFETCH])
@@ -364,7 +381,7 @@ int resolve(const Cfg& c, const kcg_compile_opts* opts, Resolved* r) {
     // one 128-row tile per cluster of LOCAL_SPLIT_U CTAs, partial tiles reduced in shared memory
     const int split = c[KCG_CFG_LOCAL_SPLIT_U];
     if (bm != 128) return fail(KCG_E_BAD_CONFIG, "the cluster split-K kernel needs BLOCK_SIZE_M = 128");
-    if (split > K / bk) return fail(KCG_E_BAD_CONFIG, "LOCAL_SPLIT_U %d exceeds the %d K blocks", split, K / bk);
+    if (split > blocks_of(K, bk)) return fail(KCG_E_BAD_CONFIG, "LOCAL_SPLIT_U %d exceeds the %d K blocks", split, blocks_of(K, bk));
     auto ok = [&](int st) { return kcg::ck_config_error(dt, bn, bk, st, split) == 0; };
     int st = (opts && opts->num_stages > 0) ? opts->num_stages : 2;
     if (!(opts && opts->num_stages > 0)) {
@@ -610,7 +627,7 @@ int fill_info(const Cfg& c, const Resolved& r, const std::string& name, const st
   const int bm = c[KCG_CFG_BLOCK_SIZE_M], bn = c[KCG_CFG_BLOCK_SIZE_N], bk = c[KCG_CFG_BLOCK_SIZE_K];
   const int M = c[KCG_CFG_M_SIZE], N = c[KCG_CFG_N_SIZE], K = c[KCG_CFG_K_SIZE];
   const int lsu = c[KCG_CFG_LOCAL_SPLIT_U] > 0 ? c[KCG_CFG_LOCAL_SPLIT_U] : 1;
-  const int tiles = (M / bm) * (N / bn);
+  const int tiles = blocks_of(M, bm) * blocks_of(N, bn);
   out->grid[1] = out->grid[2] = out->block[1] = out->block[2] = 1;
   out->cluster[0] = out->cluster[1] = out->cluster[2] = 1;
   if (r.kernel == KCG_KERNEL_TCGEN05 || r.kernel == KCG_KERNEL_TF32X1) {
@@ -731,8 +748,8 @@ SplitPlan plan_split(const kcg_kernel_info* info, bool fused_epilogue, int batch
   // KCG_TAIL_SPLIT=0 turns the split off, =2 selects the even split, =3 / =4 stream-K / the even
   // split without the cost gate, =5 stream-K over the remainder alone BEFORE the whole tiles (the
   // last arriver sums a tile; no gate; an experiment that measured no consistent gain).
-  const int T = (M / info->bm) * (N / info->bn);
-  const int num_kb = K / info->bk;
+  const int T = blocks_of(M, info->bm) * blocks_of(N, info->bn);
+  const int num_kb = blocks_of(K, info->bk);
   const int nsm = info->reserved[0] > 0 ? info->reserved[0] : 148;
   const int G = pair ? nsm / 2 : nsm;  // work units that run at once (CTAs, or CTA pairs)
   int first = T, factor = 1, sk_per = 0, sk_ranges = 0;
@@ -1083,6 +1100,9 @@ static int launch_impl(uint64_t function, const kcg_kernel_info* info, int devic
     if (!tc) return fail(KCG_E_BAD_CONFIG, "batched launches need a tcgen05 kernel (KERNEL_VARIANT 2, 3, 4 or 5)");
     if (static_cast<int64_t>(info->m) * batch > 0x7fffffff || static_cast<int64_t>(info->k) * batch > 0x7fffffff)
       return fail(KCG_E_TOO_LARGE, "batch * M and batch * K must fit 31 bits");
+    // past the end of one batch lie the next batch's rows, not zeros
+    if (info->m % info->bm || info->k % info->bk)
+      return fail(KCG_E_BAD_CONFIG, "a batched launch needs M and K divisible by BLOCK_SIZE_M and BLOCK_SIZE_K");
   }
   if (n_peers < 0 || n_peers > KCG_MAX_PEERS || (n_peers > 0 && !peer_c))
     return fail(KCG_E_BAD_ARG, "n_peers must be 0..%d with their addresses", KCG_MAX_PEERS);
@@ -1137,7 +1157,7 @@ static int launch_impl(uint64_t function, const kcg_kernel_info* info, int devic
   p.ldb = static_cast<int>(ldb);
   p.ldc = static_cast<int>(ldc);
   p.status = reinterpret_cast<unsigned int*>(slot->status);
-  p.split_first_tile = (M / (info->bm > 0 ? info->bm : 1)) * (N / (info->bn > 0 ? info->bn : 1));
+  p.split_first_tile = blocks_of(M, info->bm) * blocks_of(N, info->bn);
   p.split_factor = 1;
   p.alpha = 1.f;
   if (epi) {
@@ -1171,8 +1191,9 @@ static int launch_impl(uint64_t function, const kcg_kernel_info* info, int devic
   };
   if (info->kernel == KCG_KERNEL_TCGEN05_CLUSTERK) {
     // One cluster per tile; the K split and its reduction stay inside the cluster (no workspace).
-    if (int e = encode_operands(kcg::make_tc_layout(info->dtype, info->bm, info->bn, info->bk, info->atrans))) return e;
-    grid0 = (M / info->bm) * (N / info->bn) * info->splitk;
+    if (int e = encode_operands(kcg::make_tc_layout(info->dtype, info->bm, info->bn, info->bk, info->atrans, btrans)))
+      return e;
+    grid0 = blocks_of(M, info->bm) * blocks_of(N, info->bn) * info->splitk;
   }
   if (info->kernel == KCG_KERNEL_TCGEN05 || info->kernel == KCG_KERNEL_TF32X1 || pair) {
     // the pair kernel loads per-CTA slices: BM/2 rows of A, BN/2 columns of B
@@ -1322,7 +1343,7 @@ int kcg_matmul_host(uint64_t function, const kcg_kernel_info* info, int device, 
   // transfers in both directions and the kernels overlap; B goes in first. Tiles do not straddle
   // slabs: a slab is a multiple of BLOCK_SIZE_M rows.
   const int bm = info->bm > 0 ? info->bm : 1;
-  const int tiles_m = info->m / bm;
+  const int tiles_m = blocks_of(info->m, bm);
   const bool tensor_core = info->kernel == KCG_KERNEL_TCGEN05 || info->kernel == KCG_KERNEL_TF32X1 ||
                            info->kernel == KCG_KERNEL_TCGEN05_PAIR;
   int nslabs = 1;
@@ -1383,7 +1404,8 @@ int kcg_matmul_host(uint64_t function, const kcg_kernel_info* info, int device, 
   const int base_tiles = tiles_m / nslabs, extra = tiles_m % nslabs;
   size_t row0 = 0;
   for (int i = 0; i < nslabs && rc == 0; ++i) {
-    const size_t rows = static_cast<size_t>(base_tiles + (i < extra ? 1 : 0)) * bm;
+    size_t rows = static_cast<size_t>(base_tiles + (i < extra ? 1 : 0)) * bm;
+    if (row0 + rows > static_cast<size_t>(info->m)) rows = info->m - row0;  // a tile row that hangs over the edge
     const size_t a_off = row0 * info->k * eb, c_off = row0 * info->n * eb_c;
     if (!step(d.p_cuMemcpyHtoDAsync(s->hbuf[0] + a_off, static_cast<const char*>(hostA) + a_off, rows * info->k * eb,
                                     s_in), "cuMemcpyHtoDAsync(A)"))

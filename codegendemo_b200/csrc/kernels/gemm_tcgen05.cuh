@@ -538,6 +538,9 @@ struct TcGemm {
             const int row0 = w.m0 + row_base + t * 128 + q * 32;
 #pragma unroll 1
             for (int g = 0; g < kBN / SCOLS; ++g, ++stg_it) {
+              // A tile that hangs over C's edge: the blocks past it are left out as a whole. (The buffer rotation
+              // counts one bulk group per filled buffer, so a block must not be staged without being stored.)
+              if (row0 >= p.M || w.n0 + g * SCOLS >= p.N) break;
               uint8_t* buf = stg + (stg_it & 1u) * STG_BYTES;
               KCG_TLC(c_e0);
               if (lane == 0) tma_store_wait_read<1>();  // the store that last read `buf` is done
@@ -556,6 +559,7 @@ struct TcGemm {
                 va[i] = __uint_as_float(ra[i]);
                 if constexpr (SCOLS == 64) vb[i] = __uint_as_float(rb[i]);
               }
+              // (N is a multiple of a staging block's columns wherever tiles may hang over: a block is inside or outside)
               if (p.epi_flags != 0u && row0 + lane < p.M) {
                 epi_span<OutT, 32>(p, va, row0 + lane, w.n0 + g * SCOLS);
                 if constexpr (SCOLS == 64) epi_span<OutT, 32>(p, vb, row0 + lane, w.n0 + g * SCOLS + 32);
@@ -590,8 +594,8 @@ struct TcGemm {
               fence_proxy_async_smem();  // generic-proxy writes visible to the TMA engine
               __syncwarp();
               const int col0 = w.n0 + g * SCOLS;
-              if (lane == 0 && row0 < p.M && col0 < p.N) {
-                tma_store_2d(&p.tmC, buf, col0, row0);  // rows / columns past the edge are clipped
+              if (lane == 0) {
+                tma_store_2d(&p.tmC, buf, col0, row0);  // rows past the edge are clipped
                 tma_store_commit();
               }
               if (warp == 2 && lane == 0) KCG_TLC_ADD(23, c_e3);
@@ -752,8 +756,9 @@ struct TcGemm {
               constexpr int PPR = SCOLS / 4;               // 16-byte pieces of a partial per block row
               constexpr int PIECES = 32 * PPR;             // ... per block
               constexpr int UNR = 8, JB = 2;  // pieces per lane and partials fetched before any is added
-              for (int blk = b_lo + (warp - 2); blk < b_hi; blk += 4, ++stg_it) {
+              for (int blk = b_lo + (warp - 2); blk < b_hi; blk += 4) {
                 const int rb = blk / BLK_PER_ROWBLOCK, g = blk - rb * BLK_PER_ROWBLOCK;
+                if (w.m0 + row_base + rb * 32 >= p.M || w.n0 + g * SCOLS >= p.N) continue;  // past C's edge
                 uint8_t* buf = stg + (stg_it & 1u) * STG_BYTES;
                 if (lane == 0) tma_store_wait_read<1>();  // the store that last read `buf` is done
                 __syncwarp();
@@ -824,10 +829,11 @@ struct TcGemm {
                 fence_proxy_async_smem();  // generic-proxy writes visible to the TMA engine
                 __syncwarp();
                 const int row0 = w.m0 + row_base + rb * 32, col0 = w.n0 + g * SCOLS;
-                if (lane == 0 && row0 < p.M && col0 < p.N) {
-                  tma_store_2d(&p.tmC, buf, col0, row0);  // rows / columns past the edge are clipped
+                if (lane == 0) {
+                  tma_store_2d(&p.tmC, buf, col0, row0);  // rows past the edge are clipped
                   tma_store_commit();
                 }
+                ++stg_it;
               }
             };
             // Shares are runs of such blocks when every split unit of the launch is followed by whole

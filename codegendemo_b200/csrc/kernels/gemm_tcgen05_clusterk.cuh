@@ -40,12 +40,13 @@
 
 namespace kcg {
 
-template <int kDType, int kBN, int kBK, int kStages, int kATrans, int kSplit, int kGroup>
+// kBTrans = 1: B stored N x K, as in gemm_tcgen05.cuh.
+template <int kDType, int kBN, int kBK, int kStages, int kATrans, int kSplit, int kGroup, int kBTrans = 0>
 struct TcGemmClusterK {
   static constexpr int kBM = 128;
   static_assert(ck_config_error(kDType, kBN, kBK, kStages, kSplit) == 0,
                 "config not buildable by the cluster split-K kernel");
-  static constexpr TcLayout L = make_tc_layout(kDType, kBM, kBN, kBK, kATrans);
+  static constexpr TcLayout L = make_tc_layout(kDType, kBM, kBN, kBK, kATrans, kBTrans);
   static constexpr int EB = 2;
   static constexpr int UMMA_K = 16;
   static constexpr int KSTEPS = kBK / UMMA_K;
@@ -67,7 +68,7 @@ struct TcGemmClusterK {
   static constexpr int SMEM_BYTES = ck_smem_bytes(kBN, kBK, kStages);
   static_assert(RECV_BYTES + STAGE_OUT_BYTES <= kStages * STAGE_BYTES, "the ring must hold the exchange buffers");
   static constexpr uint32_t FMT = (kDType == KCG_DT_BF16) ? FMT_BF16 : FMT_F16;
-  static constexpr uint32_t IDESC = make_instr_desc(FMT, kATrans ? 1u : 0u, 1u, 128u, kBN);
+  static constexpr uint32_t IDESC = make_instr_desc(FMT, kATrans ? 1u : 0u, kBTrans ? 0u : 1u, 128u, kBN);
 
   struct Barriers {
     uint64_t full[kStages];
@@ -232,8 +233,13 @@ struct TcGemmClusterK {
             }
           }
 #pragma unroll
-          for (int j = 0; j < L.b_boxes; ++j)
-            tma_load_2d(sb + j * L.b_box_bytes, &p.tmB, &bars->full[s], w.n0 + j * L.atom, kb_row);
+          for (int j = 0; j < L.b_boxes; ++j) {
+            if constexpr (kBTrans) {  // N x K storage: the batch selects N rows
+              tma_load_2d(sb + j * L.b_box_bytes, &p.tmB, &bars->full[s], k0 + j * L.b_box_inner, w.n0 + w.nofs);
+            } else {
+              tma_load_2d(sb + j * L.b_box_bytes, &p.tmB, &bars->full[s], w.n0 + j * L.atom, kb_row);
+            }
+          }
           if (kb == 0) KCG_CTL(2);
         }
       }
@@ -270,7 +276,13 @@ struct TcGemmClusterK {
               constexpr int swb = (kBK * EB < 128) ? kBK * EB : 128;
               a_off = ((ks * 32) / swb) * L.a_box_bytes + ((ks * 32) % swb);
             }
-            const uint32_t b_off = ks * UMMA_K * 128;
+            uint32_t b_off;
+            if constexpr (kBTrans) {
+              constexpr int swb = (kBK * EB < 128) ? kBK * EB : 128;
+              b_off = ((ks * 32) / swb) * L.b_box_bytes + ((ks * 32) % swb);
+            } else {
+              b_off = ks * UMMA_K * 128;
+            }
             const uint64_t adesc = make_smem_desc(sa + a_off, L.a_lbo, L.a_sbo, L.a_desc_swizzle);
             const uint64_t bdesc = make_smem_desc(sb + b_off, L.b_lbo, L.b_sbo, L.b_desc_swizzle);
             umma_ss<false>(tmem_base, adesc, bdesc, IDESC, (kb > 0 || ks > 0) ? 1u : 0u);

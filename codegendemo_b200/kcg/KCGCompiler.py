@@ -22,10 +22,11 @@ def compile_kernel_matmul(*args, num_stages: int = 0, kernel: int = 0, num_sms: 
 
 
 def compile_info(cfg31, num_stages: int = 0, kernel: int = 0, num_sms: int = 0, force: bool = False,
-                 b_trans: int = 0, serpentine: int = 0) -> _lib.KernelInfo:
+                 b_trans: int = 0, serpentine: int = 0, edge_tiles: int = 0) -> _lib.KernelInfo:
     lib = _lib.get_lib()
     opts = _lib.CompileOpts(kernel=int(kernel), num_stages=int(num_stages), num_sms=int(num_sms), force=int(bool(force)),
-                            b_trans=int(bool(b_trans)), serpentine=int(bool(serpentine)))
+                            b_trans=int(bool(b_trans)), serpentine=int(bool(serpentine)),
+                            edge_tiles=int(bool(edge_tiles)))
     info = _lib.KernelInfo()
     _lib.check(lib.kcg_compile_matmul_ex(_lib.cfg_array(cfg31), ctypes.byref(opts), ctypes.byref(info)))
     return info
@@ -38,7 +39,7 @@ class KCGCompiler:
 
     def compileKernel(self, param: KernelArgMatmul) -> list:
         info = compile_info(param.compileArgs(), num_stages=param.NUM_STAGES, kernel=param.KERNEL_VARIANT,
-                            b_trans=param.IS_BTRANS, serpentine=param.RASTER_SERPENTINE)
+                            b_trans=param.IS_BTRANS, serpentine=param.RASTER_SERPENTINE, edge_tiles=param.EDGE_TILES)
         self.lastInfo = info.to_dict()
         return [(info.path.decode(), info.name.decode(), info.grid[0], info.grid[1], info.grid[2],
                  info.block[0], info.block[1], info.block[2])]

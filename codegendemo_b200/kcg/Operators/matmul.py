@@ -32,7 +32,8 @@ _ATTR_TO_KEY = {
     "REDUCE_C_CONTINUOUS": ConfigKeywords.KEY_REDUCE_C_CONTINUOUS,
 }
 _OPTIONAL = {"NUM_STAGES": ConfigKeywords.KEY_NUM_STAGES, "KERNEL_VARIANT": ConfigKeywords.KEY_KERNEL_VARIANT,
-             "IS_BTRANS": ConfigKeywords.KEY_IS_B_TRANSPOSE, "RASTER_SERPENTINE": ConfigKeywords.KEY_RASTER_SERPENTINE}
+             "IS_BTRANS": ConfigKeywords.KEY_IS_B_TRANSPOSE, "RASTER_SERPENTINE": ConfigKeywords.KEY_RASTER_SERPENTINE,
+             "EDGE_TILES": ConfigKeywords.KEY_EDGE_TILES}
 
 # Shared memory one CTA may use on sm_100a (the reference asserts 64 KiB for gfx906).
 MAX_SHARED_BYTES = 227 * 1024
@@ -87,6 +88,7 @@ class KernelArgMatmul:
         self.NUM_STAGES = 0       # 0 = derive from SHARED_PREFETCH
         self.KERNEL_VARIANT = 0   # 0 = auto
         self.IS_BTRANS = 0        # 1 = B is stored N x K (tcgen05 16-bit kernels)
+        self.EDGE_TILES = 0       # 1 = M, N, K need not be multiples of the tile (tcgen05 kernels)
         self.RASTER_SERPENTINE = 0  # 1 = odd tile columns of a BLOCK_MAPPING group walk its rows upwards
 
     def jsonfy(self) -> Dict:
@@ -124,9 +126,14 @@ class KernelArgMatmul:
 
     def check(self, verbose: bool = False) -> None:
         # problem size check
-        assert self.M % self.BLOCK_SIZE_M == 0
-        assert self.N % self.BLOCK_SIZE_N == 0
-        assert self.K % self.BLOCK_SIZE_K == 0
+        if self.EDGE_TILES:  # tiles hang over the edges; the store works in whole blocks of 32 (fp32) or 64 columns
+            assert self.usesTensorCores()
+            assert self.N % (32 if sizeof(self.__dataType_A) == 4 else 64) == 0
+            assert (self.K * sizeof(self.__dataType_A)) % 16 == 0
+        else:
+            assert self.M % self.BLOCK_SIZE_M == 0
+            assert self.N % self.BLOCK_SIZE_N == 0
+            assert self.K % self.BLOCK_SIZE_K == 0
         if not self.usesTensorCores():
             # warp-block validation check (the thread-level keys drive the SIMT kernel only)
             assert self.BLOCK_SIZE_M % self.THREAD_SIZE_M == 0

@@ -36,15 +36,114 @@ def default_config(M: int, N: int, K: int, dtype: EnumKernelDType, out_dtype=Non
     return kpm
 
 
-def tuned_config(M: int, N: int, K: int, dtype: EnumKernelDType, isATranspose: int = 0, db=None) -> KernelArgMatmul:
-    """Best known config of a shape: the kernel database's entry when the shape was tuned, else a
-    rule of thumb from the B200 measurements (CTA-pair kernels once their larger tiles still fill
-    the 74 pairs for several waves, single-CTA 256x256 / 128x256 tiles otherwise)."""
+# Tiles of the 16-bit kernels the rule below chooses from: (KERNEL_VARIANT, BLOCK_SIZE_M, N, K) -> microseconds
+# {fixed, per K block, per tile beyond its K blocks}. Fitted to 4 900 device timings (CUDA-graph replay, operands
+# rotating) of 36 tiles on 127 shapes of 128..32768 x 512..16384 x 256..16384, B stored either way; on the same
+# shapes the tile the fit picks is within 1 % of the best measured one on average (worst 10 %), where the former
+# rule - tiles had to divide the problem - averaged 22 % behind it (1664 x 2752 x 1472: 33 -> 12.9 us;
+# 11136 x 7488 x 1792: 608 -> 205 us; 128 x 1344 x 3072: 17.3 -> 7.7 us). For the cluster split-K kernel the third
+# figure is one per LOCAL_SPLIT_U of 2, 3, 4.
+_TILE_COST = {
+    (2, 128, 64, 128): (2.85, 0.433, 0.54),
+    (2, 128, 128, 128): (2.94, 0.499, 0.53),
+    (2, 128, 192, 64): (3.03, 0.344, 0.78),
+    (2, 128, 256, 64): (2.81, 0.384, 1.28),
+    (2, 256, 192, 64): (2.30, 0.57, 2.70),
+    (2, 256, 256, 64): (1.77, 0.645, 4.13),
+    (4, 256, 128, 128): (3.38, 0.469, 1.04),
+    (4, 256, 256, 64): (3.37, 0.35, 1.58),
+    (4, 256, 256, 128): (3.21, 0.663, 1.68),
+    (4, 512, 256, 64): (2.02, 0.62, 5.45),
+    (5, 128, 64, 128): (1.0, 0.45, (3.10,)),
+    (5, 128, 128, 128): (1.0, 0.505, (4.24, 4.65, 4.69)),
+    (5, 128, 192, 64): (1.0, 0.322, (5.15, 5.60, 6.32)),
+    (5, 128, 256, 64): (1.0, 0.379, (5.77, 6.37, 6.61)),
+}
+_CLUSTERS = {2: 74, 3: 45, 4: 33}  # clusters of 2, 3, 4 CTAs at 200 KB of shared memory each that run at once
+
+
+def _tile_us(tile, split, M, N, K, batch=1, sms=148):
+    """Estimated time of a 16-bit product with one of the tiles above, in microseconds."""
+    variant, bm, bn, bk = tile
+    fixed, per_block, per_tile = _TILE_COST[tile]
+    tiles, blocks = batch * -(-M // bm) * -(-N // bn), -(-K // bk)
+    stream = 2.0 + 2e-6 * batch * (M * K + K * N + M * N) / 5.5  # operands and result through HBM at 5.5 TB/s
+    if variant == 5:
+        return max(stream, fixed + -(-blocks // split) * per_block + per_tile[split - 2])
+    at_once = sms // 2 if variant == 4 else sms
+    waves, rest = -(-tiles // at_once), tiles % at_once
+    f = min(8, at_once // rest) if rest else 0
+    while f >= 2 and -(-blocks // f) * (f - 1) >= blocks:
+        f -= 1
+    if tiles > at_once and f >= 2:  # the launcher cuts the remainder tiles into f K ranges when that pays
+        rows = bm // 2 if variant == 4 else bm
+        tile_us = 2e-7 * rows * bn * K
+        if tile_us * (1.0 - 1.0 / f) > 1.25 * (3.0 + max(0.0, 1.5 + 0.14 * rows * bn / 256 - tile_us)):
+            waves = tiles // at_once + 1.0 / f + 3.0 / tile_us
+    return max(stream, fixed + waves * (blocks * per_block + per_tile))
+
+
+def _cheapest_tile(M, N, K, batch=1):
+    """(estimate, tile, split) of the tile with the smallest estimate. Tiles may hang over the edges of the problem,
+    except over M and K of a batched one, past whose matrices the next batch lies."""
+    best = None
+    for tile in _TILE_COST:
+        variant, bm, bn, bk = tile
+        if batch > 1 and (M % bm or K % bk):
+            continue
+        for split in (2, 3, 4) if variant == 5 else (1,):
+            if variant == 5 and (split > len(_TILE_COST[tile][2]) + 1 or -(-K // bk) < 2 * split or
+                                 batch * -(-M // bm) * -(-N // bn) > _CLUSTERS[split]):
+                continue
+            us = _tile_us(tile, split, M, N, K, batch)
+            if best is None or us < best[0]:
+                best = (us, tile, split)
+    return best
+
+
+def tuned_config(M: int, N: int, K: int, dtype: EnumKernelDType, isATranspose: int = 0, db=None, batch: int = 1,
+                 b_transposed: bool = False) -> KernelArgMatmul:
+    """Best known config of a shape: the kernel database's entry when the shape was tuned; else, for the 16-bit
+    types, the tile with the smallest estimated time - the plain rule's choice is kept while the estimate puts it
+    within 5 % of that, twice what estimates of equally fast tiles differ by. ``batch`` > 1: M, N, K are one
+    batch's, and the config fits all batches' tiles walked together. ``b_transposed``: B is stored N x K."""
     from codegendemo_b200.kcg.InfoDb import KernelDb
-    db = db if db is not None else KernelDb()
-    hit = db.lookup(M, N, K, int(dtype), isATranspose)
-    if hit is not None:
-        return KernelArgMatmul.fromJson(hit["config"])
+    if batch == 1:
+        db = db if db is not None else KernelDb()
+        hit = db.lookup(M, N, K, int(dtype), isATranspose)
+        if hit is not None:
+            return _with_b_transposed(KernelArgMatmul.fromJson(hit["config"])) if b_transposed else \
+                KernelArgMatmul.fromJson(hit["config"])
+    plain = _plain_rule(batch * M, N, K, dtype, isATranspose)
+    if M % plain.BLOCK_SIZE_M:
+        plain = _plain_rule(M, N, K, dtype, isATranspose)
+    plain.M = M
+    if int(dtype) != int(EnumKernelDType.float32) and M % 128 == 0 and N % 64 == 0 and K % 64 == 0:
+        us, tile, split = _cheapest_tile(M, N, K, batch)
+        have = (plain.KERNEL_VARIANT or 2, plain.BLOCK_SIZE_M, plain.BLOCK_SIZE_N, plain.BLOCK_SIZE_K)
+        if have not in _TILE_COST or _tile_us(have, plain.LOCAL_SPLIT_U, M, N, K, batch) > 1.05 * us:
+            variant, bm, bn, bk = tile
+            stages = dict(NUM_STAGES=4) if bm == 512 else {}
+            plain = default_config(M, N, K, dtype, KERNEL_VARIANT=variant, BLOCK_SIZE_M=bm, BLOCK_SIZE_N=bn,
+                                   BLOCK_SIZE_K=bk, LOCAL_SPLIT_U=split, isATranspose=isATranspose,
+                                   EDGE_TILES=int(M % bm != 0 or N % bn != 0 or K % bk != 0), **stages)
+    return _with_b_transposed(plain) if b_transposed else plain
+
+
+def _with_b_transposed(kpm):
+    """The same config for a B stored N x K: an automatic choice of the kernel is made explicit; the cluster split-K
+    kernel takes such a B under the rules of EDGE_TILES."""
+    if kpm.KERNEL_VARIANT == 0 and kpm.usesTensorCores():
+        kpm.KERNEL_VARIANT = 2
+    if kpm.KERNEL_VARIANT == 5:
+        kpm.EDGE_TILES = 1
+    kpm.IS_BTRANS = 1
+    return kpm
+
+
+def _plain_rule(M: int, N: int, K: int, dtype: EnumKernelDType, isATranspose: int = 0) -> KernelArgMatmul:
+    """A rule of thumb over tiles that divide the problem (CTA-pair kernels once their larger tiles still fill
+    the 74 pairs for several waves, single-CTA tiles otherwise)."""
     pairs = 74
     if int(dtype) == int(EnumKernelDType.float32):
         if M % 256 == 0 and N % 256 == 0 and K % 32 == 0 and (M // 256) * (N // 256) >= pairs:
@@ -157,10 +256,13 @@ def matmul(a, b, c=None, alpha=1.0, beta=0.0, bias=None, relu=False, b_transpose
     key = (M, N, K, int(dt), dev, tuple(sorted(keys.items())), bool(b_transposed))
     kern = _KERNELS.get(key)
     if kern is None:
-        kpm = default_config(M, N, K, dt, **keys) if keys else tuned_config(M, N, K, dt)
-        if b_transposed:
-            kpm = _single_pass_16bit(kpm, M, N, K, dt)
-            kpm.IS_BTRANS = 1
+        if keys:
+            kpm = default_config(M, N, K, dt, **keys)
+            if b_transposed:
+                kpm = _single_pass_16bit(kpm, M, N, K, dt)
+                kpm.IS_BTRANS = 1
+        else:
+            kpm = tuned_config(M, N, K, dt, b_transposed=b_transposed)
         _, kern = build_kernel(kpm, dev)
         _KERNELS[key] = kern
     contiguous = lda == K and ldb == (K if b_transposed else N) and ldc == N
@@ -206,7 +308,7 @@ def attention(q, k, v, scale=None, out=None):
     kerns = _KERNELS.get(key)
     if kerns is None:
         def tile_for(m, n, kk, scores_step):
-            kpm = tuned_config(H * m, n, kk, dt)
+            kpm = tuned_config(m, n, kk, dt, batch=H)
             if m % kpm.BLOCK_SIZE_M or kpm.KERNEL_VARIANT not in (0, 2, 4):
                 kpm = default_config(m, n, kk, dt)
             kpm.M = m
@@ -288,12 +390,8 @@ def bmm(a, b, c=None, alpha=1.0, beta=0.0, bias=None, relu=False, **keys):
         if keys:
             kpm = default_config(M, N, K, dt, **keys)
         else:
-            # the launch walks all batches' tiles as one tall problem: pick the tile for that much work,
-            # as long as a batch holds a whole number of tile rows
-            kpm = tuned_config(batch * M, N, K, dt)
-            if M % kpm.BLOCK_SIZE_M:
-                kpm = tuned_config(M, N, K, dt)
-            kpm.M = M
+            # the launch walks all batches' tiles as one tall problem: the tile is picked for that much work
+            kpm = tuned_config(M, N, K, dt, batch=batch)
         _, kern = build_kernel(kpm, dev)
         _KERNELS[key] = kern
     kern.run(a, b, c, alpha=alpha, beta=beta, bias=bias, relu=relu, batch=batch)

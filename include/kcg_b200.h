@@ -96,7 +96,10 @@ typedef struct kcg_compile_opts {
                           The reference stores B as K x N only (src/lib/Operators/Matmul.cc:93-121). */
   int32_t serpentine;  /* 1 = inside a BLOCK_MAPPING group, odd tile columns walk the rows upwards (the reference's
                           serpentine twin, matmul.cpp:1279-1287); tcgen05 kernels, BLOCK_MAPPING >= 2 */
-  int32_t reserved[2];
+  int32_t edge_tiles;  /* 1 = M, N and K need not be multiples of the tile: tiles hang over the edges (TMA fills with
+                          zeros and clips); N a multiple of 64 (fp32: 32), rows of 16-byte units, tcgen05 kernels. Also
+                          admits b_trans with KCG_KERNEL_TCGEN05_CLUSTERK. */
+  int32_t reserved[1];
 } kcg_compile_opts;
 
 typedef struct kcg_device_props {
