@@ -17,6 +17,7 @@
 // pipe works for one tile while the other is in its softmax. Four single-tile forms are kept for comparison
 // (AttnFwd: one query tile per CTA with two S buffers, 64- or 128-key steps, one or two threads per row, P through
 // shared or tensor memory; S issued one step ahead - two steps ahead, with a third buffer, measured slower).
+// Up to 64 query rows per head: a form of its own (kernels/attn_decode.cuh).
 // Every wait is bounded (ptx_sm100.cuh); a wait that runs out records a code in a status word the host can read
 // (kcg_attention_status), raises the CTA's abort flag and all roles fall through to the exit.
 #include <cuda.h>
@@ -793,6 +794,8 @@ struct AttnFwd2 {
   }
 };
 
+#include "kernels/attn_decode.cuh"
+
 template <int kD, bool kBf16>
 __global__ void __launch_bounds__(320, 1) kcg_attention2_kernel(const __grid_constant__ AttnParams p) {
   AttnFwd2<kD, kBf16>::run(p);
@@ -808,7 +811,7 @@ using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, voi
                               const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                               CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 EncodeFn g_encode = nullptr;
-bool g_ready[16][20];  // [device][kernel instance]: dynamic shared memory opted in
+bool g_ready[16][32];  // [device][kernel instance]: dynamic shared memory opted in
 std::mutex g_mutex;
 
 int fail(int code, const std::string& msg) { return kcg_internal_fail(code, msg.c_str()); }
@@ -910,6 +913,71 @@ int launch2(int device, int slot, cudaStream_t st, const Problem& pb) {
   return 0;
 }
 
+// CTAs that share a head's keys in the decode form (one cluster). Two CTAs of this size fit an SM, but a cluster has to
+// fit one GPC: beyond about 264 CTAs some clusters wait for a second wave (32 heads x 8192 x 128: 8 CTAs per head
+// 26 us, 9 35 us; 100 heads x 4096: 2 per head 37 us, 3 46 us), pairs alone pack all 296 places. More than 8 per head
+// pay only where fewer heads leave SMs idle (8 heads x 16384: 8 per head 21.2 us, 12 19.5, 16 18.6; 20 heads x 8192:
+// 8 23.9, 10 21.7, 16 33.9 us). At least two stages of 64 keys each: below that the joining costs what the walk saves.
+int decode_splits(int heads, int sk) {
+  const int tiles = (sk + 63) / 64;
+  int s = heads <= 148 && heads > 132 ? 2 : 264 / heads;
+  if (s > 8) s = 200 / heads > 8 ? 200 / heads : 8;
+  if (s > 16) s = 16;
+  if (s > tiles / 2) s = tiles / 2;
+  return s < 1 ? 1 : s;
+}
+
+template <int kD, bool kBf16, int kRowGroups>
+int launch_decode(int device, int slot, cudaStream_t st, const Problem& pb) {
+  using Kern = AttnDecode<kD, kBf16, kRowGroups>;
+  const auto kernel = kcg_attention_decode_kernel<kD, kBf16, kRowGroups>;
+  {
+    std::lock_guard<std::mutex> lock(g_mutex);
+    if (!g_ready[device][slot]) {
+      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Kern::SMEM_BYTES);
+      if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(MaxDynamicSharedMemorySize)");
+      e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(NonPortableClusterSizeAllowed)");
+      g_ready[device][slot] = true;
+    }
+  }
+  AttnDecodeParams p{};
+  if (int r = encode3(&p.tmK, kBf16, pb.K, kD, pb.sk, pb.heads, 64)) return r;
+  if (int r = encode3(&p.tmV, kBf16, pb.V, kD, pb.sk, pb.heads, 64)) return r;
+  p.Q = reinterpret_cast<const void*>(pb.Q);
+  p.O = reinterpret_cast<void*>(pb.O);
+  p.sq = pb.sq;
+  p.sk = pb.sk;
+  p.splits = decode_splits(pb.heads, pb.sk);
+  p.scale_log2 = pb.scale * 1.4426950408889634f;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(pb.heads) * p.splits);
+  cfg.blockDim = dim3(Kern::NUM_THREADS);
+  cfg.dynamicSmemBytes = Kern::SMEM_BYTES;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = p.splits;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
+  if (e != cudaSuccess) return cuda_fail(e, "attention launch");
+  kcg_internal_count_launch();
+  return 0;
+}
+
+template <int kRowGroups>
+int launch_decode_shape(int device, int base_slot, cudaStream_t st, const Problem& pb) {
+  if (pb.d == 128)
+    return pb.bf16 ? launch_decode<128, true, kRowGroups>(device, base_slot, st, pb)
+                   : launch_decode<128, false, kRowGroups>(device, base_slot + 1, st, pb);
+  return pb.bf16 ? launch_decode<64, true, kRowGroups>(device, base_slot + 2, st, pb)
+                 : launch_decode<64, false, kRowGroups>(device, base_slot + 3, st, pb);
+}
+
 template <int kBC, int kSplit, int kPTmem>
 int launch_shape(int device, int base_slot, cudaStream_t st, const Problem& pb) {
   if (pb.d == 128)
@@ -955,8 +1023,18 @@ extern "C" int kcg_attention_fwd(int device, uint64_t stream, uint64_t Q, uint64
   // through shared memory.
   static const int form = [] {
     const char* v = getenv("KCG_ATTN_FORM");
-    return v ? atoi(v) & 7 : 0;
+    return v ? atoi(v) & 15 : 0;
   }();
+  // KCG_ATTN_FORM=8: the 256-row kernel for every number of queries. Up to 32 rows it loses everywhere to the form that
+  // shares a head's keys among CTAs (32 heads x 1 x 8192 x 128: 148 against 26 us, 128 x 16 x 256: 9.9 / 8.3 us); up to
+  // 64 rows it loses where that walk is long (32 x 64 x 8192: 148 / 41 us, 140 x 64 x 4096: 85 / 72 us) but not where
+  // a head's keys are few (128 x 64 x 512: 15.4 / 18.9 us, 48 x 64 x 256: 8.8 / 10.8 us). At 65 rows the warps would
+  // have to walk the keys twice.
+  if (form == 0 && (sq <= 32 || (sq <= 64 && (sk >= 2048 || (heads <= 64 && sk >= 512))))) {
+    if (sq <= 16) return launch_decode_shape<1>(device, 20, st, pb);
+    if (sq <= 32) return launch_decode_shape<2>(device, 24, st, pb);
+    return launch_decode_shape<4>(device, 28, st, pb);
+  }
   switch (form) {
     case 4: return launch_shape<128, 2, 1>(device, 0, st, pb);
     case 5: return launch_shape<64, 1, 1>(device, 4, st, pb);

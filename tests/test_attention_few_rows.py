@@ -1,0 +1,59 @@
+"""The fused attention entry at up to 64 query rows: a head's keys are shared by the CTAs of a cluster."""
+import pytest
+import torch
+
+# (heads, sq, sk, d): one row and one key; the last row group full, one short, one past it (16, 32, 64 rows per
+# kernel form; 65 = the 256-row kernel); a last stage of one key; fewer stages than warps or CTAs; a cluster of 16, an
+# odd one, one CTA per head; a warp whose keys are all past the end
+SHAPES = [(1, 1, 1, 128), (3, 1, 63, 64), (2, 16, 64, 128), (2, 17, 65, 128), (5, 15, 129, 64), (2, 32, 1000, 128),
+          (2, 33, 4097, 64), (4, 64, 2049, 128), (4, 65, 2049, 128), (8, 5, 16384, 128), (8, 3, 8209, 64),
+          (40, 2, 3001, 128), (100, 7, 300, 64), (300, 1, 513, 128)]
+
+
+def _inputs(heads, sq, sk, d, dtype, seed=7):
+    gen = torch.Generator().manual_seed(seed)
+    return [torch.randn((heads, n, d), generator=gen).to(dtype) for n in (sq, sk, sk)]
+
+
+def _reference(q, k, v, scale):
+    p = torch.softmax(q.double() @ k.double().transpose(1, 2) * scale, dim=-1)
+    return p @ v.double()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "x".join(map(str, s)))
+def test_few_rows_match_the_composition_in_64_bits(shape, dtype):
+    from codegendemo_b200.kcg.matmul_op import attention_fused, attention_status
+    heads, sq, sk, d = shape
+    q, k, v = _inputs(heads, sq, sk, d, dtype)
+    out = torch.full((heads, sq, d), float("nan"), dtype=dtype, device="cuda")
+    attention_fused(q.cuda(), k.cuda(), v.cuda(), out=out)
+    attention_status(0)
+    ref = _reference(q, k, v, d ** -0.5)
+    # probabilities and the result are each rounded once to 16 bits: half a unit of the largest value, twice; the
+    # 32-bit sums and exponentials stay two orders below that
+    half_unit = 2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12
+    bound = 2.1 * half_unit * v.abs().max().item()
+    assert (out.cpu().double() - ref).abs().max().item() <= bound
+    again = torch.empty_like(out)
+    attention_fused(q.cuda(), k.cuda(), v.cuda(), out=again)
+    assert torch.equal(out, again)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sq", [1, 20, 64])
+def test_few_rows_and_extreme_scores(sq):
+    """Scores of +-2000 (all weight on one key of a late stage), and a NaN key: the rows that see it are NaN."""
+    from codegendemo_b200.kcg.matmul_op import attention_fused
+    q, k, v = _inputs(2, sq, 1500, 64, torch.bfloat16)
+    q[:] = 0
+    q[:, :, 0] = 2000.0
+    k[:] = 0
+    k[:, :, 0] = -1.0
+    k[:, 1441, 0] = 1.0
+    out = attention_fused(q.cuda(), k.cuda(), v.cuda(), scale=1.0).cpu()
+    assert torch.equal(out, v[:, 1441:1442].expand(2, sq, 64))
+    k[1, 700, 0] = float("nan")
+    out = attention_fused(q.cuda(), k.cuda(), v.cuda(), scale=1.0).cpu()
+    assert torch.equal(out[0], v[0, 1441:1442].expand(sq, 64)) and out[1].isnan().all()
