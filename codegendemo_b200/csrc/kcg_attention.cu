@@ -4,17 +4,23 @@
 // The three-launch form (matmul_op.attention: batched Q K^T with fp32 scores, row softmax, batched P V) stays as
 // the path whose parity is pinned to the composition; this kernel is checked against the same composition.
 //
-// Default form (AttnFwd2): one CTA per (head, 256 query rows) = two query tiles of 128 rows, 320 threads:
+// Default form (AttnFwd2): one CTA per (head, 256 query rows) = two query tiles of 128 rows, 384 threads:
 //   warp 0    TMA producer: both Q tiles once, then K and V tiles of 128 keys through two-stage rings, shared by
 //             the two query tiles
 //   warp 1    tcgen05.mma issuer and TMEM owner; per tile t: S_t = Q_t K_j^T (both K-major) into the tile's S
 //             buffer, O_t += P_t V_j with P_t read from tensor memory and V as the MN-major operand
-//   warps 2-5 softmax of tile 0, warps 6-9 of tile 1, one query row per thread: read S_t from TMEM, running
-//             maximum and sum in the exp2 domain, P_t as packed 16-bit pairs over the S columns just read, O_t
-//             rescaled in TMEM by exp2(m_old - m_new) only by warps that saw a new maximum; at the end O / sum to
-//             global memory
-// A tile's chain is serial (scores, softmax, P V, next scores) and the two tiles' chains interleave, so the tensor
-// pipe works for one tile while the other is in its softmax. Four single-tile forms are kept for comparison
+//   warps 4-7 softmax of tile 0, warps 8-11 of tile 1, one query row per thread: read S_t from TMEM, exponentials in
+//             the exp2 domain against a maximum that follows the running one in steps of at least 8, P_t as packed
+//             16-bit pairs over the S columns just read; at the end O / sum to global memory
+// A tile's chain is serial (scores, softmax, P V, next scores) and the two tiles' chains take turns, so the tensor
+// pipe works for one tile while the other is in its softmax. What bounds it is that chain: per step and tile 512 + 512
+// cycles of products (the scores' operands fill the shared-memory port, 128 bytes a cycle) and 1024 of exponentials,
+// of which about 3100 cycles for two tiles' steps remain exposed against 2048 of the tensor pipe alone. Measured (B200,
+// bf16), a form with votes of all softmax warps, O rescaled at every new maximum and a one-lane issuer against this
+// one: 32 heads x 4096 x 4096 x 128 322 -> 246 us (1119 TFLOP/s), x 64 287 -> 210 us, 16 x 2048 x 2048 x 128 46 -> 36 us.
+// Tried without gain: exponentials of every eighth to third pair as a polynomial on the FMA pipe (2 to 8 % slower: one
+// warp per scheduler and tile is bound by its own latencies, not by the exponential pipe).
+// Four single-tile forms are kept for comparison
 // (AttnFwd: one query tile per CTA with two S buffers, 64- or 128-key steps, one or two threads per row, P through
 // shared or tensor memory; S issued one step ahead - two steps ahead, with a third buffer, measured slower).
 // Up to 64 query rows per head: a form of its own (kernels/attn_decode.cuh).
@@ -67,6 +73,46 @@ __device__ __forceinline__ void tmem_st_32x32b_x32(uint32_t taddr, const uint32_
         "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
       : "memory");
 }
+__device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      :
+      : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+// Ties the registers of an earlier tmem_ld to the wait before it: no use of them may be scheduled ahead of this.
+__device__ __forceinline__ void pin_32(uint32_t (&r)[32]) {
+#pragma unroll
+  for (int i = 0; i < 32; ++i) asm volatile("" : "+r"(r[i]));
+}
+// Two fp32 operations per instruction on register pairs (one rounding each, like the scalar forms).
+__device__ __forceinline__ uint64_t f32x2(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 f32x2_split(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // D[tmem] (+)= A[tmem] * B[smem], 16-bit operands: A is read from tensor memory (lane = row, one 32-bit column =
@@ -88,6 +134,17 @@ __device__ __forceinline__ float ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+
+template <bool kBf16>
+__device__ __forceinline__ uint32_t pack_pair(float lo, float hi) {
+  if constexpr (kBf16) {
+    __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<uint32_t*>(&v);
+  } else {
+    __half2 v = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<uint32_t*>(&v);
+  }
 }
 
 struct AttnParams {
@@ -491,13 +548,14 @@ template <int kD, bool kBf16>
 struct AttnFwd2 {
   static constexpr int BR = 128, BC = 128, TILES = 2;
   static constexpr int K_STAGES = 2, V_STAGES = 2;
-  static constexpr int NUM_THREADS = 64 + TILES * 128;
+  static constexpr int NUM_THREADS = 128 + TILES * 128;  // whole warpgroups, for setmaxnreg
   static constexpr int BOXES = kD / 64;
   static constexpr int QBOX_BYTES = BR * 128, KVBOX_BYTES = BC * 128;
   static constexpr int Q_BYTES = BR * kD * 2, KV_BYTES = BC * kD * 2;
   static constexpr int OFF_K = TILES * Q_BYTES, OFF_V = OFF_K + K_STAGES * KV_BYTES;
   static constexpr int RING_BYTES = OFF_V + V_STAGES * KV_BYTES;
   static constexpr int SMEM_BYTES = RING_BYTES + 2048;  // 1 KB alignment slack + barriers
+  static constexpr int P_PART = 96;  // keys of a step after which P V starts
   static constexpr uint32_t COL_O = TILES * BC, TMEM_COLS = 512;
   static constexpr uint32_t FMT = kBf16 ? FMT_BF16 : FMT_F16;
   static constexpr uint32_t IDESC_S = make_instr_desc(FMT, 0u, 0u, 128u, BC);
@@ -508,8 +566,9 @@ struct AttnFwd2 {
     uint64_t q_full;
     uint64_t k_full[K_STAGES], k_empty[K_STAGES], v_full[V_STAGES], v_empty[V_STAGES];
     uint64_t s_full[TILES];   // S_t of the current step is complete
-    uint64_t p_full[TILES];   // P_t is in tensor memory and O_t is rescaled (4 warps arrive)
-    uint64_t pv_done[TILES];  // P_t V of the current step has retired
+    uint64_t p_part[TILES];   // the first P_PART keys of P_t are in tensor memory and O_t is rescaled (4 warps arrive)
+    uint64_t p_full[TILES];   // all of P_t is (4 warps arrive)
+    uint64_t o_full[TILES];   // the last P_t V has retired
     uint32_t tmem_base;
     volatile uint32_t abort_flag;
   };
@@ -549,8 +608,9 @@ struct AttnFwd2 {
       }
       for (int t = 0; t < TILES; ++t) {
         mbar_init(&bars->s_full[t], 1);
+        mbar_init(&bars->p_part[t], 4);
         mbar_init(&bars->p_full[t], 4);
-        mbar_init(&bars->pv_done[t], 1);
+        mbar_init(&bars->o_full[t], 1);
       }
       bars->abort_flag = 0u;
       fence_mbar_init();
@@ -565,185 +625,237 @@ struct AttnFwd2 {
     tc_fence_after_sync();
     const uint32_t tmem_base = bars->tmem_base;
 
-    if (warp == 0) {
-      // ------------------------------------------------------------------ producer
-      if (lane == 0) {
-        mbar_expect_tx(&bars->q_full, TILES * Q_BYTES);
-#pragma unroll
-        for (int t = 0; t < TILES; ++t)
-#pragma unroll
-          for (int b = 0; b < BOXES; ++b)
-            tma_load_3d(smem + t * Q_BYTES + b * QBOX_BYTES, &p.tmQ, &bars->q_full, b * 64, q0 + t * BR, head);
-        for (int j = 0; j < nkv; ++j) {
-          const int ks = j % K_STAGES, vs = j % V_STAGES;
-          if (!mbar_wait(&bars->k_empty[ks], ((j / K_STAGES) & 1u) ^ 1u, &bars->abort_flag)) {
-            report(bars, ATTN_TIMEOUT_PRODUCER, j, 0u);
-            break;
+    // Registers: 384 threads are launched with 168 each; the control warpgroup keeps 56, the softmax warpgroups take
+    // 224 (56 + 2 * 224 = 3 * 168), which a row's 128 scores need.
+    if (warp < 4) {
+      asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+      if (warp == 0) {
+        // ------------------------------------------------------------------ producer
+        if (lane == 0) {
+          mbar_expect_tx(&bars->q_full, TILES * Q_BYTES);
+  #pragma unroll
+          for (int t = 0; t < TILES; ++t)
+  #pragma unroll
+            for (int b = 0; b < BOXES; ++b)
+              tma_load_3d(smem + t * Q_BYTES + b * QBOX_BYTES, &p.tmQ, &bars->q_full, b * 64, q0 + t * BR, head);
+          for (int j = 0; j < nkv; ++j) {
+            const int ks = j % K_STAGES, vs = j % V_STAGES;
+            if (!mbar_wait(&bars->k_empty[ks], ((j / K_STAGES) & 1u) ^ 1u, &bars->abort_flag)) {
+              report(bars, ATTN_TIMEOUT_PRODUCER, j, 0u);
+              break;
+            }
+            mbar_expect_tx(&bars->k_full[ks], KV_BYTES);
+  #pragma unroll
+            for (int b = 0; b < BOXES; ++b)
+              tma_load_3d(smem + OFF_K + ks * KV_BYTES + b * KVBOX_BYTES, &p.tmK, &bars->k_full[ks], b * 64, j * BC, head);
+            if (!mbar_wait(&bars->v_empty[vs], ((j / V_STAGES) & 1u) ^ 1u, &bars->abort_flag)) {
+              report(bars, ATTN_TIMEOUT_PRODUCER, j, 1u);
+              break;
+            }
+            mbar_expect_tx(&bars->v_full[vs], KV_BYTES);
+  #pragma unroll
+            for (int b = 0; b < BOXES; ++b)
+              tma_load_3d(smem + OFF_V + vs * KV_BYTES + b * KVBOX_BYTES, &p.tmV, &bars->v_full[vs], b * 64, j * BC, head);
           }
-          mbar_expect_tx(&bars->k_full[ks], KV_BYTES);
-#pragma unroll
-          for (int b = 0; b < BOXES; ++b)
-            tma_load_3d(smem + OFF_K + ks * KV_BYTES + b * KVBOX_BYTES, &p.tmK, &bars->k_full[ks], b * 64, j * BC, head);
-          if (!mbar_wait(&bars->v_empty[vs], ((j / V_STAGES) & 1u) ^ 1u, &bars->abort_flag)) {
-            report(bars, ATTN_TIMEOUT_PRODUCER, j, 1u);
-            break;
-          }
-          mbar_expect_tx(&bars->v_full[vs], KV_BYTES);
-#pragma unroll
-          for (int b = 0; b < BOXES; ++b)
-            tma_load_3d(smem + OFF_V + vs * KV_BYTES + b * KVBOX_BYTES, &p.tmV, &bars->v_full[vs], b * 64, j * BC, head);
         }
-      }
-    } else if (warp == 1) {
-      // ---------------------------------------------------------------- MMA issuer
-      if (lane == 0) {
+      } else if (warp == 1) {
+        // ---------------------------------------------------------------- MMA issuer
+        // The issuer is on the critical path: its waits cost 100 to 200 cycles each while operand reads fill the
+        // shared-memory port, so each is made once per step, not once per tile. The whole warp walks the loop and elects
+        // one lane for each batch of instructions: their descriptors are then warp-uniform values. (With the loop
+        // inside an if (lane == 0) every tcgen05.mma took about 125 cycles to issue, twice what a 128 x 128 x 16
+        // product takes to run.) One issuer per tile was slower: the tiles' products then mix on the pipe instead of
+        // taking turns, and both softmaxes wait and work at the same time.
         bool ok = mbar_wait(&bars->q_full, 0u, &bars->abort_flag);
-        if (!ok) report(bars, ATTN_TIMEOUT_MMA, 0u, 0u);
-        tc_fence_after_sync();
+        if (!ok && lane == 0) report(bars, ATTN_TIMEOUT_MMA, 0u, 0u);
+        ok = __all_sync(0xffffffffu, ok);
+        const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
+        const uint64_t qdesc = make_smem_desc(smem_u32(smem), 16, 1024, SWZ_128B);
+        const uint64_t kdesc = make_smem_desc(smem_u32(smem + OFF_K), 16, 1024, SWZ_128B);
+        const uint64_t vdesc = make_smem_desc(smem_u32(smem + OFF_V), KVBOX_BYTES, 1024, SWZ_128B);
+        // waits of a whole warp; false (after the report) when one of them ran out
+        auto wait = [&](uint64_t* bar, uint32_t parity, uint32_t what, int i) -> bool {
+          const bool got = __all_sync(0xffffffffu, mbar_wait(bar, parity, &bars->abort_flag));
+          if (!got && lane == 0) report(bars, ATTN_TIMEOUT_MMA, what, static_cast<uint32_t>(i));
+          return got;
+        };
         // S_t of step i. Issued after P_t V of step i - 1 (program order), which is what has read the P that
         // these scores overwrite; the softmax warps of tile t have read the old scores before they wrote that P.
-        auto issue_s = [&](int t, int i) -> bool {
-          const int s = i % K_STAGES;
-          if (!mbar_wait(&bars->k_full[s], (i / K_STAGES) & 1u, &bars->abort_flag)) {
-            report(bars, ATTN_TIMEOUT_MMA, 1u, static_cast<uint32_t>(i));
-            return false;
-          }
-          tc_fence_after_sync();
-          const uint32_t sq_addr = smem_u32(smem + t * Q_BYTES);
-          const uint32_t sk_addr = smem_u32(smem + OFF_K + s * KV_BYTES);
+        auto issue_s = [&](int t, int i) {
+          const uint64_t ad = qdesc + t * (Q_BYTES >> 4), bd = kdesc + (i % K_STAGES) * (KV_BYTES >> 4);
 #pragma unroll
           for (int ks = 0; ks < kD / 16; ++ks) {
             const uint32_t in_row = (ks * 32) % 128, box = (ks * 32) / 128;
-            const uint64_t adesc = make_smem_desc(sq_addr + box * QBOX_BYTES + in_row, 16, 1024, SWZ_128B);
-            const uint64_t bdesc = make_smem_desc(sk_addr + box * KVBOX_BYTES + in_row, 16, 1024, SWZ_128B);
-            umma_ss<false>(tmem_base + t * BC, adesc, bdesc, IDESC_S, ks > 0 ? 1u : 0u);
+            umma_ss<false>(tmem + t * BC, ad + ((box * QBOX_BYTES + in_row) >> 4),
+                           bd + ((box * KVBOX_BYTES + in_row) >> 4), IDESC_S, ks > 0 ? 1u : 0u);
           }
-          if (t == TILES - 1) umma_commit(&bars->k_empty[s]);  // both tiles have read this K tile
           umma_commit(&bars->s_full[t]);
-          return true;
+          if (t == TILES - 1) umma_commit(&bars->k_empty[i % K_STAGES]);  // both tiles have read this K tile
         };
-        for (int t = 0; t < TILES && ok; ++t) ok = issue_s(t, 0);
-        for (int j = 0; j < nkv && ok; ++j) {
-          const int vs = j % V_STAGES;
-          for (int t = 0; t < TILES && ok; ++t) {
-            if (!mbar_wait(&bars->p_full[t], j & 1u, &bars->abort_flag) ||
-                !mbar_wait(&bars->v_full[vs], (j / V_STAGES) & 1u, &bars->abort_flag)) {
-              report(bars, ATTN_TIMEOUT_MMA, 2u, static_cast<uint32_t>(j));
-              ok = false;
-              break;
-            }
-            tc_fence_after_sync();
-            const uint32_t sv_addr = smem_u32(smem + OFF_V + vs * KV_BYTES);
+        auto issue_pv = [&](int t, int j, int ks0, int ks1) {
+          const uint64_t vd = vdesc + (j % V_STAGES) * (KV_BYTES >> 4);
 #pragma unroll
-            for (int ks = 0; ks < BC / 16; ++ks) {
-              const uint64_t bdesc = make_smem_desc(sv_addr + ks * 16 * 128, KVBOX_BYTES, 1024, SWZ_128B);
-              umma_ts_f16(tmem_base + COL_O + t * kD, tmem_base + t * BC + ks * 8, bdesc, IDESC_O,
+          for (int ks = 0; ks < BC / 16; ++ks)
+            if (ks >= ks0 && ks < ks1)
+              umma_ts_f16(tmem + COL_O + t * kD, tmem + t * BC + ks * 8, vd + ((ks * 16 * 128) >> 4), IDESC_O,
                           (j > 0 || ks > 0) ? 1u : 0u);
+        };
+        if (ok) ok = wait(&bars->k_full[0], 0u, 1u, 0);
+        if (ok) {
+          tc_fence_after_sync();
+          if (elect_one()) {
+            issue_s(0, 0);
+            issue_s(1, 0);
+          }
+          __syncwarp();
+        }
+        for (int j = 0; j < nkv && ok; ++j) {
+          const int vs = j % V_STAGES, ks = (j + 1) % K_STAGES;
+          ok = wait(&bars->v_full[vs], (j / V_STAGES) & 1u, 2u, j);
+          if (ok && j + 1 < nkv) ok = wait(&bars->k_full[ks], ((j + 1) / K_STAGES) & 1u, 1u, j + 1);
+#pragma unroll
+          for (int t = 0; t < TILES; ++t) {
+            if (ok) ok = wait(&bars->p_part[t], j & 1u, 3u, j);
+            if (!ok) break;
+            tc_fence_after_sync();
+            if (elect_one()) issue_pv(t, j, 0, P_PART / 16);
+            __syncwarp();
+            ok = wait(&bars->p_full[t], j & 1u, 4u, j);
+            if (!ok) break;
+            tc_fence_after_sync();
+            if (elect_one()) {
+              issue_pv(t, j, P_PART / 16, BC / 16);
+              if (t == TILES - 1) umma_commit(&bars->v_empty[vs]);
+              if (j + 1 < nkv) {
+                issue_s(t, j + 1);
+              } else {
+                umma_commit(&bars->o_full[t]);
+              }
             }
-            if (t == TILES - 1) umma_commit(&bars->v_empty[vs]);
-            umma_commit(&bars->pv_done[t]);
-            if (j + 1 < nkv) ok = issue_s(t, j + 1);
+            __syncwarp();
           }
         }
-      }
+      }  // (warps 2 and 3 only give their registers)
     } else {
+      asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
       // ------------------------------------------------- softmax, correction, epilogue
       const int q = warp & 3;           // TMEM lane quarter this warp may access
-      const int t = (warp - 2) >> 2;    // query tile of this warp
+      const int t = (warp - 4) >> 2;    // query tile of this warp
       const int row = q * 32 + lane;    // query row of this thread inside its tile
       const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
       const uint32_t col_s = tmem_base + lane_addr + t * BC, col_o = tmem_base + lane_addr + COL_O + t * kD;
-      float m = -INFINITY, l = 0.f;
+      // m: the maximum the exponentials are taken against, in the exp2 domain. It follows the running maximum only
+      // when that has moved by more than 8 for some row of the warp: until then the exponentials are at most 2^8,
+      // which neither the 16-bit P nor the 32-bit sums notice, and O need not be rescaled.
+      float m = -INFINITY;
+      uint64_t sum2[2] = {f32x2(0.f, 0.f), f32x2(0.f, 0.f)};
       bool ok = true;
+      const uint64_t scale2 = f32x2(p.scale_log2, p.scale_log2);
       for (int j = 0; j < nkv; ++j) {
-        bool got = mbar_wait(&bars->s_full[t], j & 1u, &bars->abort_flag);
-        if (!named_bar_all(2 + t, 128, got)) {
-          if (!got) report(bars, ATTN_TIMEOUT_SOFTMAX, 0u, static_cast<uint32_t>(j));
+        const bool got = mbar_wait(&bars->s_full[t], j & 1u, &bars->abort_flag);
+        if (!__all_sync(0xffffffffu, got)) {
+          if (lane == 0) report(bars, ATTN_TIMEOUT_SOFTMAX, 0u, static_cast<uint32_t>(j));
           ok = false;
           break;
         }
         tc_fence_after_sync();
-        // all four 32-column reads of the row in flight, one wait
-        uint32_t sr[BC / 32][32];
+        uint32_t sr[4][32];
 #pragma unroll
-        for (int c = 0; c < BC / 32; ++c) tmem_ld_32x32b_x32(col_s + c * 32, sr[c]);
+        for (int c = 0; c < 4; ++c) tmem_ld_32x32b_x32(col_s + c * 32, sr[c]);
         tmem_ld_wait();
-        float s[BC];
 #pragma unroll
-        for (int c = 0; c < BC / 32; ++c)
-#pragma unroll
-          for (int i = 0; i < 32; ++i) s[c * 32 + i] = __uint_as_float(sr[c][i]);
+        for (int c = 0; c < 4; ++c) pin_32(sr[c]);
         const int valid = p.sk - j * BC;
         if (valid < BC) {
 #pragma unroll
-          for (int i = 0; i < BC; ++i)
-            if (i >= valid) s[i] = -INFINITY;
+          for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (c * 32 + i >= valid) sr[c][i] = __float_as_uint(-INFINITY);
         }
         float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        auto max_of = [&](int c) {
 #pragma unroll
-        for (int i = 0; i < BC; i += 4) {
-          mx4[0] = fmaxf(mx4[0], s[i]);
-          mx4[1] = fmaxf(mx4[1], s[i + 1]);
-          mx4[2] = fmaxf(mx4[2], s[i + 2]);
-          mx4[3] = fmaxf(mx4[3], s[i + 3]);
-        }
-        const float mx = fmaxf(m, fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2);
-        const float alpha = ex2(m - mx);  // 0 on the first step (m = -inf)
-        const bool rescale = j > 0 && __any_sync(0xffffffffu, alpha != 1.f);
-        float sum4[4] = {0.f, 0.f, 0.f, 0.f};
-        // exponentials and P, 64 keys at a time: packed pairs over the S columns this thread has read
+          for (int i = 0; i < 32; i += 2)
+            mx4[(i >> 1) & 3] = max3(mx4[(i >> 1) & 3], __uint_as_float(sr[c][i]), __uint_as_float(sr[c][i + 1]));
+        };
+        // Exponentials and P of 32 keys: packed pairs over the S columns this thread has read.
+        auto exponentials = [&](int c) {
+          const uint64_t base2 = f32x2(-m, -m);
+          uint32_t w[16];
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          uint32_t w[32];
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const float e0 = ex2(fmaf(s[half * 64 + 2 * i], p.scale_log2, -mx));
-            const float e1 = ex2(fmaf(s[half * 64 + 2 * i + 1], p.scale_log2, -mx));
-            sum4[i & 3] += e0 + e1;
-            if constexpr (kBf16) {
-              __nv_bfloat162 v2 = __floats2bfloat162_rn(e0, e1);
-              w[i] = *reinterpret_cast<uint32_t*>(&v2);
-            } else {
-              __half2 v2 = __floats2half2_rn(e0, e1);
-              w[i] = *reinterpret_cast<uint32_t*>(&v2);
-            }
+          for (int i = 0; i < 16; ++i) {
+            float2 e = f32x2_split(fma_f32x2(f32x2(__uint_as_float(sr[c][2 * i]), __uint_as_float(sr[c][2 * i + 1])),
+                                             scale2, base2));
+            e.x = ex2(e.x);
+            e.y = ex2(e.y);
+            sum2[i & 1] = add_f32x2(sum2[i & 1], f32x2(e.x, e.y));
+            w[i] = pack_pair<kBf16>(e.x, e.y);
           }
-          tmem_st_32x32b_x32(col_s + half * 32, w);
+          tmem_st_32x32b_x16(col_s + c * 16, w);
+        };
+        auto row_max = [&]() {  // (the scale is positive: checked by the host)
+          return fmaxf(m, fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2);
+        };
+        if (j == 0) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) max_of(c);
+          m = row_max();
         }
-        l = l * alpha + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
-        m = mx;
-        if (rescale) {
-          // O_t <- alpha * O_t for this row: the previous P_t V has retired (the scores of this step were issued
-          // behind it), which the barrier confirms
-          got = mbar_wait(&bars->pv_done[t], (j & 1u) ^ 1u, &bars->abort_flag);
-          if (got) {
-            tc_fence_after_sync();
-            uint32_t orr[kD / 32][32];
-#pragma unroll
-            for (int c = 0; c < kD / 32; ++c) tmem_ld_32x32b_x32(col_o + c * 32, orr[c]);
-            tmem_ld_wait();
-#pragma unroll
+        // The first half is exponentiated against the maximum so far while the maximum of this step is being taken
+        // (comparisons fit between the exponentials, which occupy their pipe for eight cycles each); in the rare step
+        // whose maximum has moved too far that half is done again.
+        const uint64_t sum_before[2] = {sum2[0], sum2[1]};
+        max_of(0);
+        max_of(1);
+        exponentials(0);
+        max_of(2);
+        max_of(3);
+        exponentials(1);
+        const float mx = row_max();
+        if (__any_sync(0xffffffffu, mx > m + 8.f)) {
+          const float alpha = ex2(m - mx);
+          m = mx;
+          const uint64_t alpha2 = f32x2(alpha, alpha), zero2 = f32x2(0.f, 0.f);
+          sum2[0] = fma_f32x2(sum_before[0], alpha2, zero2);
+          sum2[1] = fma_f32x2(sum_before[1], alpha2, zero2);
+          if (j > 0) {
+            // O_t <- alpha * O_t. The previous P_t V has retired: the scores just read were issued behind it.
+#pragma unroll 1
             for (int c = 0; c < kD / 32; ++c) {
+              uint32_t orr[32];
+              tmem_ld_32x32b_x32(col_o + c * 32, orr);
+              tmem_ld_wait();
+              pin_32(orr);
 #pragma unroll
-              for (int i = 0; i < 32; ++i) orr[c][i] = __float_as_uint(__uint_as_float(orr[c][i]) * alpha);
-              tmem_st_32x32b_x32(col_o + c * 32, orr[c]);
+              for (int i = 0; i < 32; ++i) orr[i] = __float_as_uint(__uint_as_float(orr[i]) * alpha);
+              tmem_st_32x32b_x32(col_o + c * 32, orr);
             }
           }
+          exponentials(0);
+          exponentials(1);
         }
-        tmem_st_wait();
-        if (!named_bar_all(2 + t, 128, got)) {
-          if (!got) report(bars, ATTN_TIMEOUT_SOFTMAX, 1u, static_cast<uint32_t>(j));
-          ok = false;
-          break;
-        }
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bars->p_full[t]);
+        auto publish = [&](uint64_t* bar) {
+          tmem_st_wait();
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar);
+        };
+        // P V starts on the first 96 keys while the others are still being exponentiated (32 heads x 4096 x 4096 x 128:
+        // 246 us; after 64 keys 259 us, the product then waits for the rest with the pipe in its hands; after all 128
+        // 266 us)
+        static_assert(P_PART == 96, "three pieces of 32 keys");
+        exponentials(2);
+        publish(&bars->p_part[t]);
+        exponentials(3);
+        publish(&bars->p_full[t]);
       }
+      const float2 s01 = f32x2_split(add_f32x2(sum2[0], sum2[1]));
+      const float l = s01.x + s01.y;
       if (ok) {
-        bool got = mbar_wait(&bars->pv_done[t], (nkv - 1) & 1u, &bars->abort_flag);
-        if (!named_bar_all(2 + t, 128, got)) {
-          if (!got) report(bars, ATTN_TIMEOUT_SOFTMAX, 2u, 0u);
+        const bool got = mbar_wait(&bars->o_full[t], 0u, &bars->abort_flag);
+        if (!__all_sync(0xffffffffu, got)) {
+          if (lane == 0) report(bars, ATTN_TIMEOUT_SOFTMAX, 2u, 0u);
           ok = false;
         }
       }
@@ -797,7 +909,7 @@ struct AttnFwd2 {
 #include "kernels/attn_decode.cuh"
 
 template <int kD, bool kBf16>
-__global__ void __launch_bounds__(320, 1) kcg_attention2_kernel(const __grid_constant__ AttnParams p) {
+__global__ void __launch_bounds__(384, 1) kcg_attention2_kernel(const __grid_constant__ AttnParams p) {
   AttnFwd2<kD, kBf16>::run(p);
 }
 

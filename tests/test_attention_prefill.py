@@ -1,0 +1,60 @@
+"""The 256-row fused attention kernel where its maxima, its last steps and its second query tile can go wrong."""
+import pytest
+import torch
+
+
+def _reference(q, k, v, scale):
+    p = torch.softmax(q.double() @ k.double().transpose(1, 2) * scale, dim=-1)
+    return p @ v.double()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+# one step; keys that end in each of a step's four pieces; an odd number of steps; a second tile of one row or none
+@pytest.mark.parametrize("shape", [(3, 256, 128, 128), (2, 129, 1, 64), (2, 128, 33, 128), (2, 257, 193, 64),
+                                   (1, 300, 353, 128), (2, 255, 384, 128)], ids=lambda s: "x".join(map(str, s)))
+def test_rows_match_the_composition_in_64_bits(shape, dtype):
+    from codegendemo_b200.kcg.matmul_op import attention_fused, attention_status
+    heads, sq, sk, d = shape
+    gen = torch.Generator().manual_seed(3)
+    q, k, v = [torch.randn((heads, n, d), generator=gen).to(dtype) for n in (sq, sk, sk)]
+    out = torch.full((heads, sq, d), float("nan"), dtype=dtype, device="cuda")
+    attention_fused(q.cuda(), k.cuda(), v.cuda(), out=out)
+    attention_status(0)
+    # probabilities and the result are each rounded once to 16 bits (half a unit of the largest value, twice)
+    half_unit = 2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12
+    assert (out.cpu().double() - _reference(q, k, v, d ** -0.5)).abs().max().item() <= 2.1 * half_unit * v.abs().max().item()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("step", [0.02, 0.5, 7.9, 8.1, 40.0])
+def test_maximum_that_climbs_with_every_step(step):
+    """Scores that grow by `step` (in the exp2 domain) from one 128-key step to the next, in some rows only: the
+    maximum the exponentials refer to is left behind by up to 8 or moved, and O and the sums follow."""
+    from codegendemo_b200.kcg.matmul_op import attention_fused, attention_status
+    heads, sq, sk, d = 2, 256, 1280, 64
+    gen = torch.Generator().manual_seed(4)
+    q, k, v = [0.1 * torch.randn((heads, n, d), generator=gen) for n in (sq, sk, sk)]
+    q[:, :, 0] = 1.0
+    q[:, 1::3, 0] = -1.0
+    q[:, 2::3, 0] = 0.0
+    k[:, :, 0] = (torch.arange(sk) // 128 * step * 0.6931471805599453)[None]
+    q, k, v = q.half(), k.half(), v.half()
+    out = attention_fused(q.cuda(), k.cuda(), v.cuda(), scale=1.0)
+    attention_status(0)
+    assert (out.cpu().double() - _reference(q, k, v, 1.0)).abs().max().item() <= 2.1 * 2.0 ** -12 * v.abs().max().item()
+
+
+@pytest.mark.gpu
+def test_nan_and_infinite_scores_stay_in_their_rows():
+    from codegendemo_b200.kcg.matmul_op import attention_fused
+    gen = torch.Generator().manual_seed(5)
+    q, k, v = [torch.randn((2, n, 64), generator=gen).bfloat16() for n in (256, 512, 512)]
+    clean = attention_fused(q.cuda(), k.cuda(), v.cuda()).cpu()
+    q[0, 5, 3] = float("nan")
+    q[1, 200, 3] = float("inf")
+    out = attention_fused(q.cuda(), k.cuda(), v.cuda()).cpu()
+    assert out[0, 5].isnan().all() and out[1, 200].isnan().all()
+    clean[0, 5] = out[0, 5]
+    clean[1, 200] = out[1, 200]
+    assert torch.equal(out.nan_to_num(7.0), clean.nan_to_num(7.0))
