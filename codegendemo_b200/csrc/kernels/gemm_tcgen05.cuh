@@ -307,7 +307,11 @@ struct TcGemm {
       }
     } else if (warp == 1) {
       // -------------------------- MMA issuer (in a pair: the leader CTA only)
-      if (lane == 0 && rank == 0u) {
+      if (rank == 0u) {
+        // The whole warp walks this loop and elects one lane per batch of instructions, so that their descriptors are
+        // warp-uniform values: inside an if (lane == 0) every tcgen05.mma takes about 125 cycles to issue (measured in
+        // the fused attention kernel), as long as a 128 x 256 x 16 product runs.
+        const uint32_t tmem_base_u = __shfl_sync(0xffffffffu, tmem_base, 0);
         uint32_t it = 0, acc_it = 0;
         bool ok = true;
         Iter units(p, unit0, unit_stride, tiles_m, tiles_n, num_kb);
@@ -364,12 +368,12 @@ struct TcGemm {
         for (; ok && units.next(w); ++acc_it) {
           const uint32_t ab = acc_it % NACC;
           const uint32_t aph = (acc_it / NACC) & 1u;
-          if (!mbar_wait(&bars->tmem_empty[ab], aph ^ 1u, &bars->abort_flag)) {
+          if (!mbar_wait_warp(&bars->tmem_empty[ab], aph ^ 1u, &bars->abort_flag)) {
             report(p, bars, KCG_ST_TIMEOUT_MMA, 0x100u + ab, acc_it);
             break;
           }
           tc_fence_after_sync();
-          const uint32_t tmem_acc = tmem_base + ab * ACC_COLS;
+          const uint32_t tmem_acc = tmem_base_u + ab * ACC_COLS;
           int kb = 0;
           if constexpr (HALF) {
             // Accumulator 0 is drained (the wait above), accumulator 1 maybe not yet: run the first
@@ -379,24 +383,28 @@ struct TcGemm {
             for (int j = 0; j < pro; ++j) {
               const uint32_t s = (it + j) % kStages;
               const uint32_t ph = ((it + j) / kStages) & 1u;
-              if (!mbar_wait(&bars->full[s], ph, &bars->abort_flag)) {
+              if (!mbar_wait_warp(&bars->full[s], ph, &bars->abort_flag)) {
                 report(p, bars, KCG_ST_TIMEOUT_MMA, it + j, s);
                 ok = false;
                 break;
               }
               tc_fence_after_sync();
-              issue(s, j, 0, 1, tmem_acc);
+              if (elect_one()) issue(s, j, 0, 1, tmem_acc);
+              __syncwarp();
             }
             if (!ok) break;
-            if (!mbar_wait(&bars->tmem_empty[1], aph ^ 1u, &bars->abort_flag)) {
+            if (!mbar_wait_warp(&bars->tmem_empty[1], aph ^ 1u, &bars->abort_flag)) {
               report(p, bars, KCG_ST_TIMEOUT_MMA, 0x101u, acc_it);
               break;
             }
             tc_fence_after_sync();
             for (int j = 0; j < pro; ++j) {
               const uint32_t s = (it + j) % kStages;
-              issue(s, j, 1, 2, tmem_acc);
-              free_stage(s);
+              if (elect_one()) {
+                issue(s, j, 1, 2, tmem_acc);
+                free_stage(s);
+              }
+              __syncwarp();
             }
             it += pro;
             kb = pro;
@@ -405,7 +413,7 @@ struct TcGemm {
             const uint32_t s = it % kStages;
             const uint32_t ph = (it / kStages) & 1u;
             KCG_TLC(c_wait);
-            if (!mbar_wait(&bars->full[s], ph, &bars->abort_flag)) {
+            if (!mbar_wait_warp(&bars->full[s], ph, &bars->abort_flag)) {
               report(p, bars, KCG_ST_TIMEOUT_MMA, it, s);
               ok = false;
               break;
@@ -414,13 +422,16 @@ struct TcGemm {
             tc_fence_after_sync();
             if (it == 0) KCG_TL(3);
             KCG_TLC(c_issue);
-            issue(s, kb, 0, MT, tmem_acc);
-            free_stage(s);
+            if (elect_one()) {
+              issue(s, kb, 0, MT, tmem_acc);
+              free_stage(s);
+            }
+            __syncwarp();
             KCG_TLC_ADD(13, c_issue);
           }
           if (acc_it == 0) KCG_TL(4);
           if (acc_it < 4) KCG_TL(24 + acc_it);  // MMAs of the CTA's first four units issued
-          if (ok) {
+          if (ok && elect_one()) {
             if constexpr (kPair) {
               umma_commit_pair(smem_u32(&bars->tmem_full[ab]));
               umma_commit_pair(map_to_cta(smem_u32(&bars->tmem_full[ab]), 1u));
@@ -428,6 +439,7 @@ struct TcGemm {
               umma_commit(&bars->tmem_full[ab]);
             }
           }
+          __syncwarp();
         }
       }
     } else if (warp >= 6) {

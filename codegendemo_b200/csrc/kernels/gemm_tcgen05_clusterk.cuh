@@ -254,12 +254,16 @@ struct TcGemmClusterK {
       cluster_arrive_relaxed();  // second phase (see the epilogue warps)
     } else if (warp == 1) {
       // ---------------------------------------------------------- MMA issuer
-      if (lane == 0) {
+      {
+        // The whole warp walks this loop and elects one lane per batch of instructions, so that their descriptors are
+        // warp-uniform values: inside an if (lane == 0) every tcgen05.mma takes about 125 cycles to issue (measured in
+        // the fused attention kernel), as long as a 128 x 256 x 16 product runs.
+        const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
         bool ok = true;
         for (int kb = 0; kb < kbn; ++kb) {
           const uint32_t s = kb % kStages;
           const uint32_t ph = (kb / kStages) & 1u;
-          if (!mbar_wait(&bars->full[s], ph, &bars->abort_flag)) {
+          if (!mbar_wait_warp(&bars->full[s], ph, &bars->abort_flag)) {
             report(p, bars, KCG_ST_TIMEOUT_MMA, kb, s);
             ok = false;
             break;
@@ -267,30 +271,33 @@ struct TcGemmClusterK {
           tc_fence_after_sync();
           const uint32_t sa = smem_u32(smem + s * STAGE_BYTES);
           const uint32_t sb = sa + L.a_bytes;
+          if (elect_one()) {
 #pragma unroll
-          for (int ks = 0; ks < KSTEPS; ++ks) {
-            uint32_t a_off;
-            if constexpr (kATrans) {
-              a_off = ks * UMMA_K * 128;
-            } else {
-              constexpr int swb = (kBK * EB < 128) ? kBK * EB : 128;
-              a_off = ((ks * 32) / swb) * L.a_box_bytes + ((ks * 32) % swb);
+            for (int ks = 0; ks < KSTEPS; ++ks) {
+              uint32_t a_off;
+              if constexpr (kATrans) {
+                a_off = ks * UMMA_K * 128;
+              } else {
+                constexpr int swb = (kBK * EB < 128) ? kBK * EB : 128;
+                a_off = ((ks * 32) / swb) * L.a_box_bytes + ((ks * 32) % swb);
+              }
+              uint32_t b_off;
+              if constexpr (kBTrans) {
+                constexpr int swb = (kBK * EB < 128) ? kBK * EB : 128;
+                b_off = ((ks * 32) / swb) * L.b_box_bytes + ((ks * 32) % swb);
+              } else {
+                b_off = ks * UMMA_K * 128;
+              }
+              const uint64_t adesc = make_smem_desc(sa + a_off, L.a_lbo, L.a_sbo, L.a_desc_swizzle);
+              const uint64_t bdesc = make_smem_desc(sb + b_off, L.b_lbo, L.b_sbo, L.b_desc_swizzle);
+              umma_ss<false>(tmem_u, adesc, bdesc, IDESC, (kb > 0 || ks > 0) ? 1u : 0u);
             }
-            uint32_t b_off;
-            if constexpr (kBTrans) {
-              constexpr int swb = (kBK * EB < 128) ? kBK * EB : 128;
-              b_off = ((ks * 32) / swb) * L.b_box_bytes + ((ks * 32) % swb);
-            } else {
-              b_off = ks * UMMA_K * 128;
-            }
-            const uint64_t adesc = make_smem_desc(sa + a_off, L.a_lbo, L.a_sbo, L.a_desc_swizzle);
-            const uint64_t bdesc = make_smem_desc(sb + b_off, L.b_lbo, L.b_sbo, L.b_desc_swizzle);
-            umma_ss<false>(tmem_base, adesc, bdesc, IDESC, (kb > 0 || ks > 0) ? 1u : 0u);
+            umma_commit(&bars->empty[s]);
           }
-          umma_commit(&bars->empty[s]);
+          __syncwarp();
         }
         KCG_CTL(3);
-        if (ok && kbn > 0) umma_commit(&bars->tmem_full);
+        if (ok && kbn > 0 && elect_one()) umma_commit(&bars->tmem_full);
       }
       __syncwarp();
       cluster_wait();

@@ -195,8 +195,12 @@ struct TcGemmF32x3 {
           }
         }
         griddep_launch_dependents();  // every load is issued: the stream's next kernel may be brought in
-      } else if (warp == 1 && lane == 0 && rank == 0u) {
+      } else if (warp == 1 && rank == 0u) {
         // ---------------------------- MMA issuer (in a pair: the leader CTA only)
+        // The whole warp walks this loop and elects one lane per batch of instructions, so that their descriptors are
+        // warp-uniform values: inside an if (lane == 0) every tcgen05.mma takes about 125 cycles to issue (measured in
+        // the fused attention kernel), as long as a 128 x 256 x 16 product runs.
+        const uint32_t tmem_base_u = __shfl_sync(0xffffffffu, tmem_base, 0);
         uint32_t it = 0, chunk_it = 0;
         bool ok = true;
         Iter units(p, unit0, unit_stride, tiles_m, tiles_n, num_kb);
@@ -205,20 +209,20 @@ struct TcGemmF32x3 {
           for (int kb0 = 0; kb0 < w.kbn && ok; kb0 += kChunk, ++chunk_it) {
             const uint32_t ab = chunk_it & 1u;
             const uint32_t aph = (chunk_it >> 1) & 1u;
-            if (!mbar_wait(&bars->tmem_empty[ab], aph ^ 1u, &bars->abort_flag)) {
+            if (!mbar_wait_warp(&bars->tmem_empty[ab], aph ^ 1u, &bars->abort_flag)) {
               report(p, bars, KCG_ST_TIMEOUT_MMA, 0x100u + ab, chunk_it);
               ok = false;
               break;
             }
             tc_fence_after_sync();
-            const uint32_t tmem_acc = tmem_base + ab * ACC_COLS;
+            const uint32_t tmem_acc = tmem_base_u + ab * ACC_COLS;
             const int kb1 = (kb0 + kChunk < w.kbn) ? kb0 + kChunk : w.kbn;
             for (int kb = kb0; kb < kb1; ++kb, ++it) {
               const uint32_t s = it % kStages;
               const uint32_t sl = it % LO_STAGES;
               const uint32_t phl = (it / LO_STAGES) & 1u;
               // the lo twin is written after the hi stage has landed (in both CTAs of a pair)
-              if (!mbar_wait(&bars->split_full[sl], phl, &bars->abort_flag)) {
+              if (!mbar_wait_warp(&bars->split_full[sl], phl, &bars->abort_flag)) {
                 report(p, bars, KCG_ST_TIMEOUT_MMA, it, s);
                 ok = false;
                 break;
@@ -228,50 +232,53 @@ struct TcGemmF32x3 {
               const uint32_t sb = sa + L.a_bytes;
               const uint32_t sa_lo = smem_u32(smem + LO_RING + sl * STAGE_HI);
               const uint32_t sb_lo = sa_lo + L.a_bytes;
+              if (elect_one()) {
 #pragma unroll
-              for (int ks = 0; ks < KSTEPS; ++ks) {
-                uint32_t a_off;
-                if constexpr (kATrans) {
-                  a_off = ks * UMMA_K * 128;
-                } else {
-                  constexpr int swb = (kBK * 4 < 128) ? kBK * 4 : 128;
-                  a_off = ((ks * 32) / swb) * L.a_box_bytes + ((ks * 32) % swb);
-                }
-                const uint32_t b_off = ks * UMMA_K * 128;
-                const uint32_t first = (kb > kb0 || ks > 0) ? 1u : 0u;
-                const uint64_t bdesc = make_smem_desc(sb + b_off, L.b_lbo, L.b_sbo, L.b_desc_swizzle);
-                const uint64_t bdesc_lo =
-                    make_smem_desc(sb_lo + b_off, L.b_lbo, L.b_sbo, L.b_desc_swizzle);
-#pragma unroll
-                for (int t = 0; t < MT; ++t) {
-                  const uint32_t a_t = kATrans ? t * (128 / L.atom) * L.a_box_bytes
-                                               : t * 128 * (L.a_box_bytes / R);
-                  const uint64_t adesc =
-                      make_smem_desc(sa + a_t + a_off, L.a_lbo, L.a_sbo, L.a_desc_swizzle);
-                  const uint64_t adesc_lo = make_smem_desc(sa_lo + a_t + a_off, L.a_lbo,
-                                                           L.a_sbo, L.a_desc_swizzle);
-                  const uint32_t d = tmem_acc + t * kBN;
-                  if constexpr (kPair) {
-                    umma_ss_pair<true>(d, adesc_lo, bdesc, IDESC, first);
-                    umma_ss_pair<true>(d, adesc, bdesc_lo, IDESC, 1u);
-                    umma_ss_pair<true>(d, adesc, bdesc, IDESC, 1u);
+                for (int ks = 0; ks < KSTEPS; ++ks) {
+                  uint32_t a_off;
+                  if constexpr (kATrans) {
+                    a_off = ks * UMMA_K * 128;
                   } else {
-                    umma_ss<true>(d, adesc_lo, bdesc, IDESC, first);
-                    umma_ss<true>(d, adesc, bdesc_lo, IDESC, 1u);
-                    umma_ss<true>(d, adesc, bdesc, IDESC, 1u);
+                    constexpr int swb = (kBK * 4 < 128) ? kBK * 4 : 128;
+                    a_off = ((ks * 32) / swb) * L.a_box_bytes + ((ks * 32) % swb);
+                  }
+                  const uint32_t b_off = ks * UMMA_K * 128;
+                  const uint32_t first = (kb > kb0 || ks > 0) ? 1u : 0u;
+                  const uint64_t bdesc = make_smem_desc(sb + b_off, L.b_lbo, L.b_sbo, L.b_desc_swizzle);
+                  const uint64_t bdesc_lo =
+                      make_smem_desc(sb_lo + b_off, L.b_lbo, L.b_sbo, L.b_desc_swizzle);
+#pragma unroll
+                  for (int t = 0; t < MT; ++t) {
+                    const uint32_t a_t = kATrans ? t * (128 / L.atom) * L.a_box_bytes
+                                                 : t * 128 * (L.a_box_bytes / R);
+                    const uint64_t adesc =
+                        make_smem_desc(sa + a_t + a_off, L.a_lbo, L.a_sbo, L.a_desc_swizzle);
+                    const uint64_t adesc_lo = make_smem_desc(sa_lo + a_t + a_off, L.a_lbo,
+                                                             L.a_sbo, L.a_desc_swizzle);
+                    const uint32_t d = tmem_acc + t * kBN;
+                    if constexpr (kPair) {
+                      umma_ss_pair<true>(d, adesc_lo, bdesc, IDESC, first);
+                      umma_ss_pair<true>(d, adesc, bdesc_lo, IDESC, 1u);
+                      umma_ss_pair<true>(d, adesc, bdesc, IDESC, 1u);
+                    } else {
+                      umma_ss<true>(d, adesc_lo, bdesc, IDESC, first);
+                      umma_ss<true>(d, adesc, bdesc_lo, IDESC, 1u);
+                      umma_ss<true>(d, adesc, bdesc, IDESC, 1u);
+                    }
                   }
                 }
+                // the hi stage, and with it the lo stage of this K block, is free in both CTAs
+                // once these MMAs retire
+                if constexpr (kPair) {
+                  umma_commit_pair(smem_u32(&bars->empty[s]));
+                  umma_commit_pair(map_to_cta(smem_u32(&bars->empty[s]), 1u));
+                } else {
+                  umma_commit(&bars->empty[s]);
+                }
               }
-              // the hi stage, and with it the lo stage of this K block, is free in both CTAs
-              // once these MMAs retire
-              if constexpr (kPair) {
-                umma_commit_pair(smem_u32(&bars->empty[s]));
-                umma_commit_pair(map_to_cta(smem_u32(&bars->empty[s]), 1u));
-              } else {
-                umma_commit(&bars->empty[s]);
-              }
+              __syncwarp();
             }
-            if (ok) {
+            if (ok && elect_one()) {
               if constexpr (kPair) {
                 umma_commit_pair(smem_u32(&bars->tmem_full[ab]));
                 umma_commit_pair(map_to_cta(smem_u32(&bars->tmem_full[ab]), 1u));
@@ -279,6 +286,7 @@ struct TcGemmF32x3 {
                 umma_commit(&bars->tmem_full[ab]);
               }
             }
+            __syncwarp();
           }
         }
       }

@@ -95,6 +95,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
   }
 }
 
+// mbar_wait made by a whole (converged) warp: true only if every lane saw the phase complete.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+}
+
 // --------------------------------------------------------------------- fences
 // Generic-proxy writes to shared memory -> visible to the async proxy
 // (TMA stores, tcgen05.mma operand reads).
