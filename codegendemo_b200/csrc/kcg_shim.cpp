@@ -138,6 +138,25 @@ struct StreamSlot {
 };
 constexpr size_t kMaxStreamSlots = 32;
 
+// What a 2-D tensor map depends on.
+struct MapKey {
+  uint64_t ptr, inner, outer, row_bytes;
+  int32_t dtype, box_inner, box_outer, swizzle;
+  bool operator==(const MapKey& o) const { return memcmp(this, &o, sizeof(MapKey)) == 0; }
+};
+static_assert(sizeof(MapKey) == 48, "compared and hashed as bytes: no padding");
+struct MapKeyHash {
+  size_t operator()(const MapKey& k) const {
+    uint64_t w[sizeof(MapKey) / 8], h = 0;
+    memcpy(w, &k, sizeof(k));
+    for (uint64_t v : w) {  // xor-multiply-shift per word
+      h = (h ^ v) * 0x9e3779b97f4a7c15ull;
+      h ^= h >> 32;
+    }
+    return static_cast<size_t>(h);
+  }
+};
+
 struct DeviceState {
   bool init = false;
   CUcontext ctx = nullptr;
@@ -147,7 +166,7 @@ struct DeviceState {
   size_t hbuf_bytes[3] = {0, 0, 0};
   CUstream hstream[3] = {nullptr, nullptr, nullptr};  // kcg_matmul_host: copy-in, compute, copy-out
   std::vector<CUevent> hevents;                       // slab hand-off events of kcg_matmul_host
-  std::unordered_map<std::string, CUtensorMap> tmaps;
+  std::unordered_map<MapKey, CUtensorMap, MapKeyHash> tmaps;
 };
 constexpr int kMaxDevices = 16;
 DeviceState g_dev[kMaxDevices];
@@ -695,10 +714,7 @@ int fill_info(const Cfg& c, const Resolved& r, const std::string& name, const st
 
 int encode_map(DeviceState* s, CUtensorMap* out, int dtype, uint64_t ptr, uint64_t inner, uint64_t outer,
                uint64_t row_bytes, int box_inner, int box_outer, int swizzle) {
-  char key[160];
-  snprintf(key, sizeof(key), "%d:%llx:%llu:%llu:%llu:%d:%d:%d", dtype, (unsigned long long)ptr,
-           (unsigned long long)inner, (unsigned long long)outer, (unsigned long long)row_bytes, box_inner,
-           box_outer, swizzle);
+  const MapKey key{ptr, inner, outer, row_bytes, dtype, box_inner, box_outer, swizzle};
   auto it = s->tmaps.find(key);  // the caller holds g_dev_mutex
   if (it != s->tmaps.end()) {
     *out = it->second;

@@ -60,53 +60,41 @@ class CudaLauncher:
         device addresses or tensors shaped like c) also receive every finished tile: the fused
         all-gather of an M-sharded product. The reference's launcher has no such arguments and the plain
         call behaves as the reference's."""
-        rt = self._getWrapper()
+        rt = self.m_runtime
+        if rt is None:
+            rt = self._getWrapper()
         if len(args) != 3:
             raise TypeError("matmul kernel takes (a, b, c)")
         if stream is None:
             stream = DeviceInfo.get_cuda_stream(device)
-        a, b, c = (_pointer_of(x) for x in args)
+        a, b, c = args
         lib = _lib.get_lib()
-        if lda or ldb or ldc:
-            # operands that are sub-matrices of wider row-major arrays: elements between rows (0 = contiguous)
-            if peers:
-                raise ValueError("a strided launch has no fused all-gather")
-            fused = not (alpha == 1.0 and beta == 0.0 and bias is None and not relu)
-            epi = _lib.Epilogue(float(alpha), float(beta), _pointer_of(bias) if bias is not None else 0,
-                                int(bool(relu))) if fused else None
-            _lib.check(lib.kcg_launch_gemm_strided(ctypes.c_uint64(rt.m_function), ctypes.byref(self.m_cInfo),
-                                                   int(device), ctypes.c_uint64(int(stream)), ctypes.c_uint64(a),
-                                                   ctypes.c_uint64(b), ctypes.c_uint64(c), int(lda), int(ldb),
-                                                   int(ldc), int(batch), ctypes.byref(epi) if fused else None))
-            return
-        if batch != 1:
-            # (a, b, c) hold `batch` contiguous problems of the kernel's M, N, K (torch.bmm layout)
-            if peers:
-                raise ValueError("a batched launch has no fused all-gather")
-            fused = not (alpha == 1.0 and beta == 0.0 and bias is None and not relu)
-            epi = _lib.Epilogue(float(alpha), float(beta), _pointer_of(bias) if bias is not None else 0,
-                                int(bool(relu))) if fused else None
-            _lib.check(lib.kcg_launch_gemm_batched(ctypes.c_uint64(rt.m_function), ctypes.byref(self.m_cInfo),
-                                                   int(device), ctypes.c_uint64(int(stream)), ctypes.c_uint64(a),
-                                                   ctypes.c_uint64(b), ctypes.c_uint64(c), int(batch),
-                                                   ctypes.byref(epi) if fused else None))
-            return
-        if alpha == 1.0 and beta == 0.0 and bias is None and not relu and not peers:
-            _lib.check(lib.kcg_launch_gemm(ctypes.c_uint64(rt.m_function), ctypes.byref(self.m_cInfo),
-                                           int(device), ctypes.c_uint64(int(stream)),
-                                           ctypes.c_uint64(a), ctypes.c_uint64(b), ctypes.c_uint64(c)))
-            return
-        epi = _lib.Epilogue(float(alpha), float(beta), _pointer_of(bias) if bias is not None else 0, int(bool(relu)))
+        epi = None
+        if alpha != 1.0 or beta != 0.0 or bias is not None or relu:
+            epi = ctypes.byref(_lib.Epilogue(float(alpha), float(beta), _pointer_of(bias) if bias is not None else 0,
+                                             int(bool(relu))))
         if peers:
+            if lda or ldb or ldc:
+                raise ValueError("a strided launch has no fused all-gather")
+            if batch != 1:
+                raise ValueError("a batched launch has no fused all-gather")
+            if epi is None:
+                epi = ctypes.byref(_lib.Epilogue(1.0, 0.0, 0, 0))
             arr = (ctypes.c_uint64 * len(peers))(*[_pointer_of(x) for x in peers])
-            _lib.check(lib.kcg_launch_gemm_allgather(ctypes.c_uint64(rt.m_function), ctypes.byref(self.m_cInfo),
-                                                     int(device), ctypes.c_uint64(int(stream)), ctypes.c_uint64(a),
-                                                     ctypes.c_uint64(b), ctypes.c_uint64(c), ctypes.byref(epi),
-                                                     arr, len(peers)))
-            return
-        _lib.check(lib.kcg_launch_gemm_ex(ctypes.c_uint64(rt.m_function), ctypes.byref(self.m_cInfo),
-                                          int(device), ctypes.c_uint64(int(stream)), ctypes.c_uint64(a),
-                                          ctypes.c_uint64(b), ctypes.c_uint64(c), ctypes.byref(epi)))
+            status = lib.kcg_launch_gemm_allgather(rt.m_function, ctypes.byref(self.m_cInfo), int(device), int(stream),
+                                                   _pointer_of(a), _pointer_of(b), _pointer_of(c), epi, arr, len(peers))
+        elif lda or ldb or ldc or batch == 1:
+            # one entry for plain launches and for operands that are sub-matrices of wider row-major arrays (elements
+            # between rows; 0 = contiguous)
+            status = lib.kcg_launch_gemm_strided(rt.m_function, ctypes.byref(self.m_cInfo), int(device), int(stream),
+                                                 _pointer_of(a), _pointer_of(b), _pointer_of(c), int(lda), int(ldb),
+                                                 int(ldc), int(batch), epi)
+        else:
+            # (a, b, c) hold `batch` contiguous problems of the kernel's M, N, K (torch.bmm layout)
+            status = lib.kcg_launch_gemm_batched(rt.m_function, ctypes.byref(self.m_cInfo), int(device), int(stream),
+                                                 _pointer_of(a), _pointer_of(b), _pointer_of(c), int(batch), epi)
+        if status:
+            _lib.check(status)
 
     def runHost(self, device, hostA, hostB, hostC, stream=None):
         """Whole operator on host buffers (H2D, kernel, D2H, synchronise)."""

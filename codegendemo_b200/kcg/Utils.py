@@ -6,6 +6,7 @@ Same names and meanings as the reference: ``EnumKernelDType`` (:198-209, plus ``
 time (the reference calls ``torch.cuda.current_device()`` while importing), so compile workers and
 CPU-only tests can import the package freely.
 """
+import functools
 import json
 import os
 import pickle
@@ -103,18 +104,23 @@ def is_hip() -> bool:
     return False
 
 
+@functools.lru_cache(maxsize=None)
+def _raw_stream_getter():
+    import torch
+    try:
+        from torch._C import _cuda_getCurrentRawStream
+        return _cuda_getCurrentRawStream
+    except ImportError:
+        return lambda idx: torch.cuda.current_stream(idx).cuda_stream
+
+
 class DeviceInfo:
     @staticmethod
     def get_cuda_stream(idx=None) -> int:
         """Raw CUstream of torch's current stream on device ``idx`` (what the launcher launches on)."""
-        import torch
         if idx is None:
             idx = DeviceInfo.get_current_device()
-        try:
-            from torch._C import _cuda_getCurrentRawStream
-            return _cuda_getCurrentRawStream(idx)
-        except ImportError:
-            return torch.cuda.current_stream(idx).cuda_stream
+        return _raw_stream_getter()(idx)
 
     @staticmethod
     def get_current_device() -> int:
