@@ -18,6 +18,7 @@
 // of which about 3100 cycles for two tiles' steps remain exposed against 2048 of the tensor pipe alone. Measured (B200,
 // bf16), a form with votes of all softmax warps, O rescaled at every new maximum and a one-lane issuer against this
 // one: 32 heads x 4096 x 4096 x 128 322 -> 246 us (1119 TFLOP/s), x 64 287 -> 210 us, 16 x 2048 x 2048 x 128 46 -> 36 us.
+// A key-split form of it (kKeySplit) shares a group's keys among the CTAs of a cluster where groups do not fill a wave.
 // Tried without gain: exponentials of every eighth to third pair as a polynomial on the FMA pipe (2 to 8 % slower: one
 // warp per scheduler and tile is bound by its own latencies, not by the exponential pipe).
 // Four single-tile forms are kept for comparison
@@ -152,9 +153,14 @@ struct AttnParams {
   void* O;                    // heads x sq x d, contiguous
   int sq, sk;
   float scale_log2;           // scale * log2(e): the softmax runs on exp2
+  int first_group;            // AttnFwd2: group of 256 rows of the first CTA (cluster)
+  int splits;                 // AttnFwd2, key-split form: CTAs that share a group's keys
+  int tail_follows;           // AttnFwd2: the groups after this launch's are run by a key-split launch right behind it
 };
 
 enum : uint32_t { ATTN_TIMEOUT_PRODUCER = 1, ATTN_TIMEOUT_MMA = 2, ATTN_TIMEOUT_SOFTMAX = 3 };
+
+#include "kernels/attn_decode.cuh"
 
 // kBC = keys per step (64 or 128); kSplit = threads per query row (1 or 2). With 64 keys per step and one
 // thread per row a CTA needs 96 KB of shared memory (d = 128), 256 TMEM columns and 192 threads, so TWO CTAs
@@ -544,7 +550,7 @@ struct AttnFwd {
 // per thread and step. A tile's chain is serial (S, softmax, P V, next S: the next scores overwrite P, and the
 // tensor pipe runs its instructions in order), the two chains interleave. The MMA warp serves the tiles in a fixed
 // order (serving whichever P is ready first measured no faster).
-template <int kD, bool kBf16>
+template <int kD, bool kBf16, bool kKeySplit>
 struct AttnFwd2 {
   static constexpr int BR = 128, BC = 128, TILES = 2;
   static constexpr int K_STAGES = 2, V_STAGES = 2;
@@ -589,9 +595,17 @@ struct AttnFwd2 {
     Barriers* bars = reinterpret_cast<Barriers*>(smem + RING_BYTES);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int q_groups = (p.sq + TILES * BR - 1) / (TILES * BR);
-    const int head = static_cast<int>(blockIdx.x) / q_groups;
-    const int q0 = (static_cast<int>(blockIdx.x) % q_groups) * (TILES * BR);
-    const int nkv = (p.sk + BC - 1) / BC;
+    const int rank = kKeySplit ? static_cast<int>(cluster_cta_rank()) : 0;
+    const int group = p.first_group + static_cast<int>(blockIdx.x) / (kKeySplit ? p.splits : 1);
+    const int head = group / q_groups;
+    const int q0 = (group % q_groups) * (TILES * BR);
+    // steps of this CTA: [key0 / BC, key0 / BC + nkv); splits <= steps, so every CTA has at least one
+    const int steps = (p.sk + BC - 1) / BC;
+    const int step0 = kKeySplit ? static_cast<int>(static_cast<long long>(steps) * rank / p.splits) : 0;
+    const int nkv =
+        (kKeySplit ? static_cast<int>(static_cast<long long>(steps) * (rank + 1) / p.splits) : steps) - step0;
+    const int key0 = step0 * BC;
+    if (!kKeySplit && p.tail_follows) griddep_launch_dependents();
 
     if (threadIdx.x == 0) {
       tma_prefetch_desc(&p.tmQ);
@@ -647,7 +661,7 @@ struct AttnFwd2 {
             mbar_expect_tx(&bars->k_full[ks], KV_BYTES);
   #pragma unroll
             for (int b = 0; b < BOXES; ++b)
-              tma_load_3d(smem + OFF_K + ks * KV_BYTES + b * KVBOX_BYTES, &p.tmK, &bars->k_full[ks], b * 64, j * BC, head);
+              tma_load_3d(smem + OFF_K + ks * KV_BYTES + b * KVBOX_BYTES, &p.tmK, &bars->k_full[ks], b * 64, key0 + j * BC, head);
             if (!mbar_wait(&bars->v_empty[vs], ((j / V_STAGES) & 1u) ^ 1u, &bars->abort_flag)) {
               report(bars, ATTN_TIMEOUT_PRODUCER, j, 1u);
               break;
@@ -655,7 +669,7 @@ struct AttnFwd2 {
             mbar_expect_tx(&bars->v_full[vs], KV_BYTES);
   #pragma unroll
             for (int b = 0; b < BOXES; ++b)
-              tma_load_3d(smem + OFF_V + vs * KV_BYTES + b * KVBOX_BYTES, &p.tmV, &bars->v_full[vs], b * 64, j * BC, head);
+              tma_load_3d(smem + OFF_V + vs * KV_BYTES + b * KVBOX_BYTES, &p.tmV, &bars->v_full[vs], b * 64, key0 + j * BC, head);
           }
         }
       } else if (warp == 1) {
@@ -736,6 +750,11 @@ struct AttnFwd2 {
           }
         }
       }  // (warps 2 and 3 only give their registers)
+      if constexpr (kKeySplit) {  // the two meetings of the cluster that join the partial results
+        __syncwarp();
+        cluster_sync_all();
+        cluster_sync_all();
+      }
     } else {
       asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
       // ------------------------------------------------- softmax, correction, epilogue
@@ -765,7 +784,7 @@ struct AttnFwd2 {
         tmem_ld_wait();
 #pragma unroll
         for (int c = 0; c < 4; ++c) pin_32(sr[c]);
-        const int valid = p.sk - j * BC;
+        const int valid = p.sk - key0 - j * BC;
         if (valid < BC) {
 #pragma unroll
           for (int c = 0; c < 4; ++c)
@@ -859,32 +878,99 @@ struct AttnFwd2 {
           ok = false;
         }
       }
-      if (ok) {
-        tc_fence_after_sync();
-        const float inv = 1.f / l;
-        const int grow = q0 + t * BR + row;
-        T* out = reinterpret_cast<T*>(p.O) + (static_cast<size_t>(head) * p.sq + grow) * kD;
+      if constexpr (kKeySplit) {
+        // Partial results: once the products of BOTH tiles have retired, the operand ring holds this CTA's O rows
+        // (fp32, not normalised, 16-byte units XOR-swizzled by the row: a warp writes 32 rows at a time) and their
+        // {maximum, sum}; then each CTA joins an equal share of the output over the cluster's shared memories.
+        constexpr int UNITS = kD / 4;  // 16-byte units of a row
+        constexpr int OFF_ML = TILES * BR * kD * 4;
+        static_assert(OFF_ML + TILES * BR * 8 <= RING_BYTES, "the partial result must fit the ring");
+        if (ok) {
+          const bool got = mbar_wait(&bars->o_full[t ^ 1], 0u, &bars->abort_flag);
+          if (!__all_sync(0xffffffffu, got)) {
+            if (lane == 0) report(bars, ATTN_TIMEOUT_SOFTMAX, 3u, 0u);
+            ok = false;
+          }
+        }
+        if (ok) {
+          tc_fence_after_sync();
+          const int r = t * BR + row;
+          uint8_t* mine = smem + r * kD * 4;
 #pragma unroll
-        for (int c = 0; c < kD / 32; ++c) {
-          uint32_t r[32];
-          tmem_ld_32x32b_x32(col_o + c * 32, r);
-          tmem_ld_wait();
-          if (grow < p.sq) {
+          for (int c = 0; c < kD / 32; ++c) {
+            uint32_t o[32];
+            tmem_ld_32x32b_x32(col_o + c * 32, o);
+            tmem_ld_wait();
+            pin_32(o);
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              uint32_t w[4];
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const float a = __uint_as_float(r[u * 8 + 2 * e]) * inv, bb = __uint_as_float(r[u * 8 + 2 * e + 1]) * inv;
-                if constexpr (kBf16) {
-                  __nv_bfloat162 v2 = __floats2bfloat162_rn(a, bb);
-                  w[e] = *reinterpret_cast<uint32_t*>(&v2);
-                } else {
-                  __half2 v2 = __floats2half2_rn(a, bb);
-                  w[e] = *reinterpret_cast<uint32_t*>(&v2);
+            for (int u = 0; u < 8; ++u)
+              *reinterpret_cast<uint4*>(mine + (((c * 8 + u) ^ (r & (UNITS - 1))) << 4)) =
+                  make_uint4(o[4 * u], o[4 * u + 1], o[4 * u + 2], o[4 * u + 3]);
+          }
+          reinterpret_cast<float2*>(smem + OFF_ML)[r] = make_float2(m, l);
+        }
+        __syncwarp();
+        cluster_sync_all();
+        if (ok) {
+          const int rows = p.sq - q0 < TILES * BR ? p.sq - q0 : TILES * BR;
+          const int u0 = rows * UNITS * rank / p.splits, u1 = rows * UNITS * (rank + 1) / p.splits;
+          const uint32_t base_addr = smem_u32(smem);
+          T* out = reinterpret_cast<T*>(p.O) + (static_cast<size_t>(head) * p.sq + q0) * kD;
+          for (int i = u0 + static_cast<int>(threadIdx.x) - 128; i < u1; i += TILES * 128) {
+            const int r = i / UNITS, u = i % UNITS;
+            const uint32_t ml_addr = base_addr + OFF_ML + r * 8;
+            const uint32_t o_addr = base_addr + r * kD * 4 + ((u ^ (r & (UNITS - 1))) << 4);
+            float top = -INFINITY;
+            for (int c = 0; c < p.splits; ++c) top = fmaxf(top, ld_cluster_f2(map_to_cta(ml_addr, c)).x);
+            float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+            float sum = 0.f;
+#pragma unroll 4
+            for (int c = 0; c < p.splits; ++c) {
+              const float2 ml = ld_cluster_f2(map_to_cta(ml_addr, c));
+              const float4 x = ld_cluster_f4(map_to_cta(o_addr, c));
+              const float f = ml.x == -INFINITY ? 0.f : ex2(ml.x - top);
+              a.x = fmaf(f, x.x, a.x);
+              a.y = fmaf(f, x.y, a.y);
+              a.z = fmaf(f, x.z, a.z);
+              a.w = fmaf(f, x.w, a.w);
+              sum = fmaf(f, ml.y, sum);
+            }
+            const float inv = 1.f / sum;
+            *reinterpret_cast<uint2*>(out + 4 * static_cast<size_t>(i)) =
+                make_uint2(pack_pair<kBf16>(a.x * inv, a.y * inv), pack_pair<kBf16>(a.z * inv, a.w * inv));
+          }
+        }
+        __syncwarp();
+        cluster_sync_all();  // the other CTAs read this one's shared memory until here
+        griddep_wait();      // behind a launch of whole groups: complete after it, so that what follows waits for both
+      } else {
+        if (ok) {
+          tc_fence_after_sync();
+          const float inv = 1.f / l;
+          const int grow = q0 + t * BR + row;
+          T* out = reinterpret_cast<T*>(p.O) + (static_cast<size_t>(head) * p.sq + grow) * kD;
+  #pragma unroll
+          for (int c = 0; c < kD / 32; ++c) {
+            uint32_t r[32];
+            tmem_ld_32x32b_x32(col_o + c * 32, r);
+            tmem_ld_wait();
+            if (grow < p.sq) {
+  #pragma unroll
+              for (int u = 0; u < 4; ++u) {
+                uint32_t w[4];
+  #pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  const float a = __uint_as_float(r[u * 8 + 2 * e]) * inv, bb = __uint_as_float(r[u * 8 + 2 * e + 1]) * inv;
+                  if constexpr (kBf16) {
+                    __nv_bfloat162 v2 = __floats2bfloat162_rn(a, bb);
+                    w[e] = *reinterpret_cast<uint32_t*>(&v2);
+                  } else {
+                    __half2 v2 = __floats2half2_rn(a, bb);
+                    w[e] = *reinterpret_cast<uint32_t*>(&v2);
+                  }
                 }
+                *reinterpret_cast<uint4*>(out + c * 32 + u * 8) = make_uint4(w[0], w[1], w[2], w[3]);
               }
-              *reinterpret_cast<uint4*>(out + c * 32 + u * 8) = make_uint4(w[0], w[1], w[2], w[3]);
             }
           }
         }
@@ -906,11 +992,9 @@ struct AttnFwd2 {
   }
 };
 
-#include "kernels/attn_decode.cuh"
-
-template <int kD, bool kBf16>
+template <int kD, bool kBf16, bool kKeySplit>
 __global__ void __launch_bounds__(384, 1) kcg_attention2_kernel(const __grid_constant__ AttnParams p) {
-  AttnFwd2<kD, kBf16>::run(p);
+  AttnFwd2<kD, kBf16, kKeySplit>::run(p);
 }
 
 template <int kD, bool kBf16, int kBC, int kSplit, int kPTmem>
@@ -923,7 +1007,7 @@ using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, voi
                               const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                               CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 EncodeFn g_encode = nullptr;
-bool g_ready[16][32];  // [device][kernel instance]: dynamic shared memory opted in
+bool g_ready[16][36];  // [device][kernel instance]: dynamic shared memory opted in
 std::mutex g_mutex;
 
 int fail(int code, const std::string& msg) { return kcg_internal_fail(code, msg.c_str()); }
@@ -997,16 +1081,53 @@ int launch(int device, int slot, cudaStream_t st, const Problem& pb) {
   return 0;
 }
 
+// How many clusters of 2 .. 8 CTAs of the key-split kernel run at once (asked once per device and kernel).
+int g_clusters[16][4][9];
+
+// The largest number of CTAs, 2 to 8, that `groups` groups of 256 rows can share their keys among with every cluster
+// running at once and at least four steps of 128 keys per CTA (joining costs what two steps do); 1 = none.
+int key_splits(const int (&clusters)[9], long long groups, int sk) {
+  const int steps = (sk + 127) / 128;
+  for (int s = 8; s >= 2; --s)
+    if (groups <= clusters[s] && steps >= 4 * s) return s;
+  return 1;
+}
+
 template <int kD, bool kBf16>
-int launch2(int device, int slot, cudaStream_t st, const Problem& pb) {
-  using Kern = AttnFwd2<kD, kBf16>;
+int launch2(int device, int kind, cudaStream_t st, const Problem& pb) {
+  using Kern = AttnFwd2<kD, kBf16, false>;
+  using Split = AttnFwd2<kD, kBf16, true>;
+  const auto whole = kcg_attention2_kernel<kD, kBf16, false>;
+  const auto split = kcg_attention2_kernel<kD, kBf16, true>;
+  cudaLaunchConfig_t cfg{};
+  cfg.blockDim = dim3(Split::NUM_THREADS);
+  cfg.dynamicSmemBytes = Split::SMEM_BYTES;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
   {
     std::lock_guard<std::mutex> lock(g_mutex);
-    if (!g_ready[device][slot]) {
-      const cudaError_t e = cudaFuncSetAttribute(kcg_attention2_kernel<kD, kBf16>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, Kern::SMEM_BYTES);
+    if (!g_ready[device][16 + kind]) {
+      cudaError_t e = cudaFuncSetAttribute(whole, cudaFuncAttributeMaxDynamicSharedMemorySize, Kern::SMEM_BYTES);
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(split, cudaFuncAttributeMaxDynamicSharedMemorySize, Split::SMEM_BYTES);
       if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(MaxDynamicSharedMemorySize)");
-      g_ready[device][slot] = true;
+      for (int s = 2; s <= 8; ++s) {
+        attr[0].val.clusterDim.x = s;
+        cfg.gridDim = dim3(s);
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, split, &cfg) != cudaSuccess) {
+          cudaGetLastError();  // not known: this size is not used
+          n = 0;
+        }
+        g_clusters[device][kind][s] = n;
+      }
+      g_ready[device][16 + kind] = true;
     }
   }
   AttnParams p{};
@@ -1017,11 +1138,33 @@ int launch2(int device, int slot, cudaStream_t st, const Problem& pb) {
   p.sq = pb.sq;
   p.sk = pb.sk;
   p.scale_log2 = pb.scale * 1.4426950408889634f;
-  const int grid = pb.heads * ((pb.sq + 255) / 256);
-  kcg_attention2_kernel<kD, kBf16><<<grid, Kern::NUM_THREADS, Kern::SMEM_BYTES, st>>>(p);
-  const cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_fail(e, "attention launch");
-  kcg_internal_count_launch();
+  // A group of 256 rows keeps one SM for the whole walk over the keys, so 148 groups are a wave. What does not fill a
+  // wave - the remainder of a large problem, all of a small one - shares its keys among the SMs that would stand idle:
+  // (bf16) 32 heads x 4096 x 4096 x 128, 3.46 waves: 246 -> 230 us; 8 x 300 x 16384 x 128, 16 groups: 224 -> 55 us; 8 x 65
+  // x 16384 x 64, 8 groups: 33 us.
+  // The remainder is a launch of its own right behind the whole groups, allowed to start as soon as all of those have.
+  const long long groups = static_cast<long long>(pb.heads) * ((pb.sq + 255) / 256);
+  const long long rest = groups % 148;
+  const int s = rest ? key_splits(g_clusters[device][kind], rest, pb.sk) : 1;
+  const long long full = s > 1 ? groups - rest : groups;
+  if (full > 0) {
+    p.tail_follows = s > 1 ? 1 : 0;
+    whole<<<static_cast<unsigned>(full), Kern::NUM_THREADS, Kern::SMEM_BYTES, st>>>(p);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return cuda_fail(e, "attention launch");
+    kcg_internal_count_launch();
+  }
+  if (s > 1) {
+    p.first_group = static_cast<int>(full);
+    p.splits = s;
+    p.tail_follows = 0;
+    attr[0].val.clusterDim.x = s;
+    cfg.gridDim = dim3(static_cast<unsigned>(rest * s));
+    cfg.numAttrs = full > 0 ? 2 : 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, split, p);
+    if (e != cudaSuccess) return cuda_fail(e, "attention launch");
+    kcg_internal_count_launch();
+  }
   return 0;
 }
 
@@ -1153,8 +1296,8 @@ extern "C" int kcg_attention_fwd(int device, uint64_t stream, uint64_t Q, uint64
     case 6: return launch_shape<128, 2, 0>(device, 8, st, pb);
     case 7: return launch_shape<64, 1, 0>(device, 12, st, pb);
     default:
-      if (pb.d == 128) return pb.bf16 ? launch2<128, true>(device, 16, st, pb) : launch2<128, false>(device, 17, st, pb);
-      return pb.bf16 ? launch2<64, true>(device, 18, st, pb) : launch2<64, false>(device, 19, st, pb);
+      if (pb.d == 128) return pb.bf16 ? launch2<128, true>(device, 0, st, pb) : launch2<128, false>(device, 1, st, pb);
+      return pb.bf16 ? launch2<64, true>(device, 2, st, pb) : launch2<64, false>(device, 3, st, pb);
   }
 }
 

@@ -58,3 +58,31 @@ def test_nan_and_infinite_scores_stay_in_their_rows():
     clean[0, 5] = out[0, 5]
     clean[1, 200] = out[1, 200]
     assert torch.equal(out.nan_to_num(7.0), clean.nan_to_num(7.0))
+
+
+@pytest.mark.gpu
+# groups of 256 rows that do not fill a wave share their keys among 2 to 8 CTAs; 150 and 220 groups: whole groups and a
+# remainder behind them; a last CTA whose only step has one key; a group of one row; too few keys to share
+@pytest.mark.parametrize("shape", [(2, 300, 4097, 128), (1, 65, 8000, 64), (20, 257, 1100, 128), (150, 100, 1025, 64),
+                                   (55, 1000, 2049, 128), (40, 256, 1024, 128), (3, 256, 1023, 64)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_groups_that_share_their_keys(shape):
+    from codegendemo_b200.kcg.matmul_op import attention_fused, attention_status
+    heads, sq, sk, d = shape
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    q, k, v = [torch.randn((heads, n, d), generator=gen, device="cuda").bfloat16() for n in (sq, sk, sk)]
+    k[:, sk // 2:] *= 3.0  # the later keys' maxima are the larger ones
+    out = torch.full((heads, sq, d), float("nan"), dtype=torch.bfloat16, device="cuda")
+    attention_fused(q, k, v, out=out)
+    # ordered behind both launches: a copy, and the same call over the same buffer
+    copy = out.clone()
+    attention_fused(q, k, v, out=out)
+    attention_status(0)
+    assert torch.equal(copy, out)
+    bound = 2.1 * 2.0 ** -9 * v.abs().max().item()  # two roundings to 16 bits, of the probabilities and the result
+    for h in range(0, heads, max(1, heads // 8)):
+        ref = _reference(q[h:h + 1], k[h:h + 1], v[h:h + 1], d ** -0.5)
+        assert (out[h:h + 1].double() - ref).abs().max().item() <= bound
+    last = heads - 1
+    ref = _reference(q[last:], k[last:], v[last:], d ** -0.5)
+    assert (out[last:].double() - ref).abs().max().item() <= bound
