@@ -101,10 +101,55 @@ def _cheapest_tile(M, N, K, batch=1):
     return best
 
 
+# Tiles of the 3xTF32 kernels the rule below chooses from: (KERNEL_VARIANT, BLOCK_SIZE_M, N, K) -> (microseconds
+# {fixed, per 1000 values of K, per tile beyond them, per cut into K ranges}, stages). Fitted to 170 device timings
+# (graph replay, rotating operands) on 18 shapes of 128..6784 x 512..11008 x 256..8704, plain and with every tile cut
+# into 2 to 8 ranges: the tile the fit picks is 4 % behind the best measured one on average (the former rule, tiles that
+# divide the problem and the widest first, 22 %: 256x1024x256 18.4 -> 9.3 us, 256x2048x512 28.5 -> 14.8,
+# 384x3520x8128 197 -> 128, 6272x640x6144 325 -> 254 us).
+_TILE_COST_F32 = {
+    (2, 128, 64, 32): (2.63, 20.3, 1.94, 3.38, 4),
+    (2, 128, 128, 32): (3.25, 26.8, 3.85, 4.13, 3),
+    (2, 128, 256, 16): (2.74, 39.3, 9.36, 6.83, 4),
+    (4, 256, 128, 32): (2.80, 37.0, 3.05, 5.59, 4),
+    (4, 256, 256, 32): (1.98, 38.2, 10.80, 6.81, 3),
+}
+
+
+def _tile_us_f32(tile, split, M, N, K, sms=148):
+    """Estimated time of an fp32 product with one of the tiles above, in microseconds."""
+    variant, bm, bn, bk = tile
+    fixed, per_k, per_tile, per_cut, _ = _TILE_COST_F32[tile]
+    tiles, k_us = -(-M // bm) * -(-N // bn), per_k * K / 1000
+    at_once = sms // 2 if variant == 4 else sms
+    if split > 1:
+        return fixed + -(-tiles * split // at_once) * (k_us / split + per_tile) + per_cut
+    us = fixed + -(-tiles // at_once) * (k_us + per_tile)
+    f = min(8, at_once // (tiles % at_once)) if tiles % at_once else 0
+    if f >= 2:  # the launcher cuts the remainder tiles into f K ranges when that pays
+        us = min(us, fixed + tiles // at_once * (k_us + per_tile) + k_us / f + per_tile + per_cut)
+    return us
+
+
+def _cheapest_tile_f32(M, N, K, sms=148):
+    """(estimate, tile, split); a split only where all its units run at once, with four K blocks each or more."""
+    best = None
+    for tile in _TILE_COST_F32:
+        variant, bm, bn, bk = tile
+        tiles, at_once = -(-M // bm) * -(-N // bn), sms // 2 if variant == 4 else sms
+        for split in (1, 2, 3, 4, 6, 8):
+            if split > 1 and (tiles * split > at_once or K // bk < 4 * split):
+                continue
+            us = _tile_us_f32(tile, split, M, N, K)
+            if best is None or us < best[0]:
+                best = (us, tile, split)
+    return best
+
+
 def tuned_config(M: int, N: int, K: int, dtype: EnumKernelDType, isATranspose: int = 0, db=None, batch: int = 1,
                  b_transposed: bool = False) -> KernelArgMatmul:
-    """Best known config of a shape: the kernel database's entry when the shape was tuned; else, for the 16-bit
-    types, the tile with the smallest estimated time - the plain rule's choice is kept while the estimate puts it
+    """Best known config of a shape: the kernel database's entry when the shape was tuned; else (16-bit types, and
+    single fp32 products) the tile with the smallest estimated time - the plain rule's choice is kept while the estimate puts it
     within 10 % of that: the estimates of the two largest tiles are up to that much too low where a remainder is cut up
     (2048x11008x4096: 512x256x64 estimated 110, 256x256x128 118 us; measured 142 and 135, and 165 and 148 once the
     power cap holds the clock down). ``batch`` > 1: M, N, K are one
@@ -129,6 +174,14 @@ def tuned_config(M: int, N: int, K: int, dtype: EnumKernelDType, isATranspose: i
             plain = default_config(M, N, K, dtype, KERNEL_VARIANT=variant, BLOCK_SIZE_M=bm, BLOCK_SIZE_N=bn,
                                    BLOCK_SIZE_K=bk, LOCAL_SPLIT_U=split, isATranspose=isATranspose,
                                    EDGE_TILES=int(M % bm != 0 or N % bn != 0 or K % bk != 0), **stages)
+    elif batch == 1 and not isATranspose and M % 128 == 0 and N % 64 == 0 and K % 64 == 0:
+        us, tile, split = _cheapest_tile_f32(M, N, K)
+        have = (plain.KERNEL_VARIANT or 2, plain.BLOCK_SIZE_M, plain.BLOCK_SIZE_N, plain.BLOCK_SIZE_K)
+        if have not in _TILE_COST_F32 or _tile_us_f32(have, 1, M, N, K) > 1.1 * us:
+            variant, bm, bn, bk = tile
+            plain = default_config(M, N, K, dtype, KERNEL_VARIANT=variant, BLOCK_SIZE_M=bm, BLOCK_SIZE_N=bn,
+                                   BLOCK_SIZE_K=bk, LOCAL_SPLIT_U=split, NUM_STAGES=_TILE_COST_F32[tile][4],
+                                   EDGE_TILES=int(M % bm != 0 or N % bn != 0 or K % bk != 0))
     return _with_b_transposed(plain) if b_transposed else plain
 
 

@@ -55,6 +55,49 @@ def test_edge_tiles_are_an_option_with_rules_of_their_own():
             compile_info(default_config(128, N, K, E.bfloat16, BLOCK_SIZE_N=128).compileArgs(), kernel=kernel, edge_tiles=1)
 
 
+def test_every_fp32_shape_gets_a_config_the_kernels_can_build():
+    import ctypes
+    rng = random.Random(8)
+    lib = _lib.get_lib()
+    for i in range(200):
+        M, N, K = 128 * rng.randint(1, 64), 64 * rng.randint(1, 172), 64 * rng.randint(1, 172)
+        kpm = tuned_config(M, N, K, E.float32)
+        kpm.check()
+        assert (kpm.M, kpm.N, kpm.K) == (M, N, K)
+        opts = _lib.CompileOpts(kernel=kpm.KERNEL_VARIANT, num_stages=kpm.NUM_STAGES, edge_tiles=kpm.EDGE_TILES)
+        buf = ctypes.create_string_buffer(1024)
+        _lib.check(lib.kcg_kernel_name(_lib.cfg_array(kpm.compileArgs()), ctypes.byref(opts), buf, 1024))
+
+
+@pytest.mark.gpu
+# a tile of every kind the fp32 rule can pick, over the edges of M, N and K, whole and cut into K ranges
+@pytest.mark.parametrize("shape", [(128, 64, 64), (384, 320, 192), (640, 832, 1088)], ids=lambda s: "x".join(map(str, s)))
+def test_fp32_tiles_over_the_edges(shape):
+    from codegendemo_b200.kcg.matmul_op import _TILE_COST_F32
+    M, N, K = shape
+    gen = torch.Generator().manual_seed(2)
+    a, b = [torch.rand(s, generator=gen) * 2 - 1 for s in ((M, K), (K, N))]
+    bias = torch.rand(N, generator=gen)
+    ref = a.double() @ b.double()
+    for tile, cost in _TILE_COST_F32.items():
+        for split in (1, 3):
+            if split > 1 and K // tile[3] < 4 * split:
+                continue
+            kpm = default_config(M, N, K, E.float32, KERNEL_VARIANT=tile[0], BLOCK_SIZE_M=tile[1], BLOCK_SIZE_N=tile[2],
+                                 BLOCK_SIZE_K=tile[3], NUM_STAGES=cost[4], LOCAL_SPLIT_U=split, EDGE_TILES=1)
+            _, kern = build_kernel(kpm, 0)
+            wide = torch.full((M + 2, N + 64), float("nan"), device="cuda")
+            c = wide[1:1 + M, 32:32 + N]
+            for kw, want in ((dict(), ref), (dict(bias=bias.cuda(), relu=True), (ref + bias.double()).clamp(min=0))):
+                kern.run(a.cuda(), b.cuda(), c, ldc=N + 64, **kw)
+                kern.checkStatus()
+                # three TF32 products: 2^-21 of the operands' lengths' product, which |row| * |column| bounds
+                bound = 2.0 ** -20 * a.double().norm(dim=1)[:, None] * b.double().norm(dim=0)[None] + 2.0 ** -22
+                assert ((c.cpu().double() - want).abs() <= bound).all(), (tile, split)
+            wide[1:1 + M, 32:32 + N] = float("nan")
+            assert wide.isnan().all(), (tile, split)
+
+
 TILES = [(t, s) for t in _TILE_COST for s in ((2, 3, 4)[:len(_TILE_COST[t][2])] if t[0] == 5 else (1,))]
 # one tile short of everything; one block past a tile in N, half a K block past the last; several tiles and waves
 SHAPES = [(128, 64, 64), (384, 320, 192), (640, 832, 1088)]
