@@ -24,7 +24,7 @@
 // Four single-tile forms are kept for comparison
 // (AttnFwd: one query tile per CTA with two S buffers, 64- or 128-key steps, one or two threads per row, P through
 // shared or tensor memory; S issued one step ahead - two steps ahead, with a third buffer, measured slower).
-// Up to 64 query rows per head: a form of its own (kernels/attn_decode.cuh).
+// Few query rows per head (up to 64): a form of its own (kernels/attn_decode.cuh).
 // Every wait is bounded (ptx_sm100.cuh); a wait that runs out records a code in a status word the host can read
 // (kcg_attention_status), raises the CTA's abort flag and all roles fall through to the exit.
 #include <cuda.h>
@@ -1280,12 +1280,14 @@ extern "C" int kcg_attention_fwd(int device, uint64_t stream, uint64_t Q, uint64
     const char* v = getenv("KCG_ATTN_FORM");
     return v ? atoi(v) & 15 : 0;
   }();
-  // KCG_ATTN_FORM=8: the 256-row kernel for every number of queries. Up to 32 rows it loses everywhere to the form that
-  // shares a head's keys among CTAs (32 heads x 1 x 8192 x 128: 148 against 26 us, 128 x 16 x 256: 9.9 / 8.3 us); up to
-  // 64 rows it loses where that walk is long (32 x 64 x 8192: 148 / 41 us, 140 x 64 x 4096: 85 / 72 us) but not where
-  // a head's keys are few (128 x 64 x 512: 15.4 / 18.9 us, 48 x 64 x 256: 8.8 / 10.8 us). At 65 rows the warps would
-  // have to walk the keys twice.
-  if (form == 0 && (sq <= 32 || (sq <= 64 && (sk >= 2048 || (heads <= 64 && sk >= 512))))) {
+  // KCG_ATTN_FORM=8: the 256-row kernel for every number of queries. Up to 32 rows it loses everywhere to the few-row
+  // form (32 heads x 1 x 8192 x 128: 148 against 26 us, 32 x 32 x 8192 x 128 38 / 28 us, 100 x 32 x 4096 61 / 40 us,
+  // 128 x 16 x 256 9.9 / 8.3 us). Up to 64 rows it loses where few heads meet a middling number of keys (8 x 48 x 700 x 64
+  // 13.5 / 6.8 us, 16 x 40 x 2048 x 64 13.3 / 9.9 us, 32 x 64 x 512 x 128 11.6 / 11.9 us) but wins on long walks, where
+  // each of the few-row form's warps reads all keys from shared memory (32 x 64 x 8192 38.8 / 41.4 us, 70 x 64 x 16384
+  // 138 / 167 us), and on short ones of many heads (128 x 64 x 512 15.4 / 18.9 us). At 65 rows the warps would have to
+  // walk the keys twice.
+  if (form == 0 && (sq <= 32 || (sq <= 64 && heads <= 64 && sk >= 512 && sk < 4096))) {
     if (sq <= 16) return launch_decode_shape<1>(device, 20, st, pb);
     if (sq <= 32) return launch_decode_shape<2>(device, 24, st, pb);
     return launch_decode_shape<4>(device, 28, st, pb);

@@ -13,8 +13,8 @@
 // Each warp keeps its own running maximum, sum and O rows; they meet at the end: key groups of the CTA through
 // shared memory, then the CTAs of the cluster, each CTA summing one share of the output elements.
 // Measured (B200, bf16, back to back from a graph), this form against the 256-row kernel: 32 heads x 1 x 8192 x 128
-// 26 us = 5.2 TB/s (148 us), 128 x 1 x 8192 x 128 81 us = 6.6 TB/s, 8 x 1 x 16384 x 128 18.5 us, 32 x 64 x 8192 x 128
-// 41 us (148 us). A launch costs about 4 us however short its walk.
+// 26 us = 5.2 TB/s (148 us), 128 x 1 x 8192 x 128 81 us = 6.6 TB/s, 8 x 1 x 16384 x 128 18.5 us, 32 x 32 x 8192 x 128
+// 28 us. A launch costs about 4 us however short its walk.
 // Waits are bounded as everywhere; the launch is ordered behind the kernel before it by griddep_wait.
 #pragma once
 
