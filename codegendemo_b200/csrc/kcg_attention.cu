@@ -10,8 +10,8 @@
 //   warp 1    tcgen05.mma issuer and TMEM owner; per tile t: S_t = Q_t K_j^T (both K-major) into the tile's S
 //             buffer, O_t += P_t V_j with P_t read from tensor memory and V as the MN-major operand
 //   warps 4-7 softmax of tile 0, warps 8-11 of tile 1, one query row per thread: read S_t from TMEM, exponentials in
-//             the exp2 domain against a maximum that follows the running one in steps of at least 8, P_t as packed
-//             16-bit pairs over the S columns just read; at the end O / sum to global memory
+//             the exp2 domain against the running maximum, P_t as packed 16-bit pairs over the S columns just read, O_t
+//             rescaled where that maximum has moved; at the end O / sum to global memory
 // A tile's chain is serial (scores, softmax, P V, next scores) and the two tiles' chains take turns, so the tensor
 // pipe works for one tile while the other is in its softmax. What bounds it is that chain: per step and tile 512 + 512
 // cycles of products (the scores' operands fill the shared-memory port, 128 bytes a cycle) and 1024 of exponentials,
@@ -763,9 +763,10 @@ struct AttnFwd2 {
       const int row = q * 32 + lane;    // query row of this thread inside its tile
       const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
       const uint32_t col_s = tmem_base + lane_addr + t * BC, col_o = tmem_base + lane_addr + COL_O + t * kD;
-      // m: the maximum the exponentials are taken against, in the exp2 domain. It follows the running maximum only
-      // when that has moved by more than 8 for some row of the warp: until then the exponentials are at most 2^8,
-      // which neither the 16-bit P nor the 32-bit sums notice, and O need not be rescaled.
+      // m: the row's running maximum, which the exponentials of a step are taken against, in the exp2 domain. It has to
+      // be the maximum itself: the largest probability is then exactly 1 and does not lose a bit to the 16-bit P. A
+      // reference that lagged behind by up to 8 spared most rescaling (32 heads x 4096 x 4096 x 128: 230 against 238 us)
+      // but cost 1 to 4 % of the error against 64 bits on normal scores and 15 to 25 % where few keys dominate.
       float m = -INFINITY;
       uint64_t sum2[2] = {f32x2(0.f, 0.f), f32x2(0.f, 0.f)};
       bool ok = true;
@@ -798,9 +799,17 @@ struct AttnFwd2 {
           for (int i = 0; i < 32; i += 2)
             mx4[(i >> 1) & 3] = max3(mx4[(i >> 1) & 3], __uint_as_float(sr[c][i]), __uint_as_float(sr[c][i + 1]));
         };
+#pragma unroll
+        for (int c = 0; c < 4; ++c) max_of(c);
+        // (the scale is positive: checked by the host)
+        const float mx = fmaxf(m, fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2);
+        const float alpha = ex2(m - mx);
+        m = mx;
+        const uint64_t alpha2 = f32x2(alpha, alpha), zero2 = f32x2(0.f, 0.f), base2 = f32x2(-m, -m);
+        sum2[0] = fma_f32x2(sum2[0], alpha2, zero2);
+        sum2[1] = fma_f32x2(sum2[1], alpha2, zero2);
         // Exponentials and P of 32 keys: packed pairs over the S columns this thread has read.
         auto exponentials = [&](int c) {
-          const uint64_t base2 = f32x2(-m, -m);
           uint32_t w[16];
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
@@ -813,46 +822,39 @@ struct AttnFwd2 {
           }
           tmem_st_32x32b_x16(col_s + c * 16, w);
         };
-        auto row_max = [&]() {  // (the scale is positive: checked by the host)
-          return fmaxf(m, fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2);
-        };
-        if (j == 0) {
+        // O_t <- alpha * O_t, where a row of the warp has a new maximum. The previous P_t V has retired: the scores just
+        // read were issued behind it. The reads of O travel while the exponentials of the next piece are taken
+        // (rescaling the second half of O behind them all: 243 us, a warpgroup of its own that rescales: 258 us).
+        if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
+          auto scale_store = [&](uint32_t (&o)[32], int c) {
+            pin_32(o);
 #pragma unroll
-          for (int c = 0; c < 4; ++c) max_of(c);
-          m = row_max();
-        }
-        // The first half is exponentiated against the maximum so far while the maximum of this step is being taken
-        // (comparisons fit between the exponentials, which occupy their pipe for eight cycles each); in the rare step
-        // whose maximum has moved too far that half is done again.
-        const uint64_t sum_before[2] = {sum2[0], sum2[1]};
-        max_of(0);
-        max_of(1);
-        exponentials(0);
-        max_of(2);
-        max_of(3);
-        exponentials(1);
-        const float mx = row_max();
-        if (__any_sync(0xffffffffu, mx > m + 8.f)) {
-          const float alpha = ex2(m - mx);
-          m = mx;
-          const uint64_t alpha2 = f32x2(alpha, alpha), zero2 = f32x2(0.f, 0.f);
-          sum2[0] = fma_f32x2(sum_before[0], alpha2, zero2);
-          sum2[1] = fma_f32x2(sum_before[1], alpha2, zero2);
-          if (j > 0) {
-            // O_t <- alpha * O_t. The previous P_t V has retired: the scores just read were issued behind it.
-#pragma unroll 1
-            for (int c = 0; c < kD / 32; ++c) {
-              uint32_t orr[32];
-              tmem_ld_32x32b_x32(col_o + c * 32, orr);
-              tmem_ld_wait();
-              pin_32(orr);
+            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+            tmem_st_32x32b_x32(col_o + c * 32, o);
+          };
 #pragma unroll
-              for (int i = 0; i < 32; ++i) orr[i] = __float_as_uint(__uint_as_float(orr[i]) * alpha);
-              tmem_st_32x32b_x32(col_o + c * 32, orr);
-            }
+          for (int c = 0; c < 2; ++c) {
+            uint32_t o[32];
+            tmem_ld_32x32b_x32(col_o + c * 32, o);
+            exponentials(c);
+            tmem_ld_wait();
+            scale_store(o, c);
           }
+          if constexpr (kD == 128) {
+            uint32_t o[2][32];
+            tmem_ld_32x32b_x32(col_o + 64, o[0]);
+            tmem_ld_32x32b_x32(col_o + 96, o[1]);
+            exponentials(2);
+            tmem_ld_wait();
+            scale_store(o[0], 2);
+            scale_store(o[1], 3);
+          } else {
+            exponentials(2);
+          }
+        } else {
           exponentials(0);
           exponentials(1);
+          exponentials(2);
         }
         auto publish = [&](uint64_t* bar) {
           tmem_st_wait();
@@ -860,11 +862,10 @@ struct AttnFwd2 {
           __syncwarp();
           if (lane == 0) mbar_arrive(bar);
         };
-        // P V starts on the first 96 keys while the others are still being exponentiated (32 heads x 4096 x 4096 x 128:
-        // 246 us; after 64 keys 259 us, the product then waits for the rest with the pipe in its hands; after all 128
-        // 266 us)
+        // P V starts on the first 96 keys while the others are still being exponentiated (measured on 32 heads x 4096 x
+        // 4096 x 128 with every key in one launch: 246 us; after 64 keys 259 us, the product then waits for the rest with
+        // the pipe in its hands; after all 128 266 us)
         static_assert(P_PART == 96, "three pieces of 32 keys");
-        exponentials(2);
         publish(&bars->p_part[t]);
         exponentials(3);
         publish(&bars->p_full[t]);

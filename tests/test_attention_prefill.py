@@ -30,7 +30,7 @@ def test_rows_match_the_composition_in_64_bits(shape, dtype):
 @pytest.mark.parametrize("step", [0.02, 0.5, 7.9, 8.1, 40.0])
 def test_maximum_that_climbs_with_every_step(step):
     """Scores that grow by `step` (in the exp2 domain) from one 128-key step to the next, in some rows only: the
-    maximum the exponentials refer to is left behind by up to 8 or moved, and O and the sums follow."""
+    maximum moves by a little or a lot, and O and the sums follow."""
     from codegendemo_b200.kcg.matmul_op import attention_fused, attention_status
     heads, sq, sk, d = 2, 256, 1280, 64
     gen = torch.Generator().manual_seed(4)
@@ -43,6 +43,31 @@ def test_maximum_that_climbs_with_every_step(step):
     out = attention_fused(q.cuda(), k.cuda(), v.cuda(), scale=1.0)
     attention_status(0)
     assert (out.cpu().double() - _reference(q, k, v, 1.0)).abs().max().item() <= 2.1 * 2.0 ** -12 * v.abs().max().item()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("sk", [512, 4096], ids=["whole", "key_split"])
+def test_the_largest_probability_is_not_rounded(sk, dtype):
+    """Two keys carry all the weight, and the larger one comes later by 0.3 to 7.8 in the exp2 domain: taken against the
+    running maximum its probability is 1 in 16 bits as well, so only the smaller one and the result are rounded."""
+    from codegendemo_b200.kcg.matmul_op import attention_fused
+    heads, sq, d = 16, 128, 128
+    gen = torch.Generator().manual_seed(6)
+    v = torch.randn((heads, sk, d), generator=gen).to(dtype)
+    q, k = torch.zeros((heads, sq, d), dtype=dtype), torch.zeros((heads, sk, d), dtype=dtype)
+    q[:, :, 0] = 1.0
+    k[:, :, 0] = -200.0
+    k[:, 5, 0] = 0.0
+    k[:, 300, 0] = (0.3 + 0.5 * torch.arange(heads)) * 0.6931471805599453
+    out = attention_fused(q.cuda(), k.cuda(), v.cuda(), scale=1.0).cpu().double()
+    p = torch.softmax(q.double() @ k.double().transpose(1, 2), dim=-1)
+    ref = p @ v.double()
+    half_unit = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    # half a unit of the result and of the smaller probability; the 32-bit part (exponentials, sums, the joining of
+    # the CTAs' parts) within 2^-18 of the largest value
+    bound = half_unit * (ref.abs() + p[:, :, 5:6] * v[:, 5:6].double().abs()) + 2.0 ** -18 * v.abs().max().item()
+    assert ((out - ref).abs() <= bound).all()
 
 
 @pytest.mark.gpu
