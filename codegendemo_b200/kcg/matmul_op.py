@@ -275,7 +275,7 @@ def build_kernel(kpm: KernelArgMatmul, deviceId: int = 0):
     return inConfig, CompiledKernelFactory.getKernel(inConfig, deviceId)
 
 
-_KERNELS = {}
+_KERNELS = {}  # (operator, shape, dtype, device, options) -> kernel; True == 1, so operators must not share keys
 
 
 def _row_pitch(t, what: str) -> int:
@@ -308,7 +308,7 @@ def matmul(a, b, c=None, alpha=1.0, beta=0.0, bias=None, relu=False, b_transpose
         c = a.new_empty((M, N))
     ldc = _row_pitch(c, "c")
     dev = a.device.index or 0
-    key = (M, N, K, a.dtype, dev, tuple(sorted(keys.items())) if keys else (), bool(b_transposed))
+    key = ("mm", M, N, K, a.dtype, dev, tuple(sorted(keys.items())) if keys else (), bool(b_transposed))
     kern = _KERNELS.get(key)
     if kern is None:
         dt = FromTorchType(a.dtype)
@@ -437,7 +437,7 @@ def bmm(a, b, c=None, alpha=1.0, beta=0.0, bias=None, relu=False, **keys):
             raise ValueError("beta != 0 needs the c to scale")
         c = a.new_empty((batch, M, N))
     dev = a.device.index or 0
-    key = (M, N, K, a.dtype, dev, tuple(sorted(keys.items())) if keys else (), 0 if keys else batch)
+    key = ("bmm", M, N, K, a.dtype, dev, tuple(sorted(keys.items())) if keys else (), 0 if keys else batch)
     kern = _KERNELS.get(key)
     if kern is None:
         dt = FromTorchType(a.dtype)
