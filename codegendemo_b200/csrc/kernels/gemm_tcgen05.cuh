@@ -927,7 +927,9 @@ struct TcGemm {
                         float o[4] = {sum[u].x, sum[u].y, sum[u].z, sum[u].w};
                         if (p.epi_flags != 0u) {
                           const int idx = r0 * F4_PER_ROW + i;
-                          epi_span<OutT, 4>(p, o, w.m0 + row_base + idx / F4_PER_ROW, w.n0 + (idx % F4_PER_ROW) * 4);
+                          const int row = w.m0 + row_base + idx / F4_PER_ROW;
+                          // (a tile may hang over M: beta reads C, which ends there)
+                          if (row < p.M) epi_span<OutT, 4>(p, o, row, w.n0 + (idx % F4_PER_ROW) * 4);
                         }
                         if constexpr (sizeof(OutT) == 4) {
                           asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(out + static_cast<uint32_t>(i) * 16u),

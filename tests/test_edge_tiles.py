@@ -130,6 +130,30 @@ def test_edge_tiles_match_the_oracle_and_stay_inside_c(tile, split):
 
 
 @pytest.mark.gpu
+# every tile cut into K ranges that are summed out of the operand ring, rows past M among them; N inside the tiles (bulk
+# copies of the sums) and past them (plain stores)
+@pytest.mark.parametrize("shape", [(384, 512, 8192), (640, 320, 4096)], ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("tile,split", [((4, 256, 256, 64), 8), ((4, 512, 256, 64), 4), ((2, 256, 192, 64), 4),
+                                        ((4, 256, 128, 128), 3)], ids=lambda v: str(v).replace(", ", "x"))
+def test_split_edge_tiles_scale_and_add_c(shape, tile, split):
+    """c = alpha a b + beta c with C a corner of a larger matrix: C is read inside its rows only, nothing else changes."""
+    M, N, K = shape
+    A, B = oracle.make_inputs(M, N, K, torch.bfloat16, "normal", seed=22)
+    kpm = _cfg(tile, split, M, N, K)
+    _, kern = build_kernel(kpm, 0)
+    big = torch.randn((M + 512, N + 256), generator=torch.Generator().manual_seed(3)).to(torch.bfloat16)
+    want = 0.5 * (A.double() @ B.double()) - 2.0 * big[:M, :N].double()
+    dev = big.cuda()
+    kern.run(A.cuda(), B.cuda(), dev[:M, :N], ldc=N + 256, alpha=0.5, beta=-2.0)
+    kern.checkStatus()
+    out = dev.cpu()
+    # one rounding to bf16 (half a unit of the result), 32-bit sums of terms whose sizes add up to |A| |B|
+    bound = 2.0 ** -8 * want.abs() + 2.0 ** -18 * (A.double().abs() @ B.double().abs())
+    assert ((out[:M, :N].double() - want).abs() <= bound).all()
+    assert torch.equal(out[M:], big[M:]) and torch.equal(out[:, N:], big[:, N:])
+
+
+@pytest.mark.gpu
 def test_edge_tiles_hold_over_many_waves_and_repeat_bitwise():
     """Several waves of tiles that hang over both edges, every element checked against a device fp32 product: the
     staging buffers of skipped blocks must not be counted as stored (a fifth of the tiles came out wrong)."""
