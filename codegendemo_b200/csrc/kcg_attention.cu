@@ -803,9 +803,11 @@ struct AttnFwd2 {
         for (int c = 0; c < 4; ++c) max_of(c);
         // (the scale is positive: checked by the host)
         const float mx = fmaxf(m, fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2);
-        const float alpha = ex2(m - mx);
+        // (without a finite score so far the probabilities are 0, not -inf - -inf: a CTA may see excluded keys only)
+        const float base = mx == -INFINITY ? 0.f : mx;
+        const float alpha = ex2(m - base);
         m = mx;
-        const uint64_t alpha2 = f32x2(alpha, alpha), zero2 = f32x2(0.f, 0.f), base2 = f32x2(-m, -m);
+        const uint64_t alpha2 = f32x2(alpha, alpha), zero2 = f32x2(0.f, 0.f), base2 = f32x2(-base, -base);
         sum2[0] = fma_f32x2(sum2[0], alpha2, zero2);
         sum2[1] = fma_f32x2(sum2[1], alpha2, zero2);
         // Exponentials and P of 32 keys: packed pairs over the S columns this thread has read.

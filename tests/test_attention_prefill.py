@@ -71,6 +71,26 @@ def test_the_largest_probability_is_not_rounded(sk, dtype):
 
 
 @pytest.mark.gpu
+# one CTA per 256 rows, and 2 to 8 that share its keys; the few-row form; excluded: whole first or last ranges of a CTA
+@pytest.mark.parametrize("shape", [(2, 128, 512), (2, 300, 4096), (2, 1, 4096), (2, 20, 4096), (2, 40, 2048)],
+                         ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("first", [True, False])
+def test_keys_of_minus_infinity_weigh_nothing(shape, first):
+    from codegendemo_b200.kcg.matmul_op import attention_fused
+    heads, sq, sk = shape
+    gen = torch.Generator().manual_seed(8)
+    q, k, v = [torch.randn((heads, n, 64), generator=gen) for n in (sq, sk, sk)]
+    q[:, :, 0] = 1.0
+    k[:, :sk // 2 + 60, 0] = -float("inf")
+    if not first:
+        k = k.flip(1)
+    q, k, v = q.half(), k.half(), v.half()
+    out = attention_fused(q.cuda(), k.cuda(), v.cuda()).cpu().double()
+    # probabilities and the result are each rounded once to 16 bits (half a unit of the largest value, twice)
+    assert (out - _reference(q, k, v, 64 ** -0.5)).abs().max().item() <= 2.1 * 2.0 ** -12 * v.abs().max().item()
+
+
+@pytest.mark.gpu
 def test_nan_and_infinite_scores_stay_in_their_rows():
     from codegendemo_b200.kcg.matmul_op import attention_fused
     gen = torch.Generator().manual_seed(5)
