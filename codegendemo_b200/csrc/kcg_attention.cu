@@ -1185,6 +1185,25 @@ int decode_splits(int heads, int sk) {
   return s < 1 ? 1 : s;
 }
 
+// Whether the few-row form takes a call. Up to 32 rows always: the 256-row kernel loses everywhere (32 heads x 1 x 8192 x
+// 128: 148 against 26 us, 32 x 32 x 8192 x 128 38 / 28 us, 100 x 32 x 4096 61 / 40 us, 128 x 16 x 256 9.9 / 8.3 us). At 33
+// to 64 rows each of its four warps reads all keys from shared memory, which costs most at d = 128. Measured on 8 to 128
+// heads x 40 and 64 rows x 256 to 8192 keys, bf16, few-row time over that of the 256-row kernel:
+//   d = 64   0.47 to 0.95 from 512 keys on, whatever the heads (32 x 64 x 4096 16 / 22 us, 128 x 64 x 8192 69 / 103 us);
+//            at 256 keys 0.80 to 1.11 (7 us either way)
+//   d = 128  up to 32 heads 0.66 to 1.04 from 512 to 1536 keys (8 x 64 x 1024 11 / 16 us), then 0.97 to 1.14 (with 8 heads
+//            only from 3072 keys on); where at least three CTAs share a head (up to 88 heads) 0.77 to 1.02 from 1536 keys on
+//            (48 x 64 x 4096 36 / 40 us, 80 x 64 x 4096 51 / 61 us) and 0.93 to 1.49 below; with 100 and 128 heads 1.00 to
+//            1.45.
+// At 65 rows the warps would have to walk the keys twice.
+bool few_rows_form(int heads, int sq, int sk, int d) {
+  if (sq <= 32) return true;
+  if (sq > 64 || sk < 512) return false;
+  if (d == 64) return true;
+  if (heads <= 32) return sk < (heads <= 8 ? 3072 : 2048);
+  return heads <= 88 && sk >= 1536;
+}
+
 template <int kD, bool kBf16, int kRowGroups>
 int launch_decode(int device, int slot, cudaStream_t st, const Problem& pb) {
   using Kern = AttnDecode<kD, kBf16, kRowGroups>;
@@ -1247,6 +1266,11 @@ int launch_shape(int device, int base_slot, cudaStream_t st, const Problem& pb) 
 
 }  // namespace
 
+// For tests of the host logic: 1 where kcg_attention_fwd takes the few-row form for a call, else 0.
+extern "C" int kcg_internal_attention_few_rows(int heads, int sq, int sk, int d) {
+  return few_rows_form(heads, sq, sk, d) ? 1 : 0;
+}
+
 extern "C" int kcg_attention_fwd(int device, uint64_t stream, uint64_t Q, uint64_t K, uint64_t V, uint64_t O, int dtype,
                                  int heads, int sq, int sk, int d, float scale) {
   if (!Q || !K || !V || !O) return fail(KCG_E_BAD_ARG, "null device pointer");
@@ -1283,14 +1307,8 @@ extern "C" int kcg_attention_fwd(int device, uint64_t stream, uint64_t Q, uint64
     const char* v = getenv("KCG_ATTN_FORM");
     return v ? atoi(v) & 15 : 0;
   }();
-  // KCG_ATTN_FORM=8: the 256-row kernel for every number of queries. Up to 32 rows it loses everywhere to the few-row
-  // form (32 heads x 1 x 8192 x 128: 148 against 26 us, 32 x 32 x 8192 x 128 38 / 28 us, 100 x 32 x 4096 61 / 40 us,
-  // 128 x 16 x 256 9.9 / 8.3 us). Up to 64 rows it loses where few heads meet a middling number of keys (8 x 48 x 700 x 64
-  // 13.5 / 6.8 us, 16 x 40 x 2048 x 64 13.3 / 9.9 us, 32 x 64 x 512 x 128 11.6 / 11.9 us) but wins on long walks, where
-  // each of the few-row form's warps reads all keys from shared memory (32 x 64 x 8192 38.8 / 41.4 us, 70 x 64 x 16384
-  // 138 / 167 us), and on short ones of many heads (128 x 64 x 512 15.4 / 18.9 us). At 65 rows the warps would have to
-  // walk the keys twice.
-  if (form == 0 && (sq <= 32 || (sq <= 64 && heads <= 64 && sk >= 512 && sk < 4096))) {
+  // KCG_ATTN_FORM=8: the 256-row kernel for every number of queries.
+  if (form == 0 && few_rows_form(heads, sq, sk, d)) {
     if (sq <= 16) return launch_decode_shape<1>(device, 20, st, pb);
     if (sq <= 32) return launch_decode_shape<2>(device, 24, st, pb);
     return launch_decode_shape<4>(device, 28, st, pb);

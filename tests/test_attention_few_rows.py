@@ -1,13 +1,28 @@
-"""The fused attention entry at up to 64 query rows: a head's keys are shared by the CTAs of a cluster."""
+"""The fused attention entry at few query rows, where a head's keys are shared by the CTAs of a cluster."""
+import ctypes
+
 import pytest
 import torch
 
-# (heads, sq, sk, d): one row and one key; the last row group full, one short, one past it (16, 32, 64 rows per
-# kernel form; 65 = the 256-row kernel); a last stage of one key; fewer stages than warps or CTAs; a cluster of 16, an
-# odd one, one CTA per head; a warp whose keys are all past the end
-SHAPES = [(1, 1, 1, 128), (3, 1, 63, 64), (2, 16, 64, 128), (2, 17, 65, 128), (5, 15, 129, 64), (2, 32, 1000, 128),
-          (2, 33, 4097, 64), (4, 64, 2049, 128), (4, 65, 2049, 128), (8, 5, 16384, 128), (8, 3, 8209, 64),
-          (40, 2, 3001, 128), (100, 7, 300, 64), (300, 1, 513, 128)]
+from codegendemo_b200 import _lib
+
+# (heads, sq, sk, d) of the few-row form: one row and one key; the last row group full, one short, one past it (16, 32,
+# 64 rows per kernel form); a last stage of one key; fewer stages than warps or CTAs; a cluster of 16, an odd one, one CTA
+# per head; a warp whose keys are all past the end; 33 to 64 rows at every line of the rule that admits them
+FEW = [(1, 1, 1, 128), (3, 1, 63, 64), (2, 16, 64, 128), (2, 17, 65, 128), (5, 15, 129, 64), (2, 32, 1000, 128),
+       (8, 5, 16384, 128), (8, 3, 8209, 64), (40, 2, 3001, 128), (100, 7, 300, 64), (300, 1, 513, 128),
+       (2, 33, 4097, 64), (64, 63, 700, 64), (130, 50, 512, 64), (4, 64, 2049, 128), (5, 47, 513, 128), (8, 63, 3071, 128),
+       (9, 34, 2047, 128), (33, 64, 1537, 128), (88, 49, 1536, 128)]
+# their neighbours on the other side of each line, which the 256-row kernel takes
+MANY = [(4, 65, 2049, 128), (2, 33, 511, 64), (5, 47, 511, 128), (8, 63, 3072, 128), (9, 34, 2048, 128),
+        (33, 64, 1535, 128), (89, 49, 1536, 128)]
+SHAPES = FEW + MANY
+
+
+def test_the_shapes_lie_on_their_side_of_the_rule():
+    few = _lib.get_lib().kcg_internal_attention_few_rows
+    few.argtypes = [ctypes.c_int] * 4
+    assert [few(*s) for s in SHAPES] == [1] * len(FEW) + [0] * len(MANY)
 
 
 def _inputs(heads, sq, sk, d, dtype, seed=7):
