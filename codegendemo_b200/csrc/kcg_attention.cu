@@ -1084,6 +1084,9 @@ int launch(int device, int slot, cudaStream_t st, const Problem& pb) {
   return 0;
 }
 
+// Clusters of 1 .. 16 CTAs of the few-row kernels that run at once (asked once per device, kernel and size; -1 = none).
+int g_few_clusters[16][12][17];
+
 // How many clusters of 2 .. 8 CTAs of the key-split kernel run at once (asked once per device and kernel).
 int g_clusters[16][4][9];
 
@@ -1143,7 +1146,7 @@ int launch2(int device, int kind, cudaStream_t st, const Problem& pb) {
   p.scale_log2 = pb.scale * 1.4426950408889634f;
   // A group of 256 rows keeps one SM for the whole walk over the keys, so 148 groups are a wave. What does not fill a
   // wave - the remainder of a large problem, all of a small one - shares its keys among the SMs that would stand idle:
-  // (bf16) 32 heads x 4096 x 4096 x 128, 3.46 waves: 246 -> 230 us; 8 x 300 x 16384 x 128, 16 groups: 224 -> 55 us; 8 x 65
+  // (bf16) 32 heads x 4096 x 4096 x 128, 3.46 waves, then 246 -> 230 us; 8 x 300 x 16384 x 128, 16 groups: 224 -> 59 us; 8 x 65
   // x 16384 x 64, 8 groups: 33 us.
   // The remainder is a launch of its own right behind the whole groups, allowed to start as soon as all of those have.
   const long long groups = static_cast<long long>(pb.heads) * ((pb.sq + 255) / 256);
@@ -1176,12 +1179,15 @@ int launch2(int device, int kind, cudaStream_t st, const Problem& pb) {
 // 26 us, 9 35 us; 100 heads x 4096: 2 per head 37 us, 3 46 us), pairs alone pack all 296 places. More than 8 per head
 // pay only where fewer heads leave SMs idle (8 heads x 16384: 8 per head 21.2 us, 12 19.5, 16 18.6; 20 heads x 8192:
 // 8 23.9, 10 21.7, 16 33.9 us). At least two stages of 64 keys each: below that the joining costs what the walk saves.
-int decode_splits(int heads, int sk) {
+// A cluster of more CTAs than any GPC can hold (`fits`: fewer SMs than a whole GPU's) is not asked for.
+template <typename Fits>
+int decode_splits(int heads, int sk, Fits&& fits) {
   const int tiles = (sk + 63) / 64;
   int s = heads <= 148 && heads > 132 ? 2 : 264 / heads;
   if (s > 8) s = 200 / heads > 8 ? 200 / heads : 8;
   if (s > 16) s = 16;
   if (s > tiles / 2) s = tiles / 2;
+  while (s > 1 && !fits(s)) --s;
   return s < 1 ? 1 : s;
 }
 
@@ -1208,6 +1214,17 @@ template <int kD, bool kBf16, int kRowGroups>
 int launch_decode(int device, int slot, cudaStream_t st, const Problem& pb) {
   using Kern = AttnDecode<kD, kBf16, kRowGroups>;
   const auto kernel = kcg_attention_decode_kernel<kD, kBf16, kRowGroups>;
+  cudaLaunchConfig_t cfg{};
+  cfg.blockDim = dim3(Kern::NUM_THREADS);
+  cfg.dynamicSmemBytes = Kern::SMEM_BYTES;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  AttnDecodeParams p{};
   {
     std::lock_guard<std::mutex> lock(g_mutex);
     if (!g_ready[device][slot]) {
@@ -1217,28 +1234,27 @@ int launch_decode(int device, int slot, cudaStream_t st, const Problem& pb) {
       if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(NonPortableClusterSizeAllowed)");
       g_ready[device][slot] = true;
     }
+    p.splits = decode_splits(pb.heads, pb.sk, [&](int s) {
+      int& known = g_few_clusters[device][slot - 20][s];
+      if (known == 0) {
+        attr[0].val.clusterDim.x = s;
+        cfg.gridDim = dim3(s);
+        cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&known, kernel, &cfg) != cudaSuccess) cudaGetLastError();
+        if (known <= 0) known = -1;
+      }
+      return known > 0;
+    });
   }
-  AttnDecodeParams p{};
   if (int r = encode3(&p.tmK, kBf16, pb.K, kD, pb.sk, pb.heads, 64)) return r;
   if (int r = encode3(&p.tmV, kBf16, pb.V, kD, pb.sk, pb.heads, 64)) return r;
   p.Q = reinterpret_cast<const void*>(pb.Q);
   p.O = reinterpret_cast<void*>(pb.O);
   p.sq = pb.sq;
   p.sk = pb.sk;
-  p.splits = decode_splits(pb.heads, pb.sk);
   p.scale_log2 = pb.scale * 1.4426950408889634f;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(static_cast<unsigned>(pb.heads) * p.splits);
-  cfg.blockDim = dim3(Kern::NUM_THREADS);
-  cfg.dynamicSmemBytes = Kern::SMEM_BYTES;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = p.splits;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
+  cfg.gridDim = dim3(static_cast<unsigned>(pb.heads) * p.splits);
   cfg.numAttrs = 2;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
   if (e != cudaSuccess) return cuda_fail(e, "attention launch");
@@ -1269,6 +1285,11 @@ int launch_shape(int device, int base_slot, cudaStream_t st, const Problem& pb) 
 // For tests of the host logic: 1 where kcg_attention_fwd takes the few-row form for a call, else 0.
 extern "C" int kcg_internal_attention_few_rows(int heads, int sq, int sk, int d) {
   return few_rows_form(heads, sq, sk, d) ? 1 : 0;
+}
+
+// For tests of the host logic: the CTAs per head of the few-row form where bit s of `fitting` says that a cluster of s fits.
+extern "C" int kcg_internal_attention_splits(int heads, int sk, unsigned int fitting) {
+  return decode_splits(heads, sk, [&](int s) { return (fitting >> s & 1u) != 0u; });
 }
 
 extern "C" int kcg_attention_fwd(int device, uint64_t stream, uint64_t Q, uint64_t K, uint64_t V, uint64_t O, int dtype,

@@ -25,6 +25,15 @@ def test_the_shapes_lie_on_their_side_of_the_rule():
     assert [few(*s) for s in SHAPES] == [1] * len(FEW) + [0] * len(MANY)
 
 
+def test_no_larger_cluster_than_fits():
+    """On a whole GPU up to 16 CTAs share a head's keys; where larger clusters do not fit, the largest that does."""
+    splits = _lib.get_lib().kcg_internal_attention_splits
+    splits.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_uint]
+    assert [splits(h, 16384, 0x1ffff) for h in (1, 8, 12, 20, 32, 100, 140, 300)] == [16, 16, 16, 10, 8, 2, 2, 1]
+    assert [splits(h, 16384, 0x1ff) for h in (1, 8, 12, 20, 32, 100, 140, 300)] == [8, 8, 8, 8, 8, 2, 2, 1]
+    assert [splits(8, 16384, mask) for mask in (0b1011111, 0b111, 0b1, 0)] == [6, 2, 1, 1]
+
+
 def _inputs(heads, sq, sk, d, dtype, seed=7):
     gen = torch.Generator().manual_seed(seed)
     return [torch.randn((heads, n, d), generator=gen).to(dtype) for n in (sq, sk, sk)]
