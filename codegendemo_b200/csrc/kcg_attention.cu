@@ -1018,6 +1018,15 @@ int cuda_fail(cudaError_t e, const char* what) {
   return fail(static_cast<int>(e), std::string(what) + ": " + cudaGetErrorString(e));
 }
 
+// KCG_PDL=0 turns programmatic dependent launch off (read once, at the first launch of the process).
+bool pdl_on() {
+  static const bool on = [] {
+    const char* e = getenv("KCG_PDL");
+    return !(e && e[0] == '0');
+  }();
+  return on;
+}
+
 struct DeviceGuard {
   int prev = -1;
   bool switched = false;
@@ -1166,7 +1175,7 @@ int launch2(int device, int kind, cudaStream_t st, const Problem& pb) {
     p.tail_follows = 0;
     attr[0].val.clusterDim.x = s;
     cfg.gridDim = dim3(static_cast<unsigned>(rest * s));
-    cfg.numAttrs = full > 0 ? 2 : 1;
+    cfg.numAttrs = full > 0 && pdl_on() ? 2 : 1;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, split, p);
     if (e != cudaSuccess) return cuda_fail(e, "attention launch");
     kcg_internal_count_launch();
@@ -1255,7 +1264,7 @@ int launch_decode(int device, int slot, cudaStream_t st, const Problem& pb) {
   p.scale_log2 = pb.scale * 1.4426950408889634f;
   attr[0].val.clusterDim.x = p.splits;
   cfg.gridDim = dim3(static_cast<unsigned>(pb.heads) * p.splits);
-  cfg.numAttrs = 2;
+  cfg.numAttrs = pdl_on() ? 2 : 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
   if (e != cudaSuccess) return cuda_fail(e, "attention launch");
   kcg_internal_count_launch();

@@ -1,5 +1,8 @@
 """The fused attention entry at few query rows, where a head's keys are shared by the CTAs of a cluster."""
 import ctypes
+import os
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -32,6 +35,35 @@ def test_no_larger_cluster_than_fits():
     assert [splits(h, 16384, 0x1ffff) for h in (1, 8, 12, 20, 32, 100, 140, 300)] == [16, 16, 16, 10, 8, 2, 2, 1]
     assert [splits(h, 16384, 0x1ff) for h in (1, 8, 12, 20, 32, 100, 140, 300)] == [8, 8, 8, 8, 8, 2, 2, 1]
     assert [splits(8, 16384, mask) for mask in (0b1011111, 0b111, 0b1, 0)] == [6, 2, 1, 1]
+
+
+_EDGES = """
+import ctypes, torch
+from codegendemo_b200.kcg.matmul_op import attention_fused
+q, k, v = [torch.zeros((h, n, 64), dtype=torch.float16, device="cuda") for h, n in ((150, 256), (150, 1024), (150, 1024))]
+few = q[:, :1].contiguous()
+for x in (few, q):
+    attention_fused(x, k, v)
+graph = torch.cuda.CUDAGraph(keep_graph=True)
+with torch.cuda.graph(graph):
+    for x in (few, few, q):  # (the last: whole groups, and a remainder of two that share their keys, behind them)
+        attention_fused(x, k, v)
+edges = ctypes.CDLL("libcuda.so.1").cuGraphGetEdges_v2
+n = ctypes.c_size_t(8)
+ends, data = [(ctypes.c_void_p * 8)() for _ in range(2)], (ctypes.c_ubyte * 64)()  # 8 bytes an edge, its type the third
+assert edges(ctypes.c_void_p(graph.raw_cuda_graph()), *ends, data, ctypes.byref(n)) == 0 and n.value == 3, n
+print(sum(data[8 * i + 2] == 1 for i in range(3)))  # CU_GRAPH_DEPENDENCY_TYPE_PROGRAMMATIC
+"""
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("pdl,programmatic", [("1", 2), ("0", 0)])
+def test_programmatic_launch_can_be_turned_off(pdl, programmatic):
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _EDGES], cwd=root, env=dict(os.environ, KCG_PDL=pdl), text=True,
+                       capture_output=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    assert int(r.stdout.split()[-1]) == programmatic
 
 
 def _inputs(heads, sq, sk, d, dtype, seed=7):
