@@ -1096,8 +1096,9 @@ int launch(int device, int slot, cudaStream_t st, const Problem& pb) {
 // Clusters of 1 .. 16 CTAs of the few-row kernels that run at once (asked once per device, kernel and size; -1 = none).
 int g_few_clusters[16][12][17];
 
-// How many clusters of 2 .. 8 CTAs of the key-split kernel run at once (asked once per device and kernel).
+// How many clusters of 2 .. 8 CTAs of the key-split kernel run at once (asked once per device and kernel), and SMs.
 int g_clusters[16][4][9];
+int g_sms[16];
 
 // The largest number of CTAs, 2 to 8, that `groups` groups of 256 rows can share their keys among with every cluster
 // running at once and at least four steps of 128 keys per CTA (joining costs what two steps do); 1 = none.
@@ -1142,6 +1143,8 @@ int launch2(int device, int kind, cudaStream_t st, const Problem& pb) {
         }
         g_clusters[device][kind][s] = n;
       }
+      e = cudaDeviceGetAttribute(&g_sms[device], cudaDevAttrMultiProcessorCount, device);
+      if (e != cudaSuccess) return cuda_fail(e, "cudaDeviceGetAttribute(MultiProcessorCount)");
       g_ready[device][16 + kind] = true;
     }
   }
@@ -1153,13 +1156,13 @@ int launch2(int device, int kind, cudaStream_t st, const Problem& pb) {
   p.sq = pb.sq;
   p.sk = pb.sk;
   p.scale_log2 = pb.scale * 1.4426950408889634f;
-  // A group of 256 rows keeps one SM for the whole walk over the keys, so 148 groups are a wave. What does not fill a
+  // A group of 256 rows keeps one SM for the whole walk over the keys, so a wave is one group per SM. What does not fill a
   // wave - the remainder of a large problem, all of a small one - shares its keys among the SMs that would stand idle:
   // (bf16) 32 heads x 4096 x 4096 x 128, 3.46 waves, then 246 -> 230 us; 8 x 300 x 16384 x 128, 16 groups: 224 -> 59 us; 8 x 65
   // x 16384 x 64, 8 groups: 33 us.
   // The remainder is a launch of its own right behind the whole groups, allowed to start as soon as all of those have.
   const long long groups = static_cast<long long>(pb.heads) * ((pb.sq + 255) / 256);
-  const long long rest = groups % 148;
+  const long long rest = groups % g_sms[device];
   const int s = rest ? key_splits(g_clusters[device][kind], rest, pb.sk) : 1;
   const long long full = s > 1 ? groups - rest : groups;
   if (full > 0) {
