@@ -61,7 +61,9 @@ int fail(int code, const char* fmt, ...) {
   X(cuLaunchKernelEx) X(cuTensorMapEncodeTiled) X(cuMemAlloc) X(cuMemFree) X(cuMemsetD32)      \
   X(cuMemcpyHtoDAsync) X(cuMemcpyDtoHAsync) X(cuMemcpyDtoH) X(cuMemcpyHtoD)                    \
   X(cuStreamSynchronize) X(cuStreamCreate) X(cuStreamDestroy) X(cuStreamWaitEvent) X(cuEventCreate)        \
-  X(cuEventRecord) X(cuEventDestroy) X(cuIpcGetMemHandle) X(cuIpcOpenMemHandle) X(cuIpcCloseMemHandle)
+  X(cuEventRecord) X(cuEventDestroy) X(cuIpcGetMemHandle) X(cuIpcOpenMemHandle) X(cuIpcCloseMemHandle) \
+  X(cuMemsetD32Async) X(cuStreamGetCaptureInfo_v3) X(cuThreadExchangeStreamCaptureMode)                  \
+  X(cuUserObjectCreate) X(cuUserObjectRelease) X(cuGraphRetainUserObject)
 
 struct Driver {
   void* handle = nullptr;
@@ -126,7 +128,8 @@ int need_driver() {
 // launches on one stream run in order and may share them, launches on different streams of one
 // GPU may overlap and must not. Slots are created on a stream's first launch and recycled
 // least-recently-used beyond kMaxStreamSlots (a freed buffer is released with cuMemFree, which
-// waits for the work that still uses it).
+// waits for the work that still uses it). Launches that are captured into a graph take their
+// workspace and counters from a GraphBuffer instead (the status block stays the stream's).
 struct StreamSlot {
   CUstream stream = nullptr;
   CUdeviceptr status = 0;      // 4 x u32
@@ -137,6 +140,20 @@ struct StreamSlot {
   uint64_t last_use = 0;
 };
 constexpr size_t kMaxStreamSlots = 32;
+
+// Workspace and tile counters of the launches that one capture queued on one stream. The graph
+// runs on any stream, beside any other graph and as often as it likes, long after the stream's own
+// buffer has moved: so the buffer belongs to the graph. It is handed over as a user object, and is
+// free for the next capture once the graph and what was instantiated from it are gone.
+struct GraphBuffer {
+  CUdeviceptr ws = 0;  // the counters follow the workspace
+  size_t ws_bytes = 0, counters_n = 0;
+  CUstream stream = nullptr;
+  unsigned long long capture = 0;
+  std::atomic<bool> held{false};
+  CUdeviceptr counters() const { return ws + ((ws_bytes + 255) / 256) * 256; }
+};
+constexpr size_t kMaxFreeGraphBuffers = 4;  // freed ones that are kept
 
 // What a 2-D tensor map depends on.
 struct MapKey {
@@ -162,6 +179,8 @@ struct DeviceState {
   CUcontext ctx = nullptr;
   std::vector<StreamSlot> slots;
   uint64_t use_clock = 0;
+  std::vector<GraphBuffer*> graph_buffers;
+  CUstream aux = nullptr;  // non-blocking: clears buffers while other streams are being captured
   CUdeviceptr hbuf[3] = {0, 0, 0};  // device copies for kcg_matmul_host
   size_t hbuf_bytes[3] = {0, 0, 0};
   CUstream hstream[3] = {nullptr, nullptr, nullptr};  // kcg_matmul_host: copy-in, compute, copy-out
@@ -194,8 +213,16 @@ int ensure_device(int device, DeviceState** out) {
   return 0;
 }
 
+// While this lives the thread may allocate and free device memory although a stream is being captured.
+struct RelaxedCapture {
+  CUstreamCaptureMode mode = CU_STREAM_CAPTURE_MODE_RELAXED;
+  RelaxedCapture() { driver().p_cuThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { driver().p_cuThreadExchangeStreamCaptureMode(&mode); }
+};
+
 int grow(CUdeviceptr* p, size_t* have, size_t need) {
   if (*have >= need) return 0;
+  RelaxedCapture relaxed;
   if (*p) DRV(cuMemFree(*p));
   *p = 0;
   *have = 0;
@@ -204,7 +231,76 @@ int grow(CUdeviceptr* p, size_t* have, size_t need) {
   return 0;
 }
 
+// Zeroes n words and waits until they are, without touching a stream that may be in a capture.
+int zero_words(DeviceState* s, CUdeviceptr p, size_t n) {
+  RelaxedCapture relaxed;
+  if (!s->aux) DRV(cuStreamCreate(&s->aux, CU_STREAM_NON_BLOCKING));
+  DRV(cuMemsetD32Async(p, 0, n, s->aux));
+  DRV(cuStreamSynchronize(s->aux));
+  return 0;
+}
+
+// Runs when the last graph that holds the buffer is gone. (No driver calls are allowed here. The structure itself is
+// never freed: a graph may outlive kcg_shutdown.)
+void CUDA_CB release_graph_buffer(void* p) { static_cast<GraphBuffer*>(p)->held.store(false); }
+
+// The buffer of capture `id` on `stream` with room for `need` bytes and `counters_n` counters; `graph` will hold it.
+// Call with g_dev_mutex held.
+int graph_buffer(DeviceState* s, CUstream stream, unsigned long long id, CUgraph graph, size_t need, size_t counters_n,
+                 GraphBuffer** out) {
+  GraphBuffer* best = nullptr;
+  size_t free_ones = 0;
+  for (GraphBuffer* b : s->graph_buffers) {
+    const bool held = b->held.load();
+    const bool fits = b->ws_bytes >= need && b->counters_n >= counters_n;
+    if (held && fits && b->stream == stream && b->capture == id) {  // an earlier launch of this capture and stream
+      *out = b;
+      return 0;
+    }
+    if (held) continue;
+    ++free_ones;
+    if (fits && (!best || b->ws_bytes < best->ws_bytes)) best = b;
+  }
+  RelaxedCapture relaxed;
+  if (!best) {
+    for (size_t i = 0; i < s->graph_buffers.size() && free_ones > kMaxFreeGraphBuffers;) {
+      GraphBuffer* b = s->graph_buffers[i];
+      if (b->held.load()) {
+        ++i;
+        continue;
+      }
+      DRV(cuMemFree(b->ws));
+      s->graph_buffers.erase(s->graph_buffers.begin() + i);
+      delete b;
+      --free_ones;
+    }
+    best = new GraphBuffer;
+    best->ws_bytes = need;
+    best->counters_n = counters_n;
+    const CUresult r = driver().p_cuMemAlloc(&best->ws, ((need + 255) / 256) * 256 + counters_n * 4);
+    if (r != CUDA_SUCCESS) {
+      delete best;
+      return drv_fail(r, "cuMemAlloc(workspace of a captured launch)");
+    }
+    s->graph_buffers.push_back(best);
+  }
+  if (int e = zero_words(s, best->counters(), best->counters_n)) return e;
+  CUuserObject obj = nullptr;
+  DRV(cuUserObjectCreate(&obj, best, release_graph_buffer, 1, CU_USER_OBJECT_NO_DESTRUCTOR_SYNC));
+  best->held.store(true);
+  best->stream = stream;
+  best->capture = id;
+  const CUresult r = driver().p_cuGraphRetainUserObject(graph, obj, 1, CU_GRAPH_USER_OBJECT_MOVE);
+  if (r != CUDA_SUCCESS) {
+    driver().p_cuUserObjectRelease(obj, 1);
+    return drv_fail(r, "cuGraphRetainUserObject");
+  }
+  *out = best;
+  return 0;
+}
+
 int free_slot(StreamSlot& sl) {
+  RelaxedCapture relaxed;
   if (sl.status) DRV(cuMemFree(sl.status));
   if (sl.ws) DRV(cuMemFree(sl.ws));
   if (sl.counters) DRV(cuMemFree(sl.counters));
@@ -237,8 +333,9 @@ int slot_for(DeviceState* s, CUstream stream, bool create, StreamSlot** out) {
     dst = &s->slots.back();
   }
   dst->stream = stream;
+  RelaxedCapture relaxed;
   DRV(cuMemAlloc(&dst->status, 16));
-  DRV(cuMemsetD32(dst->status, 0, 4));
+  if (int e = zero_words(s, dst->status, 4)) return e;
   dst->last_use = ++s->use_clock;
   *out = dst;
   return 0;
@@ -1239,33 +1336,51 @@ static int launch_impl(uint64_t function, const kcg_kernel_info* info, int devic
     p.split_factor = factor;
     p.sk_per = sk_per;
     p.split_units_first = plan.units_first;
+    CUdeviceptr ws = 0;
+    size_t ws_bytes = 0;
     if (factor > 1 || ws_epilogue || sk_per > 0) {
       // slots: one per (tile, split) of an even split; range index + tile index under stream-K
       const size_t slots = sk_per > 0 ? static_cast<size_t>(sk_ranges) + (T - first)
                                       : static_cast<size_t>(T - first) * factor;
       const size_t need = slots * info->bm * info->bn * sizeof(float);
-      if (slot->ws_bytes < need) {
-        s->tmaps.clear();  // drops the maps of the workspace that is about to move
-        if (int e = grow(&slot->ws, &slot->ws_bytes, need)) return e;
-      }
       const size_t tiles = static_cast<size_t>(T - first) * (pair ? 2 : 1);  // one counter per CTA half
-      if (slot->counters_n < tiles) {
-        size_t have = slot->counters_n * 4;
-        slot->counters_n = 0;
-        if (int e = grow(&slot->counters, &have, tiles * 4)) return e;
-        slot->counters_n = tiles;
-        DRV(cuMemsetD32(slot->counters, 0, tiles));
+      CUstreamCaptureStatus capturing = CU_STREAM_CAPTURE_STATUS_NONE;
+      cuuint64_t id = 0;
+      CUgraph graph = nullptr;
+      // (an error means that the launch itself is not allowed now, and says so)
+      if (driver().p_cuStreamGetCaptureInfo_v3(reinterpret_cast<CUstream>(stream), &capturing, &id, &graph, nullptr,
+                                               nullptr, nullptr) == CUDA_SUCCESS &&
+          capturing == CU_STREAM_CAPTURE_STATUS_ACTIVE) {
+        GraphBuffer* buf = nullptr;
+        if (int e = graph_buffer(s, reinterpret_cast<CUstream>(stream), id, graph, need, tiles, &buf)) return e;
+        ws = buf->ws;
+        ws_bytes = buf->ws_bytes;
+        p.tile_counters = reinterpret_cast<unsigned int*>(buf->counters());
+      } else {
+        if (slot->ws_bytes < need) {
+          s->tmaps.clear();  // drops the maps of the workspace that is about to move
+          if (int e = grow(&slot->ws, &slot->ws_bytes, need)) return e;
+        }
+        if (slot->counters_n < tiles) {
+          size_t have = slot->counters_n * 4;
+          slot->counters_n = 0;
+          if (int e = grow(&slot->counters, &have, tiles * 4)) return e;
+          slot->counters_n = tiles;
+          if (int e = zero_words(s, slot->counters, tiles)) return e;
+        }
+        ws = slot->ws;
+        ws_bytes = slot->ws_bytes;
+        p.tile_counters = reinterpret_cast<unsigned int*>(slot->counters);
       }
-      p.splitk_ws = reinterpret_cast<float*>(slot->ws);
-      p.tile_counters = reinterpret_cast<unsigned int*>(slot->counters);
+      p.splitk_ws = reinterpret_cast<float*>(ws);
     }
     if (!x3 && (factor > 1 || sk_per > 0)) {
       // The single-pass kernel writes its partial tiles with TMA stores: the workspace as one tall
       // fp32 matrix of BN columns (every row the buffer holds, so that the map is reused while the
       // buffer is), 32 x 32 boxes with the 128B swizzle of the staging buffers.
       const uint64_t row_bytes = static_cast<uint64_t>(info->bn) * 4;
-      if (int e = encode_map(s, &p.tmWs, KCG_DTYPE_FLOAT32, static_cast<uint64_t>(slot->ws), info->bn,
-                             slot->ws_bytes / row_bytes, row_bytes, 32, 32, 3))
+      if (int e = encode_map(s, &p.tmWs, KCG_DTYPE_FLOAT32, static_cast<uint64_t>(ws), info->bn, ws_bytes / row_bytes,
+                             row_bytes, 32, 32, 3))
         return e;
     }
   }
@@ -1315,13 +1430,15 @@ static int launch_impl(uint64_t function, const kcg_kernel_info* info, int devic
 
 // Reads (and clears) the status block of a stream's slot after synchronising the stream.
 // Call with g_dev_mutex held.
-static int read_status(StreamSlot* sl) {
+static int read_status(const DeviceState* s, StreamSlot* sl) {
   unsigned int st[4] = {0, 0, 0, 0};
   DRV(cuMemcpyDtoH(st, sl->status, sizeof(st)));
   if (st[0] != 0) {
     DRV(cuMemsetD32(sl->status, 0, 4));
     // a timed-out split-K launch may leave counters mid-count
     if (sl->counters) DRV(cuMemsetD32(sl->counters, 0, sl->counters_n));
+    for (const GraphBuffer* b : s->graph_buffers)
+      if (b->held.load() && b->stream == sl->stream) DRV(cuMemsetD32(b->counters(), 0, b->counters_n));
     static const char* role[] = {"", "TMA producer", "MMA issuer", "epilogue", "splitter", "shape", "push warp"};
     return fail(KCG_E_DEVICE_TIMEOUT, "kernel gave up in a bounded wait: role %s (code %u), block %u, detail %u/%u",
                 st[0] < 7 ? role[st[0]] : "?", st[0], st[1], st[2], st[3]);
@@ -1337,7 +1454,7 @@ int kcg_check_status(int device, uint64_t stream) {
   StreamSlot* sl = nullptr;
   if (int e = slot_for(s, reinterpret_cast<CUstream>(stream), false, &sl)) return e;
   if (!sl) return 0;  // nothing was ever launched on this stream
-  return read_status(sl);
+  return read_status(s, sl);
 }
 
 int kcg_matmul_host(uint64_t function, const kcg_kernel_info* info, int device, uint64_t stream,
@@ -1376,7 +1493,7 @@ int kcg_matmul_host(uint64_t function, const kcg_kernel_info* info, int device, 
     std::lock_guard<std::mutex> g(g_dev_mutex);
     StreamSlot* sl = nullptr;
     if (int e = slot_for(s, ran_on, false, &sl)) return e;
-    return sl ? read_status(sl) : 0;
+    return sl ? read_status(s, sl) : 0;
   };
   if (nslabs == 1) {
     DRV(cuMemcpyHtoDAsync(s->hbuf[0], hostA, bytes[0], st));
@@ -1465,6 +1582,8 @@ int kcg_shutdown(void) {
       if (sl.ws) d.p_cuMemFree(sl.ws);
       if (sl.counters) d.p_cuMemFree(sl.counters);
     }
+    for (GraphBuffer* b : s.graph_buffers) d.p_cuMemFree(b->ws);
+    if (s.aux) d.p_cuStreamDestroy(s.aux);
     for (int j = 0; j < 3; ++j) {
       if (s.hbuf[j]) d.p_cuMemFree(s.hbuf[j]);
       if (s.hstream[j]) d.p_cuStreamDestroy(s.hstream[j]);

@@ -140,8 +140,9 @@ int kcg_device_properties(int device, kcg_device_props* out);
  * Replaces the generated launcher's launch() (Runtime/python/kcg/HIPLauncher.py:189-238):
  * asynchronous on `stream` (a CUstream as integer; 0 = default stream), pointers are
  * device addresses borrowed for the call. Tensor maps for TMA are built (and cached per
- * pointer/shape) inside. Split-K kernels use a per-device workspace the library
- * allocates on first use. C is overwritten (alpha = 1, beta = 0). */
+ * pointer/shape) inside. Launches that cut tiles into K ranges use a workspace the
+ * library allocates on first use: the stream's, or, where the launch is captured, one
+ * that the graph holds. C is overwritten (alpha = 1, beta = 0). */
 int kcg_launch_gemm(uint64_t function, const kcg_kernel_info* info, int device, uint64_t stream,
                     uint64_t A, uint64_t B, uint64_t C);
 /* Fused epilogue: C = act(alpha * (A*B) + beta * C + bias[col]), fp32 arithmetic in that order,
