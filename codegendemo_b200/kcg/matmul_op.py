@@ -159,8 +159,12 @@ def tuned_config(M: int, N: int, K: int, dtype: EnumKernelDType, isATranspose: i
         db = db if db is not None else KernelDb()
         hit = db.lookup(M, N, K, int(dtype), isATranspose)
         if hit is not None:
-            return _with_b_transposed(KernelArgMatmul.fromJson(hit["config"])) if b_transposed else \
-                KernelArgMatmul.fromJson(hit["config"])
+            kpm = KernelArgMatmul.fromJson(hit["config"])
+            if not b_transposed:
+                return kpm
+            if kpm.KERNEL_VARIANT in (2, 4, 5) or (kpm.KERNEL_VARIANT == 0 and kpm.usesTensorCores()):
+                return _with_b_transposed(kpm)
+            # (the other kernels read a B stored K x N only: the rule decides)
     plain = _plain_rule(batch * M, N, K, dtype, isATranspose)
     if M % plain.BLOCK_SIZE_M:
         plain = _plain_rule(M, N, K, dtype, isATranspose)

@@ -39,6 +39,25 @@ def test_a_batch_of_one_and_a_transposed_b_do_not_share_a_kernel(stubs, bmm_firs
     assert sorted(k.kpm.IS_BTRANS for k in stubs) == [0, 1]
 
 
+def test_a_stored_config_that_cannot_read_a_transposed_b_gives_way():
+    """The kernel database may hold an FFMA config for a 16-bit shape; b_transposed then takes the rule's tile."""
+    from codegendemo_b200.kcg.KCGCompiler import compile_info
+    from codegendemo_b200.kcg.Utils import EnumKernelDType as E
+
+    class Db:
+        def lookup(self, *key):
+            simt = dict(KERNEL_VARIANT=1, BLOCK_SIZE_M=128, BLOCK_SIZE_N=128, BLOCK_SIZE_K=16, THREAD_SIZE_M=8,
+                        THREAD_SIZE_N=8, WARP_SCATTER_WIDTH_A=4, WARP_SCATTER_WIDTH_B=4, THREAD_SCATTER_WIDTH_A=4,
+                        THREAD_SCATTER_WIDTH_B=4)
+            return {"config": matmul_op.default_config(256, 256, 256, E.bfloat16, **simt).jsonfy()}
+    assert matmul_op.tuned_config(256, 256, 256, E.bfloat16, db=Db()).KERNEL_VARIANT == 1
+    kpm = matmul_op.tuned_config(256, 256, 256, E.bfloat16, db=Db(), b_transposed=True)
+    kpm.check()
+    assert kpm.KERNEL_VARIANT in (2, 4, 5) and kpm.IS_BTRANS == 1
+    compile_info(kpm.compileArgs(), num_stages=kpm.NUM_STAGES, kernel=kpm.KERNEL_VARIANT, b_trans=1,
+                 edge_tiles=kpm.EDGE_TILES)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("bmm_first", [False, True])
 def test_a_batch_of_one_and_a_transposed_b_on_one_shape(bmm_first, monkeypatch):
