@@ -83,13 +83,14 @@ def _tile_us(tile, split, M, N, K, batch=1, sms=148):
     return max(stream, fixed + waves * (blocks * per_block + per_tile))
 
 
-def _cheapest_tile(M, N, K, batch=1):
+def _cheapest_tile(M, N, K, batch=1, single_pass=False):
     """(estimate, tile, split) of the tile with the smallest estimate. Tiles may hang over the edges of the problem,
-    except over M and K of a batched one, past whose matrices the next batch lies."""
+    except over M and K of a batched one, past whose matrices the next batch lies. ``single_pass``: without the cluster
+    split-K kernel."""
     best = None
     for tile in _TILE_COST:
         variant, bm, bn, bk = tile
-        if batch > 1 and (M % bm or K % bk):
+        if batch > 1 and (M % bm or K % bk) or single_pass and variant == 5:
             continue
         for split in (2, 3, 4) if variant == 5 else (1,):
             if variant == 5 and (split > len(_TILE_COST[tile][2]) + 1 or -(-K // bk) < 2 * split or
@@ -147,32 +148,35 @@ def _cheapest_tile_f32(M, N, K, sms=148):
 
 
 def tuned_config(M: int, N: int, K: int, dtype: EnumKernelDType, isATranspose: int = 0, db=None, batch: int = 1,
-                 b_transposed: bool = False) -> KernelArgMatmul:
+                 b_transposed: bool = False, single_pass: bool = False) -> KernelArgMatmul:
     """Best known config of a shape: the kernel database's entry when the shape was tuned; else (16-bit types, and
-    single fp32 products) the tile with the smallest estimated time - the plain rule's choice is kept while the estimate puts it
-    within 10 % of that: the estimates of the two largest tiles are up to that much too low where a remainder is cut up
-    (2048x11008x4096: 512x256x64 estimated 110, 256x256x128 118 us; measured 142 and 135, and 165 and 148 once the
-    power cap holds the clock down). ``batch`` > 1: M, N, K are one
-    batch's, and the config fits all batches' tiles walked together. ``b_transposed``: B is stored N x K."""
+    single fp32 products) the tile with the smallest estimated time - the plain rule's choice is kept while the estimate
+    puts it within 10 % of that: the estimates of the two largest tiles are up to that much too low where a remainder is
+    cut up (2048x11008x4096: 512x256x64 estimated 110, 256x256x128 118 us; measured 142 and 135, and 165 and 148 once the
+    power cap holds the clock down). ``batch`` > 1: M, N, K are one batch's, the config fits all batches' tiles walked
+    together, and the database, which holds single products, is not asked. ``b_transposed``: B is stored N x K.
+    ``single_pass``: a config of the single-pass kernels (KERNEL_VARIANT 2 and 4), which alone can store fp32 results of
+    16-bit operands; 16-bit types."""
     from codegendemo_b200.kcg.InfoDb import KernelDb
     if batch == 1:
         db = db if db is not None else KernelDb()
         hit = db.lookup(M, N, K, int(dtype), isATranspose)
         if hit is not None:
             kpm = KernelArgMatmul.fromJson(hit["config"])
-            if not b_transposed:
-                return kpm
-            if kpm.KERNEL_VARIANT in (2, 4, 5) or (kpm.KERNEL_VARIANT == 0 and kpm.usesTensorCores()):
-                return _with_b_transposed(kpm)
-            # (the other kernels read a B stored K x N only: the rule decides)
+            takes = (2, 4) if single_pass else (2, 4, 5)
+            if not (b_transposed or single_pass) or kpm.KERNEL_VARIANT in takes or \
+                    (kpm.KERNEL_VARIANT == 0 and kpm.usesTensorCores()):
+                return _with_b_transposed(kpm) if b_transposed else kpm
+            # (a kernel that cannot do what is asked: the rule decides)
     plain = _plain_rule(batch * M, N, K, dtype, isATranspose)
     if M % plain.BLOCK_SIZE_M:
         plain = _plain_rule(M, N, K, dtype, isATranspose)
     plain.M = M
     if int(dtype) != int(EnumKernelDType.float32) and M % 128 == 0 and N % 64 == 0 and K % 64 == 0:
-        us, tile, split = _cheapest_tile(M, N, K, batch)
+        us, tile, split = _cheapest_tile(M, N, K, batch, single_pass)
         have = (plain.KERNEL_VARIANT or 2, plain.BLOCK_SIZE_M, plain.BLOCK_SIZE_N, plain.BLOCK_SIZE_K)
-        if have not in _TILE_COST or _tile_us(have, plain.LOCAL_SPLIT_U, M, N, K, batch) > 1.1 * us:
+        if have not in _TILE_COST or single_pass and have[0] == 5 or \
+                _tile_us(have, plain.LOCAL_SPLIT_U, M, N, K, batch) > 1.1 * us:
             variant, bm, bn, bk = tile
             stages = dict(NUM_STAGES=4) if bm == 512 else {}
             plain = default_config(M, N, K, dtype, KERNEL_VARIANT=variant, BLOCK_SIZE_M=bm, BLOCK_SIZE_N=bn,
@@ -341,6 +345,16 @@ def _single_pass_16bit(kpm, M, N, K, dt):
     return default_config(M, N, K, dt, KERNEL_VARIANT=2)
 
 
+def _attention_tile(heads, m, n, kk, dt, scores):
+    """Config of one of the attention chain's batched products, per head m x n x kk. ``scores``: q k^T with k as stored;
+    the scores leave as fp32: rounded to 16 bits first, their error (up to 2^-9 of a score of several units) would be
+    amplified by the softmax's exp."""
+    kpm = tuned_config(m, n, kk, dt, batch=heads, b_transposed=scores, single_pass=True)
+    if scores:
+        kpm.setOutputDtype(EnumKernelDType.float32)
+    return kpm
+
+
 def attention(q, k, v, scale=None, out=None):
     """``softmax(scale * q @ k^T) @ v`` per head, the attention-shaped chain, as three launches on the current
     stream: a batched product with k taken as stored (keys x head_dim, no transposed copy) whose epilogue applies
@@ -365,18 +379,8 @@ def attention(q, k, v, scale=None, out=None):
     key = ("attn", H, Sq, Sk, D, int(dt), dev)
     kerns = _KERNELS.get(key)
     if kerns is None:
-        def tile_for(m, n, kk, scores_step):
-            kpm = tuned_config(m, n, kk, dt, batch=H)
-            if m % kpm.BLOCK_SIZE_M or kpm.KERNEL_VARIANT not in (0, 2, 4):
-                kpm = default_config(m, n, kk, dt)
-            kpm.M = m
-            if scores_step:
-                # q k^T with k as stored; the scores leave as fp32: rounded to 16 bits first, their error
-                # (up to 2^-9 of a score of several units) would be amplified by the softmax's exp
-                kpm = _single_pass_16bit(kpm, m, n, kk, dt)
-                kpm.IS_BTRANS = 1
-                kpm.setOutputDtype(EnumKernelDType.float32)
-            return build_kernel(kpm, dev)[1]
+        def tile_for(m, n, kk, scores):
+            return build_kernel(_attention_tile(H, m, n, kk, dt, scores), dev)[1]
         kerns = (tile_for(Sq, Sk, D, True), tile_for(Sq, D, Sk, False))
         _KERNELS[key] = kerns
     scores = torch.empty((H, Sq, Sk), dtype=torch.float32, device=q.device)

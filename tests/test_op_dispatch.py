@@ -58,6 +58,37 @@ def test_a_stored_config_that_cannot_read_a_transposed_b_gives_way():
                  edge_tiles=kpm.EDGE_TILES)
 
 
+# heads, queries, keys, head dimension of the three-launch attention; the first two are where the rule over all kernels
+# prefers the cluster split-K kernel for a product
+ATTENTION = [(8, 512, 2048, 128), (32, 128, 8192, 128), (16, 2048, 2048, 128), (4, 128, 1024, 64), (1, 384, 320, 64),
+             (2, 256, 192, 64)]
+
+
+def test_attention_takes_the_best_single_pass_tile():
+    from codegendemo_b200.kcg.Utils import EnumKernelDType as E
+    for heads, sq, sk, d in ATTENTION:
+        for m, n, k, scores in ((sq, sk, d, True), (sq, d, sk, False)):
+            kpm = matmul_op._attention_tile(heads, m, n, k, E.bfloat16, scores)
+            kpm.check()
+            tile = (kpm.KERNEL_VARIANT or 2, kpm.BLOCK_SIZE_M, kpm.BLOCK_SIZE_N, kpm.BLOCK_SIZE_K)
+            best = matmul_op._cheapest_tile(m, n, k, heads, single_pass=True)[0]
+            assert tile[0] in (2, 4) and kpm.IS_BTRANS == int(scores)
+            assert matmul_op._tile_us(tile, 1, m, n, k, heads) <= 1.1 * best, (heads, m, n, k)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", ATTENTION, ids=lambda s: "x".join(map(str, s)))
+def test_attention_in_three_launches(shape):
+    heads, sq, sk, d = shape
+    gen = torch.Generator().manual_seed(2)
+    q, k, v = [torch.randn((heads, n, d), generator=gen).to(torch.bfloat16) for n in (sq, sk, sk)]
+    out = matmul_op.attention(q.cuda(), k.cuda(), v.cuda()).cpu().double()
+    p = torch.softmax(q.double() @ k.double().transpose(1, 2) * d ** -0.5, dim=-1)
+    # probabilities and the result are each rounded once to bf16: half a unit each; 32-bit sums far below that
+    bound = 2.0 ** -8 * (p @ v.double()).abs() + 2.0 ** -8 * (p @ v.double().abs()) + 1e-5
+    assert ((out - p @ v.double()).abs() <= bound).all()
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("bmm_first", [False, True])
 def test_a_batch_of_one_and_a_transposed_b_on_one_shape(bmm_first, monkeypatch):
