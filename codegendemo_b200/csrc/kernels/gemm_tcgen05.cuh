@@ -308,9 +308,7 @@ struct TcGemm {
     } else if (warp == 1) {
       // -------------------------- MMA issuer (in a pair: the leader CTA only)
       if (rank == 0u) {
-        // The whole warp walks this loop and elects one lane per batch of instructions, so that their descriptors are
-        // warp-uniform values: inside an if (lane == 0) every tcgen05.mma takes about 125 cycles to issue (measured in
-        // the fused attention kernel), as long as a 128 x 256 x 16 product runs.
+        // whole warp, one elected lane per batch of instructions (see elect_one)
         const uint32_t tmem_base_u = __shfl_sync(0xffffffffu, tmem_base, 0);
         uint32_t it = 0, acc_it = 0;
         bool ok = true;

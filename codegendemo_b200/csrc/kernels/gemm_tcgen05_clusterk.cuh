@@ -255,9 +255,7 @@ struct TcGemmClusterK {
     } else if (warp == 1) {
       // ---------------------------------------------------------- MMA issuer
       {
-        // The whole warp walks this loop and elects one lane per batch of instructions, so that their descriptors are
-        // warp-uniform values: inside an if (lane == 0) every tcgen05.mma takes about 125 cycles to issue (measured in
-        // the fused attention kernel), as long as a 128 x 256 x 16 product runs.
+        // whole warp, one elected lane per batch of instructions (see elect_one)
         const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
         bool ok = true;
         for (int kb = 0; kb < kbn; ++kb) {

@@ -197,9 +197,7 @@ struct TcGemmF32x3 {
         griddep_launch_dependents();  // every load is issued: the stream's next kernel may be brought in
       } else if (warp == 1 && rank == 0u) {
         // ---------------------------- MMA issuer (in a pair: the leader CTA only)
-        // The whole warp walks this loop and elects one lane per batch of instructions, so that their descriptors are
-        // warp-uniform values: inside an if (lane == 0) every tcgen05.mma takes about 125 cycles to issue (measured in
-        // the fused attention kernel), as long as a 128 x 256 x 16 product runs.
+        // whole warp, one elected lane per batch of instructions (see elect_one)
         const uint32_t tmem_base_u = __shfl_sync(0xffffffffu, tmem_base, 0);
         uint32_t it = 0, chunk_it = 0;
         bool ok = true;
