@@ -52,6 +52,8 @@ def getMatmulSignature(dtypeA, dtypeB, dtypeC) -> dict:
 
 
 class KernelArgMatmul:
+    EDGE_TILES = 0  # (configs pickled before the key existed do not carry it)
+
     def __init__(self, m, n, k, typeA: EnumKernelDType, typeB: EnumKernelDType, typeC: EnumKernelDType):
         self.BLOCK_SIZE_M = 64
         self.BLOCK_SIZE_N = 64

@@ -55,6 +55,16 @@ def test_edge_tiles_are_an_option_with_rules_of_their_own():
             compile_info(default_config(128, N, K, E.bfloat16, BLOCK_SIZE_N=128).compileArgs(), kernel=kernel, edge_tiles=1)
 
 
+def test_a_config_pickled_before_the_option_existed():
+    """An autotune run that was interrupted leaves pickled configs behind; those of an older version lack the key."""
+    import pickle
+    kpm = default_config(128, 128, 64, E.bfloat16)
+    del kpm.__dict__["EDGE_TILES"]
+    old = pickle.loads(pickle.dumps(kpm))
+    old.check()
+    assert old.jsonfy() == default_config(128, 128, 64, E.bfloat16).jsonfy()
+
+
 def test_every_fp32_shape_gets_a_config_the_kernels_can_build():
     import ctypes
     rng = random.Random(8)
