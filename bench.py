@@ -12,13 +12,14 @@ tcgen05 kernel.
 
 Outside the timed region every rank checks its result against the CPU oracle (``oracle_check``): eight random
 128-row blocks of its slab at every N, and every row at N=1; a failed check ends the run with a non-zero exit
-code. At N=1 the line also carries, under ``other_workloads``, the other single-GPU configs - fp32 1024^3 and
+code. At N=1 a second JSON line, on stderr, carries under ``other_workloads`` the other single-GPU configs - fp32 1024^3 and
 4096^3 (3xTF32 and FFMA SIMT), bf16 8192^3 and the rectangular sweep M in {128, 512, 2048} x N, K in {4096, 11008}
 x {fp32, bf16} (24 points) - each with its roofline and the same shape through cuBLAS (``torch.matmul`` on the device) timed
 the same way, and the operators around the product (batched, strided, the attention-shaped chain as three launches
 and as one fused kernel), each beside its PyTorch library call and checked against the host composition at fp32.
 
-Prints ONE JSON line on rank 0 (metric: GEMM TFLOP/s, device-timed with CUDA events, max over ranks).
+Prints ONE JSON line on rank 0's stdout (metric: GEMM TFLOP/s, device-timed with CUDA events, max over ranks), of a few
+KB: readers that keep the end of the output keep all of it.
 ``--impl reference`` times the reference's CPU path for the same metric: ``torch.matmul`` on host tensors (the
 reference's own correctness oracle, Runtime/python/kcg/KCGTask.py:94) with all host threads, operands built
 once before the clock starts, only the call between the two timestamps (KCGTask.py:124-130).
@@ -787,8 +788,11 @@ def main():
             "oracle_check": check, "cpu_baseline": cpu_base, "e2e": e2e,
             "gpu_launches": int(launches), "clocks": clocks, "e2e_matches_device_result": same,
             "e2e_max_diff_vs_device_rel": e2e_diff,
-            "other_workloads": extras, "other_workloads_clocks": group_clocks, "allgather_c": allgather,
+            "allgather_c": allgather,
         }
+        if extras is not None:
+            sys.stderr.write(json.dumps({"other_workloads": extras, "other_workloads_clocks": group_clocks}) + "\n")
+            sys.stderr.flush()
         print(json.dumps(line), flush=True)
     ok = check["ok"] and e2e["oracle_check"]["ok"]
     if world > 1:
