@@ -1,5 +1,5 @@
-// Fused attention for up to 64 query rows per head over a long list of keys (the step that appends one or a few
-// tokens to a cache), fp16 / bf16, head dimension 64 or 128.
+// Fused attention for few query rows per head over a long list of keys (the step that appends one or a few tokens to a
+// cache), fp16 / bf16, head dimension 64 or 128: up to 64 rows, and all calls of up to 32 (few_rows_form draws the line).
 //
 // What bounds it: K and V are read once, 2 * sk * d values per head, and every value meets at most 64 queries, so
 // HBM does. The 256-row kernel gives a head ONE CTA, which is a serial walk over all keys with most tensor rows

@@ -59,7 +59,8 @@ _TILE_COST = {
     (5, 128, 192, 64): (1.0, 0.322, (5.15, 5.60, 6.32)),
     (5, 128, 256, 64): (1.0, 0.379, (5.77, 6.37, 6.61)),
 }
-_CLUSTERS = {2: 74, 3: 45, 4: 33}  # clusters of 2, 3, 4 CTAs at 200 KB of shared memory each that run at once
+# clusters of 2, 3, 4 CTAs at 200 KB of shared memory each that run at once on the GPU the table is fitted to (148 SMs)
+_CLUSTERS = {2: 74, 3: 45, 4: 33}
 
 
 def _tile_us(tile, split, M, N, K, batch=1, sms=148):
@@ -396,8 +397,8 @@ def attention(q, k, v, scale=None, out=None):
 
 
 def attention_fused(q, k, v, scale=None, out=None):
-    """``softmax(scale * q @ k^T) @ v`` per head as ONE kernel (``kcg_attention_fwd``): scores and probabilities
-    stay in tensor memory and shared memory. ``q`` is (heads, Sq, d), ``k`` and ``v`` are (heads, Sk, d), all
+    """``softmax(scale * q @ k^T) @ v`` per head, fused (``kcg_attention_fwd``, one or two launches): scores and
+    probabilities stay on the SM. ``q`` is (heads, Sq, d), ``k`` and ``v`` are (heads, Sk, d), all
     contiguous fp16 / bf16 with d = 64 or 128; any Sq and Sk. Returns (heads, Sq, d). ``attention`` above is the
     three-launch form of the same chain."""
     import math

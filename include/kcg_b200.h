@@ -201,13 +201,15 @@ int kcg_softmax_rows(int device, uint64_t stream, uint64_t X, int64_t rows, int 
 int kcg_softmax_rows_ex(int device, uint64_t stream, uint64_t X, int dtype_in, int64_t ldx, uint64_t Y,
                         int dtype_out, int64_t ldy, int64_t rows, int cols, float scale);
 
-/* ---- the same chain as ONE kernel ------------------------------------------------------
+/* ---- the same chain fused --------------------------------------------------------------
  * O[h] = softmax(scale * Q[h] K[h]^T) V[h] for h in [0, heads): Q and O are heads x sq x d, K and V
  * heads x sk x d, all contiguous, float16 or bfloat16 (`dtype`), d = 64 or 128. Scores and
- * probabilities stay in tensor memory and shared memory (tcgen05.mma for both products, running
- * maximum and sum per query row); nothing of size sq x sk is written. Asynchronous on `stream`;
- * allocates nothing. `scale` must be positive. The first call per device and data type opts the kernel in
- * to its dynamic shared memory (a function attribute): make it before capturing the stream into a graph.
+ * probabilities stay on the SM (running maximum and sum per query row); nothing of size sq x sk is
+ * written. Both products run on tcgen05.mma, 256 query rows to a CTA; groups of 256 rows that do not fill
+ * a wave share their keys in a second launch, and few query rows (up to 32, some shapes up to 64) take a
+ * kernel of their own (mma.sync, a head's keys shared by a cluster). Asynchronous on `stream`; allocates
+ * nothing. `scale` must be positive. The first call per device, data type and form opts the kernel in to its
+ * dynamic shared memory (a function attribute): make it before capturing the stream into a graph.
  * No counterpart in the reference (see the note on kcg_softmax_rows). */
 int kcg_attention_fwd(int device, uint64_t stream, uint64_t Q, uint64_t K, uint64_t V, uint64_t O, int dtype,
                       int heads, int sq, int sk, int d, float scale);
