@@ -87,6 +87,7 @@ def test_buffers_of_graphs_that_are_gone_serve_the_next():
         graph.reset()
         torch.cuda.synchronize()
         used.append(torch.cuda.mem_get_info()[1] - torch.cuda.mem_get_info()[0])
-    # (one buffer of this product is 18 MB; what torch keeps for a graph stays under 4 MB)
-    assert used[-1] - used[2] < 4 << 20, used
+    # A buffer of this product is 18 MB. It comes back when the driver has run the graph's destructor, which may be after
+    # the next capture has begun: two or three take turns then, but not one for each of twelve graphs.
+    assert used[-1] - used[0] <= 60 << 20, used
     assert torch.equal(c, want)
