@@ -14,10 +14,10 @@
 //             rescaled where that maximum has moved; at the end O / sum to global memory
 // A tile's chain is serial (scores, softmax, P V, next scores) and the two tiles' chains take turns, so the tensor
 // pipe works for one tile while the other is in its softmax. What bounds it is that chain: per step and tile 512 + 512
-// cycles of products (the scores' operands fill the shared-memory port, 128 bytes a cycle) and 1024 of exponentials,
-// of which about 3100 cycles for two tiles' steps remain exposed against 2048 of the tensor pipe alone. Measured (B200,
-// bf16), a form with votes of all softmax warps, O rescaled at every new maximum and a one-lane issuer against this
-// one: 32 heads x 4096 x 4096 x 128 322 -> 246 us (1119 TFLOP/s), x 64 287 -> 210 us, 16 x 2048 x 2048 x 128 46 -> 36 us.
+// cycles of products (the scores' operands fill the shared-memory port, 128 bytes a cycle) and 1024 of exponentials;
+// both tiles' steps take about 3600 cycles against 2048 of the tensor pipe alone. Measured (B200, bf16), a form with
+// votes of all softmax warps and a one-lane issuer against this one with its key-split form: 32 heads x 4096 x 4096 x
+// 128 322 -> 239 us (1150 TFLOP/s), x 64 287 -> 202 us, 16 x 2048 x 2048 x 128 46 -> 38 us.
 // A key-split form of it (kKeySplit) shares a group's keys among the CTAs of a cluster where groups do not fill a wave.
 // Tried without gain: exponentials of every eighth to third pair as a polynomial on the FMA pipe (2 to 8 % slower: one
 // warp per scheduler and tile is bound by its own latencies, not by the exponential pipe).
