@@ -61,28 +61,6 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* t
       : "memory");
 }
 
-// registers -> TMEM: each thread of the warp writes 32 consecutive fp32 columns of its own lane (row)
-__device__ __forceinline__ void tmem_st_32x32b_x32(uint32_t taddr, const uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-      :
-      : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]),
-        "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]),
-        "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-      : "memory");
-}
-__device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-      :
-      : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
-}
 // Ties the registers of an earlier tmem_ld to the wait before it: no use of them may be scheduled ahead of this.
 __device__ __forceinline__ void pin_32(uint32_t (&r)[32]) {
 #pragma unroll
@@ -114,23 +92,6 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
   return r;
 }
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
-// D[tmem] (+)= A[tmem] * B[smem], 16-bit operands: A is read from tensor memory (lane = row, one 32-bit column =
-// two consecutive K values), B through a shared-memory descriptor. Issued by ONE thread.
-__device__ __forceinline__ void umma_ts_f16(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
-                                            uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-      "}\n"
-      :
-      : "r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
 __device__ __forceinline__ float ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -332,7 +293,7 @@ struct AttnFwd {
             const uint64_t bdesc = make_smem_desc(sv_addr + ks * 16 * 128, KVBOX_BYTES, 1024, SWZ_128B);
             if constexpr (kPTmem) {
               // 16 keys = 8 columns of packed pairs in the S buffer of this step
-              umma_ts_f16(tmem_base + COL_O, tmem_base + (j & 1) * BC + ks * 8, bdesc, IDESC_O,
+              umma_ts<false>(tmem_base + COL_O, tmem_base + (j & 1) * BC + ks * 8, bdesc, IDESC_O,
                           (j > 0 || ks > 0) ? 1u : 0u);
             } else {
               const uint32_t a_off = ((ks * 32) / 128) * (BR * 128) + ((ks * 32) % 128);  // boxes of 64 keys
@@ -711,7 +672,7 @@ struct AttnFwd2 {
 #pragma unroll
           for (int ks = 0; ks < BC / 16; ++ks)
             if (ks >= ks0 && ks < ks1)
-              umma_ts_f16(tmem + COL_O + t * kD, tmem + t * BC + ks * 8, vd + ((ks * 16 * 128) >> 4), IDESC_O,
+              umma_ts<false>(tmem + COL_O + t * kD, tmem + t * BC + ks * 8, vd + ((ks * 16 * 128) >> 4), IDESC_O,
                           (j > 0 || ks > 0) ? 1u : 0u);
         };
         if (ok) ok = wait(&bars->k_full[0], 0u, 1u, 0);

@@ -486,7 +486,7 @@ int resolve(const Cfg& c, const kcg_compile_opts* opts, Resolved* r) {
       return fail(KCG_E_BAD_CONFIG, "accumulators of the tile exceed the TMEM columns available");
     const int splitk = c[KCG_CFG_LOCAL_SPLIT_U] > 0 ? c[KCG_CFG_LOCAL_SPLIT_U] : 1;
     if (splitk > blocks_of(K, bk)) return fail(KCG_E_BAD_CONFIG, "LOCAL_SPLIT_U %d exceeds the %d K blocks", splitk, blocks_of(K, bk));
-    auto ok = [&](int st) { return bn % 2 == 0 && kcg::tc_config_error(dt, bm / 2, bn / 2, bk, st, f32) == 0; };
+    auto ok = [&](int st) { return bn % 2 == 0 && kcg::tc_config_error(dt, bm / 2, bn / 2, bk, st, 2 * f32) == 0; };
     int st = (opts && opts->num_stages > 0) ? opts->num_stages : 2;
     if (!(opts && opts->num_stages > 0) && c[KCG_CFG_SHARED_PREFETCH])
       while (st < 7 && ok(st + 1)) ++st;
@@ -759,8 +759,8 @@ int fill_info(const Cfg& c, const Resolved& r, const std::string& name, const st
     const int pairs = units < r.num_sms / 2 ? units : r.num_sms / 2;
     out->grid[0] = 2 * pairs;  // persistent clusters of two CTAs
     out->cluster[0] = 2;
-    out->block[0] = f32 ? 512 : 256;
-    out->smem_bytes = kcg::tc_smem_bytes(c[KCG_CFG_DATATYPE_A], bm / 2, bn / 2, bk, r.stages, f32);
+    out->block[0] = f32 ? kcg::tc_x3_threads(kcg::tc_x3_tmem_a(bm / 2, bn / 2, bk, r.stages, 2), 2) : 256;
+    out->smem_bytes = kcg::tc_smem_bytes(c[KCG_CFG_DATATYPE_A], bm / 2, bn / 2, bk, r.stages, 2 * f32);
   } else if (r.kernel == KCG_KERNEL_TCGEN05_CLUSTERK) {
     out->grid[0] = tiles * lsu;  // one cluster of LOCAL_SPLIT_U CTAs per tile
     out->cluster[0] = lsu;

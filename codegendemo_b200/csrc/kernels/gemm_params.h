@@ -190,11 +190,30 @@ constexpr int tc_staging_bytes(int dtype, int x3) {
 // every shorter lo ring measured slower. So the lo ring is as deep as the hi ring.
 constexpr int tc_lo_stages(int stages) { return stages; }
 
-// Bytes of the operand rings: single-pass kernel stages * (A + B tile); 3xTF32 adds the lo ring.
+// `x3` of the rules below: 0 = single-pass kernel, 1 = 3xTF32 kernel, 2 = 3xTF32 on CTA pairs, whose BN here is one
+// CTA's half of the tile's columns.
+//
+// 3xTF32 kernel: K blocks of A (hi and lo parts, BK columns each) that tensor memory holds beside the two accumulator
+// buffers, or 0 where fewer than two fit (tiles of 256 columns, two accumulators): A then stays in shared memory.
+constexpr int tc_x3_tmem_a(int BM, int BN, int BK, int stages, int x3) {
+  if (x3 == 0 || BM != 128 || !(BK == 16 || BK == 32)) return 0;
+  const int fit = (512 - 2 * BN * x3) / (2 * BK);
+  const int n = kc_min(kc_min(fit, stages), 4);
+  return n >= 2 ? n : 0;
+}
+
+// Threads of a 3xTF32 CTA: control, splitter (two warpgroups in the pair form with A in tensor memory) and two
+// accumulating warpgroups.
+constexpr int tc_x3_threads(int tmem_a, int x3) { return tmem_a > 0 && x3 == 2 ? 640 : 512; }
+
+// Bytes of the operand rings: single-pass kernel stages * (A + B tile); 3xTF32 adds the lo ring, without A where that
+// goes through tensor memory.
 constexpr int tc_ring_bytes(int dtype, int BM, int BN, int BK, int stages, int x3) {
   const int eb = (dtype == KCG_DT_F32) ? 4 : 2;
   const int stage = (BM + BN) * BK * eb;
-  return stage * (stages + ((eb == 4 && x3) ? tc_lo_stages(stages) : 0));
+  if (!(eb == 4 && x3)) return stage * stages;
+  const int lo = tc_x3_tmem_a(BM, BN, BK, stages, x3) > 0 ? BN * BK * eb : stage;
+  return stage * stages + lo * tc_lo_stages(stages);
 }
 
 // Shape rules of the tcgen05 kernels; returns 0 when the config is buildable.
@@ -205,7 +224,7 @@ constexpr int tc_config_error(int dtype, int BM, int BN, int BK, int stages, int
   if (BN < 128 / eb || BN > 256 || (BN % (128 / eb)) != 0 || (BN % 16) != 0) return 3;
   if ((BM / 128) * BN > 512) return 4;
   // 3xTF32: two TMEM accumulator buffers and MT*BN/2 register accumulators per epilogue thread
-  if (eb == 4 && x3 && ((BM / 128) * BN > 256 || (BN % 64) != 0)) return 9;
+  if (eb == 4 && x3 && ((BM / 128) * BN > 256 || ((BN % 64) != 0 && !(x3 == 2 && BN == 96)))) return 9;
   const int rowb = BK * eb;
   if (!(rowb == 32 || rowb == 64 || (rowb % 128) == 0) || rowb > 512) return 5;
   if ((BK % (32 / eb)) != 0 || (BK % 8) != 0) return 6;

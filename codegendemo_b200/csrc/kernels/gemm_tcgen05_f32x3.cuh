@@ -3,9 +3,9 @@
 //
 // Why two extra mechanisms on top of the plain tcgen05 pipeline:
 //  * kind::tf32 reads fp32 words and ignores the low 13 mantissa bits, so
-//    hi = x needs no work; lo = tf32_rn(x - trunc_tf32(x)) is written by splitter
-//    warps into a twin of every landed stage, and each K step issues
-//    lo*hi + hi*lo + hi*hi (lo*lo, ~2^-22 relative, is dropped).
+//    hi = x needs no work; splitter warps write lo = tf32_rn(x - trunc_tf32(x)), for B
+//    into a twin of every landed stage, for A - hi and lo - into tensor memory, and each
+//    K step issues lo*hi + hi*lo + hi*hi (lo*lo, ~2^-22 relative, is dropped).
 //  * The tensor core adds into its fp32 accumulator with truncation, a bias that
 //    grows linearly with the number of accumulated K steps (measured: 3e-5
 //    normwise at K = 4096). So the MMA warp restarts a fresh accumulator every
@@ -13,12 +13,23 @@
 //    warps add each finished chunk into register accumulators with ordinary
 //    round-to-nearest FADDs while the next chunk is being multiplied.
 //
-// Warp roles (512 threads, four warpgroups so that setmaxnreg can move registers
-// from the control warps to the accumulating warps):
+// What bounds it. Every K block crosses the shared-memory port (~128 bytes a cycle) several times: written by TMA, read
+// and its lo twin written by the splitter, read by three products. With A in shared memory a CTA's half of a
+// 256x256x32 pair block moves about 230 KB and takes 1770 cycles against 1536 of the tensor pipe. A through registers
+// into tensor memory (hi and lo; 2 x BK columns a block) takes its lo twin and its reads by the products off the port:
+// 104 KB for 256x128 (1060 cycles measured against 768 of the pipe), 140 KB for 256x192. Tiles of 256 columns, whose two
+// accumulator buffers fill all 512 columns, and two-accumulator CTAs keep A in shared memory.
+// What the splitter cost before it was written like this, 256x256x32 pair block: rounding by cvt.rna.tf32 15 cycles per
+// warp instruction, arrivals at the leader with release at cluster scope 950 cycles, loads that waited for the stores
+// before them; 2500 cycles in all. 4096^3 585 -> 505 us, 2048x4096x4096 323 -> 262, 512x11008x4096 219 -> 190,
+// 1024^3 24.5 -> 20.9, 640x2624x1024 31 -> 25 (graph replay, B200).
+//
+// Warp roles (512 threads, 640 in the pair form with A in tensor memory; whole warpgroups so that setmaxnreg can move
+// registers from the control warps to the accumulating warps):
 //   WG0  warp 0 TMA producer, warp 1 MMA issuer + TMEM owner, warps 2-3 idle
-//   WG1  warps 4-7   splitter (lo twin of each stage)
-//   WG2/3 warps 8-15 accumulate + epilogue; warp w reads TMEM lane quarter w%4,
-//         column half (w-8)/4; kAccPerThread = MT*BN/2 fp32 registers per thread
+//   WG1 (and WG2)  splitter (lo twin of each stage; A through registers into tensor memory)
+//   the last two  accumulate + epilogue; warp w reads TMEM lane quarter w%4, column half by warpgroup;
+//         MT*BN/2 fp32 register accumulators per thread
 //
 // Same work decomposition, raster, split-K reduction and bounded waits as
 // gemm_tcgen05.cuh.
@@ -43,7 +54,8 @@ struct TcGemmF32x3 {
   static constexpr int NCTA = kPair ? 2 : 1;
   static constexpr int R = kBM / NCTA;     // rows of the tile held by one CTA
   static constexpr int BNL = kBN / NCTA;   // B columns loaded by one CTA
-  static_assert(tc_config_error(kDType, R, BNL, kBK, kStages, 1) == 0,
+  static constexpr int X3 = kPair ? 2 : 1;
+  static_assert(tc_config_error(kDType, R, BNL, kBK, kStages, X3) == 0,
                 "config not buildable by the 3xTF32 kernel");
   static constexpr TcLayout L = make_tc_layout(kDType, R, BNL, kBK, kATrans);
   static constexpr int UMMA_K = 8;
@@ -51,24 +63,39 @@ struct TcGemmF32x3 {
   static constexpr int ACC_COLS = MT * kBN;
   static_assert(2 * ACC_COLS <= 512, "two accumulator buffers must fit the 512 TMEM columns");
   static_assert(kBN % 64 == 0, "each epilogue warp drains whole 32-column pieces of its column half");
-  static constexpr int TMEM_COLS = kc_pow2_ceil(2 * ACC_COLS);
+  // K blocks of A in tensor memory, behind the accumulators: [hi: kBK columns][lo: kBK columns] each
+  static constexpr int TA = tc_x3_tmem_a(R, BNL, kBK, kStages, X3);
+  static constexpr uint32_t COL_A = 2 * ACC_COLS;
+  static constexpr int TMEM_COLS = kc_pow2_ceil(2 * ACC_COLS + TA * 2 * kBK);
+  static_assert(TMEM_COLS <= 512, "accumulators and A blocks must fit the 512 TMEM columns");
   static constexpr int STAGE_HI = L.stage_hi_bytes;
   // Two rings: kStages stages of TMA-landed hi operands (deep, to cover the load latency) and
   // LO_STAGES stages of their lo twins, written just in time by the splitter warps: lo stage
   // it % LO_STAGES is free again as soon as the MMAs of K block it - LO_STAGES have retired.
   static constexpr int LO_STAGES = tc_lo_stages(kStages);
   static constexpr int LO_RING = kStages * STAGE_HI;  // byte offset of the lo ring
-  static constexpr int RING_BYTES = (kStages + LO_STAGES) * STAGE_HI;
+  static constexpr int LO_BYTES = TA > 0 ? L.b_bytes : STAGE_HI;  // a lo stage: without A where that is in TMEM
+  static constexpr int LO_A_BYTES = TA > 0 ? 0 : L.a_bytes;
+  static constexpr int RING_BYTES = kStages * STAGE_HI + LO_STAGES * LO_BYTES;
   static constexpr int KSTEPS = kBK / UMMA_K;
-  static constexpr int NUM_THREADS = 512;
-  static constexpr int NUM_SPLIT_THREADS = 128;
+  // Splitter warpgroups; two take every other K block each. One, at about 1200 cycles a block, is slower than the products
+  // of a pair tile's block with A in tensor memory (768 for 128 columns).
+  static constexpr int NUM_THREADS = tc_x3_threads(TA, X3);
+  static constexpr int SPLIT_WGS = NUM_THREADS / 128 - 3;
+  static constexpr int FIRST_ACC_WARP = 4 + 4 * SPLIT_WGS;
+  static constexpr int NUM_SPLIT_THREADS = 128;  // of one warpgroup
   static constexpr int NUM_EPI_THREADS = 256;
+  // registers of a thread after setmaxnreg; the CTA is launched with 96 each (640 threads) or 128 (512)
+  static constexpr int CTL_REGS = SPLIT_WGS == 2 ? 48 : 56, SPLIT_REGS = TA > 0 && SPLIT_WGS == 1 ? 104 : 72;
+  static constexpr int ACC_REGS = SPLIT_WGS == 2 ? 144 : TA > 0 ? 176 : 192;
+  static_assert(CTL_REGS + SPLIT_WGS * SPLIT_REGS + 2 * ACC_REGS == (SPLIT_WGS == 2 ? 5 * 96 : 4 * 128), "register split");
   static constexpr int HALF_COLS = kBN / 2;
   static constexpr int PIECES = HALF_COLS / 32;
   static constexpr int ACC_PER_THREAD = MT * HALF_COLS;
   static_assert(ACC_PER_THREAD <= 128, "register accumulators per thread");
-  static constexpr int SMEM_BYTES = tc_smem_bytes(kDType, R, BNL, kBK, kStages, 1);
-  static constexpr uint32_t IDESC = make_instr_desc(FMT_TF32, kATrans ? 1u : 0u, 1u, kPair ? 256u : 128u, kBN);
+  static constexpr int SMEM_BYTES = tc_smem_bytes(kDType, R, BNL, kBK, kStages, X3);
+  static constexpr uint32_t IDESC =
+      make_instr_desc(FMT_TF32, kATrans && TA == 0 ? 1u : 0u, 1u, kPair ? 256u : 128u, kBN);
 
   struct Barriers {
     uint64_t full[kStages];
@@ -154,7 +181,7 @@ struct TcGemmF32x3 {
     const int bcol_base = static_cast<int>(rank) * BNL;  // this CTA's first B column inside the tile
 
     if (warp < 4) {
-      reg_dec<56>();
+      reg_dec<CTL_REGS>();
       if (warp == 0 && lane == 0) {
         // ---------------------------------------------------------- producer
         tma_prefetch_desc(&p.tmA);
@@ -200,7 +227,13 @@ struct TcGemmF32x3 {
         // whole warp, one elected lane per batch of instructions (see elect_one)
         const uint32_t tmem_base_u = __shfl_sync(0xffffffffu, tmem_base, 0);
         uint32_t it = 0, chunk_it = 0;
-        bool ok = true;
+        bool ok = true, ready = false;  // ready: block `it` has been waited for
+        // the lo twin is written after the hi stage has landed (in both CTAs of a pair)
+        auto wait_split = [&](uint32_t i) -> bool {
+          const bool got = mbar_wait_warp(&bars->split_full[i % LO_STAGES], (i / LO_STAGES) & 1u, &bars->abort_flag);
+          if (!got) report(p, bars, KCG_ST_TIMEOUT_MMA, i, i % kStages);
+          return got;
+        };
         Iter units(p, unit0, unit_stride, tiles_m, tiles_n, num_kb);
         Unit w;
         while (ok && units.next(w)) {
@@ -216,23 +249,26 @@ struct TcGemmF32x3 {
             const uint32_t tmem_acc = tmem_base_u + ab * ACC_COLS;
             const int kb1 = (kb0 + kChunk < w.kbn) ? kb0 + kChunk : w.kbn;
             for (int kb = kb0; kb < kb1; ++kb, ++it) {
+              if (!ready && !(ok = wait_split(it))) break;
+              ready = false;
+              tc_fence_after_sync();
               const uint32_t s = it % kStages;
               const uint32_t sl = it % LO_STAGES;
-              const uint32_t phl = (it / LO_STAGES) & 1u;
-              // the lo twin is written after the hi stage has landed (in both CTAs of a pair)
-              if (!mbar_wait_warp(&bars->split_full[sl], phl, &bars->abort_flag)) {
-                report(p, bars, KCG_ST_TIMEOUT_MMA, it, s);
-                ok = false;
-                break;
-              }
-              tc_fence_after_sync();
               const uint32_t sa = smem_u32(smem + s * STAGE_HI);
               const uint32_t sb = sa + L.a_bytes;
-              const uint32_t sa_lo = smem_u32(smem + LO_RING + sl * STAGE_HI);
-              const uint32_t sb_lo = sa_lo + L.a_bytes;
-              if (elect_one()) {
-#pragma unroll
-                for (int ks = 0; ks < KSTEPS; ++ks) {
+              const uint32_t sa_lo = smem_u32(smem + LO_RING + sl * LO_BYTES);
+              const uint32_t sb_lo = sa_lo + LO_A_BYTES;
+              const uint32_t ta = tmem_base_u + COL_A + it % (TA > 0 ? TA : 1) * 2 * kBK;
+              auto issue = [&](int ks) {  // the products of one K step
+                const uint32_t b_off = ks * UMMA_K * 128;
+                const uint32_t first = (kb > kb0 || ks > 0) ? 1u : 0u;
+                const uint64_t bdesc = make_smem_desc(sb + b_off, L.b_lbo, L.b_sbo, L.b_desc_swizzle);
+                const uint64_t bdesc_lo = make_smem_desc(sb_lo + b_off, L.b_lbo, L.b_sbo, L.b_desc_swizzle);
+                if constexpr (TA > 0) {
+                  umma_ts<true, NCTA>(tmem_acc, ta + kBK + ks * UMMA_K, bdesc, IDESC, first);
+                  umma_ts<true, NCTA>(tmem_acc, ta + ks * UMMA_K, bdesc_lo, IDESC, 1u);
+                  umma_ts<true, NCTA>(tmem_acc, ta + ks * UMMA_K, bdesc, IDESC, 1u);
+                } else {
                   uint32_t a_off;
                   if constexpr (kATrans) {
                     a_off = ks * UMMA_K * 128;
@@ -240,11 +276,6 @@ struct TcGemmF32x3 {
                     constexpr int swb = (kBK * 4 < 128) ? kBK * 4 : 128;
                     a_off = ((ks * 32) / swb) * L.a_box_bytes + ((ks * 32) % swb);
                   }
-                  const uint32_t b_off = ks * UMMA_K * 128;
-                  const uint32_t first = (kb > kb0 || ks > 0) ? 1u : 0u;
-                  const uint64_t bdesc = make_smem_desc(sb + b_off, L.b_lbo, L.b_sbo, L.b_desc_swizzle);
-                  const uint64_t bdesc_lo =
-                      make_smem_desc(sb_lo + b_off, L.b_lbo, L.b_sbo, L.b_desc_swizzle);
 #pragma unroll
                   for (int t = 0; t < MT; ++t) {
                     const uint32_t a_t = kATrans ? t * (128 / L.atom) * L.a_box_bytes
@@ -265,6 +296,18 @@ struct TcGemmF32x3 {
                     }
                   }
                 }
+              };
+              if (elect_one()) {
+#pragma unroll
+                for (int ks = 0; ks < KSTEPS - 1; ++ks) issue(ks);
+              }
+              __syncwarp();
+              // Is the next block there? Asked here, while the tensor pipe still has products to run, and not after the
+              // last of them: where loads and splitter keep ahead, the question costs the pipe nothing.
+              if (kb + 1 < w.kbn)
+                ready = mbar_test_warp(&bars->split_full[(it + 1) % LO_STAGES], ((it + 1) / LO_STAGES) & 1u);
+              if (elect_one()) {
+                issue(KSTEPS - 1);
                 // the hi stage, and with it the lo stage of this K block, is free in both CTAs
                 // once these MMAs retire
                 if constexpr (kPair) {
@@ -288,16 +331,18 @@ struct TcGemmF32x3 {
           }
         }
       }
-    } else if (warp < 8) {
+    } else if (warp < FIRST_ACC_WARP) {
       // --------------------------------------------------------------- splitter
-      reg_dec<56>();
-      const int stid = threadIdx.x - 128;
+      reg_dec<SPLIT_REGS>();
+      const int stid = threadIdx.x & 127;
+      const uint32_t turn = static_cast<uint32_t>(warp >> 2) - 1u;  // of this warpgroup among the K blocks
       uint32_t it = 0;
       bool ok = true;
       Iter units(p, unit0, unit_stride, tiles_m, tiles_n, num_kb);
       Unit w;
       while (ok && units.next(w)) {
         for (int kb = 0; kb < w.kbn; ++kb, ++it) {
+          if (it % SPLIT_WGS != turn) continue;
           const uint32_t s = it % kStages;
           const uint32_t ph = (it / kStages) & 1u;
           const uint32_t sl = it % LO_STAGES;
@@ -311,28 +356,65 @@ struct TcGemmF32x3 {
             got = mbar_wait(&bars->empty[prev % kStages], (prev / kStages) & 1u, &bars->abort_flag);
           }
           if (got) got = mbar_wait(&bars->full[s], ph, &bars->abort_flag);
+          got = __all_sync(0xffffffffu, got);
+          constexpr int FIRST = TA > 0 ? L.a_bytes : 0;  // the part of the stage that gets a twin in shared memory
+          constexpr int PER_THREAD = (STAGE_HI - FIRST) / 16 / NUM_SPLIT_THREADS;
+          constexpr int BATCH = PER_THREAD % 8 == 0 ? 8 : PER_THREAD % 6 == 0 ? 6 : PER_THREAD % 4 == 0 ? 4 : 1;
+          static_assert(PER_THREAD % BATCH == 0 && (STAGE_HI - FIRST) % (16 * NUM_SPLIT_THREADS) == 0, "whole batches");
+          if (got) {
+            const uint4* hi = reinterpret_cast<const uint4*>(smem + s * STAGE_HI + FIRST) + stid;
+            uint4* lo = reinterpret_cast<uint4*>(smem + LO_RING + sl * LO_BYTES) + stid;
+            // (a batch's loads are all in flight before its first store: the compiler may not move a load above a store)
+#pragma unroll
+            for (int b = 0; b < PER_THREAD; b += BATCH) {
+              uint4 x[BATCH];
+#pragma unroll
+              for (int u = 0; u < BATCH; ++u) x[u] = hi[(b + u) * NUM_SPLIT_THREADS];
+#pragma unroll
+              for (int u = 0; u < BATCH; ++u)
+                lo[(b + u) * NUM_SPLIT_THREADS] =
+                    make_uint4(lo_part(x[u].x), lo_part(x[u].y), lo_part(x[u].z), lo_part(x[u].w));
+            }
+            fence_proxy_async_smem();
+          }
+          if constexpr (TA > 0) {
+            uint32_t a[kBK];
+            if (got) load_a_row(smem + s * STAGE_HI, (warp & 3) * 32 + lane, a);
+            // TMEM block it % TA was last read by the MMAs of K block it - TA (as above, their stage's `empty`). The
+            // stores to tensor memory are made by whole warps, which therefore leave the loop as one.
+            if (got && TA < kStages && it >= static_cast<uint32_t>(TA)) {
+              const uint32_t prev = it - TA;
+              got = mbar_wait(&bars->empty[prev % kStages], (prev / kStages) & 1u, &bars->abort_flag);
+            }
+            got = __all_sync(0xffffffffu, got);
+            if (got) {
+              tc_fence_after_sync();
+              const uint32_t ta =
+                  tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + COL_A + (it % TA) * 2 * kBK;
+#pragma unroll
+              for (int k0 = 0; k0 < kBK; k0 += 16) {
+                uint32_t h[16], l[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                  h[i] = a[k0 + i];
+                  l[i] = lo_part(a[k0 + i]);
+                }
+                tmem_st_32x32b_x16(ta + k0, h);
+                tmem_st_32x32b_x16(ta + kBK + k0, l);
+              }
+              tmem_st_wait();
+              tc_fence_before_sync();
+            }
+          }
           if (!got) {
             if (lane == 0) report(p, bars, KCG_ST_TIMEOUT_SPLITTER, it, s);
             ok = false;
             break;
           }
-          const uint4* hi = reinterpret_cast<const uint4*>(smem + s * STAGE_HI);
-          uint4* lo = reinterpret_cast<uint4*>(smem + LO_RING + sl * STAGE_HI);
-#pragma unroll 4
-          for (int i = stid; i < STAGE_HI / 16; i += NUM_SPLIT_THREADS) {
-            const uint4 x = hi[i];
-            uint4 l;
-            l.x = lo_part(x.x);
-            l.y = lo_part(x.y);
-            l.z = lo_part(x.z);
-            l.w = lo_part(x.w);
-            lo[i] = l;
-          }
-          fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
             if constexpr (kPair) {
-              mbar_arrive_cluster(map_to_cta(smem_u32(&bars->split_full[sl]), 0u));
+              mbar_arrive_cluster_cta(map_to_cta(smem_u32(&bars->split_full[sl]), 0u));
             } else {
               mbar_arrive(&bars->split_full[sl]);
             }
@@ -341,11 +423,11 @@ struct TcGemmF32x3 {
       }
     } else {
       // --------------------------------------------------- accumulate + epilogue
-      reg_inc<200>();
+      reg_inc<ACC_REGS>();
       griddep_wait();  // C, the workspace and the counters may still be in use by the kernel before
       const int q = warp & 3;
-      const int half = (warp - 8) >> 2;
-      const int epi_tid = threadIdx.x - 256;
+      const int half = (warp - FIRST_ACC_WARP) >> 2;
+      const int epi_tid = threadIdx.x - 32 * FIRST_ACC_WARP;
       const int row_in_acc = q * 32 + lane;
       const int col_half0 = half * HALF_COLS;
       float* Cout = reinterpret_cast<float*>(p.C);
@@ -390,7 +472,7 @@ struct TcGemmF32x3 {
           __syncwarp();
           if (lane == 0) {
             if constexpr (kPair) {
-              mbar_arrive_cluster(map_to_cta(smem_u32(&bars->tmem_empty[ab]), 0u));
+              mbar_arrive_cluster_relaxed(map_to_cta(smem_u32(&bars->tmem_empty[ab]), 0u));  // ("read" is all it says)
             } else {
               mbar_arrive(&bars->tmem_empty[ab]);
             }
@@ -513,13 +595,37 @@ struct TcGemmF32x3 {
     }
   }
 
-  // tf32_rn(x - trunc_tf32(x)) on raw bits; the subtraction is exact in fp32.
+  // One thread's row of a landed A block.
+  __device__ static __forceinline__ void load_a_row(const uint8_t* a, int row, uint32_t (&x)[kBK]) {
+    if constexpr (kATrans) {
+      // boxes of 32 rows x kBK values of K, 128 bytes per value; 32-byte units XORed with K mod 4
+      const uint8_t* col = a + (row >> 5) * L.a_box_bytes + (row & 7) * 4;
+#pragma unroll
+      for (int k = 0; k < kBK; ++k)
+        x[k] = *reinterpret_cast<const uint32_t*>(col + k * 128 + ((((row >> 3) & 3) ^ (k & 3)) << 5));
+    } else {
+      // boxes of `swb` bytes of K x R rows; 16-byte units XORed with the row's number within the swizzle's repeat
+      constexpr int swb = (kBK * 4 < 128) ? kBK * 4 : 128;
+      const int flip = (row * swb / 128) & (swb / 16 - 1);
+#pragma unroll
+      for (int u = 0; u < kBK / 4; ++u) {
+        const uint8_t* line = a + (u * 16 / swb) * L.a_box_bytes + row * swb;
+        const uint4 v = *reinterpret_cast<const uint4*>(line + (((u % (swb / 16)) ^ flip) << 4));
+        x[4 * u] = v.x;
+        x[4 * u + 1] = v.y;
+        x[4 * u + 2] = v.z;
+        x[4 * u + 3] = v.w;
+      }
+    }
+  }
+
+  // tf32_rna(x - trunc_tf32(x)) on raw bits, in its upper 19 bits: half of the last bit kept is added and kind::tf32
+  // ignores the rest. The subtraction is exact in fp32; x * 0 turns the lo part of an infinite or NaN x into NaN (the
+  // integer sum would wrap). cvt.rna.tf32.f32 - same bits - takes 15 cycles per warp instruction.
   __device__ static __forceinline__ uint32_t lo_part(uint32_t xbits) {
     const float x = __uint_as_float(xbits);
     const float hi = __uint_as_float(xbits & 0xffffe000u);
-    uint32_t l;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(l) : "f"(x - hi));
-    return l;
+    return __float_as_uint(__fmaf_rn(x, 0.f, __uint_as_float(__float_as_uint(x - hi) + 0x1000u)));
   }
 };
 

@@ -104,6 +104,22 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
 
+// Has the phase completed? Asked once, without waiting, by a whole (converged) warp; the acquire of a true answer is a
+// wait's.
+__device__ __forceinline__ bool mbar_test_warp(uint64_t* bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred P;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, P;\n\t"
+      "}\n"
+      : "=r"(done)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return __all_sync(0xffffffffu, done != 0u);
+}
+
 // --------------------------------------------------------------------- fences
 // Generic-proxy writes to shared memory -> visible to the async proxy
 // (TMA stores, tcgen05.mma operand reads).
@@ -297,6 +313,58 @@ __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// registers -> TMEM: each thread of the warp writes consecutive 32-bit columns of its own lane (row)
+__device__ __forceinline__ void tmem_st_32x32b_x32(uint32_t taddr, const uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+      :
+      : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]),
+        "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]),
+        "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      :
+      : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// D[tmem] (+)= A[tmem] * B[smem]: A is read from tensor memory (lane = row; one 32-bit column = one fp32 value or two
+// consecutive 16-bit values of K), B through a shared-memory descriptor. Issued by ONE thread. kCtas = 2: the CTA-pair
+// form, each CTA's tensor memory holding its own 128 rows of A at the same columns.
+template <bool kTf32, int kCtas = 1>
+__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
+                                        uint32_t accumulate) {
+#define KCG_UMMA_TS(group, kind)                                                       \
+  asm volatile(                                                                        \
+      "{\n\t"                                                                          \
+      ".reg .pred p;\n\t"                                                              \
+      "setp.ne.b32 p, %4, 0;\n\t"                                                      \
+      "tcgen05.mma.cta_group::" group ".kind::" kind " [%0], [%1], %2, %3, p;\n\t"     \
+      "}\n"                                                                            \
+      :                                                                                \
+      : "r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)              \
+      : "memory")
+  if constexpr (kTf32 && kCtas == 2) {
+    KCG_UMMA_TS("2", "tf32");
+  } else if constexpr (kTf32) {
+    KCG_UMMA_TS("1", "tf32");
+  } else if constexpr (kCtas == 2) {
+    KCG_UMMA_TS("2", "f16");
+  } else {
+    KCG_UMMA_TS("1", "f16");
+  }
+#undef KCG_UMMA_TS
+}
+
 }  // namespace kcg
 
 // ===================================================================== CTA pairs
@@ -346,6 +414,13 @@ __device__ __forceinline__ void named_bar_arrive(uint32_t id, uint32_t nthreads)
 __device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr)
                : "memory");
+}
+// Arrival on a barrier of the CTA that issues a pair's products, behind writes to THIS CTA's own shared or tensor memory
+// which those products read here: the writer has put them in order for the tensor core (proxy fence, tcgen05.wait::st)
+// before this, so release at CTA scope, the instruction's default, is enough. (Release at cluster scope waits for the
+// thread's memory traffic: 950 cycles behind a K block of the 3xTF32 splitter, against 30.)
+__device__ __forceinline__ void mbar_arrive_cluster_cta(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // Arrive on an mbarrier that lives in another CTA of the cluster.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {

@@ -104,17 +104,19 @@ def _cheapest_tile(M, N, K, batch=1, single_pass=False):
 
 
 # Tiles of the 3xTF32 kernels the rule below chooses from: (KERNEL_VARIANT, BLOCK_SIZE_M, N, K) -> (microseconds
-# {fixed, per 1000 values of K, per tile beyond them, per cut into K ranges}, stages). Fitted to 170 device timings
-# (graph replay, rotating operands) on 18 shapes of 128..6784 x 512..11008 x 256..8704, plain and with every tile cut
-# into 2 to 8 ranges: the tile the fit picks is 4 % behind the best measured one on average (the former rule, tiles that
-# divide the problem and the widest first, 22 %: 256x1024x256 18.4 -> 9.3 us, 256x2048x512 28.5 -> 14.8,
-# 384x3520x8128 197 -> 128, 6272x640x6144 325 -> 254 us).
+# {fixed, per 1000 values of K, per tile beyond them, per cut into K ranges}, stages). Fitted to 180 device timings
+# (graph replay, rotating operands) on 18 shapes of 128..6272 x 512..11008 x 256..11008, plain and with every tile cut
+# into 2 to 8 ranges: the tile the fit picks is 2.5 % behind the best measured one on average. The pair tiles of 128 and
+# 192 columns, whose A goes through tensor memory, are ahead on the middling shapes (640x2624x1024 25 us against 31 with
+# the best of the others, 896x1536x6144 80 / 83, 6272x640x6144 223 / 281 with 256 columns), 128 rows by 256 columns on
+# few rows and long K (128x11008x11008 170 / 226), 256 by 256 on the largest (4096^3 509 / 552 with 192 columns).
 _TILE_COST_F32 = {
-    (2, 128, 64, 32): (2.63, 20.3, 1.94, 3.38, 4),
-    (2, 128, 128, 32): (3.25, 26.8, 3.85, 4.13, 3),
-    (2, 128, 256, 16): (2.74, 39.3, 9.36, 6.83, 4),
-    (4, 256, 128, 32): (2.80, 37.0, 3.05, 5.59, 4),
-    (4, 256, 256, 32): (1.98, 38.2, 10.80, 6.81, 3),
+    (2, 128, 64, 32): (2.88, 17.2, 1.44, 4.62, 6),
+    (2, 128, 128, 32): (2.46, 20.2, 3.48, 6.14, 4),
+    (2, 128, 256, 16): (1.65, 40.0, 7.11, 12.14, 4),
+    (4, 256, 128, 32): (2.48, 17.3, 3.49, 6.43, 6),
+    (4, 256, 192, 32): (2.32, 21.4, 6.75, 7.64, 5),
+    (4, 256, 256, 32): (1.55, 30.4, 7.85, 10.70, 3),
 }
 
 
