@@ -494,11 +494,12 @@ int resolve(const Cfg& c, const kcg_compile_opts* opts, Resolved* r) {
     if (N % 8) return fail(KCG_E_BAD_CONFIG, "N must be a multiple of 8 for TMA row strides");
     r->stages = st;
   } else if (want == KCG_KERNEL_TCGEN05_CLUSTERK) {
-    // one 128-row tile per cluster of LOCAL_SPLIT_U CTAs, partial tiles reduced in shared memory
-    const int split = c[KCG_CFG_LOCAL_SPLIT_U];
-    if (bm != 128) return fail(KCG_E_BAD_CONFIG, "the cluster split-K kernel needs BLOCK_SIZE_M = 128");
+    // one 128-row tile per cluster of LOCAL_SPLIT_U CTAs (256 rows: CTA pairs), partial tiles reduced in shared memory
+    const int split = c[KCG_CFG_LOCAL_SPLIT_U], ck_pair = bm == 256 ? 1 : 0;
+    if (bm != 128 && !(ck_pair && split == 2))
+      return fail(KCG_E_BAD_CONFIG, "the cluster split-K kernel needs BLOCK_SIZE_M = 128, or 256 with LOCAL_SPLIT_U = 2");
     if (split > blocks_of(K, bk)) return fail(KCG_E_BAD_CONFIG, "LOCAL_SPLIT_U %d exceeds the %d K blocks", split, blocks_of(K, bk));
-    auto ok = [&](int st) { return kcg::ck_config_error(dt, bn, bk, st, split) == 0; };
+    auto ok = [&](int st) { return kcg::ck_config_error(dt, bn, bk, st, split, ck_pair) == 0; };
     int st = (opts && opts->num_stages > 0) ? opts->num_stages : 2;
     if (!(opts && opts->num_stages > 0)) {
       while (st < 8 && !ok(st)) ++st;                                   // the ring must hold the received slices
@@ -506,9 +507,9 @@ int resolve(const Cfg& c, const kcg_compile_opts* opts, Resolved* r) {
     }
     if (!ok(st))
       return fail(KCG_E_BAD_CONFIG,
-                  "tile 128x%dx%d / %d stages / LOCAL_SPLIT_U %d not buildable by the cluster split-K kernel (rule %d: "
+                  "tile %dx%dx%d / %d stages / LOCAL_SPLIT_U %d not buildable by the cluster split-K kernel (rule %d: "
                   "fp16 / bf16, split 2..4 and at most BLOCK_SIZE_N / 32, ring large enough for the exchange buffers)",
-                  bn, bk, st, split, kcg::ck_config_error(dt, bn, bk, st, split));
+                  bm, bn, bk, st, split, kcg::ck_config_error(dt, bn, bk, st, split, ck_pair));
     if (N % 8) return fail(KCG_E_BAD_CONFIG, "N must be a multiple of 8 for TMA row strides");
     r->stages = st;
   } else if (want == KCG_KERNEL_SIMT) {
@@ -762,10 +763,10 @@ int fill_info(const Cfg& c, const Resolved& r, const std::string& name, const st
     out->block[0] = f32 ? kcg::tc_x3_threads(kcg::tc_x3_tmem_a(bm / 2, bn / 2, bk, r.stages, 2), 2) : 256;
     out->smem_bytes = kcg::tc_smem_bytes(c[KCG_CFG_DATATYPE_A], bm / 2, bn / 2, bk, r.stages, 2 * f32);
   } else if (r.kernel == KCG_KERNEL_TCGEN05_CLUSTERK) {
-    out->grid[0] = tiles * lsu;  // one cluster of LOCAL_SPLIT_U CTAs per tile
-    out->cluster[0] = lsu;
+    out->grid[0] = tiles * lsu * (bm / 128);  // one cluster of LOCAL_SPLIT_U CTAs (CTA pairs) per tile
+    out->cluster[0] = lsu * (bm / 128);
     out->block[0] = 192;  // producer, MMA, four epilogue warps
-    out->smem_bytes = kcg::ck_smem_bytes(bn, bk, r.stages);
+    out->smem_bytes = kcg::ck_smem_bytes(bn, bk, r.stages, bm == 256 ? 1 : 0);
   } else if (r.kernel == KCG_KERNEL_SIMT) {
     // grid/block as the reference derives them (Optimizer.cc:20,336; Rewriter.cc:726-761)
     out->grid[0] = tiles;
@@ -1304,9 +1305,10 @@ static int launch_impl(uint64_t function, const kcg_kernel_info* info, int devic
   };
   if (info->kernel == KCG_KERNEL_TCGEN05_CLUSTERK) {
     // One cluster per tile; the K split and its reduction stay inside the cluster (no workspace).
-    if (int e = encode_operands(kcg::make_tc_layout(info->dtype, info->bm, info->bn, info->bk, info->atrans, btrans)))
+    const int ctas = info->bm / 128;  // that share a K range, each loading 128 rows of A and as large a part of B
+    if (int e = encode_operands(kcg::make_tc_layout(info->dtype, 128, info->bn / ctas, info->bk, info->atrans, btrans)))
       return e;
-    grid0 = blocks_of(M, info->bm) * blocks_of(N, info->bn) * info->splitk;
+    grid0 = blocks_of(M, info->bm) * blocks_of(N, info->bn) * info->splitk * ctas;
   }
   if (info->kernel == KCG_KERNEL_TCGEN05 || info->kernel == KCG_KERNEL_TF32X1 || pair) {
     // the pair kernel loads per-CTA slices: BM/2 rows of A, BN/2 columns of B

@@ -75,7 +75,7 @@ KCG_KERNEL_NAME(const __grid_constant__ KcgGemmParams p) {
 }
 #elif KCG_VARIANT == KCG_VARIANT_TCGEN05_CLUSTERK
 #include "gemm_tcgen05_clusterk.cuh"
-using Gemm = kcg::TcGemmClusterK<KCG_DTYPE, KCG_BN, KCG_BK, KCG_STAGES, KCG_ATRANS, KCG_SPLITK, KCG_GROUP, KCG_BTRANS>;
+using Gemm = kcg::TcGemmClusterK<KCG_DTYPE, KCG_BN, KCG_BK, KCG_STAGES, KCG_ATRANS, KCG_SPLITK, KCG_GROUP, KCG_BTRANS, (KCG_BM == 256)>;
 extern "C" __global__ void __launch_bounds__(Gemm::NUM_THREADS, 1)
 KCG_KERNEL_NAME(const __grid_constant__ KcgGemmParams p) {
   Gemm::run(p);

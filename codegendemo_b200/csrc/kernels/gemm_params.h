@@ -237,22 +237,24 @@ constexpr int tc_config_error(int dtype, int BM, int BN, int BK, int stages, int
 // Cluster split-K kernel (gemm_tcgen05_clusterk.cuh): a 128 x BN tile per cluster of `split` CTAs.
 // The operand ring doubles as the exchange buffers of the reduction (a staging copy of the fp32
 // accumulator, 128 x BN x 4 bytes, plus a receive slot per other CTA), so it must be at least that
-// large; no TMA-store staging.
-constexpr int ck_config_error(int dtype, int BN, int BK, int stages, int split) {
+// large; no TMA-store staging. `pair`: a 256 x BN tile per cluster of 2 * split CTAs, each loading half of B's columns;
+// clusters of more than four such CTAs do not run side by side on enough of the GPU.
+constexpr int ck_ring_bytes(int BN, int BK, int stages, int pair) { return (128 + BN / (pair ? 2 : 1)) * BK * 2 * stages; }
+constexpr int ck_config_error(int dtype, int BN, int BK, int stages, int split, int pair = 0) {
   if (!(dtype == KCG_DT_F16 || dtype == KCG_DT_BF16)) return 1;
-  if (split < 2 || split > 4) return 2;  // larger clusters do not fit the exchange buffers (nor the GPU: few run at once)
-  if (BN < 64 || BN > 256 || (BN % 64) != 0 || BN / 32 < split) return 3;
+  if (split < 2 || split > (pair ? 2 : 4)) return 2;  // larger clusters do not fit the exchange buffers (nor the GPU: few run at once)
+  if (BN < 64 || BN > 256 || (BN % (pair ? 128 : 64)) != 0 || BN / 32 < split) return 3;
   const int rowb = BK * 2;
   if (!(rowb == 32 || rowb == 64 || (rowb % 128) == 0) || rowb > 512 || (BK % 16) != 0) return 5;
   if (stages < 2 || stages > 12) return 7;
-  const int ring = (128 + BN) * BK * 2 * stages;
+  const int ring = ck_ring_bytes(BN, BK, stages, pair);
   if (ring + 2048 > 227 * 1024) return 8;
   // the ring doubles as exchange buffers: a receive slot per other CTA plus a staging copy of the accumulator
   // of the blocks that belong to other CTAs
   if (ring < ((split - 1) * ((BN / 32 + split - 1) / split) + (BN / 32 - BN / 32 / split)) * 128 * 128) return 10;
   return 0;
 }
-constexpr int ck_smem_bytes(int BN, int BK, int stages) { return (128 + BN) * BK * 2 * stages + 2048; }
+constexpr int ck_smem_bytes(int BN, int BK, int stages, int pair = 0) { return ck_ring_bytes(BN, BK, stages, pair) + 2048; }
 
 constexpr int tc_smem_bytes(int dtype, int BM, int BN, int BK, int stages, int x3) {
   // +1024 alignment slack, +1024 barriers / TMEM holder / flags, + epilogue staging

@@ -1,7 +1,7 @@
 // Split-K GEMM on thread-block clusters for problems with few output tiles (skinny M):
 // C[M,N] = A[M,K] * B[K,N], fp16 / bf16, fp32 accumulation.
 //
-// A cluster of kSplit CTAs owns ONE 128 x kBN output tile. CTA r of the cluster multiplies the
+// A cluster of kSplit CTAs (or CTA pairs, see kPair) owns ONE 128 x kBN output tile. CTA r of the cluster multiplies the
 // r-th of kSplit equal K ranges with the usual pipeline (warp 0 TMA producer, warp 1 tcgen05.mma
 // issuer, fp32 accumulator in TMEM), so kSplit times as many SMs stream B as there are tiles.
 // The partial tiles never touch global memory: the tile's columns are cut into kSplit slices
@@ -41,12 +41,21 @@
 namespace kcg {
 
 // kBTrans = 1: B stored N x K, as in gemm_tcgen05.cuh.
-template <int kDType, int kBN, int kBK, int kStages, int kATrans, int kSplit, int kGroup, int kBTrans = 0>
+//
+// kPair = 1 puts a CTA pair (cta_group::2, as in gemm_tcgen05.cuh) in the place of each CTA: a 256 x kBN tile per cluster
+// of 2 * kSplit CTAs, ranks 2 r and 2 r + 1 multiplying the r-th K range with half of the rows and half of the B tile
+// each. Everything behind the products - exchange, adding, storing - happens among the CTAs that hold the same rows. A
+// CTA then loads 128 + kBN / 2 rows of operands instead of 128 + kBN for the same products, and a cycle of the tensor
+// pipe takes 160 bytes through the shared-memory port instead of 192 (128 x 256 a CTA): 512 x 4096 x 11008 41.3 -> 36.4 us.
+template <int kDType, int kBN, int kBK, int kStages, int kATrans, int kSplit, int kGroup, int kBTrans = 0, int kPair = 0>
 struct TcGemmClusterK {
-  static constexpr int kBM = 128;
-  static_assert(ck_config_error(kDType, kBN, kBK, kStages, kSplit) == 0,
+  static constexpr int NCTA = kPair ? 2 : 1;  // CTAs that share a K range
+  static constexpr int R = 128;               // rows of the tile held by one CTA
+  static constexpr int kBM = R * NCTA;
+  static constexpr int BNL = kBN / NCTA;      // B columns loaded by one CTA
+  static_assert(ck_config_error(kDType, kBN, kBK, kStages, kSplit, kPair) == 0,
                 "config not buildable by the cluster split-K kernel");
-  static constexpr TcLayout L = make_tc_layout(kDType, kBM, kBN, kBK, kATrans, kBTrans);
+  static constexpr TcLayout L = make_tc_layout(kDType, R, BNL, kBK, kATrans, kBTrans);
   static constexpr int EB = 2;
   static constexpr int UMMA_K = 16;
   static constexpr int KSTEPS = kBK / UMMA_K;
@@ -65,16 +74,17 @@ struct TcGemmClusterK {
   __host__ __device__ static constexpr int first_block_of(int r) { return (r * NCH + kSplit - 1) / kSplit; }
   static constexpr int NUM_EPI_THREADS = 128;
   static constexpr int NUM_THREADS = 64 + NUM_EPI_THREADS;
-  static constexpr int SMEM_BYTES = ck_smem_bytes(kBN, kBK, kStages);
+  static constexpr int SMEM_BYTES = ck_smem_bytes(kBN, kBK, kStages, kPair);
   static_assert(RECV_BYTES + STAGE_OUT_BYTES <= kStages * STAGE_BYTES, "the ring must hold the exchange buffers");
   static constexpr uint32_t FMT = (kDType == KCG_DT_BF16) ? FMT_BF16 : FMT_F16;
-  static constexpr uint32_t IDESC = make_instr_desc(FMT, kATrans ? 1u : 0u, kBTrans ? 0u : 1u, 128u, kBN);
+  static constexpr uint32_t IDESC =
+      make_instr_desc(FMT, kATrans ? 1u : 0u, kBTrans ? 0u : 1u, static_cast<uint32_t>(kBM), kBN);
 
   struct Barriers {
     uint64_t full[kStages];
     uint64_t empty[kStages];
     uint64_t tmem_full;
-    uint64_t ring_free[4];  // [r]: CTA r of the cluster no longer touches its operand ring
+    uint64_t ring_free[4];  // [r]: the CTA with K range r (and this one's rows) no longer touches its operand ring
     uint64_t recv_full;     // all slices for this CTA have arrived (transaction bytes of the bulk copies)
     uint64_t staged[8];     // [f]: the four epilogue warps have laid down the f-th block that leaves this CTA
     uint32_t tmem_base;
@@ -134,16 +144,19 @@ struct TcGemmClusterK {
       fence_proxy_async_smem();
       // what the other CTAs will copy in: (kSplit - 1) senders x this CTA's blocks x 16 KB. Posted now;
       // a copy that lands before this CTA looks is simply counted.
-      const int r_me = static_cast<int>(cluster_cta_rank());
+      const int r_me = static_cast<int>(cluster_cta_rank()) / NCTA;
       const int nb_me = first_block_of(r_me + 1) - first_block_of(r_me);
       mbar_expect_tx(&bars->recv_full, static_cast<uint32_t>((kSplit - 1) * nb_me * BLOCK_BYTES));
     }
-    const uint32_t rank = cluster_cta_rank();
+    const uint32_t cta = cluster_cta_rank();
+    const uint32_t rank = cta / NCTA;  // of the K range
+    const uint32_t half = cta % NCTA;  // which rows of the tile; 0 issues a pair's products
+    auto cta_of = [&](uint32_t r) { return r * NCTA + half; };  // the CTA with K range r and the same rows
     // This cluster's tile and this CTA's K range. The raster (and a batched launch's offsets) come
     // from the iterator the other tcgen05 kernels use.
     WorkIter<kBM, kBN, kGroup, KCG_SERPENTINE> raster(p, 0, 1, tiles_m, tiles_n, num_kb);
     WorkUnit w;
-    w.tile = static_cast<int>(blockIdx.x) / kSplit;
+    w.tile = static_cast<int>(blockIdx.x) / (kSplit * NCTA);
     raster.origin(w);
     const int per = (num_kb + kSplit - 1) / kSplit;
     const int kb0 = static_cast<int>(rank) * per;
@@ -179,14 +192,19 @@ struct TcGemmClusterK {
         const uint32_t slot = rank < owner ? rank : rank - 1u;  // senders in rank order, the owner left out
         const int o_first = first_block_of(static_cast<int>(owner));
         const uint32_t dst_local = smem_u32(smem) + slot * SLICE_BYTES + (c - o_first) * BLOCK_BYTES;
-        bulk_copy_to_cta(map_to_cta(dst_local, owner), smem_u32(staged_at(c)), BLOCK_BYTES,
-                         map_to_cta(smem_u32(&bars->recv_full), owner));
+        bulk_copy_to_cta(map_to_cta(dst_local, cta_of(owner)), smem_u32(staged_at(c)), BLOCK_BYTES,
+                         map_to_cta(smem_u32(&bars->recv_full), cta_of(owner)));
       }
     };
 
     if (warp == 1) {
-      tmem_alloc(&bars->tmem_base, TMEM_COLS);
-      tmem_relinquish();
+      if constexpr (kPair) {
+        tmem_alloc_pair(&bars->tmem_base, TMEM_COLS);
+        tmem_relinquish_pair();
+      } else {
+        tmem_alloc(&bars->tmem_base, TMEM_COLS);
+        tmem_relinquish();
+      }
     }
     // Set-up meeting on named barrier 3. Warp 0 needs nothing from the others (thread 0 initialised the
     // barriers itself, and its loads signal only those), so it merely arrives and starts loading at
@@ -203,7 +221,12 @@ struct TcGemmClusterK {
     // the exchange: arrive on the cluster barrier now (thread 0's fence.mbarrier_init has published the
     // fresh barriers, so the arrival itself needs no ordering), wait for it only there (cluster_wait
     // below), and keep the main loop free of the cluster's start-up skew.
+    // (A pair's loads are counted on the leader's barriers from the first one on: it waits here.)
     cluster_arrive_relaxed();
+    auto others_set_up = [&] {
+      if constexpr (!kPair) cluster_wait();
+    };
+    if constexpr (kPair) cluster_wait();
     const uint32_t tmem_base = (warp == 0) ? 0u : bars->tmem_base;
     if (threadIdx.x == 32) KCG_CTL(1);
 
@@ -221,23 +244,33 @@ struct TcGemmClusterK {
           uint8_t* sa = smem + s * STAGE_BYTES;
           uint8_t* sb = sa + L.a_bytes;
           const int k0 = (kb0 + kb) * kBK;
-          const int am0 = kATrans ? w.mcol : w.m0;
+          const int am0 = (kATrans ? w.mcol : w.m0) + static_cast<int>(half) * R;
+          const int bn0 = w.n0 + static_cast<int>(half) * BNL;
           const int ka = kATrans ? k0 + w.kofs : k0, kb_row = k0 + w.kofs;
-          mbar_expect_tx(&bars->full[s], static_cast<uint32_t>(STAGE_BYTES));
+          // completion bytes of both CTAs of a pair land on the leader's barrier
+          const uint32_t full_leader = kPair ? map_to_cta(smem_u32(&bars->full[s]), cta - half) : 0u;
+          auto load = [&](void* dst, const CUtensorMap* tm, int c0, int c1) {
+            if constexpr (kPair) {
+              tma_load_2d_pair(dst, tm, full_leader, c0, c1);
+            } else {
+              tma_load_2d(dst, tm, &bars->full[s], c0, c1);
+            }
+          };
+          if (half == 0u) mbar_expect_tx(&bars->full[s], static_cast<uint32_t>(NCTA * STAGE_BYTES));
 #pragma unroll
           for (int j = 0; j < L.a_boxes; ++j) {
             if constexpr (kATrans) {
-              tma_load_2d(sa + j * L.a_box_bytes, &p.tmA, &bars->full[s], am0 + j * L.atom, ka);
+              load(sa + j * L.a_box_bytes, &p.tmA, am0 + j * L.atom, ka);
             } else {
-              tma_load_2d(sa + j * L.a_box_bytes, &p.tmA, &bars->full[s], ka + j * L.a_box_inner, am0);
+              load(sa + j * L.a_box_bytes, &p.tmA, ka + j * L.a_box_inner, am0);
             }
           }
 #pragma unroll
           for (int j = 0; j < L.b_boxes; ++j) {
             if constexpr (kBTrans) {  // N x K storage: the batch selects N rows
-              tma_load_2d(sb + j * L.b_box_bytes, &p.tmB, &bars->full[s], k0 + j * L.b_box_inner, w.n0 + w.nofs);
+              load(sb + j * L.b_box_bytes, &p.tmB, k0 + j * L.b_box_inner, bn0 + w.nofs);
             } else {
-              tma_load_2d(sb + j * L.b_box_bytes, &p.tmB, &bars->full[s], w.n0 + j * L.atom, kb_row);
+              load(sb + j * L.b_box_bytes, &p.tmB, bn0 + j * L.atom, kb_row);
             }
           }
           if (kb == 0) KCG_CTL(2);
@@ -245,7 +278,7 @@ struct TcGemmClusterK {
       }
       __syncwarp();
       if (lane == 0) griddep_launch_dependents();  // every load is issued: the stream's next kernel may be brought in
-      cluster_wait();  // set-up phase of the cluster barrier: the other CTAs' barriers exist
+      others_set_up();  // set-up phase of the cluster barrier: the other CTAs' barriers exist
       if (lane == 0) {
         ship(0);
         KCG_CTL(5);
@@ -253,11 +286,19 @@ struct TcGemmClusterK {
       __syncwarp();
       cluster_arrive_relaxed();  // second phase (see the epilogue warps)
     } else if (warp == 1) {
-      // ---------------------------------------------------------- MMA issuer
-      {
+      // ---------------------------------------------------------- MMA issuer (in a pair: the leader CTA only)
+      if (half == 0u) {
         // whole warp, one elected lane per batch of instructions (see elect_one)
         const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
         bool ok = true;
+        auto commit = [&](uint64_t* bar) {  // the products issued so far -> this barrier (of both CTAs of a pair)
+          if constexpr (kPair) {
+            umma_commit_pair(smem_u32(bar));
+            umma_commit_pair(map_to_cta(smem_u32(bar), cta + 1u));
+          } else {
+            umma_commit(bar);
+          }
+        };
         for (int kb = 0; kb < kbn; ++kb) {
           const uint32_t s = kb % kStages;
           const uint32_t ph = (kb / kStages) & 1u;
@@ -288,17 +329,21 @@ struct TcGemmClusterK {
               }
               const uint64_t adesc = make_smem_desc(sa + a_off, L.a_lbo, L.a_sbo, L.a_desc_swizzle);
               const uint64_t bdesc = make_smem_desc(sb + b_off, L.b_lbo, L.b_sbo, L.b_desc_swizzle);
-              umma_ss<false>(tmem_u, adesc, bdesc, IDESC, (kb > 0 || ks > 0) ? 1u : 0u);
+              if constexpr (kPair) {
+                umma_ss_pair<false>(tmem_u, adesc, bdesc, IDESC, (kb > 0 || ks > 0) ? 1u : 0u);
+              } else {
+                umma_ss<false>(tmem_u, adesc, bdesc, IDESC, (kb > 0 || ks > 0) ? 1u : 0u);
+              }
             }
-            umma_commit(&bars->empty[s]);
+            commit(&bars->empty[s]);
           }
           __syncwarp();
         }
         KCG_CTL(3);
-        if (ok && kbn > 0 && elect_one()) umma_commit(&bars->tmem_full);
+        if (ok && kbn > 0 && elect_one()) commit(&bars->tmem_full);
       }
       __syncwarp();
-      cluster_wait();
+      others_set_up();
       if (lane == 0) {
         ship(1);
         KCG_CTL(12);
@@ -316,7 +361,7 @@ struct TcGemmClusterK {
       // the four warps take every branch below together (named barrier 2 ANDs their outcomes)
       const bool have_acc = named_bar_all(2, NUM_EPI_THREADS, ok);
       if (!have_acc && !ok) report(p, bars, KCG_ST_TIMEOUT_EPILOGUE, 0u, rank);
-      cluster_wait();  // the other CTAs' barriers are initialised (all four warps, every lane)
+      others_set_up();  // the other CTAs' barriers are initialised (all four warps, every lane)
       bool all_in = false;
       if (have_acc) {
         tc_fence_after_sync();
@@ -324,7 +369,8 @@ struct TcGemmClusterK {
         // This CTA's MMAs have retired (or it had none): its ring is free to receive slices. One lane per
         // CTA of the cluster tells it so.
         if (epi_tid < kSplit)
-          mbar_arrive_cluster_relaxed(map_to_cta(smem_u32(&bars->ring_free[rank]), static_cast<uint32_t>(epi_tid)));
+          mbar_arrive_cluster_relaxed(
+              map_to_cta(smem_u32(&bars->ring_free[rank]), cta_of(static_cast<uint32_t>(epi_tid))));
         if (epi_tid == 0) KCG_CTL(9);
         const uint32_t tmem_acc = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
         // ---- stage: the blocks that belong to other CTAs are laid down in this CTA's (idle) ring in the
@@ -381,7 +427,7 @@ struct TcGemmClusterK {
           OutT* Cout = reinterpret_cast<OutT*>(p.C);
           const int c_first = first_block_of(static_cast<int>(rank));
           const int c_end = first_block_of(static_cast<int>(rank) + 1);
-          const int grow = w.m0 + row;
+          const int grow = w.m0 + static_cast<int>(half) * R + row;
 #pragma unroll 1
           for (int c = c_first; c < c_end; ++c) {
             const int cbi = c - c_first;
@@ -457,7 +503,11 @@ struct TcGemmClusterK {
     if (warp == 1) {
       __syncwarp();
       tc_fence_after_sync();
-      tmem_dealloc(tmem_base, TMEM_COLS);
+      if constexpr (kPair) {
+        tmem_dealloc_pair(tmem_base, TMEM_COLS);
+      } else {
+        tmem_dealloc(tmem_base, TMEM_COLS);
+      }
       if (lane == 0) KCG_CTL(8);
     }
 #ifdef KCG_TIMELINE

@@ -144,7 +144,8 @@ class KernelArgMatmul:
             assert (self.BLOCK_LAYOUT_N * self.WARP_LAYOUT_N) == (self.BLOCK_SIZE_N // self.THREAD_SIZE_N)
             assert self.WARP_LAYOUT_N * self.WARP_LAYOUT_M == self.WARP_SIZE
         # shm size check
-        per_cta = 2 if self.KERNEL_VARIANT == 4 else 1  # a CTA pair splits the tile's operands
+        # a CTA pair splits the tile's operands
+        per_cta = 2 if self.KERNEL_VARIANT == 4 or self.KERNEL_VARIANT == 5 and self.BLOCK_SIZE_M == 256 else 1
         assert 2 * (self.BLOCK_SIZE_M + self.BLOCK_SIZE_N) * self.BLOCK_SIZE_K * sizeof(self.__dataType_A) // per_cta \
             <= MAX_SHARED_BYTES
         if verbose:

@@ -42,7 +42,10 @@ def default_config(M: int, N: int, K: int, dtype: EnumKernelDType, out_dtype=Non
 # shapes the tile the fit picks is within 1 % of the best measured one on average (worst 10 %), where the former
 # rule - tiles had to divide the problem - averaged 22 % behind it (1664 x 2752 x 1472: 33 -> 12.9 us;
 # 11136 x 7488 x 1792: 608 -> 205 us; 128 x 1344 x 3072: 17.3 -> 7.7 us). For the cluster split-K kernel the third
-# figure is one per LOCAL_SPLIT_U of 2, 3, 4.
+# figure is one per LOCAL_SPLIT_U of 2, 3, 4; its 256-row tiles run on CTA pairs, two K ranges only (12 shapes; against the
+# best 128-row choice 512 x 4096 x 11008 41.3 -> 36.4 us, 1024 x 2048 x 8192 29.5 -> 27.5, 256 x 4096 x 4096 14.9 -> 13.0,
+# 640 x 1280 x 2560 10.2 -> 9.6; behind it where K is short, 512 x 1024 x 1024 5.4 / 5.8, or most SMs idle, 256 x 2048 x
+# 16384 23 / 30).
 _TILE_COST = {
     (2, 128, 64, 128): (2.85, 0.433, 0.54),
     (2, 128, 128, 128): (2.94, 0.499, 0.53),
@@ -61,6 +64,8 @@ _TILE_COST = {
 }
 # clusters of 2, 3, 4 CTAs at 200 KB of shared memory each that run at once on the GPU the table is fitted to (148 SMs)
 _CLUSTERS = {2: 74, 3: 45, 4: 33}
+    (5, 256, 128, 128): (1.0, 0.56, (3.20,)),
+    (5, 256, 256, 64): (1.0, 0.35, (5.20,)),
 
 
 def _tile_us(tile, split, M, N, K, batch=1, sms=148):
@@ -95,7 +100,7 @@ def _cheapest_tile(M, N, K, batch=1, single_pass=False):
             continue
         for split in (2, 3, 4) if variant == 5 else (1,):
             if variant == 5 and (split > len(_TILE_COST[tile][2]) + 1 or -(-K // bk) < 2 * split or
-                                 batch * -(-M // bm) * -(-N // bn) > _CLUSTERS[split]):
+                                 batch * -(-M // bm) * -(-N // bn) > _CLUSTERS[split * bm // 128]):
                 continue
             us = _tile_us(tile, split, M, N, K, batch)
             if best is None or us < best[0]:
@@ -154,7 +159,8 @@ def tuned_config(M: int, N: int, K: int, dtype: EnumKernelDType, isATranspose: i
                  b_transposed: bool = False, single_pass: bool = False) -> KernelArgMatmul:
     """Best known config of a shape: the kernel database's entry when the shape was tuned; else (16-bit types, and
     single fp32 products) the tile with the smallest estimated time - the plain rule's choice is kept while the estimate
-    puts it within 10 % of that: the estimates of the two largest tiles are up to that much too low where a remainder is
+    puts it within 10 % of that (5 % for a cluster split-K tile: 512x4096x11008 39.4 estimated against 36.3 with the best
+    tile, 41.3 and 36.4 measured): the estimates of the two largest tiles are up to that much too low where a remainder is
     cut up (2048x11008x4096: 512x256x64 estimated 110, 256x256x128 118 us; measured 142 and 135, and 165 and 148 once the
     power cap holds the clock down). ``batch`` > 1: M, N, K are one batch's, the config fits all batches' tiles walked
     together, and the database, which holds single products, is not asked. ``b_transposed``: B is stored N x K.
@@ -179,7 +185,7 @@ def tuned_config(M: int, N: int, K: int, dtype: EnumKernelDType, isATranspose: i
         us, tile, split = _cheapest_tile(M, N, K, batch, single_pass)
         have = (plain.KERNEL_VARIANT or 2, plain.BLOCK_SIZE_M, plain.BLOCK_SIZE_N, plain.BLOCK_SIZE_K)
         if have not in _TILE_COST or single_pass and have[0] == 5 or \
-                _tile_us(have, plain.LOCAL_SPLIT_U, M, N, K, batch) > 1.1 * us:
+                _tile_us(have, plain.LOCAL_SPLIT_U, M, N, K, batch) > (1.05 if have[0] == 5 else 1.1) * us:
             variant, bm, bn, bk = tile
             stages = dict(NUM_STAGES=4) if bm == 512 else {}
             plain = default_config(M, N, K, dtype, KERNEL_VARIANT=variant, BLOCK_SIZE_M=bm, BLOCK_SIZE_N=bn,
