@@ -4,7 +4,8 @@
     python -m codegendemo_b200.build --lib-only
 
 The library is built with nvcc for sm_100a: its host code binds the CUDA driver lazily (so it loads without a GPU),
-and two pieces of device code are linked into it (the allocation-free split-K entry and the row softmax). The GEMM
+and pieces of device code are linked into it (the allocation-free split-K entry, the row softmax, the fused attention).
+Beside it stands ``_pycall.so``, a small extension module that launches on behalf of Python callers. The GEMM
 kernels themselves are compiled per config by the library's own compile entry with
 ``nvcc -cubin -gencode arch=compute_100a,code=sm_100a``.
 """
@@ -23,7 +24,19 @@ def _newer(target: str, sources) -> bool:
     return all(os.path.getmtime(s) <= t for s in sources)
 
 
+def build_pycall(force: bool = False) -> str:
+    """The Python extension module that makes the common launches (csrc/kcg_pycall.c)."""
+    import sysconfig
+    out = os.path.join(HERE, "_pycall.so")
+    src = os.path.join(HERE, "csrc", "kcg_pycall.c")
+    if force or not _newer(out, [src, os.path.join(os.path.dirname(HERE), "include", "kcg_b200.h")]):
+        subprocess.check_call(["gcc", "-O2", "-shared", "-fPIC", "-Wno-unused-parameter",
+                               "-I" + sysconfig.get_paths()["include"], "-o", out, src])
+    return out
+
+
 def build_library(force: bool = False) -> str:
+    build_pycall(force)
     out = os.path.join(HERE, "libkcg_b200.so")
     srcs = [os.path.join(HERE, "csrc", "kcg_shim.cpp")]
     kdir = os.path.join(HERE, "csrc", "kernels")  # the allocation-free entry instantiates a kernel from these

@@ -36,6 +36,7 @@ class CudaLauncher:
         # loaded lazily in the process that owns the GPU (launchers are pickled across processes)
         self.m_runtime = None
         self.m_cInfo = None
+        self.m_infoAddr = 0
 
     def __getstate__(self):
         st = dict(self.__dict__)
@@ -50,6 +51,7 @@ class CudaLauncher:
             info = dict(self.m_kernelInfoDict)
             info["grid"], info["block"], info["smem_bytes"] = self.m_gridDims, self.m_blockDims, self.m_shmSize
             self.m_cInfo = _lib.KernelInfo.from_dict(info)
+            self.m_infoAddr = ctypes.addressof(self.m_cInfo)
             self.m_runtime = CudaLoaderST().loadBinary(self.m_libFile)
         return self.m_runtime
 
@@ -68,12 +70,16 @@ class CudaLauncher:
         if stream is None:
             stream = DeviceInfo.get_cuda_stream(device)
         a, b, c = args
-        lib = _lib.get_lib()
-        epi = None
-        if alpha != 1.0 or beta != 0.0 or bias is not None or relu:
-            epi = ctypes.byref(_lib.Epilogue(float(alpha), float(beta), _pointer_of(bias) if bias is not None else 0,
-                                             int(bool(relu))))
-        if peers:
+        if not peers:
+            # lda, ldb, ldc: elements between rows of operands that are sub-matrices of wider row-major arrays, 0 =
+            # contiguous; with batch > 1, (a, b, c) hold `batch` problems of the kernel's M, N, K (torch.bmm layout)
+            status = _lib.pycall.gemm(rt.m_function, self.m_infoAddr, device, stream, a, b, c, lda, ldb, ldc, batch, alpha,
+                                      beta, bias, relu)
+        else:
+            epi = None
+            if alpha != 1.0 or beta != 0.0 or bias is not None or relu:
+                epi = ctypes.byref(_lib.Epilogue(float(alpha), float(beta), _pointer_of(bias) if bias is not None else 0,
+                                                 int(bool(relu))))
             if lda or ldb or ldc:
                 raise ValueError("a strided launch has no fused all-gather")
             if batch != 1:
@@ -81,18 +87,9 @@ class CudaLauncher:
             if epi is None:
                 epi = ctypes.byref(_lib.Epilogue(1.0, 0.0, 0, 0))
             arr = (ctypes.c_uint64 * len(peers))(*[_pointer_of(x) for x in peers])
-            status = lib.kcg_launch_gemm_allgather(rt.m_function, ctypes.byref(self.m_cInfo), int(device), int(stream),
-                                                   _pointer_of(a), _pointer_of(b), _pointer_of(c), epi, arr, len(peers))
-        elif lda or ldb or ldc or batch == 1:
-            # one entry for plain launches and for operands that are sub-matrices of wider row-major arrays (elements
-            # between rows; 0 = contiguous)
-            status = lib.kcg_launch_gemm_strided(rt.m_function, ctypes.byref(self.m_cInfo), int(device), int(stream),
-                                                 _pointer_of(a), _pointer_of(b), _pointer_of(c), int(lda), int(ldb),
-                                                 int(ldc), int(batch), epi)
-        else:
-            # (a, b, c) hold `batch` contiguous problems of the kernel's M, N, K (torch.bmm layout)
-            status = lib.kcg_launch_gemm_batched(rt.m_function, ctypes.byref(self.m_cInfo), int(device), int(stream),
-                                                 _pointer_of(a), _pointer_of(b), _pointer_of(c), int(batch), epi)
+            status = _lib.get_lib().kcg_launch_gemm_allgather(
+                rt.m_function, ctypes.byref(self.m_cInfo), int(device), int(stream), _pointer_of(a), _pointer_of(b),
+                _pointer_of(c), epi, arr, len(peers))
         if status:
             _lib.check(status)
 

@@ -1,10 +1,13 @@
 """Convenience wrappers over the reference-style flow
 ``KernelArgMatmul -> KCGCompiler.compileKernel -> UserInputs -> CompiledKernelFactory.getKernel``
 (the sequence of SerialCompileTask._task_compile_kernel, Runtime/python/kcg/KCGTask.py:275-297)."""
+import math
+
+from codegendemo_b200 import _lib
 from codegendemo_b200.kcg.CompiledKernelFactory import CompiledKernelFactory, EnumOperator, UserInputs
 from codegendemo_b200.kcg.KCGCompiler import KCGCompiler
 from codegendemo_b200.kcg.Operators.matmul import KernelArgMatmul
-from codegendemo_b200.kcg.Utils import EnumKernelDType, FromTorchType
+from codegendemo_b200.kcg.Utils import DeviceInfo, EnumKernelDType, FromTorchType
 
 
 def default_config(M: int, N: int, K: int, dtype: EnumKernelDType, out_dtype=None, **keys) -> KernelArgMatmul:
@@ -61,11 +64,11 @@ _TILE_COST = {
     (5, 128, 128, 128): (1.0, 0.505, (4.24, 4.65, 4.69)),
     (5, 128, 192, 64): (1.0, 0.322, (5.15, 5.60, 6.32)),
     (5, 128, 256, 64): (1.0, 0.379, (5.77, 6.37, 6.61)),
+    (5, 256, 128, 128): (1.0, 0.56, (3.20,)),
+    (5, 256, 256, 64): (1.0, 0.35, (5.20,)),
 }
 # clusters of 2, 3, 4 CTAs at 200 KB of shared memory each that run at once on the GPU the table is fitted to (148 SMs)
 _CLUSTERS = {2: 74, 3: 45, 4: 33}
-    (5, 256, 128, 128): (1.0, 0.56, (3.20,)),
-    (5, 256, 256, 64): (1.0, 0.35, (5.20,)),
 
 
 def _tile_us(tile, split, M, N, K, batch=1, sms=148):
@@ -311,19 +314,26 @@ def matmul(a, b, c=None, alpha=1.0, beta=0.0, bias=None, relu=False, b_transpose
     be views with a row pitch (column or row blocks of wider row-major tensors): their leading dimensions go
     to the strided launch entry, nothing is copied. ``b_transposed=True`` takes ``b`` stored N x K and computes
     ``a @ b.T`` (16-bit dtypes). Compiled and loaded kernels are kept per (shape, dtype, device, keys)."""
-    import torch
     M, K = a.shape
     if b_transposed:
         N, K2 = b.shape
     else:
         K2, N = b.shape
     assert K == K2
-    lda, ldb = _row_pitch(a, "a"), _row_pitch(b, "b")
-    if c is None:
+    lda = ldb = ldc = 0  # contiguous
+    if c is None and a.is_contiguous() and b.is_contiguous():
         if beta != 0.0:
             raise ValueError("beta != 0 needs the c to scale")
         c = a.new_empty((M, N))
-    ldc = _row_pitch(c, "c")
+    else:
+        lda, ldb = _row_pitch(a, "a"), _row_pitch(b, "b")
+        if c is None:
+            if beta != 0.0:
+                raise ValueError("beta != 0 needs the c to scale")
+            c = a.new_empty((M, N))
+        ldc = _row_pitch(c, "c")
+        if lda == K and ldb == (K if b_transposed else N) and ldc == N:
+            lda = ldb = ldc = 0
     dev = a.device.index or 0
     key = ("mm", M, N, K, a.dtype, dev, tuple(sorted(keys.items())) if keys else (), bool(b_transposed))
     kern = _KERNELS.get(key)
@@ -338,8 +348,6 @@ def matmul(a, b, c=None, alpha=1.0, beta=0.0, bias=None, relu=False, b_transpose
             kpm = tuned_config(M, N, K, dt, b_transposed=b_transposed)
         _, kern = build_kernel(kpm, dev)
         _KERNELS[key] = kern
-    if lda == K and ldb == (K if b_transposed else N) and ldc == N:
-        lda = ldb = ldc = 0
     kern.m_launcher.launchKernel(dev, a, b, c, alpha=alpha, beta=beta, bias=bias, relu=relu, lda=lda, ldb=ldb, ldc=ldc)
     return c
 
@@ -372,10 +380,7 @@ def attention(q, k, v, scale=None, out=None):
     (heads, Sk, d), all contiguous fp16 / bf16; ``heads`` may be batch * heads flattened. The Sq x Sk score and
     probability matrices are materialised; Sk must be a multiple of 8. Returns (heads, Sq, d)."""
     import ctypes
-    import math
     import torch
-    from codegendemo_b200 import _lib
-    from codegendemo_b200.kcg.Utils import DeviceInfo
     H, Sq, D = q.shape
     H2, Sk, D2 = k.shape
     assert H == H2 and D == D2 and tuple(v.shape) == (H, Sk, D)
@@ -409,10 +414,7 @@ def attention_fused(q, k, v, scale=None, out=None):
     probabilities stay on the SM. ``q`` is (heads, Sq, d), ``k`` and ``v`` are (heads, Sk, d), all
     contiguous fp16 / bf16 with d = 64 or 128; any Sq and Sk. Returns (heads, Sq, d). ``attention`` above is the
     three-launch form of the same chain."""
-    import math
     import torch
-    from codegendemo_b200 import _lib
-    from codegendemo_b200.kcg.Utils import DeviceInfo
     H, Sq, D = q.shape
     H2, Sk, D2 = k.shape
     assert H == H2 and D == D2 and tuple(v.shape) == (H, Sk, D)
@@ -424,9 +426,10 @@ def attention_fused(q, k, v, scale=None, out=None):
         out = q.new_empty((H, Sq, D))
     assert out.is_contiguous() and tuple(out.shape) == (H, Sq, D) and out.dtype == q.dtype
     dev = q.device.index or 0
-    status = _lib.get_lib().kcg_attention_fwd(dev, DeviceInfo.get_cuda_stream(dev), q.data_ptr(), k.data_ptr(),
-                                              v.data_ptr(), out.data_ptr(), int(FromTorchType(q.dtype)), H, Sq, Sk, D,
-                                              float(scale))
+    if _lib.pycall is None:
+        _lib.get_lib()
+    dt = EnumKernelDType.bfloat16 if q.dtype == torch.bfloat16 else EnumKernelDType.float16
+    status = _lib.pycall.attention(dev, DeviceInfo.get_cuda_stream(dev), q, k, v, out, dt, H, Sq, Sk, D, scale)
     if status:
         _lib.check(status)
     return out
@@ -435,7 +438,6 @@ def attention_fused(q, k, v, scale=None, out=None):
 def attention_status(device: int = 0) -> None:
     """Synchronises the device and raises if a bounded wait of the fused attention kernel ran out."""
     import ctypes
-    from codegendemo_b200 import _lib
     out = (ctypes.c_uint32 * 4)()
     _lib.check(_lib.get_lib().kcg_attention_status(int(device), out))
 
@@ -445,7 +447,6 @@ def bmm(a, b, c=None, alpha=1.0, beta=0.0, bias=None, relu=False, **keys):
     contiguous) as ONE launch of the kernel compiled for a single batch's M, N, K: the persistent grid
     walks the tiles of all batches, so that small per-batch problems fill the GPU together. The
     epilogue keywords are those of ``matmul`` (a bias is shared by the batches)."""
-    import torch
     batch, M, K = a.shape
     batch2, K2, N = b.shape
     assert batch == batch2 and K == K2 and a.is_contiguous() and b.is_contiguous()
