@@ -87,6 +87,11 @@ __device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float r;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
@@ -792,7 +797,11 @@ struct AttnFwd2 {
           auto scale_store = [&](uint32_t (&o)[32], int c) {
             pin_32(o);
 #pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+            for (int i = 0; i < 32; i += 2) {  // (pairs: 8 x 300 x 16384 x 128 60.3 -> 59.0 us, 32 x 4096 x 4096 x 64 199 -> 197)
+              const float2 v = f32x2_split(mul_f32x2(f32x2(__uint_as_float(o[i]), __uint_as_float(o[i + 1])), alpha2));
+              o[i] = __float_as_uint(v.x);
+              o[i + 1] = __float_as_uint(v.y);
+            }
             tmem_st_32x32b_x32(col_o + c * 32, o);
           };
 #pragma unroll
