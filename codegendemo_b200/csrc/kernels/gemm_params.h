@@ -23,7 +23,7 @@
 
 #define KCG_VARIANT_TCGEN05_PAIR 4  // tcgen05 cta_group::2 on clusters of two CTAs (fp16 / bf16)
 // K split over a thread-block cluster of LOCAL_SPLIT_U CTAs, partial tiles reduced through
-// distributed shared memory (fp16 / bf16, 128-row tiles): no workspace, no counters
+// distributed shared memory (fp16 / bf16, 128-row tiles, or 256-row tiles on CTA pairs): no workspace, no counters
 #define KCG_VARIANT_TCGEN05_CLUSTERK 5
 
 #define KCG_MAX_PEERS 7  // other GPUs of one NVSwitch domain of eight
