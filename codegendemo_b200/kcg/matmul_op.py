@@ -67,8 +67,13 @@ _TILE_COST = {
     (5, 256, 128, 128): (1.0, 0.56, (3.20,)),
     (5, 256, 256, 64): (1.0, 0.35, (5.20,)),
 }
-# clusters of 2, 3, 4 CTAs at 200 KB of shared memory each that run at once on the GPU the table is fitted to (148 SMs)
+# clusters of 2, 3, 4 CTAs at 200 KB of shared memory each that run at once on the GPU the table is fitted to (148 SMs).
+# Of 44 or 45 clusters of three some start late, and the product with them, by about 4 us whatever K and the tile: 128 x
+# N x 4096 with 128 columns 13.5, 14.1, 16.2, 17.6 us at 42 to 45 tiles; 256x4224x11008 with 192 columns in three ranges
+# 31.9, with 128 in two 28.8; 512x2112x4480 18.2 / 14.8. More clusters than run at once take a second wave: 256x4608x4096 in
+# 36 clusters of four 26.4, in 72 of two 14.6.
 _CLUSTERS = {2: 74, 3: 45, 4: 33}
+_LATE_CLUSTERS, _LATE_US = 43, 4.0
 
 
 def _tile_us(tile, split, M, N, K, batch=1, sms=148):
@@ -78,7 +83,10 @@ def _tile_us(tile, split, M, N, K, batch=1, sms=148):
     tiles, blocks = batch * -(-M // bm) * -(-N // bn), -(-K // bk)
     stream = 2.0 + 2e-6 * batch * (M * K + K * N + M * N) / 5.5  # operands and result through HBM at 5.5 TB/s
     if variant == 5:
-        return max(stream, fixed + -(-blocks // split) * per_block + per_tile[split - 2])
+        ctas = split * bm // 128
+        late = _LATE_US if ctas == 3 and _LATE_CLUSTERS < tiles <= _CLUSTERS[3] else 0.0
+        waves = -(-tiles // _CLUSTERS[ctas])
+        return max(stream, fixed + waves * (-(-blocks // split) * per_block + per_tile[split - 2]) + late)
     at_once = sms // 2 if variant == 4 else sms
     waves, rest = -(-tiles // at_once), tiles % at_once
     f = min(8, at_once // rest) if rest else 0

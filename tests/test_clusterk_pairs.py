@@ -4,7 +4,7 @@ import torch
 
 from codegendemo_b200 import _lib
 from codegendemo_b200.kcg.KCGCompiler import compile_info
-from codegendemo_b200.kcg.matmul_op import build_kernel, default_config
+from codegendemo_b200.kcg.matmul_op import _CLUSTERS, build_kernel, default_config, tuned_config
 from codegendemo_b200.kcg.Utils import EnumKernelDType as E
 from oracle import oracle
 
@@ -71,3 +71,27 @@ def test_launch_module_checks_its_arguments():
         call(0, 0, 0, 0, -1, 1, 1, *rest)
     assert call(0, 0, 0, 0, 16, 16, 16, *rest) == _lib.E_BAD_ARG  # no kernel: the library's own check
     assert _lib.pycall.attention(0, 0, 0, 16, 16, 16, 62, 1, 1, 1, 64, 0.1) == _lib.E_BAD_ARG
+
+
+class _NoDb:
+    def lookup(self, *shape):
+        return None
+
+
+def _rule(M, N, K):
+    kpm = tuned_config(M, N, K, E.bfloat16, db=_NoDb())
+    return (kpm.KERNEL_VARIANT, kpm.BLOCK_SIZE_M, kpm.BLOCK_SIZE_N, kpm.LOCAL_SPLIT_U)
+
+
+def test_rule_counts_the_clusters_that_run_at_once():
+    """Of 44 clusters of three some start late: two ranges of narrower tiles are ahead (256x4224x11008 31.9 / 28.8 us). 42
+    run at once: there the three ranges are (384x3584x11008 30.1 / 37.6). No choice is left with a second wave of clusters."""
+    for K in (9216, 11008, 14336):
+        assert _rule(256, 4224, K) == (5, 128, 128, 2)
+    assert _rule(384, 3584, 11008) == (5, 128, 256, 3)
+    for M in (128, 256, 384, 512, 640):
+        for N in range(512, 8193, 64):
+            for K in (2048, 4096, 8192):
+                variant, bm, bn, split = _rule(M, N, K)
+                if variant == 5:
+                    assert -(-M // bm) * -(-N // bn) <= _CLUSTERS[split * bm // 128], (M, N, K)
