@@ -113,6 +113,11 @@ def _cheapest_tile(M, N, K, batch=1, single_pass=False):
             if variant == 5 and (split > len(_TILE_COST[tile][2]) + 1 or -(-K // bk) < 2 * split or
                                  batch * -(-M // bm) * -(-N // bn) > _CLUSTERS[split * bm // 128]):
                 continue
+            # CTA pairs from four whole K blocks a range on. Below, the estimate leaves out up to 0.8 us of theirs (their
+            # loads wait for the cluster's start) and 64 columns a CTA are ahead: K = 704 to 768 5.8-6.1 us against 6.1-6.9
+            # on 17 shapes, K = 960 6.6-7.0 / 6.4-7.5. At 1024 they replace 128 columns, 7.2-8.0 / 6.5-7.6.
+            if variant == 5 and bm == 256 and K // bk < 4 * split:
+                continue
             us = _tile_us(tile, split, M, N, K, batch)
             if best is None or us < best[0]:
                 best = (us, tile, split)

@@ -95,3 +95,13 @@ def test_rule_counts_the_clusters_that_run_at_once():
                 variant, bm, bn, split = _rule(M, N, K)
                 if variant == 5:
                     assert -(-M // bm) * -(-N // bn) <= _CLUSTERS[split * bm // 128], (M, N, K)
+
+
+def test_rule_takes_pairs_from_four_blocks_a_range_on():
+    """K = 768: 64 columns a CTA are ahead of CTA pairs (512x2048 5.9 / 6.5 us); at 1024 and more pairs are chosen."""
+    for M, N in ((256, 3072), (512, 2048), (896, 896), (1280, 768), (768, 1344), (256, 8192)):
+        for K in (512, 640, 704, 768, 896, 960):
+            variant, bm, _, _ = _rule(M, N, K)
+            assert not (variant == 5 and bm == 256), (M, N, K)
+    for K in (1024, 1536, 2048):
+        assert _rule(512, 2048, K) == (5, 256, 128, 2)
