@@ -6,10 +6,14 @@ parameter block, so one C entry (``kcg_launch_gemm``) serves all of them and bui
 maps itself. Pointer arguments may be ints or anything with ``data_ptr()`` (HIPLauncher.py:148-187).
 """
 import ctypes
+import threading
 
 from codegendemo_b200 import _lib
 from codegendemo_b200.kcg.Loader import CudaLoaderST, KernelLibFile
 from codegendemo_b200.kcg.Utils import DeviceInfo
+
+
+_LOADING = threading.Lock()
 
 
 def _pointer_of(obj) -> int:
@@ -42,17 +46,23 @@ class CudaLauncher:
         st = dict(self.__dict__)
         st["m_runtime"] = None
         st["m_cInfo"] = None
+        st["m_infoAddr"] = 0
         return st
 
     def _getWrapper(self):
         if self.m_runtime is None:
-            if self.m_kernelInfoDict is None:
-                raise RuntimeError("KCG launcher: kernelInfo missing (compile with KCGCompiler first)")
-            info = dict(self.m_kernelInfoDict)
-            info["grid"], info["block"], info["smem_bytes"] = self.m_gridDims, self.m_blockDims, self.m_shmSize
-            self.m_cInfo = _lib.KernelInfo.from_dict(info)
-            self.m_infoAddr = ctypes.addressof(self.m_cInfo)
-            self.m_runtime = CudaLoaderST().loadBinary(self.m_libFile)
+            # One thread loads. A launch reads m_cInfo by its address, with the GIL released and no reference of its own,
+            # so the structure is never replaced, and m_runtime, which says that it is there, is set last.
+            with _LOADING:
+                if self.m_runtime is None:
+                    if self.m_kernelInfoDict is None:
+                        raise RuntimeError("KCG launcher: kernelInfo missing (compile with KCGCompiler first)")
+                    info = dict(self.m_kernelInfoDict)
+                    info["grid"], info["block"], info["smem_bytes"] = self.m_gridDims, self.m_blockDims, self.m_shmSize
+                    cInfo = _lib.KernelInfo.from_dict(info)
+                    runtime = CudaLoaderST().loadBinary(self.m_libFile)
+                    self.m_cInfo, self.m_infoAddr = cInfo, ctypes.addressof(cInfo)
+                    self.m_runtime = runtime
         return self.m_runtime
 
     def launchKernel(self, device, *args, stream=None, alpha=1.0, beta=0.0, bias=None, relu=False, peers=None,
