@@ -15,25 +15,63 @@ static GemmFn g_gemm;
 static AttentionFn g_attention;
 static PyObject* g_data_ptr;
 
-/* Address of an argument: an int, or anything with data_ptr(). */
-static int pointer_of(PyObject* o, uint64_t* out) {
-  if (PyLong_Check(o)) {
-    *out = PyLong_AsUnsignedLongLong(o);
-    return PyErr_Occurred() ? -1 : 0;
+/* int(o) and float(o) of an argument, as C numbers; the exact types first. -1 with an exception set on failure. */
+static int u64_of(PyObject* o, uint64_t* out) {
+  PyObject* i = PyLong_Check(o) ? Py_NewRef(o) : PyNumber_Long(o);
+  if (!i) return -1;
+  *out = PyLong_AsUnsignedLongLong(i);
+  Py_DECREF(i);
+  return PyErr_Occurred() ? -1 : 0;
+}
+
+static int i64_of(PyObject* o, int64_t* out) {
+  PyObject* i = PyLong_Check(o) ? Py_NewRef(o) : PyNumber_Long(o);
+  if (!i) return -1;
+  *out = PyLong_AsLongLong(i);
+  Py_DECREF(i);
+  return PyErr_Occurred() ? -1 : 0;
+}
+
+static int int_of(PyObject* o, int* out) {
+  int64_t v;
+  if (i64_of(o, &v)) return -1;
+  *out = (int)v;
+  return 0;
+}
+
+static int double_of(PyObject* o, double* out) {
+  if (PyFloat_CheckExact(o)) {
+    *out = PyFloat_AS_DOUBLE(o);
+    return 0;
   }
+  PyObject* f = PyNumber_Float(o);
+  if (!f) return -1;
+  *out = PyFloat_AS_DOUBLE(f);
+  Py_DECREF(f);
+  return 0;
+}
+
+/* Address of an argument: an int, or what its data_ptr() returns. */
+static int pointer_of(PyObject* o, uint64_t* out) {
+  if (PyLong_Check(o)) return u64_of(o, out);
   if (o == Py_None) {
     PyErr_SetString(PyExc_TypeError, "KCG launcher: pointer argument is None");
     return -1;
   }
   PyObject* r = PyObject_CallMethodNoArgs(o, g_data_ptr);
   if (!r) {
-    if (PyErr_ExceptionMatches(PyExc_AttributeError))
-      PyErr_SetString(PyExc_TypeError, "Pointer argument must be either uint64 or have data_ptr method");
+    if (PyErr_ExceptionMatches(PyExc_AttributeError)) {
+      PyObject *type, *value, *trace;
+      PyErr_Fetch(&type, &value, &trace);
+      const int has = PyObject_HasAttr(o, g_data_ptr);  /* then the error came from inside the method */
+      PyErr_Restore(type, value, trace);
+      if (!has) PyErr_SetString(PyExc_TypeError, "Pointer argument must be either uint64 or have data_ptr method");
+    }
     return -1;
   }
-  *out = PyLong_AsUnsignedLongLong(r);
+  const int e = u64_of(r, out);
   Py_DECREF(r);
-  return PyErr_Occurred() ? -1 : 0;
+  return e;
 }
 
 static PyObject* bind(PyObject* self, PyObject* args) {
@@ -50,25 +88,23 @@ static PyObject* gemm(PyObject* self, PyObject* const* a, Py_ssize_t n) {
     PyErr_SetString(PyExc_TypeError, "gemm takes 15 arguments, after bind");
     return NULL;
   }
-  const uint64_t function = PyLong_AsUnsignedLongLong(a[0]), info = PyLong_AsUnsignedLongLong(a[1]);
-  const int device = (int)PyLong_AsLong(a[2]);
-  const uint64_t stream = PyLong_AsUnsignedLongLong(a[3]);
-  if (PyErr_Occurred()) return NULL;
-  uint64_t p[3];
+  uint64_t function, info, stream, p[3];
+  int64_t ld[3];
+  int device, batch;
+  double alpha, beta;
+  if (u64_of(a[0], &function) || u64_of(a[1], &info) || int_of(a[2], &device) || u64_of(a[3], &stream)) return NULL;
   for (int i = 0; i < 3; ++i)
-    if (pointer_of(a[4 + i], &p[i])) return NULL;
-  const int64_t lda = PyLong_AsLongLong(a[7]), ldb = PyLong_AsLongLong(a[8]), ldc = PyLong_AsLongLong(a[9]);
-  const int batch = (int)PyLong_AsLong(a[10]);
-  const double alpha = PyFloat_AsDouble(a[11]), beta = PyFloat_AsDouble(a[12]);
+    if (pointer_of(a[4 + i], &p[i]) || i64_of(a[7 + i], &ld[i])) return NULL;
+  if (int_of(a[10], &batch) || double_of(a[11], &alpha) || double_of(a[12], &beta)) return NULL;
   const int relu = PyObject_IsTrue(a[14]);
-  if (PyErr_Occurred()) return NULL;
+  if (relu < 0) return NULL;
   kcg_epilogue epi = {(float)alpha, (float)beta, 0, relu, {0, 0, 0}};
   if (a[13] != Py_None && pointer_of(a[13], &epi.bias)) return NULL;
   const int fused = alpha != 1.0 || beta != 0.0 || a[13] != Py_None || relu;
   int status;
   Py_BEGIN_ALLOW_THREADS
-  status = g_gemm(function, (const kcg_kernel_info*)(uintptr_t)info, device, stream, p[0], p[1], p[2], lda, ldb, ldc, batch,
-                  fused ? &epi : NULL);
+  status = g_gemm(function, (const kcg_kernel_info*)(uintptr_t)info, device, stream, p[0], p[1], p[2], ld[0], ld[1], ld[2],
+                  batch, fused ? &epi : NULL);
   Py_END_ALLOW_THREADS
   return PyLong_FromLong(status);
 }
@@ -79,18 +115,18 @@ static PyObject* attention(PyObject* self, PyObject* const* a, Py_ssize_t n) {
     PyErr_SetString(PyExc_TypeError, "attention takes 12 arguments, after bind");
     return NULL;
   }
-  uint64_t p[4];
+  uint64_t stream, p[4];
+  int device, v[5];
+  double scale;
+  if (int_of(a[0], &device) || u64_of(a[1], &stream)) return NULL;
   for (int i = 0; i < 4; ++i)
     if (pointer_of(a[2 + i], &p[i])) return NULL;
-  const uint64_t stream = PyLong_AsUnsignedLongLong(a[1]);
-  const long v[6] = {PyLong_AsLong(a[0]), PyLong_AsLong(a[6]), PyLong_AsLong(a[7]),
-                     PyLong_AsLong(a[8]), PyLong_AsLong(a[9]), PyLong_AsLong(a[10])};
-  const double scale = PyFloat_AsDouble(a[11]);
-  if (PyErr_Occurred()) return NULL;
+  for (int i = 0; i < 5; ++i)
+    if (int_of(a[6 + i], &v[i])) return NULL;
+  if (double_of(a[11], &scale)) return NULL;
   int status;
   Py_BEGIN_ALLOW_THREADS
-  status = g_attention((int)v[0], stream, p[0], p[1], p[2], p[3], (int)v[1], (int)v[2], (int)v[3], (int)v[4], (int)v[5],
-                       (float)scale);
+  status = g_attention(device, stream, p[0], p[1], p[2], p[3], v[0], v[1], v[2], v[3], v[4], (float)scale);
   Py_END_ALLOW_THREADS
   return PyLong_FromLong(status);
 }
