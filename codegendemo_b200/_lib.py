@@ -109,12 +109,28 @@ def lib_path() -> str:
 
 
 _lib = None
-pycall = None  # extension module of the common launches (csrc/kcg_pycall.c), bound by get_lib()
+
+
+def __getattr__(name):
+    """``_lib.pycall``: the extension module that makes the common launches (csrc/kcg_pycall.c), loaded where a launch first
+    asks for it, so that compiling and the host-side entries need the library alone. Raises if it has not been built for
+    this interpreter (no fallback exists)."""
+    if name != "pycall":
+        raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
+    lib = get_lib()
+    try:
+        from codegendemo_b200 import _pycall
+    except ImportError as e:
+        raise RuntimeError("codegendemo_b200/_pycall is missing or not loadable in this interpreter: build it with "
+                           "`python -m codegendemo_b200.build`") from e
+    _pycall.bind(*(ctypes.cast(f, ctypes.c_void_p).value for f in (lib.kcg_launch_gemm_strided, lib.kcg_attention_fwd)))
+    globals()["pycall"] = _pycall
+    return _pycall
 
 
 def get_lib() -> ctypes.CDLL:
     """Loads the library once. Raises if it has not been built (no fallback exists)."""
-    global _lib, pycall
+    global _lib
     if _lib is not None:
         return _lib
     path = lib_path()
@@ -175,13 +191,6 @@ def get_lib() -> ctypes.CDLL:
                  "kcg_unload", "kcg_device_properties", "kcg_launch_gemm", "kcg_launch_gemm_ex",
                  "kcg_check_status", "kcg_matmul_host", "kcg_shutdown"):
         getattr(lib, name).restype = ctypes.c_int
-    try:
-        from codegendemo_b200 import _pycall
-    except ImportError as e:
-        raise RuntimeError("codegendemo_b200/_pycall.so is missing or not loadable: build it with "
-                           "`python -m codegendemo_b200.build`") from e
-    _pycall.bind(*(ctypes.cast(f, ctypes.c_void_p).value for f in (lib.kcg_launch_gemm_strided, lib.kcg_attention_fwd)))
-    pycall = _pycall
     _lib = lib
     return lib
 

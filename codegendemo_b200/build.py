@@ -5,8 +5,8 @@
 
 The library is built with nvcc for sm_100a: its host code binds the CUDA driver lazily (so it loads without a GPU),
 and pieces of device code are linked into it (the allocation-free split-K entry, the row softmax, the fused attention).
-Beside it stands ``_pycall.so``, a small extension module that launches on behalf of Python callers. The GEMM
-kernels themselves are compiled per config by the library's own compile entry with
+Beside it stands ``_pycall``, a small extension module for the building interpreter that launches on behalf of Python
+callers. The GEMM kernels themselves are compiled per config by the library's own compile entry with
 ``nvcc -cubin -gencode arch=compute_100a,code=sm_100a``.
 """
 import os
@@ -24,19 +24,31 @@ def _newer(target: str, sources) -> bool:
     return all(os.path.getmtime(s) <= t for s in sources)
 
 
+def pycall_path() -> str:
+    """The extension module of this interpreter: its name carries the ABI tag, so another one's is never loaded."""
+    import sysconfig
+    return os.path.join(HERE, "_pycall" + sysconfig.get_config_var("EXT_SUFFIX"))
+
+
 def build_pycall(force: bool = False) -> str:
     """The Python extension module that makes the common launches (csrc/kcg_pycall.c)."""
+    import shlex
+    import shutil
     import sysconfig
-    out = os.path.join(HERE, "_pycall.so")
+    out = pycall_path()
+    untagged = os.path.join(HERE, "_pycall.so")  # an earlier build's, for whichever interpreter
+    if os.path.exists(untagged):
+        os.remove(untagged)
     src = os.path.join(HERE, "csrc", "kcg_pycall.c")
     if force or not _newer(out, [src, os.path.join(os.path.dirname(HERE), "include", "kcg_b200.h")]):
-        subprocess.check_call(["gcc", "-O2", "-shared", "-fPIC", "-Wno-unused-parameter",
-                               "-I" + sysconfig.get_paths()["include"], "-o", out, src])
+        compilers = [shlex.split(c) for c in (os.environ.get("CC"), sysconfig.get_config_var("CC"), "cc", "gcc") if c]
+        cc = next((c for c in compilers if shutil.which(c[0])), ["cc"])
+        subprocess.check_call(cc + ["-O2", "-shared", "-fPIC", "-I" + sysconfig.get_paths()["include"], "-o", out, src])
     return out
 
 
 def build_library(force: bool = False) -> str:
-    build_pycall(force)
+    """The C-ABI library. Needs nvcc alone; :func:`build_pycall` makes what Python callers launch through."""
     out = os.path.join(HERE, "libkcg_b200.so")
     srcs = [os.path.join(HERE, "csrc", "kcg_shim.cpp")]
     kdir = os.path.join(HERE, "csrc", "kernels")  # the allocation-free entry instantiates a kernel from these
@@ -114,5 +126,6 @@ def prebuild_kernels(verbose: bool = True) -> int:
 if __name__ == "__main__":
     sys.path.insert(0, os.path.dirname(HERE))
     print(build_library(force="--force" in sys.argv))
+    print(build_pycall(force="--force" in sys.argv))
     if "--lib-only" not in sys.argv:
         prebuild_kernels()

@@ -18,6 +18,7 @@ def _built_library():
     from codegendemo_b200 import build as kbuild
     from oracle import build_oracle
     kbuild.build_library()
+    kbuild.build_pycall()
     build_oracle.build_port()
     yield
 

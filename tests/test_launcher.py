@@ -1,6 +1,9 @@
 """The launcher without a GPU (the loader and the library's entries are stand-ins): a kernel's first launch from several
 threads, and the arguments that a launch takes."""
 import ctypes
+import os
+import subprocess
+import sys
 import threading
 import types
 
@@ -117,3 +120,28 @@ def test_launch_takes_what_int_and_float_take(monkeypatch):
         assert not got
     finally:
         call.bind(*real)
+
+
+def test_library_loads_without_the_launch_module():
+    """Compiling and the host-side entries need the C library alone; a launch without the module says how to build it. The
+    module is this interpreter's own."""
+    code = """
+import sys
+sys.modules["codegendemo_b200._pycall"] = None  # importing it fails
+from codegendemo_b200 import _lib, build
+from codegendemo_b200.kcg.KCGCompiler import compile_info
+from codegendemo_b200.kcg.matmul_op import default_config
+from codegendemo_b200.kcg.Utils import EnumKernelDType as E
+assert _lib.get_lib().kcg_version()
+assert compile_info(default_config(256, 256, 256, E.bfloat16).compileArgs()).grid[0] == 2
+try:
+    _lib.pycall
+except RuntimeError as e:
+    assert "codegendemo_b200.build" in str(e)
+else:
+    raise AssertionError("no error")
+import importlib.machinery, os
+assert build.pycall_path().endswith(importlib.machinery.EXTENSION_SUFFIXES[0]) and os.path.exists(build.pycall_path())
+assert not os.path.exists(os.path.join(os.path.dirname(build.pycall_path()), "_pycall.so"))
+"""
+    subprocess.run([sys.executable, "-c", code], check=True, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
