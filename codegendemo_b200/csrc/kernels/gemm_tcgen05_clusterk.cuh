@@ -417,8 +417,10 @@ struct TcGemmClusterK {
       // Second phase of the cluster barrier, which guards the CTAs' lifetimes: this CTA has received
       // everything (or has given up), so no copy into it is in flight any more. Once every CTA of the
       // cluster has said so, all copies have landed and each may leave; the wait is at the common exit,
-      // behind the adding and storing below.
-      cluster_arrive_relaxed();
+      // behind the adding and storing below. Tensor memory is a CTA's own, but a pair gives its columns
+      // back together: there the arrival says as well that this warp has read its last accumulator, and
+      // is made behind the adding.
+      if constexpr (!kPair) cluster_arrive_relaxed();
       if (all_in) {
         const uint32_t tmem_acc = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
         {
@@ -485,6 +487,11 @@ struct TcGemmClusterK {
           }
         }
       }
+      if constexpr (kPair) {
+        tc_fence_before_sync();
+        __syncwarp();
+        cluster_arrive_relaxed();
+      }
     }
 
     // ------------------------------------------------------------ common exit
@@ -499,7 +506,9 @@ struct TcGemmClusterK {
     if (threadIdx.x == 64) KCG_CTL(7);
     tc_fence_before_sync();
     __syncthreads();
-    cluster_wait();  // no CTA leaves while another may still write into its shared memory or read from it
+    // no CTA leaves while another may still write into its shared memory or read from it, or - in a pair - reads the
+    // tensor memory that both give back
+    cluster_wait();
     if (warp == 1) {
       __syncwarp();
       tc_fence_after_sync();

@@ -105,3 +105,34 @@ def test_rule_takes_pairs_from_four_blocks_a_range_on():
             assert not (variant == 5 and bm == 256), (M, N, K)
     for K in (1024, 1536, 2048):
         assert _rule(512, 2048, K) == (5, 256, 128, 2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bn,bk,stages", [(128, 64, 3), (128, 128, 2), (256, 64, 4)])
+def test_pairs_that_share_an_sm(bn, bk, stages):
+    """Short rings leave room for several CTAs on an SM, and more clusters than fit come and go: a pair's tensor memory is
+    taken by the next CTA as soon as it is given back, so neither half may still read its accumulator by then. Launches that
+    follow one another without a wait, two kernels in turn on two streams, give the bits of launches one at a time."""
+    M = N = 2048
+    K = 320
+    a, b = [x.cuda() for x in oracle.make_inputs(M, N, K, torch.bfloat16, "normal", seed=3)]
+    _, kern = build_kernel(_cfg(M, N, K, bn, bk, NUM_STAGES=stages), 0)
+    _, other = build_kernel(default_config(M, N, K, E.bfloat16, KERNEL_VARIANT=2, BLOCK_SIZE_N=64, BLOCK_SIZE_K=64,
+                                           NUM_STAGES=2), 0)
+    alone = torch.empty((M, N), dtype=torch.bfloat16, device="cuda")
+    kern.run(a, b, alone)
+    kern.checkStatus()
+    err = oracle.rel_errors(alone, oracle.host_matmul(a.cpu(), b.cpu()))
+    assert err["max_rel"] <= oracle.tolerance_for(torch.bfloat16)
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    outs = [torch.full((2, M, N), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(8)]
+    torch.cuda.synchronize()
+    for c in outs:
+        for s in streams:
+            with torch.cuda.stream(s):
+                kern.run(a, b, c[0] if s is streams[0] else c[1])
+                other.run(a, b, torch.empty((M, N), dtype=torch.bfloat16, device="cuda"))
+    torch.cuda.synchronize()
+    kern.checkStatus()
+    for c in outs:
+        assert torch.equal(c[0], alone) and torch.equal(c[1], alone)
