@@ -532,10 +532,10 @@ struct TcGemm {
           __syncwarp();
           if (lane == 0) {
             if constexpr (kPair) {
-              // ("read" is all it says: released at cluster scope, the arrival would wait for the warp's stores to
-              // shared memory and their fence, about 950 cycles in which the leader may not start the next tile; relaxed,
-              // 16384 x 4096 x 1024 went from 106 to 99.6 us, 4096 x 4096 x 1024 from 29.0 to 28.2)
-              mbar_arrive_cluster_relaxed(map_to_cta(smem_u32(&bars->tmem_empty[idx]), 0u));
+              // (the lanes' reads are complete, tcgen05.wait::ld, and fenced above; released at cluster scope, the arrival
+              // would wait for the warp's stores to shared memory and their fence, about 950 cycles in which the leader
+              // may not start the next tile: 16384 x 4096 x 1024 106 us instead of 100, 4096 x 4096 x 1024 29.0 / 28.2)
+              mbar_arrive_cluster_cta(map_to_cta(smem_u32(&bars->tmem_empty[idx]), 0u));
             } else {
               mbar_arrive(&bars->tmem_empty[idx]);
             }

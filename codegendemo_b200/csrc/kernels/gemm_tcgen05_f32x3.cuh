@@ -475,7 +475,7 @@ struct TcGemmF32x3 {
           __syncwarp();
           if (lane == 0) {
             if constexpr (kPair) {
-              mbar_arrive_cluster_relaxed(map_to_cta(smem_u32(&bars->tmem_empty[ab]), 0u));  // ("read" is all it says)
+              mbar_arrive_cluster_cta(map_to_cta(smem_u32(&bars->tmem_empty[ab]), 0u));  // (the reads above are complete)
             } else {
               mbar_arrive(&bars->tmem_empty[ab]);
             }
