@@ -28,8 +28,10 @@ def test_config():
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("bn,bk", [(128, 64), (128, 128), (256, 64), (256, 128)])
-# one K block a range; an odd number of blocks (ranges of unequal length), the last one half full; past the ring
-@pytest.mark.parametrize("K", [256, 1248, 4096])
+# the shortest (one block of 128 a range); past the ring with equal ranges, the last block half (64) or three quarters (128)
+# full; an odd number of blocks past the ring, hence unequal ranges, of 64 (10 + 9) and of both (17 + 16, 9 + 8), the last
+# one half full (a quarter of 128 at 1184)
+@pytest.mark.parametrize("K", [256, 1248, 1184, 2112, 4096])
 def test_matches_the_oracle(bn, bk, K):
     M, N = 384, 320
     a, b = oracle.make_inputs(M, N, K, torch.bfloat16, "normal", seed=9)

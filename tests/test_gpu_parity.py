@@ -473,7 +473,10 @@ def test_abandoned_shares_of_a_split_reduction_are_summed_by_the_last_arriver(sh
     (2048, 2048, dict(KERNEL_VARIANT=4, BLOCK_SIZE_M=256, BLOCK_SIZE_N=256, BLOCK_SIZE_K=64)),
     (1024, 1024, dict(KERNEL_VARIANT=2, BLOCK_SIZE_M=128, BLOCK_SIZE_N=128, BLOCK_SIZE_K=64, LOCAL_SPLIT_U=2)),
     (512, 1024, dict(KERNEL_VARIANT=4, BLOCK_SIZE_M=256, BLOCK_SIZE_N=256, BLOCK_SIZE_K=32, dtype=E.float32)),
-], ids=["cluster-split-k", "cta-pairs", "single-cta-split-k", "fp32-3xtf32-pairs"])
+    (512, 1024, dict(KERNEL_VARIANT=5, BLOCK_SIZE_M=256, BLOCK_SIZE_N=256, BLOCK_SIZE_K=64, LOCAL_SPLIT_U=2)),
+    (512, 1024, dict(KERNEL_VARIANT=4, BLOCK_SIZE_M=256, BLOCK_SIZE_N=128, BLOCK_SIZE_K=32, dtype=E.float32)),
+], ids=["cluster-split-k", "cta-pairs", "single-cta-split-k", "fp32-3xtf32-pairs", "cluster-split-k-pairs",
+        "fp32-pairs-a-in-tensor-memory"])
 def test_back_to_back_dependent_launches_see_each_others_results(shape):
     """Launches of the tcgen05 kernels carry the programmatic-dependent-launch attribute:
     the next kernel of a stream is brought onto the GPU while the one before it drains, and waits
