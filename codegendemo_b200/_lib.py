@@ -109,28 +109,24 @@ def lib_path() -> str:
 
 
 _lib = None
+pycall = None  # extension module of the common launches (csrc/kcg_pycall.c), bound by get_lib()
 
 
-def __getattr__(name):
-    """``_lib.pycall``: the extension module that makes the common launches (csrc/kcg_pycall.c), loaded where a launch first
-    asks for it, so that compiling and the host-side entries need the library alone. Raises if it has not been built for
-    this interpreter (no fallback exists)."""
-    if name != "pycall":
-        raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
-    lib = get_lib()
-    try:
-        from codegendemo_b200 import _pycall
-    except ImportError as e:
+class _NoPycall:
+    """Stands for the extension module where this interpreter has none: compiling and the host-side entries need the library
+    alone, a launch says what is missing (no fallback exists)."""
+
+    def __init__(self, cause):
+        self.cause = cause
+
+    def __getattr__(self, name):
         raise RuntimeError("codegendemo_b200/_pycall is missing or not loadable in this interpreter: build it with "
-                           "`python -m codegendemo_b200.build`") from e
-    _pycall.bind(*(ctypes.cast(f, ctypes.c_void_p).value for f in (lib.kcg_launch_gemm_strided, lib.kcg_attention_fwd)))
-    globals()["pycall"] = _pycall
-    return _pycall
+                           "`python -m codegendemo_b200.build`") from self.cause
 
 
 def get_lib() -> ctypes.CDLL:
     """Loads the library once. Raises if it has not been built (no fallback exists)."""
-    global _lib
+    global _lib, pycall
     if _lib is not None:
         return _lib
     path = lib_path()
@@ -191,6 +187,13 @@ def get_lib() -> ctypes.CDLL:
                  "kcg_unload", "kcg_device_properties", "kcg_launch_gemm", "kcg_launch_gemm_ex",
                  "kcg_check_status", "kcg_matmul_host", "kcg_shutdown"):
         getattr(lib, name).restype = ctypes.c_int
+    try:
+        from codegendemo_b200 import _pycall
+        _pycall.bind(*(ctypes.cast(f, ctypes.c_void_p).value
+                       for f in (lib.kcg_launch_gemm_strided, lib.kcg_attention_fwd)))
+        pycall = _pycall
+    except ImportError as e:
+        pycall = _NoPycall(e)
     _lib = lib
     return lib
 

@@ -17,19 +17,27 @@ static PyObject* g_data_ptr;
 
 /* int(o) and float(o) of an argument, as C numbers; the exact types first. -1 with an exception set on failure. */
 static int u64_of(PyObject* o, uint64_t* out) {
-  PyObject* i = PyLong_Check(o) ? Py_NewRef(o) : PyNumber_Long(o);
-  if (!i) return -1;
-  *out = PyLong_AsUnsignedLongLong(i);
-  Py_DECREF(i);
-  return PyErr_Occurred() ? -1 : 0;
+  if (PyLong_Check(o)) {
+    *out = PyLong_AsUnsignedLongLong(o);
+  } else {
+    PyObject* i = PyNumber_Long(o);
+    if (!i) return -1;
+    *out = PyLong_AsUnsignedLongLong(i);
+    Py_DECREF(i);
+  }
+  return *out == (uint64_t)-1 && PyErr_Occurred() ? -1 : 0;
 }
 
 static int i64_of(PyObject* o, int64_t* out) {
-  PyObject* i = PyLong_Check(o) ? Py_NewRef(o) : PyNumber_Long(o);
-  if (!i) return -1;
-  *out = PyLong_AsLongLong(i);
-  Py_DECREF(i);
-  return PyErr_Occurred() ? -1 : 0;
+  if (PyLong_Check(o)) {
+    *out = PyLong_AsLongLong(o);
+  } else {
+    PyObject* i = PyNumber_Long(o);
+    if (!i) return -1;
+    *out = PyLong_AsLongLong(i);
+    Py_DECREF(i);
+  }
+  return *out == -1 && PyErr_Occurred() ? -1 : 0;
 }
 
 static int int_of(PyObject* o, int* out) {

@@ -439,6 +439,8 @@ def attention_fused(q, k, v, scale=None, out=None):
         out = q.new_empty((H, Sq, D))
     assert out.is_contiguous() and tuple(out.shape) == (H, Sq, D) and out.dtype == q.dtype
     dev = q.device.index or 0
+    if _lib.pycall is None:
+        _lib.get_lib()
     dt = EnumKernelDType.bfloat16 if q.dtype == torch.bfloat16 else EnumKernelDType.float16
     status = _lib.pycall.attention(dev, DeviceInfo.get_cuda_stream(dev), q, k, v, out, dt, H, Sq, Sk, D, scale)
     if status:

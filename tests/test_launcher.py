@@ -135,7 +135,7 @@ from codegendemo_b200.kcg.Utils import EnumKernelDType as E
 assert _lib.get_lib().kcg_version()
 assert compile_info(default_config(256, 256, 256, E.bfloat16).compileArgs()).grid[0] == 2
 try:
-    _lib.pycall
+    _lib.pycall.gemm
 except RuntimeError as e:
     assert "codegendemo_b200.build" in str(e)
 else:
