@@ -1,7 +1,7 @@
 /* The two launches a Python program makes most, as one C call each: tensors to addresses, Python numbers to C ones, the
- * launch, its status back. The same entries of libkcg_b200.so serve them through ctypes; converting a launch's twelve
- * arguments there took 2.2 us on a host where this takes 0.4 (the whole of `matmul` 9.3 -> 4.9 us, without the driver's
- * part). `bind` is given the entries' addresses, so this module is linked against neither the library nor torch. */
+ * launch, its status back. The same entries of libkcg_b200.so serve them through ctypes; there `launchKernel` took 4.0 us
+ * without the driver's part, here it takes 0.9 (the whole of `matmul`, whose contiguous operands also skip the row-pitch
+ * questions, 8.7 -> 3.9 on the same host). `bind` is given the entries' addresses, so this module is linked against neither the library nor torch. */
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #include <stdint.h>

@@ -1,8 +1,8 @@
 // Split-K GEMM on thread-block clusters for problems with few output tiles (skinny M):
 // C[M,N] = A[M,K] * B[K,N], fp16 / bf16, fp32 accumulation.
 //
-// A cluster of kSplit CTAs (or CTA pairs, see kPair) owns ONE 128 x kBN output tile. CTA r of the cluster multiplies the
-// r-th of kSplit equal K ranges with the usual pipeline (warp 0 TMA producer, warp 1 tcgen05.mma
+// A cluster of kSplit CTAs owns ONE 128 x kBN output tile (of kSplit CTA pairs a 256 x kBN tile, see kPair: read "CTA" as
+// "the pair's CTA with the same rows" below). CTA r of the cluster multiplies the r-th of kSplit equal K ranges with the usual pipeline (warp 0 TMA producer, warp 1 tcgen05.mma
 // issuer, fp32 accumulator in TMEM), so kSplit times as many SMs stream B as there are tiles.
 // The partial tiles never touch global memory: the tile's columns are cut into kSplit slices
 // (runs of 32-column blocks, lengths differing by at most one, so kSplit = 3 works as well as 2 and 4),

@@ -3,9 +3,10 @@
 //
 // Why two extra mechanisms on top of the plain tcgen05 pipeline:
 //  * kind::tf32 reads fp32 words and ignores the low 13 mantissa bits, so
-//    hi = x needs no work; splitter warps write lo = tf32_rn(x - trunc_tf32(x)), for B
-//    into a twin of every landed stage, for A - hi and lo - into tensor memory, and each
-//    K step issues lo*hi + hi*lo + hi*hi (lo*lo, ~2^-22 relative, is dropped).
+//    hi = x needs no work; splitter warps write lo = tf32_rn(x - trunc_tf32(x)) into a
+//    twin of every landed stage - for A, where tensor memory has room beside the
+//    accumulators, hi and lo into tensor memory instead - and each K step issues
+//    lo*hi + hi*lo + hi*hi (lo*lo, ~2^-22 relative, is dropped).
 //  * The tensor core adds into its fp32 accumulator with truncation, a bias that
 //    grows linearly with the number of accumulated K steps (measured: 3e-5
 //    normwise at K = 4096). So the MMA warp restarts a fresh accumulator every
@@ -21,8 +22,10 @@
 // accumulator buffers fill all 512 columns, and two-accumulator CTAs keep A in shared memory.
 // What the splitter cost before it was written like this, 256x256x32 pair block: rounding by cvt.rna.tf32 15 cycles per
 // warp instruction, arrivals at the leader with release at cluster scope 950 cycles, loads that waited for the stores
-// before them; 2500 cycles in all. 4096^3 585 -> 505 us, 2048x4096x4096 323 -> 262, 512x11008x4096 219 -> 190,
-// 1024^3 24.5 -> 20.9, 640x2624x1024 31 -> 25 (graph replay, B200).
+// before them; 2500 cycles in all. 4096^3 578 -> 488 us, 2048x4096x4096 338 -> 278, 512x11008x4096 220 -> 191,
+// 640x2624x1024 34.6 -> 26.6, 6272x640x6144 252 -> 221 (graph replay in turn, B200), 1024^3 23.2 -> 20.2 per call.
+// Spills (-Xptxas -v, bytes stored / loaded per thread): 256x256x32 124 / 180, 128x256x16 104 / 188, 256x192x32 24 / 44, the
+// narrower tiles none.
 //
 // Warp roles (512 threads, 640 in the pair form with A in tensor memory; whole warpgroups so that setmaxnreg can move
 // registers from the control warps to the accumulating warps):

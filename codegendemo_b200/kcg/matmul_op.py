@@ -40,15 +40,18 @@ def default_config(M: int, N: int, K: int, dtype: EnumKernelDType, out_dtype=Non
 
 
 # Tiles of the 16-bit kernels the rule below chooses from: (KERNEL_VARIANT, BLOCK_SIZE_M, N, K) -> microseconds
-# {fixed, per K block, per tile beyond its K blocks}. Fitted to 4 900 device timings (CUDA-graph replay, operands
-# rotating) of 36 tiles on 127 shapes of 128..32768 x 512..16384 x 256..16384, B stored either way; on the same
-# shapes the tile the fit picks is within 1 % of the best measured one on average (worst 10 %), where the former
-# rule - tiles had to divide the problem - averaged 22 % behind it (1664 x 2752 x 1472: 33 -> 12.9 us;
-# 11136 x 7488 x 1792: 608 -> 205 us; 128 x 1344 x 3072: 17.3 -> 7.7 us). For the cluster split-K kernel the third
-# figure is one per LOCAL_SPLIT_U of 2, 3, 4; its 256-row tiles run on CTA pairs, two K ranges only (12 shapes; against the
-# best 128-row choice 512 x 4096 x 11008 41.3 -> 36.4 us, 1024 x 2048 x 8192 29.5 -> 27.5, 256 x 4096 x 4096 14.9 -> 13.0,
-# 640 x 1280 x 2560 10.2 -> 9.6; behind it where K is short, 512 x 1024 x 1024 5.4 / 5.8, or most SMs idle, 256 x 2048 x
-# 16384 23 / 30).
+# {fixed, per K block, per tile beyond its K blocks}. For the cluster split-K kernel the third figure is one per LOCAL_SPLIT_U
+# of 2, 3, 4; its 256-row tiles run on CTA pairs, two K ranges only. Fitted to 4 900 device timings (CUDA-graph replay,
+# operands rotating) of 36 tiles on 127 single products of 128..32768 x 512..16384 x 256..16384, B stored either way - the two
+# 256-row cluster tiles later, to 12 shapes, and the KERNEL_VARIANT 4 rows are from before pairs released accumulators
+# without waiting for their stores. On 56 other shapes of that range what the rule picks is now 4 % behind the best measured tile
+# on average; more than 10 % on six, worst 10368 x 5568 x 320, 57 us against 38 with 256x256x64 pairs, whose row is too high
+# at short K. (The rule of tiles that divide the problem was 22 % behind: 1664 x 2752 x 1472 33 -> 12.9 us, 11136 x 7488 x
+# 1792 608 -> 205, 128 x 1344 x 3072 17.3 -> 7.7.) No batched products are among the fit's shapes: their times are 4 to 26 %,
+# on average 15 %, above the estimate (24 x 384x768x640 11.5 estimated, 15.6 a call), the picks 2 % behind on 12 shapes, worst
+# 10 %. The 256-row cluster tiles against the best 128-row choice: 512 x 4096 x 11008 41.3 -> 36.4 us, 1024 x 2048 x 8192
+# 29.5 -> 27.5, 256 x 4096 x 4096 14.9 -> 13.0, 640 x 1280 x 2560 10.2 -> 9.6; behind it where K is short, 512 x 1024 x 1024
+# 5.4 / 5.8, or most SMs idle, 256 x 2048 x 16384 23 / 30.
 _TILE_COST = {
     (2, 128, 64, 128): (2.85, 0.433, 0.54),
     (2, 128, 128, 128): (2.94, 0.499, 0.53),
@@ -130,7 +133,7 @@ def _cheapest_tile(M, N, K, batch=1, single_pass=False):
 # into 2 to 8 ranges: the tile the fit picks is 2.5 % behind the best measured one on average. The pair tiles of 128 and
 # 192 columns, whose A goes through tensor memory, are ahead on the middling shapes (640x2624x1024 25 us against 31 with
 # the best of the others, 896x1536x6144 80 / 83, 6272x640x6144 223 / 281 with 256 columns), 128 rows by 256 columns on
-# few rows and long K (128x11008x11008 170 / 226), 256 by 256 on the largest (4096^3 509 / 552 with 192 columns).
+# few rows and long K (128x11008x11008 170 / 226), 256 by 256 on the largest (4096^3 488 / 510 with 192 columns).
 _TILE_COST_F32 = {
     (2, 128, 64, 32): (2.88, 17.2, 1.44, 4.62, 6),
     (2, 128, 128, 32): (2.46, 20.2, 3.48, 6.14, 4),
@@ -175,10 +178,12 @@ def tuned_config(M: int, N: int, K: int, dtype: EnumKernelDType, isATranspose: i
                  b_transposed: bool = False, single_pass: bool = False) -> KernelArgMatmul:
     """Best known config of a shape: the kernel database's entry when the shape was tuned; else (16-bit types, and
     single fp32 products) the tile with the smallest estimated time - the plain rule's choice is kept while the estimate
-    puts it within 10 % of that (5 % for a cluster split-K tile: 512x4096x11008 39.4 estimated against 36.3 with the best
-    tile, 41.3 and 36.4 measured): the estimates of the two largest tiles are up to that much too low where a remainder is
+    puts it within 10 % of that: the estimates of the two largest tiles are up to that much too low where a remainder is
     cut up (2048x11008x4096: 512x256x64 estimated 110, 256x256x128 118 us; measured 142 and 135, and 165 and 148 once the
-    power cap holds the clock down). ``batch`` > 1: M, N, K are one batch's, the config fits all batches' tiles walked
+    power cap holds the clock down). A plain cluster split-K choice is kept within 5 %: of 46 shapes (128 to 512 rows, K 2048 to
+    14336) where it is 5 to 10 % behind by estimate the cheapest tile was 3 to 20 % ahead, measured, on all but those with 44
+    clusters of three (512x4096x11008 39.4 estimated against 36.3, 40.0 and 35.9 measured); within 5 % it was ahead by 4 to 16 %
+    on five shapes, behind by 10 % on one. ``batch`` > 1: M, N, K are one batch's, the config fits all batches' tiles walked
     together, and the database, which holds single products, is not asked. ``b_transposed``: B is stored N x K.
     ``single_pass``: a config of the single-pass kernels (KERNEL_VARIANT 2 and 4), which alone can store fp32 results of
     16-bit operands; 16-bit types."""
