@@ -13,6 +13,7 @@ NUM_CFG_KEYS = 31
 LIB_NAME = "libkcg_b200.so"
 
 KERNEL_AUTO, KERNEL_SIMT, KERNEL_TCGEN05, KERNEL_TF32X1, KERNEL_TCGEN05_PAIR, KERNEL_TCGEN05_CLUSTERK = 0, 1, 2, 3, 4, 5
+KERNEL_F32_SPLIT = 6
 KERNEL_NAIVE, KERNEL_WAIT_PROBE = 100, 101
 
 E_BAD_CONFIG, E_COMPILE, E_NO_DRIVER, E_IO, E_DEVICE_TIMEOUT, E_BAD_ARG, E_TOO_LARGE = (

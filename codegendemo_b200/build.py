@@ -54,8 +54,9 @@ def build_library(force: bool = False) -> str:
     kdir = os.path.join(HERE, "csrc", "kernels")  # the allocation-free entry instantiates a kernel from these
     deps = srcs + [os.path.join(kdir, f) for f in sorted(os.listdir(kdir))] + [
         os.path.join(os.path.dirname(HERE), "include", "kcg_b200.h")]
-    # device code linked into the library itself: the allocation-free split-K entry and the row softmax
-    extra = [os.path.join(HERE, "csrc", f) for f in ("kcg_noalloc.cu", "kcg_softmax.cu", "kcg_attention.cu")]
+    # device code linked into the library itself: the allocation-free split-K entry, the row softmax, the fused attention
+    # and the split of fp32 operands
+    extra = [os.path.join(HERE, "csrc", f) for f in ("kcg_noalloc.cu", "kcg_softmax.cu", "kcg_attention.cu", "kcg_f32split.cu")]
     deps += extra
     if not force and _newer(out, deps):
         return out

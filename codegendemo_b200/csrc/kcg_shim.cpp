@@ -33,6 +33,9 @@
 
 #include "../../include/kcg_b200.h"
 #include "kernels/gemm_params.h"
+#include "kernels/split_f32.h"
+
+extern "C" int kcg_internal_split_f32(uint64_t stream, const kcg::SplitF32Args* q, int pdl);  // kcg_f32split.cu
 
 extern char** environ;
 
@@ -140,6 +143,7 @@ struct StreamSlot {
   uint64_t last_use = 0;
 };
 constexpr size_t kMaxStreamSlots = 32;
+constexpr size_t kMaxWorkspaceBytes = size_t(4) << 30;  // of all streams of a device together
 
 // Workspace and tile counters of the launches that one capture queued on one stream. The graph
 // runs on any stream, beside any other graph and as often as it likes, long after the stream's own
@@ -153,7 +157,8 @@ struct GraphBuffer {
   std::atomic<bool> held{false};
   CUdeviceptr counters() const { return ws + ((ws_bytes + 255) / 256) * 256; }
 };
-constexpr size_t kMaxFreeGraphBuffers = 4;  // freed ones that are kept
+constexpr size_t kMaxFreeGraphBuffers = 4;  // freed ones that are kept ...
+constexpr size_t kMaxFreeGraphBytes = size_t(1) << 30;  // ... and their bytes
 
 // What a 2-D tensor map depends on.
 struct MapKey {
@@ -249,7 +254,7 @@ void CUDA_CB release_graph_buffer(void* p) { static_cast<GraphBuffer*>(p)->held.
 int graph_buffer(DeviceState* s, CUstream stream, unsigned long long id, CUgraph graph, size_t need, size_t counters_n,
                  GraphBuffer** out) {
   GraphBuffer* best = nullptr;
-  size_t free_ones = 0;
+  size_t free_ones = 0, free_bytes = 0;
   for (GraphBuffer* b : s->graph_buffers) {
     const bool held = b->held.load();
     const bool fits = b->ws_bytes >= need && b->counters_n >= counters_n;
@@ -259,16 +264,18 @@ int graph_buffer(DeviceState* s, CUstream stream, unsigned long long id, CUgraph
     }
     if (held) continue;
     ++free_ones;
+    free_bytes += b->ws_bytes;
     if (fits && (!best || b->ws_bytes < best->ws_bytes)) best = b;
   }
   RelaxedCapture relaxed;
   if (!best) {
-    for (size_t i = 0; i < s->graph_buffers.size() && free_ones > kMaxFreeGraphBuffers;) {
+    for (size_t i = 0; i < s->graph_buffers.size() && (free_ones > kMaxFreeGraphBuffers || free_bytes > kMaxFreeGraphBytes);) {
       GraphBuffer* b = s->graph_buffers[i];
       if (b->held.load()) {
         ++i;
         continue;
       }
+      free_bytes -= b->ws_bytes;
       DRV(cuMemFree(b->ws));
       s->graph_buffers.erase(s->graph_buffers.begin() + i);
       delete b;
@@ -297,6 +304,25 @@ int graph_buffer(DeviceState* s, CUstream stream, unsigned long long id, CUgraph
   }
   *out = best;
   return 0;
+}
+
+// Before `slot`'s workspace grows to `need` bytes: workspaces of other streams, the least recently used ones first, are
+// given back until all of them stay within kMaxWorkspaceBytes (the splits of fp32 operands are as large as the operands).
+int make_room(DeviceState* s, StreamSlot* slot, size_t need) {
+  for (;;) {
+    size_t held = need;
+    StreamSlot* oldest = nullptr;
+    for (StreamSlot& sl : s->slots) {
+      if (&sl == slot || !sl.ws) continue;
+      held += sl.ws_bytes;
+      if (!oldest || sl.last_use < oldest->last_use) oldest = &sl;
+    }
+    if (held <= kMaxWorkspaceBytes || !oldest) return 0;
+    RelaxedCapture relaxed;
+    DRV(cuMemFree(oldest->ws));  // (waits for the work that still uses it)
+    oldest->ws = 0;
+    oldest->ws_bytes = 0;
+  }
 }
 
 int free_slot(StreamSlot& sl) {
@@ -444,8 +470,9 @@ int resolve(const Cfg& c, const kcg_compile_opts* opts, Resolved* r) {
   if (r->edge) {
     // Tiles that hang over an edge: TMA reads zeros past it and clips the stores; direct stores and the fused
     // epilogue work in whole blocks of 32 (fp32) or 64 columns, which therefore must not straddle the edge.
-    if (!(want == KCG_KERNEL_TCGEN05 || want == KCG_KERNEL_TCGEN05_PAIR || want == KCG_KERNEL_TCGEN05_CLUSTERK))
-      return fail(KCG_E_BAD_CONFIG, "tiles over the edge need a tcgen05 kernel (KERNEL_VARIANT 2, 4 or 5)");
+    if (!(want == KCG_KERNEL_TCGEN05 || want == KCG_KERNEL_TCGEN05_PAIR || want == KCG_KERNEL_TCGEN05_CLUSTERK ||
+          want == KCG_KERNEL_F32_SPLIT))
+      return fail(KCG_E_BAD_CONFIG, "tiles over the edge need a tcgen05 kernel (KERNEL_VARIANT 2, 4, 5 or 6)");
     const int nstep = dt == KCG_DTYPE_FLOAT32 ? 32 : 64;
     if (N % nstep || (K * (dt == KCG_DTYPE_FLOAT32 ? 4 : 2)) % 16)
       return fail(KCG_E_BAD_CONFIG, "tiles over the edge need N a multiple of %d and rows of 16-byte units", nstep);
@@ -455,7 +482,7 @@ int resolve(const Cfg& c, const kcg_compile_opts* opts, Resolved* r) {
   r->btrans = (opts && opts->b_trans) ? 1 : 0;
   r->serpentine = (opts && opts->serpentine) ? 1 : 0;
   if (r->serpentine && !(want == KCG_KERNEL_TCGEN05 || want == KCG_KERNEL_TF32X1 || want == KCG_KERNEL_TCGEN05_PAIR ||
-                         want == KCG_KERNEL_TCGEN05_CLUSTERK))
+                         want == KCG_KERNEL_TCGEN05_CLUSTERK || want == KCG_KERNEL_F32_SPLIT))
     return fail(KCG_E_BAD_CONFIG, "the serpentine raster belongs to the tcgen05 kernels' tile walk");
   if (r->serpentine && c[KCG_CFG_BLOCK_MAPPING] < 2)
     return fail(KCG_E_BAD_CONFIG, "the serpentine raster needs BLOCK_MAPPING >= 2 (rows per group)");
@@ -493,6 +520,17 @@ int resolve(const Cfg& c, const kcg_compile_opts* opts, Resolved* r) {
     if (!ok(st)) return fail(KCG_E_BAD_CONFIG, "tile %dx%dx%d / %d stages not buildable by the CTA-pair kernel", bm, bn, bk, st);
     if (N % 8) return fail(KCG_E_BAD_CONFIG, "N must be a multiple of 8 for TMA row strides");
     r->stages = st;
+  } else if (want == KCG_KERNEL_F32_SPLIT) {
+    if (dt != KCG_DTYPE_FLOAT32 || c[KCG_CFG_IS_ATRANS])
+      return fail(KCG_E_BAD_CONFIG, "the split fp32 kernel needs float32 data and an A stored M x K");
+    if (const int e = kcg::h2_config_error(bm, bn, bk))
+      return fail(KCG_E_BAD_CONFIG, "tile %dx%dx%d not buildable by the split fp32 kernel (rule %d)", bm, bn, bk, e);
+    if (opts && opts->num_stages > 0 && opts->num_stages != kcg::h2_stages(bn))
+      return fail(KCG_E_BAD_CONFIG, "the split fp32 kernel has %d stages for tiles of %d columns", kcg::h2_stages(bn), bn);
+    const int splitk = c[KCG_CFG_LOCAL_SPLIT_U] > 0 ? c[KCG_CFG_LOCAL_SPLIT_U] : 1;
+    if (splitk > blocks_of(K, bk)) return fail(KCG_E_BAD_CONFIG, "LOCAL_SPLIT_U %d exceeds the %d K blocks", splitk, blocks_of(K, bk));
+    if (N % 64 || K % 4) return fail(KCG_E_BAD_CONFIG, "the split fp32 kernel needs N a multiple of 64 and K of 4");
+    r->stages = kcg::h2_stages(bn);
   } else if (want == KCG_KERNEL_TCGEN05_CLUSTERK) {
     // one 128-row tile per cluster of LOCAL_SPLIT_U CTAs (256 rows: CTA pairs), partial tiles reduced in shared memory
     const int split = c[KCG_CFG_LOCAL_SPLIT_U], ck_pair = bm == 256 ? 1 : 0;
@@ -762,6 +800,12 @@ int fill_info(const Cfg& c, const Resolved& r, const std::string& name, const st
     out->cluster[0] = 2;
     out->block[0] = f32 ? kcg::tc_x3_threads(kcg::tc_x3_tmem_a(bm / 2, bn / 2, bk, r.stages, 2), 2) : 256;
     out->smem_bytes = kcg::tc_smem_bytes(c[KCG_CFG_DATATYPE_A], bm / 2, bn / 2, bk, r.stages, 2 * f32);
+  } else if (r.kernel == KCG_KERNEL_F32_SPLIT) {
+    const int units = tiles * lsu, pairs = units < r.num_sms / 2 ? units : r.num_sms / 2;
+    out->grid[0] = 2 * pairs;
+    out->cluster[0] = 2;
+    out->block[0] = kcg::tc_x3_threads(kcg::tc_x3_tmem_a(128, bn / 2, 32, kcg::h2_x3_stages(bn), 2), 2);
+    out->smem_bytes = kcg::h2_smem_bytes(bn);
   } else if (r.kernel == KCG_KERNEL_TCGEN05_CLUSTERK) {
     out->grid[0] = tiles * lsu * (bm / 128);  // one cluster of LOCAL_SPLIT_U CTAs (CTA pairs) per tile
     out->cluster[0] = lsu * (bm / 128);
@@ -810,6 +854,15 @@ int fill_info(const Cfg& c, const Resolved& r, const std::string& name, const st
   return 0;
 }
 
+// KCG_PDL=0 turns programmatic dependent launch off (read once).
+bool pdl_on() {
+  static const bool on = [] {
+    const char* e = getenv("KCG_PDL");
+    return !(e && e[0] == '0');
+  }();
+  return on;
+}
+
 int encode_map(DeviceState* s, CUtensorMap* out, int dtype, uint64_t ptr, uint64_t inner, uint64_t outer,
                uint64_t row_bytes, int box_inner, int box_outer, int swizzle) {
   const MapKey key{ptr, inner, outer, row_bytes, dtype, box_inner, box_outer, swizzle};
@@ -843,8 +896,9 @@ struct SplitPlan {
 
 SplitPlan plan_split(const kcg_kernel_info* info, bool fused_epilogue, int batch = 1) {
   const int M = info->m * batch, N = info->n, K = info->k;  // a batched product is one tall problem
-  const bool pair = info->kernel == KCG_KERNEL_TCGEN05_PAIR;
-  const bool x3 = info->dtype == KCG_DTYPE_FLOAT32 && info->kernel != KCG_KERNEL_TF32X1;
+  const bool h2 = info->kernel == KCG_KERNEL_F32_SPLIT;
+  const bool pair = info->kernel == KCG_KERNEL_TCGEN05_PAIR || h2;
+  const bool x3 = info->dtype == KCG_DTYPE_FLOAT32 && info->kernel != KCG_KERNEL_TF32X1;  // sums in registers, split units last
   // K splitting. LOCAL_SPLIT_U > 1 splits every tile evenly. Otherwise the tiles that do not fill
   // a wave of the persistent grid (the remainder) can be split over the CTAs so that every SM works
   // for about the same time:
@@ -881,8 +935,8 @@ SplitPlan plan_split(const kcg_kernel_info* info, bool fused_epilogue, int batch
     if (mode != 0 && rem > 0) {
       // Worth it only when the time saved exceeds the cost of the split. A tile's main-loop time is
       // estimated from a per-SM rate in MFLOP per microsecond: 10 for 16-bit data, 1.4 useful for fp32
-      // as 3xTF32, 4.5 for the single TF32 pass.
-      const double mflop_per_us = (info->dtype == KCG_DTYPE_FLOAT32 && info->kernel != KCG_KERNEL_TF32X1) ? 1.4
+      // as 3xTF32, 4 as three fp16 products, 4.5 for the single TF32 pass.
+      const double mflop_per_us = h2 ? 4.0 : (info->dtype == KCG_DTYPE_FLOAT32 && info->kernel != KCG_KERNEL_TF32X1) ? 1.4
                                   : (info->dtype == KCG_DTYPE_FLOAT32)                                     ? 4.5
                                                                                                            : 10.0;
       const double tile_us =
@@ -967,7 +1021,7 @@ SplitPlan plan_split(const kcg_kernel_info* info, bool fused_epilogue, int batch
   // The 3xTF32 kernel applies a fused epilogue in its reduction loop only (its register file is
   // full of accumulators at the direct store), so a fused launch sends every tile through the
   // workspace as a one-way split; the tail split is not combined with it.
-  const bool ws_epilogue = x3 && fused_epilogue;
+  const bool ws_epilogue = x3 && !h2 && fused_epilogue;
   if (ws_epilogue && info->splitk <= 1) {
     first = 0;
     factor = 1;
@@ -1284,7 +1338,8 @@ static int launch_impl(uint64_t function, const kcg_kernel_info* info, int devic
   p.n_peers = n_peers;
   for (int i = 0; i < n_peers; ++i) p.peerC[i] = reinterpret_cast<void*>(peer_c[i]);
   int grid0 = info->grid[0];
-  const bool pair = info->kernel == KCG_KERNEL_TCGEN05_PAIR;
+  const bool h2 = info->kernel == KCG_KERNEL_F32_SPLIT;
+  const bool pair = info->kernel == KCG_KERNEL_TCGEN05_PAIR || h2;
   // Tensor maps of A and B for a tcgen05 kernel whose per-CTA operand slices have layout L.
   auto encode_operands = [&](const kcg::TcLayout& L) -> int {
     if (info->atrans) {
@@ -1310,9 +1365,10 @@ static int launch_impl(uint64_t function, const kcg_kernel_info* info, int devic
       return e;
     grid0 = blocks_of(M, info->bm) * blocks_of(N, info->bn) * info->splitk * ctas;
   }
-  if (info->kernel == KCG_KERNEL_TCGEN05 || info->kernel == KCG_KERNEL_TF32X1 || pair) {
+  if (info->kernel == KCG_KERNEL_TCGEN05 || info->kernel == KCG_KERNEL_TF32X1 || pair) {  // (pair: variants 4 and 6)
     // the pair kernel loads per-CTA slices: BM/2 rows of A, BN/2 columns of B
-    if (int e = encode_operands(pair ? kcg::make_tc_layout(info->dtype, info->bm / 2, info->bn / 2, info->bk,
+    // (the split fp32 kernel: the maps of the 3xTF32 kernel it falls back to, whose K blocks are 32)
+    if (int e = encode_operands(pair ? kcg::make_tc_layout(info->dtype, info->bm / 2, info->bn / 2, h2 ? 32 : info->bk,
                                                            info->atrans, btrans)
                                      : kcg::make_tc_layout(info->dtype, info->bm, info->bn, info->bk, info->atrans,
                                                            btrans)))
@@ -1329,6 +1385,7 @@ static int launch_impl(uint64_t function, const kcg_kernel_info* info, int devic
     const int T = plan.tiles, first = plan.first, factor = plan.factor, sk_per = plan.sk_per,
               sk_ranges = plan.sk_ranges, G = plan.units_at_once;
     const bool ws_epilogue = x3 && p.epi_flags != 0u;
+    p.whole_slot0 = h2 ? (T - first) * factor : -1;
     // Under stream-K the whole tiles before the tail are walked with the grid as stride: the grid
     // stays at every unit that runs at once even when the tail is cut into fewer ranges (the CTAs
     // beyond the last range then simply have no tail piece).
@@ -1340,12 +1397,22 @@ static int launch_impl(uint64_t function, const kcg_kernel_info* info, int devic
     p.split_units_first = plan.units_first;
     CUdeviceptr ws = 0;
     size_t ws_bytes = 0;
-    if (factor > 1 || ws_epilogue || sk_per > 0) {
+    kcg::SplitF32Layout parts{};
+    bool split_now = h2;  // false: no memory for the parts; the kernel then reads the fp32 operands
+    if (factor > 1 || ws_epilogue || sk_per > 0 || h2) {
       // slots: one per (tile, split) of an even split; range index + tile index under stream-K
       const size_t slots = sk_per > 0 ? static_cast<size_t>(sk_ranges) + (T - first)
-                                      : static_cast<size_t>(T - first) * factor;
-      const size_t need = slots * info->bm * info->bn * sizeof(float);
-      const size_t tiles = static_cast<size_t>(T - first) * (pair ? 2 : 1);  // one counter per CTA half
+                                      : static_cast<size_t>(T - first) * factor + (h2 && ws_epilogue ? G : 0);
+      const size_t partials = slots * info->bm * info->bn * sizeof(float);
+      size_t need = partials;
+      // one counter per CTA half; before them the two words of the split fp32 kernel
+      const size_t tiles = static_cast<size_t>(T - first) * (pair ? 2 : 1) + (h2 ? 4 : 0);
+      if (h2) {
+        parts = kcg::split_f32_layout(partials, M, N, K);
+        need = parts.end;
+        split_now = need <= kMaxWorkspaceBytes;
+        if (!split_now) need = partials;
+      }
       CUstreamCaptureStatus capturing = CU_STREAM_CAPTURE_STATUS_NONE;
       cuuint64_t id = 0;
       CUgraph graph = nullptr;
@@ -1354,14 +1421,25 @@ static int launch_impl(uint64_t function, const kcg_kernel_info* info, int devic
                                                nullptr, nullptr) == CUDA_SUCCESS &&
           capturing == CU_STREAM_CAPTURE_STATUS_ACTIVE) {
         GraphBuffer* buf = nullptr;
-        if (int e = graph_buffer(s, reinterpret_cast<CUstream>(stream), id, graph, need, tiles, &buf)) return e;
+        int e = graph_buffer(s, reinterpret_cast<CUstream>(stream), id, graph, need, tiles, &buf);
+        if (e == CUDA_ERROR_OUT_OF_MEMORY && split_now) {
+          split_now = false;
+          e = graph_buffer(s, reinterpret_cast<CUstream>(stream), id, graph, partials, tiles, &buf);
+        }
+        if (e) return e;
         ws = buf->ws;
         ws_bytes = buf->ws_bytes;
         p.tile_counters = reinterpret_cast<unsigned int*>(buf->counters());
       } else {
         if (slot->ws_bytes < need) {
           s->tmaps.clear();  // drops the maps of the workspace that is about to move
-          if (int e = grow(&slot->ws, &slot->ws_bytes, need)) return e;
+          if (int e = make_room(s, slot, need)) return e;
+          int e = grow(&slot->ws, &slot->ws_bytes, need);
+          if (e == CUDA_ERROR_OUT_OF_MEMORY && split_now) {
+            split_now = false;
+            e = grow(&slot->ws, &slot->ws_bytes, partials);
+          }
+          if (e) return e;
         }
         if (slot->counters_n < tiles) {
           size_t have = slot->counters_n * 4;
@@ -1375,6 +1453,40 @@ static int launch_impl(uint64_t function, const kcg_kernel_info* info, int devic
         p.tile_counters = reinterpret_cast<unsigned int*>(slot->counters);
       }
       p.splitk_ws = reinterpret_cast<float*>(ws);
+      if (h2) {
+        unsigned int* words = p.tile_counters;
+        p.tile_counters += 4;
+        if (split_now) p.h2_words = words;
+      }
+    }
+    if (split_now) {
+      kcg::SplitF32Args q;
+      q.A = reinterpret_cast<const float*>(A);
+      q.B = reinterpret_cast<const float*>(B);
+      q.lda = lda;
+      q.ldb = ldb;
+      q.M = M;
+      q.N = N;
+      q.K = K;
+      q.parts_a = reinterpret_cast<uint8_t*>(ws + parts.parts_a);
+      q.parts_b = reinterpret_cast<uint8_t*>(ws + parts.parts_b);
+      q.scale_a = reinterpret_cast<float*>(ws + parts.scale_a);
+      q.scale_b = reinterpret_cast<float*>(ws + parts.scale_b);
+      q.scale_lda = p.scale_lda = parts.scale_lda;
+      q.scale_ldb = p.scale_ldb = parts.scale_ldb;
+      q.words = p.h2_words;
+      q.columns = reinterpret_cast<float*>(ws + parts.columns);
+      p.columns = q.columns;
+      p.scale_a = q.scale_a;
+      p.scale_b = q.scale_b;
+      // the parts as one matrix of 64 halves a row, A's and then B's, up to the last row of B's: boxes past it read zeros
+      const uint64_t kb = blocks_of(K, kcg::H2_BK), row_b0 = (parts.parts_b - parts.parts_a) / 128;
+      p.parts_b_row = static_cast<int>(row_b0);
+      if (int e = encode_map(s, &p.tmWs, KCG_DTYPE_FLOAT16, ws + parts.parts_a, 64, row_b0 + blocks_of(N, 64) * kb * 128, 128,
+                             64, 128, 3))
+        return e;
+      if (int e = encode_map(s, &p.tmC, KCG_DTYPE_FLOAT32, C, N, M, static_cast<uint64_t>(ldc) * 4, 32, 32, 3)) return e;
+      if (int e = kcg_internal_split_f32(stream, &q, pdl_on() ? 1 : 0)) return e;
     }
     if (!x3 && (factor > 1 || sk_per > 0)) {
       // The single-pass kernel writes its partial tiles with TMA stores: the workspace as one tall
@@ -1413,13 +1525,9 @@ static int launch_impl(uint64_t function, const kcg_kernel_info* info, int devic
   // set themselves up and wait there for its completion, instead of being launched only then.
   // KCG_PDL=0 turns it off.
   {
-    static const bool pdl_on = [] {
-      const char* e = getenv("KCG_PDL");
-      return !(e && e[0] == '0');
-    }();
-    const bool guarded = info->kernel == KCG_KERNEL_TCGEN05 || info->kernel == KCG_KERNEL_TCGEN05_PAIR ||
+    const bool guarded = info->kernel == KCG_KERNEL_TCGEN05 || info->kernel == KCG_KERNEL_TCGEN05_PAIR || h2 ||
                          info->kernel == KCG_KERNEL_TF32X1 || info->kernel == KCG_KERNEL_TCGEN05_CLUSTERK;
-    if (pdl_on && guarded) {
+    if (pdl_on() && guarded) {
       attr[cfg.numAttrs].id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
       attr[cfg.numAttrs].value.programmaticStreamSerializationAllowed = 1;
       ++cfg.numAttrs;
@@ -1480,7 +1588,7 @@ int kcg_matmul_host(uint64_t function, const kcg_kernel_info* info, int device, 
   const int bm = info->bm > 0 ? info->bm : 1;
   const int tiles_m = blocks_of(info->m, bm);
   const bool tensor_core = info->kernel == KCG_KERNEL_TCGEN05 || info->kernel == KCG_KERNEL_TF32X1 ||
-                           info->kernel == KCG_KERNEL_TCGEN05_PAIR;
+                           info->kernel == KCG_KERNEL_TCGEN05_PAIR || info->kernel == KCG_KERNEL_F32_SPLIT;
   int nslabs = 1;
   if (tensor_core && !info->atrans && bytes[0] + bytes[2] >= (64u << 20) && tiles_m >= 4) {
     // up to 16 slabs, none smaller than ~16 MiB of A + C: what is not overlapped is the first

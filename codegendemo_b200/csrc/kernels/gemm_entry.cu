@@ -80,6 +80,13 @@ extern "C" __global__ void __launch_bounds__(Gemm::NUM_THREADS, 1)
 KCG_KERNEL_NAME(const __grid_constant__ KcgGemmParams p) {
   Gemm::run(p);
 }
+#elif KCG_VARIANT == KCG_VARIANT_F32H2
+#include "gemm_tcgen05_f32h2.cuh"
+using Gemm = kcg::TcGemmF32H2<KCG_BN, KCG_SPLITK, KCG_GROUP>;
+extern "C" __global__ void __launch_bounds__(Gemm::NUM_THREADS, 1)
+KCG_KERNEL_NAME(const __grid_constant__ KcgGemmParams p) {
+  Gemm::run(p);
+}
 #elif KCG_VARIANT == KCG_VARIANT_SIMT
 #include "gemm_simt.cuh"
 using Gemm = kcg::SimtGemm<KCG_T, KCG_BM, KCG_BN, KCG_BK, KCG_TM, KCG_TN, KCG_BLM, KCG_BLN, KCG_WLM,

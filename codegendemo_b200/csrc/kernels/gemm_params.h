@@ -26,6 +26,10 @@
 // distributed shared memory (fp16 / bf16, 128-row tiles, or 256-row tiles on CTA pairs): no workspace, no counters
 #define KCG_VARIANT_TCGEN05_CLUSTERK 5
 
+// fp32 through two fp16 parts per value, split in memory before the product (CTA pairs; 3xTF32 where the parts cannot
+// carry a value)
+#define KCG_VARIANT_F32H2 6
+
 #define KCG_MAX_PEERS 7  // other GPUs of one NVSwitch domain of eight
 
 // epi_flags bits
@@ -79,6 +83,17 @@ struct alignas(64) KcgGemmParams {
   float alpha, beta;
   const void* bias;
   unsigned int epi_flags;  // KCG_EPI_*
+  // fp32 kernels: workspace slots of whole tiles that go through the workspace (fused epilogue), one per CTA (pair) from
+  // this on; -1: the tile's own slot.
+  int whole_slot0;
+  // KERNEL_VARIANT 6 (gemm_tcgen05_f32h2.cuh): the factors of the parts' products, [K block][rows of A] and [K block][64
+  // columns of B] with these pitches, those of the finished columns, and {not every value splits, CTAs done}; no words:
+  // 3xTF32 throughout. tmWs maps the parts, those of B from row parts_b_row on.
+  const float* scale_a;
+  const float* scale_b;
+  const float* columns;
+  int scale_lda, scale_ldb, parts_b_row;
+  unsigned int* h2_words;
   // Fused all-gather of an M-sharded product: besides C, every finished tile is also written
   // to the same rows / columns of n_peers more matrices with C's pitch — this rank's slab inside
   // the full C of every other GPU, mapped into this process (coalesced 16-byte stores over NVLink
@@ -256,9 +271,27 @@ constexpr int ck_config_error(int dtype, int BN, int BK, int stages, int split, 
 }
 constexpr int ck_smem_bytes(int BN, int BK, int stages, int pair = 0) { return ck_ring_bytes(BN, BK, stages, pair) + 2048; }
 
+// fp32 through fp16 parts (gemm_tcgen05_f32h2.cuh): 256-row tiles on CTA pairs; the kernel it falls back to is the 3xTF32
+// pair kernel of the same tile with K blocks of 32 and h2_x3_stages stages.
+constexpr int H2_BK = 64;  // K block = chunk of one exponent
+constexpr int h2_config_error(int BM, int BN, int BK) {
+  if (BM != 256) return 2;
+  if (BN != 128 && BN != 256) return 3;
+  return BK == H2_BK ? 0 : 5;
+}
+constexpr int h2_x3_stages(int BN) { return BN == 256 ? 3 : 6; }
+constexpr int h2_stages(int BN) { return BN == 256 ? 3 : 4; }
+
 constexpr int tc_smem_bytes(int dtype, int BM, int BN, int BK, int stages, int x3) {
   // +1024 alignment slack, +1024 barriers / TMEM holder / flags, + epilogue staging
   return tc_ring_bytes(dtype, BM, BN, BK, stages, x3) + 2048 + tc_staging_bytes(dtype, x3);
+}
+
+constexpr int h2_smem_bytes(int BN) {
+  // ring, staging of the store, barriers, alignment slack; at least what the fallback takes
+  const int own = h2_stages(BN) * (128 + BN / 2) * H2_BK * 4 + 8 * 32 * 128 + 2048;
+  const int x3 = tc_smem_bytes(KCG_DT_F32, 128, BN / 2, 32, h2_x3_stages(BN), 2);
+  return own > x3 ? own : x3;
 }
 
 }  // namespace kcg

@@ -495,6 +495,8 @@ struct TcGemmF32x3 {
         // the reduction loop below, where the accumulators are dead: with all of them live
         // there are no registers left for the bias / C operands.
         const bool via_ws = w.nsplit > 1 || p.epi_flags != 0u;
+        // the tile's first contributor's; a whole tile's own, or one that all whole tiles of this CTA (pair) take in turn
+        const int slot0 = w.nsplit > 1 || p.whole_slot0 < 0 ? w.slot - w.split : p.whole_slot0 + unit0;
 #pragma unroll
         for (int t = 0; t < MT; ++t) {
           const int row = w.m0 + row_base + t * 128 + row_in_acc;
@@ -507,7 +509,7 @@ struct TcGemmF32x3 {
               // warp store (and the reducer's loads) 512 contiguous bytes. Row-major partials, 16
               // bytes per lane at a 1 KB stride, made L2 merge every sector.
               float4* d4 = via_ws ? reinterpret_cast<float4*>(p.splitk_ws +
-                                                             (static_cast<size_t>(w.slot) * kBM + row_base) * kBN) +
+                                                             (static_cast<size_t>(slot0 + w.split) * kBM + row_base) * kBN) +
                                         (t * PIECES + c) * 8 * NUM_EPI_THREADS + epi_tid
                                   : reinterpret_cast<float4*>(Cout + static_cast<size_t>(row) * p.ldc + col);
               const int step = via_ws ? NUM_EPI_THREADS : 1;
@@ -552,7 +554,7 @@ struct TcGemmF32x3 {
                 for (int s = 0; s < w.nsplit; ++s) {
                   const float4* src =
                       reinterpret_cast<const float4*>(
-                          p.splitk_ws + ((static_cast<size_t>(w.slot - w.split) + s) * kBM + row_base) * kBN) +
+                          p.splitk_ws + (static_cast<size_t>(slot0 + s) * kBM + row_base) * kBN) +
                       (t * PIECES + c) * 8 * NUM_EPI_THREADS + epi_tid;
 #pragma unroll
                   for (int i = 0; i < 8; ++i) {

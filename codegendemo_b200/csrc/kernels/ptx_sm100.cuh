@@ -48,6 +48,10 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
 }
 
 // Makes mbarrier.init visible to the async proxy (TMA, tcgen05.commit).
+// Before the memory of a barrier nobody uses any more is used for something else.
+__device__ __forceinline__ void mbar_inval(uint64_t* bar) {
+  asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 __device__ __forceinline__ void fence_mbar_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
@@ -557,6 +561,20 @@ __device__ __forceinline__ void umma_ss_pair(uint32_t tmem_d, uint64_t adesc, ui
         : "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
   }
+}
+
+// D[tmem] = A * B + D * 2^-kShift, fp16 / bf16 operands, over both CTAs of the pair.
+template <int kShift>
+__device__ __forceinline__ void umma_ss_pair_f16_scaled_d(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.b32 p, 1, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p, %4;\n\t"
+      "}\n"
+      :
+      : "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "n"(kShift)
+      : "memory");
 }
 
 // Completion of the pair MMAs issued so far -> one arrival on the barrier at

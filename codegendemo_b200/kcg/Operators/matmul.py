@@ -120,7 +120,7 @@ class KernelArgMatmul:
 
     def usesTensorCores(self) -> bool:
         """True when the config's tile is one the tcgen05 kernel can build (what AUTO resolves to)."""
-        if self.KERNEL_VARIANT in (2, 3, 4, 5):
+        if self.KERNEL_VARIANT in (2, 3, 4, 5, 6):
             return True
         if self.KERNEL_VARIANT == 1:
             return False
@@ -145,7 +145,7 @@ class KernelArgMatmul:
             assert self.WARP_LAYOUT_N * self.WARP_LAYOUT_M == self.WARP_SIZE
         # shm size check
         # a CTA pair splits the tile's operands
-        per_cta = 2 if self.KERNEL_VARIANT == 4 or self.KERNEL_VARIANT == 5 and self.BLOCK_SIZE_M == 256 else 1
+        per_cta = 2 if self.KERNEL_VARIANT in (4, 6) or self.KERNEL_VARIANT == 5 and self.BLOCK_SIZE_M == 256 else 1
         assert 2 * (self.BLOCK_SIZE_M + self.BLOCK_SIZE_N) * self.BLOCK_SIZE_K * sizeof(self.__dataType_A) // per_cta \
             <= MAX_SHARED_BYTES
         if verbose:

@@ -236,7 +236,8 @@ class ConfigKeywords:
     # Optional keys of this library (absent from the reference's JSONs; defaults apply).
     KEY_NUM_STAGES = "NUM_STAGES"          # shared-memory pipeline depth of the tcgen05 kernels
     KEY_KERNEL_VARIANT = "KERNEL_VARIANT"  # 0 auto, 1 SIMT FFMA, 2 tcgen05 (fp32: 3xTF32), 3 TF32 x1, 4 CTA pairs,
-    #                                        5 cluster split-K (LOCAL_SPLIT_U CTAs per tile, shared-memory reduction)
+    #                                        5 cluster split-K (LOCAL_SPLIT_U CTAs per tile, shared-memory reduction),
+    #                                        6 fp32 as fp16 parts split in memory
     KEY_IS_B_TRANSPOSE = "IS_BTRANS"       # 1 = B stored N x K row-major (16-bit tcgen05 kernels)
     KEY_EDGE_TILES = "EDGE_TILES"  # 1 = tiles may hang over the edges of the problem (tcgen05 kernels)
     KEY_RASTER_SERPENTINE = "RASTER_SERPENTINE"  # 1 = serpentine walk inside a BLOCK_MAPPING group (tcgen05 kernels)

@@ -174,6 +174,46 @@ def _cheapest_tile_f32(M, N, K, sms=148):
     return best
 
 
+# Tiles of the split fp32 kernel (KERNEL_VARIANT 6): BLOCK_SIZE_N -> microseconds {fixed, with the split's launch; per million
+# values of A and B for the split; per 64 values of K; per tile beyond them; per cut into K ranges}. Fitted to 111 device
+# timings (graph replay, rotating operands) on 32 shapes of 128..4864 x 512..11008 x 256..10496, 9 % rms; large products,
+# which the power cap slows down by up to a third, are estimated as much too low as the 3xTF32 tiles above.
+_TILE_COST_F32_SPLIT = {
+    128: (7.5, 1.82, 0.498, 2.4, 2.3),
+    256: (6.6, 1.74, 0.723, 6.0, 7.8),
+}
+_SPLIT_BYTES = 2 << 30  # most memory that a product's parts may take: 4 bytes a value
+
+
+def _tile_us_f32_split(bn, split, M, N, K, sms=148):
+    """Estimated time of an fp32 product on the split kernel, in microseconds."""
+    fixed, per_value, per_block, per_tile, per_cut = _TILE_COST_F32_SPLIT[bn]
+    tiles, blocks, pairs = -(-M // 256) * -(-N // bn), -(-K // 64), sms // 2
+    fixed += per_value * 1e-6 * (M * K + K * N)
+    if split > 1:
+        return fixed + -(-tiles * split // pairs) * (-(-blocks // split) * per_block + per_tile) + per_cut
+    us = fixed + -(-tiles // pairs) * (blocks * per_block + per_tile)
+    f = min(8, pairs // (tiles % pairs)) if tiles % pairs else 0
+    if f >= 2:  # the launcher cuts the remainder tiles into f K ranges when that pays
+        us = min(us, fixed + tiles // pairs * (blocks * per_block + per_tile) + -(-blocks // f) * per_block + per_tile + per_cut)
+    return us
+
+
+def _cheapest_tile_f32_split(M, N, K, sms=148):
+    """(estimate, BLOCK_SIZE_N, split), or None where the parts would take too much memory."""
+    if 4 * (M * K + K * N) > _SPLIT_BYTES:
+        return None
+    best = None
+    for bn in _TILE_COST_F32_SPLIT:
+        for split in (1, 2, 3, 4, 6, 8):
+            if split > 1 and (-(-M // 256) * -(-N // bn) * split > sms // 2 or K // 64 < 4 * split):
+                continue
+            us = _tile_us_f32_split(bn, split, M, N, K)
+            if best is None or us < best[0]:
+                best = (us, bn, split)
+    return best
+
+
 def tuned_config(M: int, N: int, K: int, dtype: EnumKernelDType, isATranspose: int = 0, db=None, batch: int = 1,
                  b_transposed: bool = False, single_pass: bool = False) -> KernelArgMatmul:
     """Best known config of a shape: the kernel database's entry when the shape was tuned; else (16-bit types, and
@@ -215,7 +255,15 @@ def tuned_config(M: int, N: int, K: int, dtype: EnumKernelDType, isATranspose: i
     elif batch == 1 and not isATranspose and M % 128 == 0 and N % 64 == 0 and K % 64 == 0:
         us, tile, split = _cheapest_tile_f32(M, N, K)
         have = (plain.KERNEL_VARIANT or 2, plain.BLOCK_SIZE_M, plain.BLOCK_SIZE_N, plain.BLOCK_SIZE_K)
-        if have not in _TILE_COST_F32 or _tile_us_f32(have, 1, M, N, K) > 1.1 * us:
+        in_parts = _cheapest_tile_f32_split(M, N, K)
+        if in_parts is not None and in_parts[0] < 0.95 * us:
+            # operands split in memory once, not in every tile that reads them: from about 512 rows on (both kernels'
+            # times in _TILE_COST_F32_SPLIT's fit: 128x4096x4096 35 us as 3xTF32, 59 split; 512x8704x2048 79 / 70; 1024x7936x768
+            # 65 / 47; 4096^3 495 / 350; of 32 shapes none that this line sends there was slower)
+            _, bn, split = in_parts
+            plain = default_config(M, N, K, dtype, KERNEL_VARIANT=6, BLOCK_SIZE_M=256, BLOCK_SIZE_N=bn, BLOCK_SIZE_K=64,
+                                   LOCAL_SPLIT_U=split, EDGE_TILES=int(M % 256 != 0 or N % bn != 0))
+        elif have not in _TILE_COST_F32 or _tile_us_f32(have, 1, M, N, K) > 1.1 * us:
             variant, bm, bn, bk = tile
             plain = default_config(M, N, K, dtype, KERNEL_VARIANT=variant, BLOCK_SIZE_M=bm, BLOCK_SIZE_N=bn,
                                    BLOCK_SIZE_K=bk, LOCAL_SPLIT_U=split, NUM_STAGES=_TILE_COST_F32[tile][4],

@@ -56,6 +56,10 @@ enum kcg_cfg_index {
 #define KCG_KERNEL_TCGEN05_CLUSTERK 5 /* fp16/bf16 128-row tiles; LOCAL_SPLIT_U (2..4) CTAs of a thread-block
                                          cluster split K and reduce through distributed shared memory; 256-row
                                          tiles: two CTA pairs (LOCAL_SPLIT_U = 2) */
+#define KCG_KERNEL_F32_SPLIT 6 /* float32 as three products of fp16 parts that a kernel in front of it writes to the
+                                  stream's workspace (4 bytes a value of A and B); 256-row tiles on CTA pairs,
+                                  BLOCK_SIZE_N 128 or 256, BLOCK_SIZE_K 64; multiplies as 3xTF32 where values do not
+                                  split or the workspace has no room */
 #define KCG_KERNEL_NAIVE 100  /* one thread per C element, on-device reference */
 #define KCG_KERNEL_WAIT_PROBE 101 /* no GEMM: one bounded wait (20 ms) that expires -> KCG_E_DEVICE_TIMEOUT */
 
@@ -286,7 +290,8 @@ int kcg_matmul_host(uint64_t function, const kcg_kernel_info* info, int device, 
 int kcg_gemm_bf16_splitk_noalloc(int device, uint64_t stream, uint64_t A, uint64_t B, uint64_t C, int M, int N,
                                  int K, int synchronize);
 
-/* Number of kernel launches issued through this library since load (all threads). */
+/* Number of kernel launches issued through this library since load (all threads); a product of KCG_KERNEL_F32_SPLIT counts
+ * as one. */
 uint64_t kcg_launch_count(void);
 /* Frees workspaces, device buffers and cached tensor maps of every device. */
 int kcg_shutdown(void);

@@ -1,0 +1,229 @@
+"""The split fp32 kernel (KERNEL_VARIANT 6): fp16 parts of both operands, written in front of the product, and the 3xTF32
+kernel in the same launch where values do not split."""
+import pytest
+import torch
+
+from codegendemo_b200 import _lib
+from codegendemo_b200.kcg.KCGCompiler import compile_info
+from codegendemo_b200.kcg.matmul_op import build_kernel, default_config, matmul, tuned_config
+from codegendemo_b200.kcg.Utils import EnumKernelDType as E
+
+
+def _kernel(M, N, K, bn, split=1):
+    return build_kernel(default_config(M, N, K, E.float32, KERNEL_VARIANT=6, BLOCK_SIZE_M=256, BLOCK_SIZE_N=bn, BLOCK_SIZE_K=64,
+                                       LOCAL_SPLIT_U=split, EDGE_TILES=1), 0)[1]
+
+
+def _as_tf32(M, N, K, bn):
+    """The kernel this one falls back to."""
+    return build_kernel(default_config(M, N, K, E.float32, KERNEL_VARIANT=4, BLOCK_SIZE_M=256, BLOCK_SIZE_N=bn, BLOCK_SIZE_K=32,
+                                       NUM_STAGES=3 if bn == 256 else 6, EDGE_TILES=1), 0)[1]
+
+
+def _bound(a, b):
+    """What 3xTF32 guarantees of a value: products left out and rounded, and sums of K terms in fp32."""
+    return 2.0 ** -20 * (a.double().abs() @ b.double().abs())
+
+
+def _split(x, axis):
+    """hi, lo and 2^-e of the split kernel, in 64 bits: 64 values along `axis` share an exponent."""
+    top = x.abs().amax(dim=axis, keepdim=True)
+    scale = torch.where(top > 0, torch.exp2(14 - torch.floor(torch.log2(torch.where(top > 0, top, torch.ones_like(top))))), 1.0)
+    y = x.double() * scale
+    hi = y.half().double()
+    return hi, ((y - hi) * 4096).half().double() / 4096, 1 / scale
+
+
+def test_two_parts_keep_21_bits():
+    """The arithmetic of the split: 2^-22 of a value is lost at most down to 2^-28 of the largest beside it, and the product
+    that is left out is below 2^-24."""
+    gen = torch.Generator().manual_seed(1)
+    x = torch.rand((256, 64), generator=gen) * 2 - 1
+    x = (x * torch.exp2(-torch.randint(0, 28, x.shape, generator=gen).float()))
+    x[:, 0] = 1.0
+    hi, lo, inv = _split(x, 1)
+    assert ((hi + lo) * inv - x.double()).abs().le(2.0 ** -22 * x.double().abs()).all()
+    assert (lo.abs() <= 2.0 ** -11 * hi.abs().clamp(min=2.0 ** -14)).all() and hi.abs().max() < 65504
+
+
+def test_configs_and_the_rule():
+    for bn, stages, threads in ((128, 4, 640), (256, 3, 512)):
+        kpm = default_config(384, 320, 192, E.float32, KERNEL_VARIANT=6, BLOCK_SIZE_M=256, BLOCK_SIZE_N=bn, BLOCK_SIZE_K=64,
+                             EDGE_TILES=1)
+        kpm.check()
+        info = compile_info(kpm.compileArgs(), kernel=6, edge_tiles=1)
+        assert (info.kernel, info.stages, info.block[0]) == (_lib.KERNEL_F32_SPLIT, stages, threads)
+        assert list(info.cluster) == [2, 1, 1] and info.smem_bytes <= 227 * 1024
+    for bad in (dict(BLOCK_SIZE_M=512), dict(BLOCK_SIZE_N=192), dict(BLOCK_SIZE_K=32), dict(isATranspose=1)):
+        keys = {**dict(KERNEL_VARIANT=6, BLOCK_SIZE_M=256, BLOCK_SIZE_N=256, BLOCK_SIZE_K=64), **bad}
+        with pytest.raises(RuntimeError):
+            compile_info(default_config(1024, 768, 512, E.float32, **keys).compileArgs(), kernel=6, edge_tiles=1)
+    with pytest.raises(RuntimeError):  # 16-bit data
+        compile_info(default_config(256, 256, 256, E.float16, KERNEL_VARIANT=6, BLOCK_SIZE_M=256, BLOCK_SIZE_K=64).compileArgs(),
+                     kernel=6)
+
+    class NoDb:
+        def lookup(self, *shape):
+            return None
+
+    def variant(M, N, K):
+        return tuned_config(M, N, K, E.float32, db=NoDb()).KERNEL_VARIANT
+    assert variant(4096, 4096, 4096) == 6 and variant(1024, 7936, 768) == 6
+    assert variant(128, 4096, 4096) != 6       # few rows: B would be written and read once more for one row of tiles
+    assert variant(65536, 8192, 8192) != 6     # 2.25 GB of parts
+
+
+@pytest.mark.gpu
+# one chunk of K; tiles and panels of rows over the edges, K no multiple of a chunk; several tiles and chunks past the ring
+@pytest.mark.parametrize("shape", [(128, 64, 64), (384, 320, 196), (640, 832, 1092)], ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("bn,split", [(128, 1), (128, 3), (256, 1), (256, 2)])
+def test_tiles_over_the_edges(shape, bn, split):
+    M, N, K = shape
+    if K < 64 * 2 * split:
+        split = 1
+    kern = _kernel(M, N, K, bn, split)
+    gen = torch.Generator().manual_seed(2)
+    wide_a, wide_b = [torch.rand(s, generator=gen).cuda() * 2 - 1 for s in ((M, K + 8), (K, N + 64))]
+    a, b = wide_a[:, 4:4 + K], wide_b[:, 64:]
+    bias = torch.rand(N, generator=gen).cuda()
+    old = torch.rand((M, N), generator=gen).cuda()
+    ref = a.double() @ b.double()
+    wide = torch.full((M + 2, N + 64), float("nan"), device="cuda")
+    c = wide[1:1 + M, 32:32 + N]
+    for kw, want in ((dict(), ref), (dict(bias=bias, relu=True), (ref + bias.double()).clamp(min=0)),
+                     (dict(alpha=0.5, beta=2.0), 0.5 * ref + 2.0 * old.double())):
+        c.copy_(old)
+        kern.run(a, b, c, lda=K + 8, ldb=N + 64, ldc=N + 64, **kw)
+        kern.checkStatus()
+        assert ((c.double() - want).abs() <= _bound(a, b) + 2.0 ** -22 * want.abs().clamp(min=1)).all(), kw
+    first = c.clone()
+    c.copy_(old)
+    kern.run(a, b, c, lda=K + 8, ldb=N + 64, ldc=N + 64, alpha=0.5, beta=2.0)
+    assert torch.equal(c, first)
+    wide[1:1 + M, 32:32 + N] = float("nan")
+    assert wide.isnan().all()
+
+
+@pytest.mark.gpu
+def test_closer_than_three_tf32_products():
+    M, N, K = 512, 512, 4096
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    a, b = [torch.rand(s, generator=gen, device="cuda") * 2 - 1 for s in ((M, K), (K, N))]
+    ref = a.double() @ b.double()
+    out = [torch.empty((M, N), device="cuda") for _ in range(2)]
+    _kernel(M, N, K, 256).run(a, b, out[0])
+    _as_tf32(M, N, K, 256).run(a, b, out[1])
+    err = [float((c.double() - ref).norm() / ref.norm()) for c in out]
+    assert err[0] < 0.5 * err[1], err  # (measured 1.9e-7 and 1.0e-6)
+
+
+def _planted(kind, a, b):
+    if kind == "inf":
+        a[3, 5], b[7, 9] = float("inf"), float("-inf")
+    elif kind == "nan":
+        b[70, 17] = float("nan")
+    elif kind == "huge":
+        a[1] *= 2.0 ** 70
+    elif kind == "tiny":
+        b[:, 2] *= 2.0 ** -70
+        b[:, 3] *= 2.0 ** -130
+    elif kind == "far below":  # a value that counts, 2^-35 of the largest beside it
+        a[9, 1], a[9, 2] = 2.0 ** 20, 1.2345678e-5
+        b[1], b[2] = 0.0, 2.0 ** 20
+    return a, b
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["inf", "nan", "huge", "tiny", "far below"])
+@pytest.mark.parametrize("bn", [128, 256])
+@pytest.mark.parametrize("fused", [False, True])
+def test_values_that_do_not_split(kind, bn, fused):
+    """The 3xTF32 kernel's results, bit for bit; and the next call on the stream is not affected."""
+    M, N, K = 384, 320, 192
+    gen = torch.Generator().manual_seed(5)
+    plain = [torch.rand(s, generator=gen) * 2 - 1 for s in ((M, K), (K, N))]
+    a, b = [t.cuda() for t in _planted(kind, *[t.clone() for t in plain])]
+    kw = dict(bias=torch.rand(N, generator=gen).cuda(), relu=True) if fused else {}
+    kern, other = _kernel(M, N, K, bn), _as_tf32(M, N, K, bn)
+    c, want = [torch.full((M, N), 7.0, device="cuda") for _ in range(2)]
+    other.run(a, b, want, **kw)
+    for _ in range(2):
+        c.fill_(7.0)
+        kern.run(a, b, c, **kw)
+        kern.checkStatus()
+        assert torch.equal(c.nan_to_num(nan=123.0), want.nan_to_num(nan=123.0))
+    a, b = [t.cuda() for t in plain]
+    kern.run(a, b, c, **kw)
+    other.run(a, b, want, **kw)
+    assert not torch.equal(c, want)  # (closer to the exact product than that)
+    ref = a.double() @ b.double()
+    ref = (ref + kw["bias"].double()).clamp(min=0) if fused else ref
+    assert ((c.double() - ref).abs() <= _bound(a, b) + 2.0 ** -22).all()
+
+
+@pytest.mark.gpu
+def test_values_that_split():
+    """Rows, columns and stretches of K of very different size, zeros, and exponents up to the limits: the split kernel's own
+    result, within what 3xTF32 guarantees."""
+    M, N, K = 256, 256, 256
+    gen = torch.Generator().manual_seed(6)
+    a, b = [torch.rand(s, generator=gen) * 2 - 1 for s in ((M, K), (K, N))]
+    a *= torch.exp2(torch.randint(-45, 46, (M, 1), generator=gen).float())
+    b *= torch.exp2(torch.randint(-18, 19, (1, N), generator=gen).float())
+    a[:, 64:128] *= 2.0 ** -3
+    b[128:192] = 0.0
+    a[5], b[:, 6] = 0.0, 0.0
+    a[7, 9:] = 0.0
+    a, b = a.cuda(), b.cuda()
+    ref = a.double() @ b.double()
+    c, other = [torch.empty((M, N), device="cuda") for _ in range(2)]
+    kern = _kernel(M, N, K, 256)
+    kern.run(a, b, c)
+    kern.checkStatus()
+    _as_tf32(M, N, K, 256).run(a, b, other)
+    assert not torch.equal(c, other)
+    assert ((c.double() - ref).abs() <= _bound(a, b)).all()
+    assert (c[5] == 0).all() and (c[:, 6] == 0).all()
+
+
+@pytest.mark.gpu
+def test_a_remainder_cut_into_ranges_and_a_graph():
+    """More tiles than run at once, the rest cut into K ranges, with a fused bias; captured, it keeps its own parts."""
+    M, N, K = 3840, 2560, 1024
+    assert tuned_config(M, N, K, E.float32).KERNEL_VARIANT == 6
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    a, b = [torch.rand(s, generator=gen, device="cuda") * 2 - 1 for s in ((M, K), (K, N))]
+    bias = torch.rand(N, generator=gen, device="cuda")
+    want = matmul(a, b, bias=bias)
+    ref = a.double() @ b.double() + bias.double()
+    assert ((want.double() - ref).abs() <= _bound(a, b) + 2.0 ** -22).all()
+    c, stream, graph = torch.empty_like(want), torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        matmul(a, b, c, bias=bias)
+    with torch.cuda.stream(stream):
+        matmul(b[:, :1024].contiguous(), a[:1024].contiguous())  # the stream's own workspace
+    c.fill_(float("nan"))
+    graph.replay()
+    assert torch.equal(c, want)
+    a.view(-1)[0] = float("nan")
+    graph.replay()
+    assert c[0].isnan().all() and not c[1:].isnan().any()
+    a.view(-1)[0] = 0.5
+    ref = matmul(a, b, bias=bias)
+    for _ in range(2):
+        graph.replay()
+        assert torch.equal(c, ref)
+
+
+@pytest.mark.gpu
+def test_parts_larger_than_any_workspace():
+    """4 GiB and more of parts: the product is taken as 3xTF32, with the same bits."""
+    M, N, K = 1 << 19, 256, 2048
+    a = torch.empty((M, K), device="cuda").uniform_(-1, 1, generator=torch.Generator(device="cuda").manual_seed(8))
+    b = a[:K, :N].contiguous()
+    c, want = [torch.empty((M, N), device="cuda") for _ in range(2)]
+    kern = _kernel(M, N, K, 256)
+    kern.run(a, b, c)
+    kern.checkStatus()
+    _as_tf32(M, N, K, 256).run(a, b, want)
+    assert torch.equal(c, want)
