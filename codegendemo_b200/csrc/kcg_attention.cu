@@ -7,17 +7,23 @@
 // Default form (AttnFwd2): one CTA per (head, 256 query rows) = two query tiles of 128 rows, 384 threads:
 //   warp 0    TMA producer: both Q tiles once, then K and V tiles of 128 keys through two-stage rings, shared by
 //             the two query tiles
+//   warp 2    waits for K and V tiles in the issuer's place
 //   warp 1    tcgen05.mma issuer and TMEM owner; per tile t: S_t = Q_t K_j^T (both K-major) into the tile's S
 //             buffer, O_t += P_t V_j with P_t read from tensor memory and V as the MN-major operand
 //   warps 4-7 softmax of tile 0, warps 8-11 of tile 1, one query row per thread: read S_t from TMEM, exponentials in
 //             the exp2 domain against the running maximum, P_t as packed 16-bit pairs over the S columns just read, O_t
 //             rescaled where that maximum has moved; at the end O / sum to global memory
 // A tile's chain is serial (scores, softmax, P V, next scores) and the two tiles' chains take turns, so the tensor
-// pipe works for one tile while the other is in its softmax. What bounds it is that chain: per step and tile 512 + 512
-// cycles of products (the scores' operands fill the shared-memory port, 128 bytes a cycle) and 1024 of exponentials;
-// both tiles' steps take about 3600 cycles against 2048 of the tensor pipe alone. Measured (B200, bf16), a form with
-// votes of all softmax warps and a one-lane issuer against this one with its key-split form: 32 heads x 4096 x 4096 x
-// 128 322 -> 239 us (1150 TFLOP/s), x 64 287 -> 202 us, 16 x 2048 x 2048 x 128 46 -> 38 us.
+// pipe works for one tile while the other is in its softmax. What bounds it is that chain, and the power cap: per step and tile
+// 512 + 512 cycles of products (the scores' operands fill the shared-memory port, 128 bytes a cycle) and 1024 of
+// exponentials; both tiles' steps take 2970 cycles against 2048 of the tensor pipe alone, of a tile's 100 to read the
+// scores, 300 for the maximum, 1170 for 96 exponentials with the rescaling, 400 for the last 32, 640 of products and 260 of
+// hand-offs. The issuer's waits are named barriers: with mbarriers a step took 3450, 32 heads x 4096 x 4096 x 128 239 us ->
+// 223 (1230 TFLOP/s), 16 x 2048 x 2048 x 128 37.5 -> 34.0, 100 x 700 x 3000 x 128 127 -> 113, 8 x 300 x 16384 x 128 57.6 ->
+// 53.9, 32 x 4096 x 4096 x 64 196 -> 191 (B200, bf16, graph replay in turn).
+// Tried without gain since: two threads a row (241 -> 276 us: the maximum through shared memory, both tiles' exponentials at
+// once), steps of 64 keys with two score buffers a tile (311: the rescaling waits for the product before), the first half of the
+// next scores under the exponentials (289: products of 64 keys read Q twice as often).
 // A key-split form of it (kKeySplit) shares a group's keys among the CTAs of a cluster where groups do not fill a wave.
 // Tried without gain: exponentials of every eighth to third pair as a polynomial on the FMA pipe (2 to 8 % slower: one
 // warp per scheduler and tile is bound by its own latencies, not by the exponential pipe).
@@ -527,7 +533,12 @@ struct AttnFwd2 {
   static constexpr int OFF_K = TILES * Q_BYTES, OFF_V = OFF_K + K_STAGES * KV_BYTES;
   static constexpr int RING_BYTES = OFF_V + V_STAGES * KV_BYTES;
   static constexpr int SMEM_BYTES = RING_BYTES + 2048;  // 1 KB alignment slack + barriers
-  static constexpr int P_PART = 96;  // keys of a step after which P V starts
+  // Keys of a step after which P V starts, and whether tile 1 starts half a step after tile 0 (the walk keeps the distance:
+  // one tile's exponentials then run while the other waits for its products, not beside the other's). Measured, 32 heads x
+  // 4096 x 4096: d = 128 after 64, 96, 112, 128 keys 236, 223, 230, 233 us, with the distance 230, 225 (its products alone keep
+  // the tiles apart); d = 64 after 64, 96, 128 keys 198, 205, 208 us, with the distance 191, 203.
+  static constexpr int P_PART = kD == 128 ? 96 : 64;
+  static constexpr bool kApart = kD == 64;
   static constexpr uint32_t COL_O = TILES * BC, TMEM_COLS = 512;
   static constexpr uint32_t FMT = kBf16 ? FMT_BF16 : FMT_F16;
   static constexpr uint32_t IDESC_S = make_instr_desc(FMT, 0u, 0u, 128u, BC);
@@ -538,12 +549,23 @@ struct AttnFwd2 {
     uint64_t q_full;
     uint64_t k_full[K_STAGES], k_empty[K_STAGES], v_full[V_STAGES], v_empty[V_STAGES];
     uint64_t s_full[TILES];   // S_t of the current step is complete
-    uint64_t p_part[TILES];   // the first P_PART keys of P_t are in tensor memory and O_t is rescaled (4 warps arrive)
-    uint64_t p_full[TILES];   // all of P_t is (4 warps arrive)
     uint64_t o_full[TILES];   // the last P_t V has retired
     uint32_t tmem_base;
     volatile uint32_t abort_flag;
   };
+
+  // Named barriers, on which the issuer meets what its products wait for. They are not in shared memory: a look at an
+  // mbarrier there takes 200 to 300 cycles while the products' operand reads fill the port, and an issuer that looked six
+  // times a step (P_t twice, K and V) was on the critical path with 900 of 3450 cycles.
+  // Every meeting takes place in every step whatever else happened: the issuer and warp 2 go on after a wait that ran out, and
+  // so do the softmax warps, whose scores then come from whatever the operands hold. These wait for their scores without
+  // looking at the abort flag, and four times as long as anybody else waits: should the scores never come, every other wait of
+  // the CTA has ended long before, so the issuer has left the step before, and the warp only comes to the meetings that
+  // are left (it must not come twice to one that the issuer has not come to).
+  static constexpr uint32_t BAR_PART = 1;  // + t: the first P_PART keys of P_t are in tensor memory and O_t is rescaled
+  static constexpr uint32_t BAR_FULL = 3;  // + t: all of P_t is (both: four softmax warps arrive, the issuer waits)
+  static constexpr uint32_t BAR_KV = 5;    // the V tile of a step and the K tile of the next have landed (warp 2 and the issuer)
+  static constexpr uint32_t PT_THREADS = 160, KV_THREADS = 64;
 
   __device__ static __forceinline__ void report(Barriers* bars, uint32_t code, uint32_t d0, uint32_t d1) {
     bars->abort_flag = 1u;
@@ -588,8 +610,6 @@ struct AttnFwd2 {
       }
       for (int t = 0; t < TILES; ++t) {
         mbar_init(&bars->s_full[t], 1);
-        mbar_init(&bars->p_part[t], 4);
-        mbar_init(&bars->p_full[t], 4);
         mbar_init(&bars->o_full[t], 1);
       }
       bars->abort_flag = 0u;
@@ -640,25 +660,18 @@ struct AttnFwd2 {
         }
       } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
-        // The issuer is on the critical path: its waits cost 100 to 200 cycles each while operand reads fill the
-        // shared-memory port, so each is made once per step, not once per tile. The whole warp walks the loop and elects
-        // one lane for each batch of instructions: their descriptors are then warp-uniform values. (With the loop
-        // inside an if (lane == 0) every tcgen05.mma took about 125 cycles to issue, twice what a 128 x 128 x 16
-        // product takes to run.) One issuer per tile was slower: the tiles' products then mix on the pipe instead of
-        // taking turns, and both softmaxes wait and work at the same time.
-        bool ok = mbar_wait(&bars->q_full, 0u, &bars->abort_flag);
-        if (!ok && lane == 0) report(bars, ATTN_TIMEOUT_MMA, 0u, 0u);
-        ok = __all_sync(0xffffffffu, ok);
+        // The whole warp walks the loop and elects one lane for each batch of instructions: their descriptors are then
+        // warp-uniform values. (With the loop inside an if (lane == 0) every tcgen05.mma took about 125 cycles to issue, twice
+        // what a 128 x 128 x 16 product takes to run.) One issuer per tile was slower: the tiles' products then mix on the
+        // pipe instead of taking turns, and both softmaxes wait and work at the same time. After a wait somewhere that ran
+        // out the loop goes on, over whatever the operands hold.
+        const bool q_there = mbar_wait(&bars->q_full, 0u, &bars->abort_flag);
+        if (!q_there && lane == 0) report(bars, ATTN_TIMEOUT_MMA, 0u, 0u);
+        __syncwarp();
         const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
         const uint64_t qdesc = make_smem_desc(smem_u32(smem), 16, 1024, SWZ_128B);
         const uint64_t kdesc = make_smem_desc(smem_u32(smem + OFF_K), 16, 1024, SWZ_128B);
         const uint64_t vdesc = make_smem_desc(smem_u32(smem + OFF_V), KVBOX_BYTES, 1024, SWZ_128B);
-        // waits of a whole warp; false (after the report) when one of them ran out
-        auto wait = [&](uint64_t* bar, uint32_t parity, uint32_t what, int i) -> bool {
-          const bool got = __all_sync(0xffffffffu, mbar_wait(bar, parity, &bars->abort_flag));
-          if (!got && lane == 0) report(bars, ATTN_TIMEOUT_MMA, what, static_cast<uint32_t>(i));
-          return got;
-        };
         // S_t of step i. Issued after P_t V of step i - 1 (program order), which is what has read the P that
         // these scores overwrite; the softmax warps of tile t have read the old scores before they wrote that P.
         auto issue_s = [&](int t, int i) {
@@ -680,32 +693,29 @@ struct AttnFwd2 {
               umma_ts<false>(tmem + COL_O + t * kD, tmem + t * BC + ks * 8, vd + ((ks * 16 * 128) >> 4), IDESC_O,
                           (j > 0 || ks > 0) ? 1u : 0u);
         };
-        if (ok) ok = wait(&bars->k_full[0], 0u, 1u, 0);
-        if (ok) {
-          tc_fence_after_sync();
-          if (elect_one()) {
-            issue_s(0, 0);
-            issue_s(1, 0);
-          }
-          __syncwarp();
+        named_bar_sync(BAR_KV, KV_THREADS);  // the first K tile
+        tc_fence_after_sync();
+        if (elect_one()) {
+          issue_s(0, 0);
+          if (!kApart) issue_s(1, 0);
         }
-        for (int j = 0; j < nkv && ok; ++j) {
-          const int vs = j % V_STAGES, ks = (j + 1) % K_STAGES;
-          ok = wait(&bars->v_full[vs], (j / V_STAGES) & 1u, 2u, j);
-          if (ok && j + 1 < nkv) ok = wait(&bars->k_full[ks], ((j + 1) / K_STAGES) & 1u, 1u, j + 1);
+        __syncwarp();
+        for (int j = 0; j < nkv; ++j) {
+          named_bar_sync(BAR_KV, KV_THREADS);
 #pragma unroll
           for (int t = 0; t < TILES; ++t) {
-            if (ok) ok = wait(&bars->p_part[t], j & 1u, 3u, j);
-            if (!ok) break;
+            named_bar_sync(BAR_PART + t, PT_THREADS);
             tc_fence_after_sync();
-            if (elect_one()) issue_pv(t, j, 0, P_PART / 16);
+            if (elect_one()) {
+              if (kApart && j == 0 && t == 0) issue_s(1, 0);
+              issue_pv(t, j, 0, P_PART / 16);
+            }
             __syncwarp();
-            ok = wait(&bars->p_full[t], j & 1u, 4u, j);
-            if (!ok) break;
+            named_bar_sync(BAR_FULL + t, PT_THREADS);
             tc_fence_after_sync();
             if (elect_one()) {
               issue_pv(t, j, P_PART / 16, BC / 16);
-              if (t == TILES - 1) umma_commit(&bars->v_empty[vs]);
+              if (t == TILES - 1) umma_commit(&bars->v_empty[j % V_STAGES]);
               if (j + 1 < nkv) {
                 issue_s(t, j + 1);
               } else {
@@ -715,7 +725,21 @@ struct AttnFwd2 {
             __syncwarp();
           }
         }
-      }  // (warps 2 and 3 only give their registers)
+      } else if (warp == 2) {
+        // ------------------------------------------- waits for K and V in the issuer's place
+        bool ok = true;
+        auto wait = [&](uint64_t* bar, uint32_t parity, uint32_t what, int i) {
+          if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar, parity, &bars->abort_flag));
+          if (!ok && lane == 0) report(bars, ATTN_TIMEOUT_MMA, what, static_cast<uint32_t>(i));
+        };
+        wait(&bars->k_full[0], 0u, 1u, 0);
+        named_bar_sync(BAR_KV, KV_THREADS);
+        for (int j = 0; j < nkv; ++j) {
+          wait(&bars->v_full[j % V_STAGES], (j / V_STAGES) & 1u, 2u, j);
+          if (j + 1 < nkv) wait(&bars->k_full[(j + 1) % K_STAGES], ((j + 1) / K_STAGES) & 1u, 1u, j + 1);
+          named_bar_sync(BAR_KV, KV_THREADS);
+        }
+      }  // (warp 3 only gives its registers)
       if constexpr (kKeySplit) {  // the two meetings of the cluster that join the partial results
         __syncwarp();
         cluster_sync_all();
@@ -737,8 +761,9 @@ struct AttnFwd2 {
       uint64_t sum2[2] = {f32x2(0.f, 0.f), f32x2(0.f, 0.f)};
       bool ok = true;
       const uint64_t scale2 = f32x2(p.scale_log2, p.scale_log2);
-      for (int j = 0; j < nkv; ++j) {
-        const bool got = mbar_wait(&bars->s_full[t], j & 1u, &bars->abort_flag);
+      int j = 0;
+      for (; j < nkv; ++j) {
+        const bool got = mbar_wait_for(&bars->s_full[t], j & 1u, 4 * KCG_WAIT_LIMIT_NS);
         if (!__all_sync(0xffffffffu, got)) {
           if (lane == 0) report(bars, ATTN_TIMEOUT_SOFTMAX, 0u, static_cast<uint32_t>(j));
           ok = false;
@@ -813,6 +838,7 @@ struct AttnFwd2 {
             scale_store(o, c);
           }
           if constexpr (kD == 128) {
+            static_assert(P_PART == 96, "the third piece of 32 keys comes before the publication");
             uint32_t o[2][32];
             tmem_ld_32x32b_x32(col_o + 64, o[0]);
             tmem_ld_32x32b_x32(col_o + 96, o[1]);
@@ -820,27 +846,26 @@ struct AttnFwd2 {
             tmem_ld_wait();
             scale_store(o[0], 2);
             scale_store(o[1], 3);
-          } else {
-            exponentials(2);
           }
         } else {
           exponentials(0);
           exponentials(1);
-          exponentials(2);
+          if constexpr (P_PART == 96) exponentials(2);
         }
-        auto publish = [&](uint64_t* bar) {
+        auto publish = [&](uint32_t bar) {
           tmem_st_wait();
           tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar);
+          named_bar_arrive(bar, PT_THREADS);
         };
-        // P V starts on the first 96 keys while the others are still being exponentiated (measured on 32 heads x 4096 x
-        // 4096 x 128 with every key in one launch: 246 us; after 64 keys 259 us, the product then waits for the rest with
-        // the pipe in its hands; after all 128 266 us)
-        static_assert(P_PART == 96, "three pieces of 32 keys");
-        publish(&bars->p_part[t]);
+        publish(BAR_PART + t);
+        if constexpr (P_PART == 64) exponentials(2);
         exponentials(3);
-        publish(&bars->p_full[t]);
+        publish(BAR_FULL + t);
+      }
+      for (; j < nkv; ++j) {  // (given up)
+        __syncwarp();
+        named_bar_sync(BAR_PART + t, PT_THREADS);
+        named_bar_sync(BAR_FULL + t, PT_THREADS);
       }
       const float2 s01 = f32x2_split(add_f32x2(sum2[0], sum2[1]));
       const float l = s01.x + s01.y;

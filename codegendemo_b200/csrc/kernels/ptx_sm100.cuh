@@ -102,6 +102,16 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
     }
   }
 }
+// Without a look at any flag: for a wait whose end other bounded waits guarantee, `limit_ns` later at most.
+__device__ __forceinline__ bool mbar_wait_for(uint64_t* bar, uint32_t parity, uint64_t limit_ns) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const uint64_t t0 = global_timer_ns();
+  uint32_t spins = 0;
+  while (true) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if ((++spins & 63u) == 0u && global_timer_ns() - t0 > limit_ns) return false;
+  }
+}
 
 // mbar_wait made by a whole (converged) warp: true only if every lane saw the phase complete.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag) {
