@@ -6,7 +6,8 @@
 The library is built with nvcc for sm_100a: its host code binds the CUDA driver lazily (so it loads without a GPU),
 and pieces of device code are linked into it (the allocation-free split-K entry, the row softmax, the fused attention).
 Beside it stands ``_pycall``, a small extension module for the building interpreter that launches on behalf of Python
-callers. The GEMM kernels themselves are compiled per config by the library's own compile entry with
+callers, and ``_torchcall``, which makes an operator's warm call in one step (optional: without it the operators go their way
+through Python). The GEMM kernels themselves are compiled per config by the library's own compile entry with
 ``nvcc -cubin -gencode arch=compute_100a,code=sm_100a``.
 """
 import os
@@ -44,6 +45,39 @@ def build_pycall(force: bool = False) -> str:
         compilers = [shlex.split(c) for c in (os.environ.get("CC"), sysconfig.get_config_var("CC"), "cc", "gcc") if c]
         cc = next((c for c in compilers if shutil.which(c[0])), ["cc"])
         subprocess.check_call(cc + ["-O2", "-shared", "-fPIC", "-I" + sysconfig.get_paths()["include"], "-o", out, src])
+    return out
+
+
+def torchcall_path() -> str:
+    import sysconfig
+    return os.path.join(HERE, "_torchcall" + sysconfig.get_config_var("EXT_SUFFIX"))
+
+
+def build_torchcall(force: bool = False):
+    """The extension module of the warm calls (csrc/kcg_torchcall.cpp), against this interpreter's torch; None where there is
+    no torch or no C++ compiler to build it with."""
+    import shlex
+    import shutil
+    import sysconfig
+    cxx = next((c for c in (os.environ.get("CXX"), sysconfig.get_config_var("CXX"), "c++", "g++")
+                if c and shutil.which(shlex.split(c)[0])), None)
+    try:
+        import torch
+    except ImportError:
+        torch = None
+    if cxx is None or torch is None or torch.version.cuda is None:
+        return None
+    out, src = torchcall_path(), os.path.join(HERE, "csrc", "kcg_torchcall.cpp")
+    root = os.path.dirname(torch.__file__)
+    deps = [src, os.path.join(os.path.dirname(HERE), "include", "kcg_b200.h"), os.path.join(root, "version.py")]
+    if force or not _newer(out, deps):
+        includes = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+                    os.path.join(CUDA_HOME, "include")]
+        subprocess.check_call(shlex.split(cxx) + ["-O2", "-std=c++17", "-shared", "-fPIC",
+                                                  f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+                                                  "-I" + sysconfig.get_paths()["include"]]
+                              + [f for i in includes for f in ("-isystem", i)] + ["-o", out, src, "-L" + os.path.join(root, "lib")]
+                              + ["-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10"])
     return out
 
 
@@ -128,5 +162,6 @@ if __name__ == "__main__":
     sys.path.insert(0, os.path.dirname(HERE))
     print(build_library(force="--force" in sys.argv))
     print(build_pycall(force="--force" in sys.argv))
+    print(build_torchcall(force="--force" in sys.argv))
     if "--lib-only" not in sys.argv:
         prebuild_kernels()

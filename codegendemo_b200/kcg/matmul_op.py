@@ -4,6 +4,7 @@
 import math
 
 from codegendemo_b200 import _lib
+from codegendemo_b200.kcg.CudaLauncher import CudaLauncher
 from codegendemo_b200.kcg.CompiledKernelFactory import CompiledKernelFactory, EnumOperator, UserInputs
 from codegendemo_b200.kcg.KCGCompiler import KCGCompiler
 from codegendemo_b200.kcg.Operators.matmul import KernelArgMatmul
@@ -361,6 +362,36 @@ def build_kernel(kpm: KernelArgMatmul, deviceId: int = 0):
     return inConfig, CompiledKernelFactory.getKernel(inConfig, deviceId)
 
 
+_warm = None  # csrc/kcg_torchcall.cpp once something was launched, False where it was not built for this torch
+
+
+def _warm_calls():
+    """The module of the warm calls, bound to the library; False without it."""
+    global _warm
+    if _warm is None:
+        import ctypes
+        import torch
+        try:
+            from codegendemo_b200 import _torchcall
+            found = _torchcall if _torchcall.TORCH_VERSION == torch.__version__.split("+")[0] else False
+        except ImportError:
+            found = False
+        if found:
+            lib = _lib.get_lib()
+            found.bind(*(ctypes.cast(f, ctypes.c_void_p).value for f in (lib.kcg_launch_gemm_strided, lib.kcg_attention_fwd)),
+                       _lib.check)
+        _warm = found
+    return _warm
+
+
+def _remember(kern, t, M, N, K, batch, b_transposed):
+    """The next call of this shape on plain contiguous tensors may be a warm one. (A launch has been made with `kern`.)"""
+    launcher, warm = getattr(kern, "m_launcher", None), _warm_calls()
+    if warm and isinstance(launcher, CudaLauncher) and t.is_cuda:
+        warm.remember(M, N, K, batch, int(FromTorchType(t.dtype)), t.device.index or 0, int(bool(b_transposed)),
+                      launcher.m_runtime.m_function, launcher.m_infoAddr, launcher)
+
+
 _KERNELS = {}  # (operator, shape, dtype, device, options) -> kernel; True == 1, so operators must not share keys
 
 
@@ -380,6 +411,10 @@ def matmul(a, b, c=None, alpha=1.0, beta=0.0, bias=None, relu=False, b_transpose
     be views with a row pitch (column or row blocks of wider row-major tensors): their leading dimensions go
     to the strided launch entry, nothing is copied. ``b_transposed=True`` takes ``b`` stored N x K and computes
     ``a @ b.T`` (16-bit dtypes). Compiled and loaded kernels are kept per (shape, dtype, device, keys)."""
+    if _warm and c is None and not keys and type(alpha) is float and alpha == 1.0 and type(beta) is float and beta == 0.0:
+        c = _warm.matmul(a, b, bias, relu, b_transposed)
+        if c is not None:
+            return c
     M, K = a.shape
     if b_transposed:
         N, K2 = b.shape
@@ -414,7 +449,12 @@ def matmul(a, b, c=None, alpha=1.0, beta=0.0, bias=None, relu=False, b_transpose
             kpm = tuned_config(M, N, K, dt, b_transposed=b_transposed)
         _, kern = build_kernel(kpm, dev)
         _KERNELS[key] = kern
+        keep = not keys
+    else:
+        keep = False
     kern.m_launcher.launchKernel(dev, a, b, c, alpha=alpha, beta=beta, bias=bias, relu=relu, lda=lda, ldb=ldb, ldc=ldc)
+    if keep:
+        _remember(kern, a, M, N, K, 0, b_transposed)
     return c
 
 
@@ -480,6 +520,10 @@ def attention_fused(q, k, v, scale=None, out=None):
     probabilities stay on the SM. ``q`` is (heads, Sq, d), ``k`` and ``v`` are (heads, Sk, d), all
     contiguous fp16 / bf16 with d = 64 or 128; any Sq and Sk. Returns (heads, Sq, d). ``attention`` above is the
     three-launch form of the same chain."""
+    if _warm and scale is None and out is None:
+        out = _warm.attention(q, k, v)
+        if out is not None:
+            return out
     import torch
     H, Sq, D = q.shape
     H2, Sk, D2 = k.shape
@@ -498,6 +542,8 @@ def attention_fused(q, k, v, scale=None, out=None):
     status = _lib.pycall.attention(dev, DeviceInfo.get_cuda_stream(dev), q, k, v, out, dt, H, Sq, Sk, D, scale)
     if status:
         _lib.check(status)
+    if _warm is None:
+        _warm_calls()
     return out
 
 
@@ -513,6 +559,10 @@ def bmm(a, b, c=None, alpha=1.0, beta=0.0, bias=None, relu=False, **keys):
     contiguous) as ONE launch of the kernel compiled for a single batch's M, N, K: the persistent grid
     walks the tiles of all batches, so that small per-batch problems fill the GPU together. The
     epilogue keywords are those of ``matmul`` (a bias is shared by the batches)."""
+    if _warm and c is None and not keys and type(alpha) is float and alpha == 1.0 and type(beta) is float and beta == 0.0:
+        c = _warm.bmm(a, b, bias, relu)
+        if c is not None:
+            return c
     batch, M, K = a.shape
     batch2, K2, N = b.shape
     assert batch == batch2 and K == K2 and a.is_contiguous() and b.is_contiguous()
@@ -532,5 +582,10 @@ def bmm(a, b, c=None, alpha=1.0, beta=0.0, bias=None, relu=False, **keys):
             kpm = tuned_config(M, N, K, dt, batch=batch)
         _, kern = build_kernel(kpm, dev)
         _KERNELS[key] = kern
+        keep = not keys
+    else:
+        keep = False
     kern.m_launcher.launchKernel(dev, a, b, c, alpha=alpha, beta=beta, bias=bias, relu=relu, batch=batch)
+    if keep:
+        _remember(kern, a, M, N, K, batch, False)
     return c

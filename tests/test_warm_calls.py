@@ -1,0 +1,115 @@
+"""The warm calls of the operators (csrc/kcg_torchcall.cpp): what they take, and that they do what the operator's own way does."""
+
+import pytest
+import torch
+
+from codegendemo_b200 import _lib
+from codegendemo_b200 import build as kbuild
+from codegendemo_b200.kcg import matmul_op
+
+
+@pytest.fixture(scope="module")
+def warm():
+    if kbuild.build_torchcall() is None or not matmul_op._warm_calls():
+        pytest.skip("no module of warm calls for this torch")
+    return matmul_op._warm_calls()
+
+
+class _Sub(torch.Tensor):
+    pass
+
+
+def test_everything_but_plain_cuda_tensors_goes_the_operators_way(warm):
+    x = torch.zeros((256, 256), dtype=torch.bfloat16)
+    for a in (x, x.as_subclass(_Sub), x.to("meta"), x.t(), x.to_sparse(), x[0], 3, None, "a"):
+        for b in (x, a):
+            assert warm.matmul(a, b, None, False, False) is None
+            assert warm.bmm(a, b, None, False) is None
+            assert warm.attention(a, b, b) is None
+    assert warm.matmul(x) is None and warm.bmm() is None and warm.attention(x, x, x, x) is None
+
+
+def test_without_the_module_the_operators_go_their_way(warm, monkeypatch):
+    class _Kernel:
+        def launchKernel(self, dev, a, b, c, **kw):
+            c.fill_(7)
+    kern = _Kernel()
+    kern.m_launcher = kern
+    for value in (None, False, warm):
+        monkeypatch.setattr(matmul_op, "_warm", value)
+        monkeypatch.setattr(matmul_op, "_KERNELS", {})
+        monkeypatch.setattr(matmul_op, "build_kernel", lambda kpm, dev=0: (None, kern))
+        x = torch.zeros((256, 256), dtype=torch.bfloat16)
+        assert (matmul_op.matmul(x, x) == 7).all() and (matmul_op.bmm(x[None], x[None]) == 7).all()
+
+
+def _calls():
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    r = lambda *s, dt=torch.bfloat16: torch.randn(s, generator=gen, device="cuda").to(dt) / 16
+    for dt in (torch.bfloat16, torch.float16, torch.float32):
+        a, b, bias = r(256, 192, dt=dt), r(192, 384, dt=dt), r(384, dt=dt)
+        yield matmul_op.matmul, (a, b), {}
+        yield matmul_op.matmul, (torch.nn.Parameter(a), b), dict(bias=bias, relu=True)
+        if dt != torch.float32:
+            yield matmul_op.matmul, (a, r(384, 192, dt=dt)), dict(b_transposed=True, relu=True)
+            yield matmul_op.bmm, (r(3, 128, 64, dt=dt), r(3, 64, 192, dt=dt)), dict(bias=r(192, dt=dt))
+            yield matmul_op.attention_fused, (r(2, 70, 64, dt=dt), r(2, 200, 64, dt=dt), r(2, 200, 64, dt=dt)), {}
+
+
+@pytest.mark.gpu
+def test_the_same_results(warm, monkeypatch):
+    """Also on another stream, under a mode that watches torch's calls, and for operands the warm call does not take."""
+    class Watch(torch.utils._python_dispatch.TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(func)
+            return func(*args, **(kwargs or {}))
+    taken = []
+
+    class Spy:
+        def __getattr__(self, name):
+            def call(*args):
+                out = getattr(warm, name)(*args)
+                taken.append(out is not None)
+                return out
+            return call if name in ("matmul", "bmm", "attention") else getattr(warm, name)
+    stream = torch.cuda.Stream()
+    for op, args, kw in _calls():
+        op(*args, **kw)
+        monkeypatch.setattr(matmul_op, "_warm", False)
+        want = op(*args, **kw)
+        monkeypatch.setattr(matmul_op, "_warm", Spy())
+        taken.clear()
+        first, second = op(*args, **kw), op(*args, **kw)
+        assert taken == [True, True], (op.__name__, kw.keys())
+        assert first.data_ptr() != second.data_ptr() and first.dtype == want.dtype and not first.requires_grad
+        with torch.cuda.stream(stream):
+            stream.wait_stream(torch.cuda.default_stream())
+            third = op(*args, **kw)
+        stream.synchronize()
+        seen = []
+        taken.clear()
+        with Watch():
+            fourth = op(*args, **kw)
+        assert taken == [False] and seen
+        for got in (first, second, third, fourth):
+            assert torch.equal(got, want), (op.__name__, kw.keys())
+        if op is matmul_op.matmul and not kw:
+            a = torch.cat([args[0], args[0]], dim=1)[:, args[0].shape[1]:]  # rows with a pitch
+            taken.clear()
+            assert torch.equal(op(a, args[1]), want) and taken == [False]
+
+
+@pytest.mark.gpu
+def test_errors_of_a_warm_call(warm):
+    """An operand that no kernel can read is refused with the library's error, and the next call is not affected."""
+    a, b = torch.ones((256, 192), device="cuda", dtype=torch.bfloat16), torch.ones((192, 256), device="cuda", dtype=torch.bfloat16)
+    want = matmul_op.matmul(a, b)
+    odd = torch.ones(256 * 192 + 1, device="cuda", dtype=torch.bfloat16)[1:].view(256, 192)  # not on 16 bytes
+    for _ in range(2):
+        with pytest.raises(_lib.KCGError):
+            matmul_op.matmul(odd, b)
+    with pytest.raises(_lib.KCGError):
+        matmul_op.matmul(a, b, bias=torch.ones(257, device="cuda", dtype=torch.bfloat16)[1:])
+    with pytest.raises(AssertionError):
+        matmul_op.matmul(a, b[:128])
+    assert torch.equal(matmul_op.matmul(a, b), want)
