@@ -67,6 +67,14 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* t
       : "memory");
 }
 
+// The tile of a later load into L2 (allowed before griddep_wait(): see tma_prefetch_2d).
+__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* tm, int32_t c0, int32_t c1, int32_t c2) {
+  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global [%0, {%1, %2, %3}];"
+               :
+               : "l"(reinterpret_cast<uint64_t>(tm)), "r"(c0), "r"(c1), "r"(c2)
+               : "memory");
+}
+
 // Ties the registers of an earlier tmem_ld to the wait before it: no use of them may be scheduled ahead of this.
 __device__ __forceinline__ void pin_32(uint32_t (&r)[32]) {
 #pragma unroll

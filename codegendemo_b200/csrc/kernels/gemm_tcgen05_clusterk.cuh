@@ -233,6 +233,17 @@ struct TcGemmClusterK {
     if (warp == 0) {
       // ------------------------------------------------------------ producer
       if (lane == 0) {
+        // The first K block starts towards L2 while the last CTAs of the kernel before this one end (gemm_tcgen05.cuh).
+        if (kbn > 0) {
+          const int k0 = kb0 * kBK, ka = kATrans ? k0 + w.kofs : k0;
+          const int am0 = (kATrans ? w.mcol : w.m0) + static_cast<int>(half) * R, bn0 = w.n0 + static_cast<int>(half) * BNL;
+#pragma unroll
+          for (int j = 0; j < L.a_boxes; ++j)
+            tma_prefetch_2d(&p.tmA, kATrans ? am0 + j * L.atom : ka + j * L.a_box_inner, kATrans ? ka : am0);
+#pragma unroll
+          for (int j = 0; j < L.b_boxes; ++j)
+            tma_prefetch_2d(&p.tmB, kBTrans ? k0 + j * L.b_box_inner : bn0 + j * L.atom, kBTrans ? bn0 + w.nofs : k0 + w.kofs);
+        }
         griddep_wait();  // the kernel before this one in the stream may have written A or B
         for (int kb = 0; kb < kbn; ++kb) {
           const uint32_t s = kb % kStages;

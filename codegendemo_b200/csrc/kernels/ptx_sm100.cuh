@@ -203,6 +203,15 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* t
       : "memory");
 }
 
+// The tile of a later load into L2. Allowed before griddep_wait(): L2 is where the kernel before this one writes, so a line
+// that it still writes is not stale there.
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* tm, int32_t c0, int32_t c1) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];"
+               :
+               : "l"(reinterpret_cast<uint64_t>(tm)), "r"(c0), "r"(c1)
+               : "memory");
+}
+
 // 2-D tiled store shared -> global (bulk-group completion).
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* tm, const void* smem_src,
                                              int32_t c0, int32_t c1) {
