@@ -894,7 +894,7 @@ struct SplitPlan {
   int tiles, first, factor, sk_per, sk_ranges, units_at_once, units_first;
 };
 
-SplitPlan plan_split(const kcg_kernel_info* info, bool fused_epilogue, int batch = 1) {
+SplitPlan plan_split(const kcg_kernel_info* info, int batch = 1) {
   const int M = info->m * batch, N = info->n, K = info->k;  // a batched product is one tall problem
   const bool h2 = info->kernel == KCG_KERNEL_F32_SPLIT;
   const bool pair = info->kernel == KCG_KERNEL_TCGEN05_PAIR || h2;
@@ -1018,15 +1018,6 @@ SplitPlan plan_split(const kcg_kernel_info* info, bool fused_epilogue, int batch
       }
     }
   }
-  // The 3xTF32 kernel applies a fused epilogue in its reduction loop only (its register file is
-  // full of accumulators at the direct store), so a fused launch sends every tile through the
-  // workspace as a one-way split; the tail split is not combined with it.
-  const bool ws_epilogue = x3 && !h2 && fused_epilogue;
-  if (ws_epilogue && info->splitk <= 1) {
-    first = 0;
-    factor = 1;
-    sk_per = 0;
-  }
   return SplitPlan{T, first, factor, sk_per, sk_ranges, G, units_first};
 }
 
@@ -1043,7 +1034,8 @@ void kcg_internal_count_launch(void) { g_launches.fetch_add(1); }
 // {tiles, split_first_tile, split_factor, sk_per, stream-K ranges, units that run at once, split units first}.
 int kcg_internal_plan_split(const kcg_kernel_info* info, int fused_epilogue, int batch, int out[7]) {
   if (!info || !out || batch < 1) return fail(KCG_E_BAD_ARG, "null argument");
-  const SplitPlan pl = plan_split(info, fused_epilogue != 0, batch);
+  (void)fused_epilogue;  // a launch is cut up in the same way with and without one
+  const SplitPlan pl = plan_split(info, batch);
   out[0] = pl.tiles;
   out[1] = pl.first;
   out[2] = pl.factor;
@@ -1381,11 +1373,19 @@ static int launch_impl(uint64_t function, const kcg_kernel_info* info, int devic
                              3 /*CU_TENSOR_MAP_SWIZZLE_128B*/))
         return e;
     }
-    const SplitPlan plan = plan_split(info, p.epi_flags != 0u, batch);
+    const SplitPlan plan = plan_split(info, batch);
     const int T = plan.tiles, first = plan.first, factor = plan.factor, sk_per = plan.sk_per,
               sk_ranges = plan.sk_ranges, G = plan.units_at_once;
+    // The 3xTF32 kernel applies a fused epilogue in its reduction loop only (its register file is full of accumulators at
+    // the direct store), so a whole tile of a fused launch passes through the workspace too: through one slot per CTA
+    // (pair), behind those of the split tiles, that its tiles take in turn and that stays in L2. (With a slot a tile,
+    // and the remainder never cut into K ranges: 128x4864x9024 with bias and ReLU 360 us, now 85; the plain product 83.)
     const bool ws_epilogue = x3 && p.epi_flags != 0u;
-    p.whole_slot0 = h2 ? (T - first) * factor : -1;
+    // slots of partials: one per (tile, split) of an even split; range index + tile index under stream-K
+    const size_t split_slots = sk_per > 0   ? static_cast<size_t>(sk_ranges) + (T - first)
+                               : factor > 1 ? static_cast<size_t>(T - first) * factor
+                                            : 0;
+    p.whole_slot0 = static_cast<int>(split_slots);
     // Under stream-K the whole tiles before the tail are walked with the grid as stride: the grid
     // stays at every unit that runs at once even when the tail is cut into fewer ranges (the CTAs
     // beyond the last range then simply have no tail piece).
@@ -1400,13 +1400,12 @@ static int launch_impl(uint64_t function, const kcg_kernel_info* info, int devic
     kcg::SplitF32Layout parts{};
     bool split_now = h2;  // false: no memory for the parts; the kernel then reads the fp32 operands
     if (factor > 1 || ws_epilogue || sk_per > 0 || h2) {
-      // slots: one per (tile, split) of an even split; range index + tile index under stream-K
-      const size_t slots = sk_per > 0 ? static_cast<size_t>(sk_ranges) + (T - first)
-                                      : static_cast<size_t>(T - first) * factor + (h2 && ws_epilogue ? G : 0);
+      const size_t whole_slots = !ws_epilogue ? 0 : sk_per > 0 ? G : first < G ? first : G;
+      const size_t slots = split_slots + whole_slots;
       const size_t partials = slots * info->bm * info->bn * sizeof(float);
       size_t need = partials;
       // one counter per CTA half; before them the two words of the split fp32 kernel
-      const size_t tiles = static_cast<size_t>(T - first) * (pair ? 2 : 1) + (h2 ? 4 : 0);
+      const size_t tiles = static_cast<size_t>(T > first ? T - first : 1) * (pair ? 2 : 1) + (h2 ? 4 : 0);
       if (h2) {
         parts = kcg::split_f32_layout(partials, M, N, K);
         need = parts.end;

@@ -84,7 +84,7 @@ struct alignas(64) KcgGemmParams {
   const void* bias;
   unsigned int epi_flags;  // KCG_EPI_*
   // fp32 kernels: workspace slots of whole tiles that go through the workspace (fused epilogue), one per CTA (pair) from
-  // this on; -1: the tile's own slot.
+  // this on.
   int whole_slot0;
   // KERNEL_VARIANT 6 (gemm_tcgen05_f32h2.cuh): the factors of the parts' products, [K block][rows of A] and [K block][64
   // columns of B] with these pitches, those of the finished columns, and {not every value splits, CTAs done}; no words:

@@ -490,13 +490,12 @@ struct TcGemmF32x3 {
         ok = named_bar_all(2, NUM_EPI_THREADS, ok);
         if (!ok) break;
         // ---- tile (or split partial) complete in registers: store. A launch with a fused
-        // epilogue sends whole-K tiles through the workspace too (every tile is then its own
-        // one-way "split": the launcher sets split_first_tile = 0) and applies the epilogue in
+        // epilogue sends whole-K tiles through the workspace too and applies the epilogue in
         // the reduction loop below, where the accumulators are dead: with all of them live
         // there are no registers left for the bias / C operands.
         const bool via_ws = w.nsplit > 1 || p.epi_flags != 0u;
-        // the tile's first contributor's; a whole tile's own, or one that all whole tiles of this CTA (pair) take in turn
-        const int slot0 = w.nsplit > 1 || p.whole_slot0 < 0 ? w.slot - w.split : p.whole_slot0 + unit0;
+        // the tile's first contributor's, or the one that all whole tiles of this CTA (pair) take in turn
+        const int slot0 = w.nsplit > 1 ? w.slot - w.split : p.whole_slot0 + unit0;
 #pragma unroll
         for (int t = 0; t < MT; ++t) {
           const int row = w.m0 + row_base + t * 128 + row_in_acc;
