@@ -934,11 +934,13 @@ SplitPlan plan_split(const kcg_kernel_info* info, int batch = 1) {
     const int rem = T % G;
     if (mode != 0 && rem > 0) {
       // Worth it only when the time saved exceeds the cost of the split. A tile's main-loop time is
-      // estimated from a per-SM rate in MFLOP per microsecond: 10 for 16-bit data, 1.4 useful for fp32
-      // as 3xTF32, 4 as three fp16 products, 4.5 for the single TF32 pass.
-      const double mflop_per_us = h2 ? 4.0 : (info->dtype == KCG_DTYPE_FLOAT32 && info->kernel != KCG_KERNEL_TF32X1) ? 1.4
-                                  : (info->dtype == KCG_DTYPE_FLOAT32)                                     ? 4.5
-                                                                                                           : 10.0;
+      // estimated from a per-SM rate in MFLOP per microsecond: 10 for 16-bit data, 4.5 for the single
+      // TF32 pass; for fp32 the useful rates of the fits behind the tile rules (matmul_op.py): as 3xTF32
+      // 0.95 on 64 columns, 1.6 on more (one CTA), 2.1 (pairs), as fp16 parts 4.2 and 5.8 (256 columns).
+      const double mflop_per_us = h2                                      ? (info->bn <= 128 ? 4.2 : 5.8)
+                                  : x3                                    ? (info->bn <= 64 ? 0.95 : pair ? 2.1 : 1.6)
+                                  : (info->dtype == KCG_DTYPE_FLOAT32) ? 4.5
+                                                                          : 10.0;
       const double tile_us =
           2.0 * (info->bm / (pair ? 2 : 1)) * info->bn * static_cast<double>(K) / 1e6 / mflop_per_us;
       const double partial_kb = (info->bm / (pair ? 2 : 1)) * static_cast<double>(info->bn) * 4.0 / 1024.0;
@@ -949,14 +951,15 @@ SplitPlan plan_split(const kcg_kernel_info* info, int batch = 1) {
       //  * hidden (whole tiles follow, single-pass kernels): a pipeline refill, plus whatever of
       //    the write + shared sum does not fit behind one whole tile's main loop;
       //  * exposed, shared (no whole tiles follow): 6 us + 0.05 us per KB of partial;
-      //  * exposed, summed by the last arriver (3xTF32): 5 us + 0.18 us per KB of partial.
+      //  * exposed, summed by the last arriver (fp32): 2.5 us + 0.07 us per KB of partial, fitted to the
+      //    cuts of 180 timings (4.6 us at 32 KB, 6.1-6.4 at 64, 7.6 at 96, 10.7-12.1 at 128).
       const bool hidden = units_first != 0 && T > G;
       auto overhead_us = [&](int contrib) {
         if (hidden) {
           const double fix = 1.5 + partial_kb * (contrib <= 8 ? 0.063 : 0.027 + 0.036 * contrib);
           return 3.0 + (fix > tile_us ? fix - tile_us : 0.0);
         }
-        return !x3 ? 6.0 + 0.05 * partial_kb : 5.0 + 0.18 * partial_kb;
+        return !x3 ? 6.0 + 0.05 * partial_kb : 2.5 + 0.07 * partial_kb;
       };
       const double margin = ungated ? 0.0 : 1.25;
       if (mode == 2) {
@@ -1379,7 +1382,7 @@ static int launch_impl(uint64_t function, const kcg_kernel_info* info, int devic
     // The 3xTF32 kernel applies a fused epilogue in its reduction loop only (its register file is full of accumulators at
     // the direct store), so a whole tile of a fused launch passes through the workspace too: through one slot per CTA
     // (pair), behind those of the split tiles, that its tiles take in turn and that stays in L2. (With a slot a tile,
-    // and the remainder never cut into K ranges: 128x4864x9024 with bias and ReLU 360 us, now 85; the plain product 83.)
+    // and the remainder never cut into K ranges: 128x4864x9024 with bias and ReLU 360 us, now 85.)
     const bool ws_epilogue = x3 && p.epi_flags != 0u;
     // slots of partials: one per (tile, split) of an even split; range index + tile index under stream-K
     const size_t split_slots = sk_per > 0   ? static_cast<size_t>(sk_ranges) + (T - first)
