@@ -13,7 +13,8 @@ from codegendemo_b200.kcg.Utils import EnumKernelDType as E
 # M, N, K, variant, tile, {whole tiles, K ranges of the others}
 CASES = [
     (128, 512, 4096, 2, (128, 64, 32), (0, 8)),      # remainder alone
-    (128, 1792, 4096, 2, (128, 256, 16), (0, 8)),    # whole fill of seven ranges' slots
+    (256, 768, 1152, 2, (128, 64, 32), (0, 6)),      # a short K
+    (128, 1792, 4096, 2, (128, 256, 16), (0, 8)),    # seven tiles of 256 columns
     (1280, 1024, 4096, 2, (128, 64, 32), (148, 8)),  # a wave of whole tiles, then twelve tiles cut up
     (2560, 2048, 2048, 4, (256, 256, 32), (74, 8)),  # the same on CTA pairs
     (5120, 2176, 256, 4, (256, 128, 32), (340, 1)),  # more whole tiles than slots, none cut up
