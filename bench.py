@@ -13,7 +13,7 @@ tcgen05 kernel.
 Outside the timed region every rank checks its result against the CPU oracle (``oracle_check``): eight random
 128-row blocks of its slab at every N, and every row at N=1; a failed check ends the run with a non-zero exit
 code. At N=1 a second JSON line, on stderr, carries under ``other_workloads`` the other single-GPU configs - fp32 1024^3 and
-4096^3 (3xTF32 and FFMA SIMT), bf16 8192^3 and the rectangular sweep M in {128, 512, 2048} x N, K in {4096, 11008}
+4096^3 (fp16 parts and FFMA SIMT), bf16 8192^3 and the rectangular sweep M in {128, 512, 2048} x N, K in {4096, 11008}
 x {fp32, bf16} (24 points) - each with its roofline and the same shape through cuBLAS (``torch.matmul`` on the device) timed
 the same way, and the operators around the product (batched, strided, the attention-shaped chain as three launches
 and as one fused kernel), each beside its PyTorch library call and checked against the host composition at fp32.
@@ -274,7 +274,7 @@ def other_workloads(device: int, peaks: dict, sampler: "ClockSampler", launches:
     f32, bf16 = (E.float32, torch.float32), (E.bfloat16, torch.bfloat16)
     groups = [
         ("square fp32", [("c1 fp32 1024^3 3xTF32", 1024, 1024, 1024, f32, "uniform", None),
-                         ("c2 fp32 4096^3 3xTF32", 4096, 4096, 4096, f32, "uniform", None),
+                         ("c2 fp32 4096^3 fp16 parts", 4096, 4096, 4096, f32, "uniform", None),
                          ("c2 fp32 4096^3 FFMA SIMT", 4096, 4096, 4096, f32, "uniform", simt)]),
         ("square bf16", [("c3 bf16 8192^3", 8192, 8192, 8192, bf16, "normal", None)]),
     ]
