@@ -265,6 +265,7 @@ def other_workloads(device: int, peaks: dict, sampler: "ClockSampler", launches:
     the largest difference between the two results. Problems that fit the L2 rotate over copies of their operands
     so that every launch starts cold. One clock sample per group of workloads."""
     import torch
+    from codegendemo_b200._lib import KERNEL_F32_SPLIT
     from codegendemo_b200.kcg import roofline as rl
     from codegendemo_b200.kcg.matmul_op import build_kernel, default_config, tuned_config
     from codegendemo_b200.kcg.Utils import EnumKernelDType as E
@@ -325,16 +326,19 @@ def other_workloads(device: int, peaks: dict, sampler: "ClockSampler", launches:
                 med, lib_med = ts[len(ts) // 2], tl[len(tl) // 2]
                 flops = rl.gemm_flops(m, n, k)
                 variant = int(inc.kernelInfo["kernel"])
-                tensor_peak = rl.tensor_peak_tflops(str(tdt).replace("torch.", ""), variant == 1, peaks)
+                parts = variant == KERNEL_F32_SPLIT  # three fp16 products a step
+                tensor_peak = (rl.tensor_peak_tflops("bfloat16", False, peaks) / 3 if parts else
+                               rl.tensor_peak_tflops(str(tdt).replace("torch.", ""), variant == 1, peaks))
                 roof = rl.shape_roofline(m, n, k, eb, tensor_peak, peaks["hbm_gbs"])
                 bound, peak = roof["bound"], roof["peak"]
                 tfl = flops / (med * 1e9)
                 out.append({
-                    "workload": tag, "dtype": "f32(3xtf32)" if (tdt == torch.float32 and variant != 1) else
+                    "workload": tag, "dtype": "f32(fp16 parts)" if parts else "f32(3xtf32)" if (tdt == torch.float32 and variant != 1) else
                     ("f32" if tdt == torch.float32 else "bf16"), "ms": round(med, 4), "ms_best": round(ts[0], 4),
                     "tflops": round(tfl, 1), "gbs": round(nbytes / med / 1e6, 0),
                     "roofline": {"bound": bound, "peak": round(peak, 1), "frac": round(tfl / peak, 4),
                                  "peak_source": ("FFMA pipe 74 TFLOP/s" if variant == 1 else
+                                                 f"{peaks['source']} bf16_tflops / 3" if parts else
                                                  "nominal TF32 1100 / 3" if tdt == torch.float32 else
                                                  f"{peaks['source']} bf16_tflops") +
                                                 (f", capped by AI x {peaks['source']} hbm_gbs" if bound == "hbm" else "")},
