@@ -916,6 +916,8 @@ SplitPlan plan_split(const kcg_kernel_info* info, int batch = 1) {
   // KCG_TAIL_SPLIT=0 turns the split off, =2 selects the even split, =3 / =4 stream-K / the even
   // split without the cost gate, =5 stream-K over the remainder alone BEFORE the whole tiles (the
   // last arriver sums a tile; no gate; an experiment that measured no consistent gain).
+  // The split fp32 kernel is never cut by stream-K: sk_per counts K blocks, and the one launch may be walked in blocks of
+  // 64 values or, by the 3xTF32 kernel it falls back to, of 32. An even split's ranges follow from each walk's own blocks.
   const int T = blocks_of(M, info->bm) * blocks_of(N, info->bn);
   const int num_kb = blocks_of(K, info->bk);
   const int nsm = info->reserved[0] > 0 ? info->reserved[0] : 148;
@@ -929,7 +931,8 @@ SplitPlan plan_split(const kcg_kernel_info* info, int batch = 1) {
     const char* e = getenv("KCG_TAIL_SPLIT");
     const bool sk_first = e && e[0] == '5' && !x3;  // stream-K ranges before the whole tiles, no gate
     const bool ungated = e && (e[0] == '3' || e[0] == '4' || e[0] == '5');
-    const int mode = (e && e[0] == '0') ? 0 : (e && (e[0] == '1' || e[0] == '3' || e[0] == '5')) ? 1 : 2;
+    const bool stream_k = e && (e[0] == '1' || e[0] == '3' || e[0] == '5') && !h2;
+    const int mode = (e && e[0] == '0') ? 0 : stream_k ? 1 : 2;
     units_first = (!x3 && (mode == 2 || sk_first)) ? 1 : 0;
     const int rem = T % G;
     if (mode != 0 && rem > 0) {

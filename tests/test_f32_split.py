@@ -1,5 +1,10 @@
 """The split fp32 kernel (KERNEL_VARIANT 6): fp16 parts of both operands, written in front of the product, and the 3xTF32
 kernel in the same launch where values do not split."""
+import ctypes
+import os
+import random
+import subprocess
+
 import pytest
 import torch
 
@@ -71,6 +76,42 @@ def test_configs_and_the_rule():
     assert variant(4096, 4096, 4096) == 6 and variant(1024, 7936, 768) == 6
     assert variant(128, 4096, 4096) != 6       # few rows: B would be written and read once more for one row of tiles
     assert variant(65536, 8192, 8192) != 6     # 2.25 GB of parts
+
+
+@pytest.mark.parametrize("bn", [128, 256])
+def test_both_kernels_of_a_launch_cover_every_tile(bn, tmp_path, monkeypatch):
+    """One plan is walked in K blocks of 64, or of 32 by the kernel that a launch falls back to: in every mode of
+    KCG_TAIL_SPLIT both walks cover every tile's K once, within the slots of the launch."""
+    lib = _lib.get_lib()
+    lib.kcg_internal_plan_split.argtypes = [ctypes.POINTER(_lib.KernelInfo), ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_int)]
+    tests = os.path.dirname(os.path.abspath(__file__))
+    kernels = os.path.join(os.path.dirname(tests), "codegendemo_b200", "csrc", "kernels")
+    for bk in (64, 32):
+        subprocess.run(["g++", "-O1", "-std=c++17", "-I/usr/local/cuda/include", "-I" + kernels, "-DWIC_BM=256", f"-DWIC_BN={bn}",
+                        f"-DWIC_BK={bk}", "-o", str(tmp_path / str(bk)), os.path.join(tests, "work_iter_check.cpp")], check=True)
+    rng = random.Random(bn)
+    layers = set()
+    for M, N, K in [(4096, 4096, 4096), (2048, 11008, 11008)] + [
+            (256 * rng.randint(1, 20), bn * rng.randint(1, 40), rng.choice([4 * rng.randint(16, 400), 64 * rng.randint(4, 172)]))
+            for _ in range(10)]:
+        for mode in (None, "1", "2", "3", "4", "5"):
+            if mode is None:
+                monkeypatch.delenv("KCG_TAIL_SPLIT", raising=False)
+            else:
+                monkeypatch.setenv("KCG_TAIL_SPLIT", mode)
+            kpm = default_config(M, N, K, E.float32, KERNEL_VARIANT=6, BLOCK_SIZE_M=256, BLOCK_SIZE_N=bn, BLOCK_SIZE_K=64, EDGE_TILES=1)
+            info = compile_info(kpm.compileArgs(), kernel=6, edge_tiles=1)
+            out = (ctypes.c_int * 7)()
+            assert lib.kcg_internal_plan_split(ctypes.byref(info), 0, 1, out) == 0
+            tiles, first, factor, sk_per, ranges, at_once, units_first = out
+            assert (sk_per, ranges) == (0, 0)
+            layers.add(factor > 1)
+            grid, slots = min(first + (tiles - first) * factor, at_once), (tiles - first) * factor
+            for bk in (64, 32):
+                r = subprocess.run([str(tmp_path / str(bk))] + [str(v) for v in (M, N, K, first, factor, sk_per, grid, slots, units_first)],
+                                   capture_output=True, text=True)
+                assert r.returncode == 0 and r.stdout.startswith("OK"), (M, N, K, mode, bk, list(out), r.stdout + r.stderr)
+    assert layers == {False, True}
 
 
 @pytest.mark.gpu
@@ -213,6 +254,26 @@ def test_a_remainder_cut_into_ranges_and_a_graph():
     for _ in range(2):
         graph.replay()
         assert torch.equal(c, ref)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["1", "3"])
+def test_stream_k_asked_for(mode, monkeypatch):
+    """More tiles than run at once, under the modes that lay K blocks end to end: values that split and values that do not."""
+    monkeypatch.setenv("KCG_TAIL_SPLIT", mode)
+    M, N, K = 2560, 2304, 1024
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    a, b = [torch.rand(s, generator=gen, device="cuda") * 2 - 1 for s in ((M, K), (K, N))]
+    kern = _kernel(M, N, K, 256)
+    for _ in range(2):
+        for value in (0.5, float("nan")):
+            a[2559, 1000] = value
+            c = torch.full((M, N), 7.0, device="cuda")
+            kern.run(a, b, c)
+            kern.checkStatus()
+            ref = a.double() @ b.double()
+            assert c[2559].isnan().all() or value == 0.5
+            assert ((c.double() - ref).abs() <= _bound(a, b))[:2559].all()
 
 
 @pytest.mark.gpu

@@ -43,7 +43,7 @@ int main(int argc, char** argv) {
   const int grid = atoi(argv[7]), slots = atoi(argv[8]);
   p.split_units_first = atoi(argv[9]);
   p.batch_rows = argc == 11 ? atoi(argv[10]) : 0;
-  const int tiles_m = p.M / WIC_BM, tiles_n = p.N / WIC_BN, num_kb = p.K / WIC_BK, tiles = tiles_m * tiles_n;
+  const int tiles_m = p.M / WIC_BM, tiles_n = p.N / WIC_BN, num_kb = (p.K + WIC_BK - 1) / WIC_BK, tiles = tiles_m * tiles_n;
   std::vector<int> cover(static_cast<size_t>(tiles) * num_kb, 0);
   struct Piece { int split, nsplit, slot, kb0, kbn, share, last; };
   std::map<int, std::vector<Piece>> by_tile;
