@@ -6,6 +6,7 @@
 // 6.5 us through Python, of them 2.2 the launch and 1.8 the result's allocation, 3.6 here; the GPU needs 4.4. Calls in a row 6.6 -> 4.3.
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/utils/object_ptr.h>
 #include <torch/version.h>
 
 #include <ATen/ATen.h>
@@ -107,6 +108,8 @@ PyObject* product(const Shape& shape, const at::Tensor& a, const at::Tensor& b, 
     fused = true;
   }
   const Kernel kernel = it->second;
+  // The launch reads the owner's info with the GIL released, and another thread may put another owner in its place.
+  const auto owner = THPObjectPtr(Py_NewRef(kernel.owner));
   const uint64_t stream = reinterpret_cast<uint64_t>(c10::cuda::getCurrentCUDAStream(a.device().index()).stream());
   at::Tensor c = at::detail::empty_cuda(sizes, a.scalar_type(), a.device(), std::nullopt);
   int status;

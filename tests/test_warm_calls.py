@@ -1,5 +1,10 @@
 """The warm calls of the operators (csrc/kcg_torchcall.cpp): what they take, and that they do what the operator's own way does."""
 
+import ctypes
+import gc
+import threading
+import weakref
+
 import pytest
 import torch
 
@@ -113,3 +118,48 @@ def test_errors_of_a_warm_call(warm):
     with pytest.raises(AssertionError):
         matmul_op.matmul(a, b[:128])
     assert torch.equal(matmul_op.matmul(a, b), want)
+
+
+class _Owner:
+    pass
+
+
+@pytest.mark.gpu
+def test_a_launch_holds_what_owns_its_kernel(warm):
+    """While a warm call is inside the launch (a stand-in that waits), another thread puts another kernel in its place."""
+    gemm_t = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_uint64, ctypes.c_void_p, ctypes.c_int, *[ctypes.c_uint64] * 4,
+                              *[ctypes.c_int64] * 3, ctypes.c_int, ctypes.c_void_p)
+    inside, go_on, functions = threading.Event(), threading.Event(), []
+
+    def gemm(function, *rest):
+        functions.append(function)
+        inside.set()
+        go_on.wait(20.0)
+        return 0
+    gemm_c, lib = gemm_t(gemm), _lib.get_lib()
+    address = lambda f: ctypes.cast(f, ctypes.c_void_p).value
+    a, b = torch.zeros((8, 24), device="cuda"), torch.zeros((24, 40), device="cuda")
+    key = (8, 40, 24, 0, 4, a.device.index, 0)
+    first, second = _Owner(), _Owner()
+    alive = weakref.ref(first)
+    warm.remember(*key, 111, 0, first)
+    warm.bind(address(gemm_c), address(lib.kcg_attention_fwd), _lib.check)
+    try:
+        got = []
+        caller = threading.Thread(target=lambda: got.append(warm.matmul(a, b, None, False, False)))
+        caller.start()
+        assert inside.wait(20.0)
+        del first
+        warm.remember(*key, 222, 0, second)
+        gc.collect()
+        held = alive() is not None
+        go_on.set()
+        caller.join(20.0)
+        assert held and not caller.is_alive() and got[0].shape == (8, 40)
+        gc.collect()
+        assert alive() is None
+        warm.matmul(a, b, None, False, False)
+        assert functions == [111, 222]
+    finally:
+        go_on.set()
+        warm.bind(address(lib.kcg_launch_gemm_strided), address(lib.kcg_attention_fwd), _lib.check)
