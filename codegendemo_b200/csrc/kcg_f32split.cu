@@ -1,7 +1,7 @@
 // Splits the operands of an fp32 product into the fp16 parts that gemm_tcgen05_f32h2.cuh multiplies:
 //   x * 2^e = hi + 2^-12 lo,
 // one exponent e for 64 values of K of a row of A, or for 64 values of K of 64 columns of B, which have been multiplied by a
-// power of two of each column's own. One pass: a CTA takes 128 rows x 64 values of K of A, or 64 values of K x 128 columns
+// power of two of each column's own, 1 or more. One pass: a CTA takes 128 rows x 64 values of K of A, or 64 values of K x 128 columns
 // of B, into registers (32 KB), finds the largest magnitudes, and writes both parts where one TMA box of the product's stage
 // will read them:
 //   A  [panel of 128 rows][64 values of K][hi, lo][row][64 halves]
@@ -37,18 +37,21 @@ __device__ __forceinline__ Scale scale_of(uint32_t top) {
   return s;
 }
 
-// The power of two that brings a value of this magnitude to about 1, within 2^+-40.
-__device__ __forceinline__ float column_power(uint32_t bits) {
-  const int e = bits == 0u ? 0 : 127 - static_cast<int>(bits >> 23);
-  return __uint_as_float(static_cast<uint32_t>(127 + min(max(e, -40), 40)) << 23);
+// The power of two, from 1 to 2^40, that brings a value of this magnitude up to the largest of its 64 columns. (Never below 1:
+// the sums that the product keeps are of the multiplied columns, and must not underflow where those of the columns do not.)
+__device__ __forceinline__ float column_power(uint32_t bits, uint32_t largest) {
+  const int up = bits == 0u ? 0 : min(static_cast<int>(largest >> 23) - static_cast<int>(bits >> 23), 40);
+  return __uint_as_float(static_cast<uint32_t>(127 + up) << 23);
 }
 
 __device__ __forceinline__ uint32_t magnitude(float x) { return __float_as_uint(x) & 0x7fffffffu; }
 
 // Four values as hi and lo parts; true where one of them keeps less than 21 bits.
-__device__ __forceinline__ bool split4(const float4& x, const float4& mult, uint2* hi, uint2* lo) {
-  const float v[4] = {x.x * mult.x, x.y * mult.y, x.z * mult.z, x.w * mult.w};
+__device__ __forceinline__ bool split4(const float4& x, float mult, uint2* hi, uint2* lo) {
+  const float v[4] = {x.x * mult, x.y * mult, x.z * mult, x.w * mult};
   bool lost = false;
+  if (mult < 1.f)  // it may turn a value to zero, of which nothing is missed below
+    lost = (v[0] == 0.f && x.x != 0.f) || (v[1] == 0.f && x.y != 0.f) || (v[2] == 0.f && x.z != 0.f) || (v[3] == 0.f && x.w != 0.f);
   uint32_t h[2], l[2];
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
@@ -99,7 +102,7 @@ __global__ void __launch_bounds__(kThreads) split_f32_kernel(const kcg::SplitF32
       for (int s = 8; s > 0; s >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, s));
       const Scale sc = scale_of(top);
       uint2 hi, lo;
-      bad |= split4(x[i], make_float4(sc.mult, sc.mult, sc.mult, sc.mult), &hi, &lo) || !sc.ok;
+      bad |= split4(x[i], sc.mult, &hi, &lo) || !sc.ok;
       const int r = r0 + 16 * i;
       *reinterpret_cast<uint2*>(block + r * 128 + k4 * 2) = hi;
       *reinterpret_cast<uint2*>(block + (kRows + r) * 128 + k4 * 2) = lo;
@@ -131,7 +134,11 @@ __global__ void __launch_bounds__(kThreads) split_f32_kernel(const kcg::SplitF32
       const uint4 v = column_top[o][lane];
       ct = make_uint4(max(ct.x, v.x), max(ct.y, v.y), max(ct.z, v.z), max(ct.w, v.w));
     }
-    const float4 cm = make_float4(column_power(ct.x), column_power(ct.y), column_power(ct.z), column_power(ct.w));
+    uint32_t largest = max(max(ct.x, ct.y), max(ct.z, ct.w));  // of this lane's 64 columns
+#pragma unroll
+    for (int s = 8; s > 0; s >>= 1) largest = max(largest, __shfl_xor_sync(0xffffffffu, largest, s));
+    const float4 cm = make_float4(column_power(ct.x, largest), column_power(ct.y, largest), column_power(ct.z, largest),
+                                  column_power(ct.w, largest));
     uint32_t top = 0u;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -150,12 +157,11 @@ __global__ void __launch_bounds__(kThreads) split_f32_kernel(const kcg::SplitF32
       if (kb == 0 && warp == 0)
         *reinterpret_cast<float4*>(q.columns + n) = make_float4(1.f / cm.x, 1.f / cm.y, 1.f / cm.z, 1.f / cm.w);
       if (warp == 0 && (lane & 15) == 0) q.scale_b[static_cast<size_t>(kb) * q.scale_ldb + (n >> 6)] = sc.inv;
-      const float4 mult = make_float4(sc.mult, sc.mult, sc.mult, sc.mult);
       uint8_t* block = q.parts_b + (static_cast<size_t>(n >> 6) * num_kb + kb) * (2 * kBK * 128) + (n & 63) * 2;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         uint2 hi, lo;
-        bad |= split4(x[i], mult, &hi, &lo);
+        bad |= split4(x[i], sc.mult, &hi, &lo);
         *reinterpret_cast<uint2*>(block + (warp + 8 * i) * 128) = hi;
         *reinterpret_cast<uint2*>(block + (kBK + warp + 8 * i) * 128) = lo;
       }

@@ -171,11 +171,20 @@ def _planted(kind, a, b):
     elif kind == "far below":  # a value that counts, 2^-35 of the largest beside it
         a[9, 1], a[9, 2] = 2.0 ** 20, 1.2345678e-5
         b[1], b[2] = 0.0, 2.0 ** 20
+    elif kind == "vanishes":  # 2^-115 beside 2^50: its factor makes it a zero
+        a[9] = 0.0
+        a[9, 1], a[9, 2] = 2.0 ** 50, 1.5 * 2.0 ** -115
+        b[1] = 0.0
+    elif kind == "column vanishes":  # 2^-112 in a column whose other values are near 2^40
+        a[:, 24], a[9] = 0.0, 0.0
+        a[9, 2] = 1.0
+        b[:, 4] *= 2.0 ** 40
+        b[2, 4] = 1.5 * 2.0 ** -112
     return a, b
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("kind", ["inf", "nan", "huge", "tiny", "far below"])
+@pytest.mark.parametrize("kind", ["inf", "nan", "huge", "tiny", "far below", "vanishes", "column vanishes"])
 @pytest.mark.parametrize("bn", [128, 256])
 @pytest.mark.parametrize("fused", [False, True])
 def test_values_that_do_not_split(kind, bn, fused):
@@ -225,6 +234,24 @@ def test_values_that_split():
     assert not torch.equal(c, other)
     assert ((c.double() - ref).abs() <= _bound(a, b)).all()
     assert (c[5] == 0).all() and (c[:, 6] == 0).all()
+
+
+@pytest.mark.gpu
+def test_small_products_of_a_large_column():
+    """A column near 2^40 whose other stretch of K is 2^-50 of that: a product near 2^-116 there, with nothing beside it."""
+    M, N, K = 256, 256, 128
+    gen = torch.Generator().manual_seed(10)
+    a, b = [torch.rand(s, generator=gen) + 1 for s in ((M, K), (K, N))]
+    b[64:] *= 2.0 ** -50
+    b[:, 5] *= 2.0 ** 40
+    a[9], b[64, 5] = 0.0, 0.0
+    a[9, 64], a[9, 66], b[66, 5] = 2.0 ** -50, 1.25 * 2.0 ** -78, 1.5 * 2.0 ** -38
+    a, b = a.cuda(), b.cuda()
+    c = torch.empty((M, N), device="cuda")
+    kern = _kernel(M, N, K, 256)
+    kern.run(a, b, c)
+    kern.checkStatus()
+    assert ((c.double() - a.double() @ b.double()).abs() <= _bound(a, b)).all()
 
 
 @pytest.mark.gpu
