@@ -55,7 +55,7 @@ def torchcall_path() -> str:
 
 def build_torchcall(force: bool = False):
     """The extension module of the warm calls (csrc/kcg_torchcall.cpp), against this interpreter's torch; None where there is
-    no torch or no C++ compiler to build it with."""
+    no torch or no C++ compiler to build it with, or where it does not compile (no Python headers, another torch's internals)."""
     import shlex
     import shutil
     import sysconfig
@@ -73,11 +73,18 @@ def build_torchcall(force: bool = False):
     if force or not _newer(out, deps):
         includes = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
                     os.path.join(CUDA_HOME, "include")]
-        subprocess.check_call(shlex.split(cxx) + ["-O2", "-std=c++17", "-shared", "-fPIC",
-                                                  f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-                                                  "-I" + sysconfig.get_paths()["include"]]
-                              + [f for i in includes for f in ("-isystem", i)] + ["-o", out, src, "-L" + os.path.join(root, "lib")]
-                              + ["-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10"])
+        if os.path.exists(out):  # (one of an older source or torch must not be what is imported if this one does not compile)
+            os.remove(out)
+        try:
+            subprocess.check_call(shlex.split(cxx) + ["-O2", "-std=c++17", "-shared", "-fPIC",
+                                                      f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+                                                      "-I" + sysconfig.get_paths()["include"]]
+                                  + [f for i in includes for f in ("-isystem", i)]
+                                  + ["-o", out, src, "-L" + os.path.join(root, "lib")]
+                                  + ["-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10"])
+        except subprocess.CalledProcessError as e:
+            print(f"{src} does not compile here (status {e.returncode}): warm calls go through Python", file=sys.stderr)
+            return None
     return out
 
 

@@ -120,6 +120,17 @@ def test_errors_of_a_warm_call(warm):
     assert torch.equal(matmul_op.matmul(a, b), want)
 
 
+def test_a_module_that_does_not_compile(tmp_path, monkeypatch):
+    """The build goes on without the warm calls, and leaves no module of an older source to be imported in their place."""
+    from codegendemo_b200 import build
+    stale = tmp_path / "_torchcall.so"
+    stale.write_bytes(b"")
+    monkeypatch.setattr(build, "torchcall_path", lambda: str(stale))
+    monkeypatch.setenv("CXX", "false")
+    assert build.build_torchcall(force=True) is None
+    assert not stale.exists()
+
+
 class _Owner:
     pass
 
