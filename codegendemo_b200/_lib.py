@@ -26,7 +26,7 @@ EXPORTED_SYMBOLS = (
     "kcg_launch_gemm_ex", "kcg_launch_gemm_batched", "kcg_launch_gemm_strided", "kcg_softmax_rows", "kcg_softmax_rows_ex",
     "kcg_attention_fwd", "kcg_attention_status",
     "kcg_launch_gemm_allgather", "kcg_peer_alloc", "kcg_peer_open", "kcg_peer_close",
-    "kcg_peer_free", "kcg_check_status", "kcg_matmul_host", "kcg_launch_count", "kcg_shutdown",
+    "kcg_peer_free", "kcg_check_status", "kcg_matmul_host", "kcg_launch_count", "kcg_trim", "kcg_shutdown",
     "kcg_last_error", "kcg_version", "kcg_gemm_bf16_splitk_noalloc",
 )
 
@@ -186,7 +186,7 @@ def get_lib() -> ctypes.CDLL:
     lib.kcg_version.restype = ctypes.c_char_p
     for name in ("kcg_compile_matmul", "kcg_compile_matmul_ex", "kcg_kernel_name", "kcg_load_binary",
                  "kcg_unload", "kcg_device_properties", "kcg_launch_gemm", "kcg_launch_gemm_ex",
-                 "kcg_check_status", "kcg_matmul_host", "kcg_shutdown"):
+                 "kcg_check_status", "kcg_matmul_host", "kcg_trim", "kcg_shutdown"):
         getattr(lib, name).restype = ctypes.c_int
     try:
         from codegendemo_b200 import _pycall

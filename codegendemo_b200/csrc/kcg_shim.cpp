@@ -61,7 +61,7 @@ int fail(int code, const char* fmt, ...) {
   X(cuInit) X(cuDeviceGet) X(cuDeviceGetCount) X(cuDeviceGetAttribute) X(cuGetErrorString)     \
   X(cuDevicePrimaryCtxRetain) X(cuCtxGetCurrent) X(cuCtxSetCurrent) X(cuModuleLoadData)        \
   X(cuModuleGetFunction) X(cuModuleUnload) X(cuFuncSetAttribute) X(cuFuncGetAttribute)         \
-  X(cuLaunchKernelEx) X(cuTensorMapEncodeTiled) X(cuMemAlloc) X(cuMemFree) X(cuMemsetD32)      \
+  X(cuLaunchKernelEx) X(cuTensorMapEncodeTiled) X(cuMemAlloc) X(cuMemFree) X(cuMemGetInfo) X(cuMemsetD32) \
   X(cuMemcpyHtoDAsync) X(cuMemcpyDtoHAsync) X(cuMemcpyDtoH) X(cuMemcpyHtoD)                    \
   X(cuStreamSynchronize) X(cuStreamCreate) X(cuStreamDestroy) X(cuStreamWaitEvent) X(cuEventCreate)        \
   X(cuEventRecord) X(cuEventDestroy) X(cuIpcGetMemHandle) X(cuIpcOpenMemHandle) X(cuIpcCloseMemHandle) \
@@ -143,7 +143,9 @@ struct StreamSlot {
   uint64_t last_use = 0;
 };
 constexpr size_t kMaxStreamSlots = 32;
-constexpr size_t kMaxWorkspaceBytes = size_t(4) << 30;  // of all streams of a device together
+constexpr size_t kMaxWorkspaceBytes = size_t(4) << 30;  // of all streams of a device together, where parts of operands are kept
+constexpr uint64_t kIdleLaunches = 256;      // a stream's workspace is idle when so many launches of the device went past it
+constexpr uint64_t kRefusedLaunches = 1024;  // no room for parts: not asked again for so many launches
 
 // Workspace and tile counters of the launches that one capture queued on one stream. The graph
 // runs on any stream, beside any other graph and as often as it likes, long after the stream's own
@@ -183,7 +185,9 @@ struct DeviceState {
   bool init = false;
   CUcontext ctx = nullptr;
   std::vector<StreamSlot> slots;
-  uint64_t use_clock = 0;
+  uint64_t use_clock = 0;  // launches (and status reads)
+  size_t refused_bytes = 0;  // the last workspace with parts that there was no memory for, and when
+  uint64_t refused_at = 0;
   std::vector<GraphBuffer*> graph_buffers;
   CUstream aux = nullptr;  // non-blocking: clears buffers while other streams are being captured
   CUdeviceptr hbuf[3] = {0, 0, 0};  // device copies for kcg_matmul_host
@@ -306,23 +310,91 @@ int graph_buffer(DeviceState* s, CUstream stream, unsigned long long id, CUgraph
   return 0;
 }
 
-// Before `slot`'s workspace grows to `need` bytes: workspaces of other streams, the least recently used ones first, are
-// given back until all of them stay within kMaxWorkspaceBytes (the splits of fp32 operands are as large as the operands).
-int make_room(DeviceState* s, StreamSlot* slot, size_t need) {
-  for (;;) {
-    size_t held = need;
-    StreamSlot* oldest = nullptr;
-    for (StreamSlot& sl : s->slots) {
-      if (&sl == slot || !sl.ws) continue;
-      held += sl.ws_bytes;
-      if (!oldest || sl.last_use < oldest->last_use) oldest = &sl;
-    }
-    if (held <= kMaxWorkspaceBytes || !oldest) return 0;
-    RelaxedCapture relaxed;
-    DRV(cuMemFree(oldest->ws));  // (waits for the work that still uses it)
-    oldest->ws = 0;
-    oldest->ws_bytes = 0;
+// Frees the workspaces of streams other than `keep`'s that `idle` launches have gone past (0: of all others), and buffers that
+// graphs have let go of. (cuMemFree waits for the work that still uses the memory.) Call with g_dev_mutex held.
+int give_back(DeviceState* s, const StreamSlot* keep, uint64_t idle, size_t* freed) {
+  *freed = 0;
+  RelaxedCapture relaxed;
+  for (StreamSlot& sl : s->slots) {
+    if (&sl == keep || !sl.ws || s->use_clock - sl.last_use < idle) continue;
+    DRV(cuMemFree(sl.ws));
+    *freed += sl.ws_bytes;
+    sl.ws = 0;
+    sl.ws_bytes = 0;
   }
+  for (size_t i = 0; i < s->graph_buffers.size();) {
+    GraphBuffer* b = s->graph_buffers[i];
+    if (b->held.load()) {
+      ++i;
+      continue;
+    }
+    DRV(cuMemFree(b->ws));
+    *freed += b->ws_bytes;
+    s->graph_buffers.erase(s->graph_buffers.begin() + i);
+    delete b;
+  }
+  return 0;
+}
+
+bool parts_refused(const DeviceState* s, size_t need) {
+  return s->refused_bytes > 0 && need >= s->refused_bytes && s->use_clock - s->refused_at < kRefusedLaunches;
+}
+
+// The workspace of a launch on the stream of `slot`: the `partials` bytes that it cannot do without or, where *in_parts, the
+// `need` bytes with the parts of its fp32 operands in them. *in_parts becomes false where there is no room for these: beside the
+// other streams' workspaces, which are given up for them only when idle (streams whose large products alternate would take the
+// memory from each other on every call, and wait for the device each time), or on the device.
+// Call with g_dev_mutex held.
+int reserve(DeviceState* s, StreamSlot* slot, size_t partials, size_t need, bool* in_parts) {
+  if (slot->ws_bytes >= (*in_parts ? need : partials)) return 0;
+  size_t freed = 0;
+  if (*in_parts) {
+    *in_parts = !parts_refused(s, need);
+    auto others = [&] {
+      size_t sum = 0;
+      for (const StreamSlot& sl : s->slots)
+        if (&sl != slot) sum += sl.ws_bytes;
+      return sum;
+    };
+    if (*in_parts && others() + need > kMaxWorkspaceBytes) {
+      if (int e = give_back(s, slot, kIdleLaunches, &freed)) return e;
+      *in_parts = others() + need <= kMaxWorkspaceBytes;
+    }
+  }
+  if (*in_parts) {
+    RelaxedCapture relaxed;
+    CUdeviceptr fresh = 0;
+    CUresult r = driver().p_cuMemAlloc(&fresh, need);  // (before the old one goes: it is kept if there is no memory)
+    if (r == CUDA_ERROR_OUT_OF_MEMORY) {
+      if (int e = give_back(s, slot, kIdleLaunches, &freed)) return e;
+      const size_t old = slot->ws ? slot->ws_bytes : 0;
+      if (old > 0) {
+        DRV(cuMemFree(slot->ws));
+        slot->ws = 0;
+        slot->ws_bytes = 0;
+      }
+      if (freed + old > 0) r = driver().p_cuMemAlloc(&fresh, need);
+    }
+    if (r == CUDA_SUCCESS) {
+      s->tmaps.clear();  // drops the maps of the workspace that moves
+      if (slot->ws) DRV(cuMemFree(slot->ws));
+      slot->ws = fresh;
+      slot->ws_bytes = need;
+      return 0;
+    }
+    if (r != CUDA_ERROR_OUT_OF_MEMORY) return drv_fail(r, "cuMemAlloc(workspace)");
+    *in_parts = false;
+    s->refused_bytes = need;
+    s->refused_at = s->use_clock;
+  }
+  if (slot->ws_bytes >= partials) return 0;
+  s->tmaps.clear();
+  int e = grow(&slot->ws, &slot->ws_bytes, partials);
+  if (e == CUDA_ERROR_OUT_OF_MEMORY) {
+    if (int g = give_back(s, slot, 0, &freed)) return g;
+    if (freed > 0) e = grow(&slot->ws, &slot->ws_bytes, partials);
+  }
+  return e;
 }
 
 int free_slot(StreamSlot& sl) {
@@ -1416,7 +1488,6 @@ static int launch_impl(uint64_t function, const kcg_kernel_info* info, int devic
         parts = kcg::split_f32_layout(partials, M, N, K);
         need = parts.end;
         split_now = need <= kMaxWorkspaceBytes;
-        if (!split_now) need = partials;
       }
       CUstreamCaptureStatus capturing = CU_STREAM_CAPTURE_STATUS_NONE;
       cuuint64_t id = 0;
@@ -1426,9 +1497,17 @@ static int launch_impl(uint64_t function, const kcg_kernel_info* info, int devic
                                                nullptr, nullptr) == CUDA_SUCCESS &&
           capturing == CU_STREAM_CAPTURE_STATUS_ACTIVE) {
         GraphBuffer* buf = nullptr;
-        int e = graph_buffer(s, reinterpret_cast<CUstream>(stream), id, graph, need, tiles, &buf);
+        split_now = split_now && !parts_refused(s, need);
+        int e = graph_buffer(s, reinterpret_cast<CUstream>(stream), id, graph, split_now ? need : partials, tiles, &buf);
+        size_t freed = 0;
+        if (e == CUDA_ERROR_OUT_OF_MEMORY) {
+          if (int g = give_back(s, nullptr, split_now ? kIdleLaunches : 0, &freed)) return g;
+          if (freed > 0) e = graph_buffer(s, reinterpret_cast<CUstream>(stream), id, graph, split_now ? need : partials, tiles, &buf);
+        }
         if (e == CUDA_ERROR_OUT_OF_MEMORY && split_now) {
           split_now = false;
+          s->refused_bytes = need;
+          s->refused_at = s->use_clock;
           e = graph_buffer(s, reinterpret_cast<CUstream>(stream), id, graph, partials, tiles, &buf);
         }
         if (e) return e;
@@ -1436,16 +1515,7 @@ static int launch_impl(uint64_t function, const kcg_kernel_info* info, int devic
         ws_bytes = buf->ws_bytes;
         p.tile_counters = reinterpret_cast<unsigned int*>(buf->counters());
       } else {
-        if (slot->ws_bytes < need) {
-          s->tmaps.clear();  // drops the maps of the workspace that is about to move
-          if (int e = make_room(s, slot, need)) return e;
-          int e = grow(&slot->ws, &slot->ws_bytes, need);
-          if (e == CUDA_ERROR_OUT_OF_MEMORY && split_now) {
-            split_now = false;
-            e = grow(&slot->ws, &slot->ws_bytes, partials);
-          }
-          if (e) return e;
-        }
+        if (int e = reserve(s, slot, partials, need, &split_now)) return e;
         if (slot->counters_n < tiles) {
           size_t have = slot->counters_n * 4;
           slot->counters_n = 0;
@@ -1682,6 +1752,51 @@ int kcg_matmul_host(uint64_t function, const kcg_kernel_info* info, int device, 
   step(r_out, "cuStreamSynchronize");
   step(r_st, "cuStreamSynchronize");
   return rc ? rc : kernel_status(s_exec);
+}
+
+int kcg_trim(int device) {
+  if (device < 0 || device >= kMaxDevices) return fail(KCG_E_BAD_ARG, "device %d out of range", device);
+  std::lock_guard<std::mutex> g(g_dev_mutex);
+  DeviceState& s = g_dev[device];
+  if (!s.init) return 0;
+  CUcontext cur = nullptr;
+  DRV(cuCtxGetCurrent(&cur));
+  DRV(cuCtxSetCurrent(s.ctx));
+  size_t freed = 0;
+  int e = give_back(&s, nullptr, 0, &freed);
+  if (freed > 0) s.tmaps.clear();
+  if (cur && cur != s.ctx) DRV(cuCtxSetCurrent(cur));
+  return e;
+}
+
+// For an allocator that is about to take memory from the device: kcg_trim when less than a quarter of it is free.
+// True if there was something to give back.
+bool kcg_internal_trim_if_low(int device) {
+  if (device < 0 || device >= kMaxDevices) return false;
+  {
+    std::lock_guard<std::mutex> g(g_dev_mutex);
+    const DeviceState& s = g_dev[device];
+    bool held = false;
+    for (const StreamSlot& sl : s.slots) held = held || sl.ws;
+    for (const GraphBuffer* b : s.graph_buffers) held = held || !b->held.load();
+    size_t free_bytes = 0, total = 0;
+    if (!held || driver().p_cuMemGetInfo(&free_bytes, &total) != CUDA_SUCCESS || free_bytes >= total / 4) return false;
+  }
+  return kcg_trim(device) == 0;
+}
+
+// reserve() for a stream, without a launch. out: {in parts, workspace bytes}.
+int kcg_internal_reserve(int device, uint64_t stream, uint64_t partials, uint64_t need, uint64_t out[2]) {
+  DeviceState* s = nullptr;
+  if (int e = ensure_device(device, &s)) return e;
+  std::lock_guard<std::mutex> guard(g_dev_mutex);
+  StreamSlot* slot = nullptr;
+  if (int e = slot_for(s, reinterpret_cast<CUstream>(stream), true, &slot)) return e;
+  bool in_parts = need > 0;
+  const int e = reserve(s, slot, partials, need, &in_parts);
+  out[0] = in_parts;
+  out[1] = slot->ws_bytes;
+  return e;
 }
 
 int kcg_shutdown(void) {

@@ -13,8 +13,11 @@
 #include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 
+#include <atomic>
 #include <cmath>
 #include <cstdint>
 #include <unordered_map>
@@ -29,6 +32,16 @@ using AttentionFn = int (*)(int, uint64_t, uint64_t, uint64_t, uint64_t, uint64_
 GemmFn g_gemm = nullptr;
 AttentionFn g_attention = nullptr;
 PyObject* g_check = nullptr;  // raises the error of a status
+
+// torch's allocator asks before it takes memory from the device: the library's workspaces, which it cannot see, are given back
+// when memory is low. (No GIL here, and no call of the library comes back to the allocator.)
+std::atomic<bool (*)(int)> g_trim{nullptr};
+struct GiveBack final : c10::FreeMemoryCallback {
+  bool Execute() override {
+    bool (*trim)(int) = g_trim.load();
+    return trim && trim(c10::cuda::current_device());
+  }
+};
 
 // What the operator chose a kernel by. Written and read with the GIL held.
 struct Shape {
@@ -202,11 +215,20 @@ PyObject* bind(PyObject*, PyObject* args) {
   Py_RETURN_NONE;
 }
 
+// bind_trim(kcg_internal_trim_if_low)
+PyObject* bind_trim(PyObject*, PyObject* args) {
+  unsigned long long trim;
+  if (!PyArg_ParseTuple(args, "K", &trim)) return nullptr;
+  g_trim = reinterpret_cast<bool (*)(int)>(static_cast<uintptr_t>(trim));
+  Py_RETURN_NONE;
+}
+
 template <typename F>
 PyCFunction fast(F f) {
   return reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f));
 }
 PyMethodDef g_methods[] = {{"bind", bind, METH_VARARGS, "addresses of the library's entries"},
+                           {"bind_trim", bind_trim, METH_VARARGS, "address of the function that gives memory back"},
                            {"remember", remember, METH_VARARGS, "a shape's kernel"},
                            {"matmul", fast(matmul), METH_FASTCALL, "a product whose kernel is known, or None"},
                            {"bmm", fast(bmm), METH_FASTCALL, "a batched one"},
@@ -215,6 +237,10 @@ PyMethodDef g_methods[] = {{"bind", bind, METH_VARARGS, "addresses of the librar
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_torchcall", nullptr, -1, g_methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace
+
+namespace c10 {
+REGISTER_FREE_MEMORY_CALLBACK("kcg_workspaces", GiveBack)
+}
 
 PyMODINIT_FUNC PyInit__torchcall() {
   PyObject* m = PyModule_Create(&g_module);

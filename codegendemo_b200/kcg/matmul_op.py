@@ -380,6 +380,7 @@ def _warm_calls():
             lib = _lib.get_lib()
             found.bind(*(ctypes.cast(f, ctypes.c_void_p).value for f in (lib.kcg_launch_gemm_strided, lib.kcg_attention_fwd)),
                        _lib.check)
+            found.bind_trim(ctypes.cast(lib.kcg_internal_trim_if_low, ctypes.c_void_p).value)
         _warm = found
     return _warm
 

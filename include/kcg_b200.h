@@ -293,6 +293,9 @@ int kcg_gemm_bf16_splitk_noalloc(int device, uint64_t stream, uint64_t A, uint64
 /* Number of kernel launches issued through this library since load (all threads); a product of KCG_KERNEL_F32_SPLIT counts
  * as one. */
 uint64_t kcg_launch_count(void);
+/* Gives back the workspaces of a device's streams and those that graphs have let go of; waits for the work that uses them.
+ * The next launch that needs one takes it again. */
+int kcg_trim(int device);
 /* Frees workspaces, device buffers and cached tensor maps of every device. */
 int kcg_shutdown(void);
 const char* kcg_last_error(void);

@@ -174,3 +174,35 @@ def test_a_launch_holds_what_owns_its_kernel(warm):
     finally:
         go_on.set()
         warm.bind(address(lib.kcg_launch_gemm_strided), address(lib.kcg_attention_fwd), _lib.check)
+
+
+@pytest.mark.gpu
+def test_the_allocator_asks_before_it_takes_memory(warm):
+    """What would give the library's workspaces back (a stand-in) is called when torch goes to the device for memory."""
+    asked = []
+    trim = ctypes.CFUNCTYPE(ctypes.c_bool, ctypes.c_int)(lambda device: bool(asked.append(device)))
+    own = ctypes.cast(_lib.get_lib().kcg_internal_trim_if_low, ctypes.c_void_p).value
+    torch.cuda.empty_cache()
+    warm.bind_trim(ctypes.cast(trim, ctypes.c_void_p).value)
+    try:
+        t = torch.empty(64 << 20, dtype=torch.uint8, device="cuda")
+    finally:
+        warm.bind_trim(own)
+    assert asked == [t.device.index]
+
+
+@pytest.mark.gpu
+def test_a_product_after_its_workspace_is_gone():
+    """Parts, partials and captured graphs after kcg_trim: the same bits."""
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    a, b = [torch.rand(s, generator=gen, device="cuda") * 2 - 1 for s in ((2048, 2048), (2048, 4096))]
+    want = matmul_op.matmul(a, b)
+    c = torch.empty_like(want)
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        matmul_op.matmul(a, b, c)
+    assert _lib.get_lib().kcg_trim(0) == 0
+    junk = [torch.full((1 << 22,), 7.0, device="cuda") for _ in range(16)]  # what is free now belongs to others
+    graph.replay()
+    assert torch.equal(c, want) and torch.equal(matmul_op.matmul(a, b), want)
+    assert all(bool((j == 7.0).all()) for j in junk)
