@@ -1099,6 +1099,28 @@ SplitPlan plan_split(const kcg_kernel_info* info, int batch = 1) {
   return SplitPlan{T, first, factor, sk_per, sk_ranges, G, units_first};
 }
 
+// CTAs (CTA pairs) of a launch, and its workspace slots of one tile each: those of the split tiles - one per (tile, split) of an
+// even split, range index + tile index under stream-K - and behind them, where whole tiles pass through the workspace too,
+// one per CTA that has any.
+struct LaunchSlots {
+  int grid;
+  size_t split, whole;
+};
+LaunchSlots launch_slots(const SplitPlan& pl, bool whole_through_workspace) {
+  LaunchSlots l;
+  // Under stream-K the whole tiles before the tail are walked with the grid as stride: the grid
+  // stays at every unit that runs at once even when the tail is cut into fewer ranges (the CTAs
+  // beyond the last range then simply have no tail piece).
+  const int units = pl.sk_per > 0 ? (pl.first > 0 ? pl.units_at_once : pl.sk_ranges) : pl.first + (pl.tiles - pl.first) * pl.factor;
+  l.grid = units < pl.units_at_once ? units : pl.units_at_once;
+  l.split = pl.sk_per > 0   ? static_cast<size_t>(pl.sk_ranges) + (pl.tiles - pl.first)
+            : pl.factor > 1 ? static_cast<size_t>(pl.tiles - pl.first) * pl.factor
+                            : 0;
+  // (a stream-K range may hold a tile whole: any CTA may have one)
+  l.whole = !whole_through_workspace ? 0 : pl.sk_per > 0 || pl.first >= pl.units_at_once ? pl.units_at_once : pl.first;
+  return l;
+}
+
 }  // namespace
 
 // ============================================================================ C ABI
@@ -1112,7 +1134,7 @@ void kcg_internal_count_launch(void) { g_launches.fetch_add(1); }
 // {tiles, split_first_tile, split_factor, sk_per, stream-K ranges, units that run at once, split units first}.
 int kcg_internal_plan_split(const kcg_kernel_info* info, int fused_epilogue, int batch, int out[7]) {
   if (!info || !out || batch < 1) return fail(KCG_E_BAD_ARG, "null argument");
-  (void)fused_epilogue;  // a launch is cut up in the same way with and without one
+  (void)fused_epilogue;  // (a launch is cut up in the same way with and without one: what it changes is kcg_internal_launch_slots)
   const SplitPlan pl = plan_split(info, batch);
   out[0] = pl.tiles;
   out[1] = pl.first;
@@ -1121,6 +1143,17 @@ int kcg_internal_plan_split(const kcg_kernel_info* info, int fused_epilogue, int
   out[4] = pl.sk_ranges;
   out[5] = pl.units_at_once;
   out[6] = pl.units_first;
+  return 0;
+}
+
+// The workspace of such a launch: {CTAs (pairs), slots of split tiles, slots of whole tiles}.
+int kcg_internal_launch_slots(const kcg_kernel_info* info, int fused_epilogue, int batch, int out[3]) {
+  if (!info || !out || batch < 1) return fail(KCG_E_BAD_ARG, "null argument");
+  const bool x3 = info->dtype == KCG_DTYPE_FLOAT32 && info->kernel != KCG_KERNEL_TF32X1;
+  const LaunchSlots l = launch_slots(plan_split(info, batch), x3 && fused_epilogue != 0);
+  out[0] = l.grid;
+  out[1] = static_cast<int>(l.split);
+  out[2] = static_cast<int>(l.whole);
   return 0;
 }
 
@@ -1452,23 +1485,15 @@ static int launch_impl(uint64_t function, const kcg_kernel_info* info, int devic
         return e;
     }
     const SplitPlan plan = plan_split(info, batch);
-    const int T = plan.tiles, first = plan.first, factor = plan.factor, sk_per = plan.sk_per,
-              sk_ranges = plan.sk_ranges, G = plan.units_at_once;
+    const int T = plan.tiles, first = plan.first, factor = plan.factor, sk_per = plan.sk_per;
     // The 3xTF32 kernel applies a fused epilogue in its reduction loop only (its register file is full of accumulators at
     // the direct store), so a whole tile of a fused launch passes through the workspace too: through one slot per CTA
     // (pair), behind those of the split tiles, that its tiles take in turn and that stays in L2. (With a slot a tile,
     // and the remainder never cut into K ranges: 128x4864x9024 with bias and ReLU 360 us, now 85.)
     const bool ws_epilogue = x3 && p.epi_flags != 0u;
-    // slots of partials: one per (tile, split) of an even split; range index + tile index under stream-K
-    const size_t split_slots = sk_per > 0   ? static_cast<size_t>(sk_ranges) + (T - first)
-                               : factor > 1 ? static_cast<size_t>(T - first) * factor
-                                            : 0;
-    p.whole_slot0 = static_cast<int>(split_slots);
-    // Under stream-K the whole tiles before the tail are walked with the grid as stride: the grid
-    // stays at every unit that runs at once even when the tail is cut into fewer ranges (the CTAs
-    // beyond the last range then simply have no tail piece).
-    const int units = sk_per > 0 ? (first > 0 ? G : sk_ranges) : first + (T - first) * factor;
-    grid0 = (units < G ? units : G) * (pair ? 2 : 1);
+    const LaunchSlots slots = launch_slots(plan, ws_epilogue);
+    p.whole_slot0 = static_cast<int>(slots.split);
+    grid0 = slots.grid * (pair ? 2 : 1);
     p.split_first_tile = first;
     p.split_factor = factor;
     p.sk_per = sk_per;
@@ -1478,9 +1503,7 @@ static int launch_impl(uint64_t function, const kcg_kernel_info* info, int devic
     kcg::SplitF32Layout parts{};
     bool split_now = h2;  // false: no memory for the parts; the kernel then reads the fp32 operands
     if (factor > 1 || ws_epilogue || sk_per > 0 || h2) {
-      const size_t whole_slots = !ws_epilogue ? 0 : sk_per > 0 ? G : first < G ? first : G;
-      const size_t slots = split_slots + whole_slots;
-      const size_t partials = slots * info->bm * info->bn * sizeof(float);
+      const size_t partials = (slots.split + slots.whole) * info->bm * info->bn * sizeof(float);
       size_t need = partials;
       // one counter per CTA half; before them the two words of the split fp32 kernel
       const size_t tiles = static_cast<size_t>(T > first ? T - first : 1) * (pair ? 2 : 1) + (h2 ? 4 : 0);

@@ -1,6 +1,8 @@
 """Fused epilogues of the 3xTF32 kernels: whole tiles through one workspace slot per CTA (pair), remainder tiles cut into K
 ranges behind them, as without an epilogue."""
 import ctypes
+import os
+import subprocess
 
 import pytest
 import torch
@@ -77,3 +79,39 @@ def test_fused_batches():
     c = bmm(a, b, bias=bias, relu=True)
     want = torch.relu(a.double() @ b.double() + bias.double())
     assert (c.double() - want).abs().le(2.0 ** -20 * (a.double().abs() @ b.double().abs()) + 2.0 ** -22 * bias.abs().max()).all()
+
+
+@pytest.mark.parametrize("mode", [None, "0", "1", "2", "3", "4", "5"])
+def test_slots_lie_inside_the_workspace(mode, tmp_path, monkeypatch):
+    """Every tile of a fused launch passes through a slot that the launch has memory for: fewer whole tiles than CTAs, more,
+    none, and K blocks laid end to end."""
+    if mode is None:
+        monkeypatch.delenv("KCG_TAIL_SPLIT", raising=False)
+    else:
+        monkeypatch.setenv("KCG_TAIL_SPLIT", mode)
+    lib = _lib.get_lib()
+    for f in (lib.kcg_internal_plan_split, lib.kcg_internal_launch_slots):
+        f.argtypes = [ctypes.POINTER(_lib.KernelInfo), ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_int)]
+    tests = os.path.dirname(os.path.abspath(__file__))
+    kernels = os.path.join(os.path.dirname(tests), "codegendemo_b200", "csrc", "kernels")
+    programs, wholes = {}, []
+    more = [(4096, 4096, 2048, 4, (256, 256, 32), None), (3456, 768, 1408, 2, (128, 128, 32), None),
+            (2048, 4096, 4096, 4, (256, 128, 32), None), (256, 256, 512, 4, (256, 128, 32), None)]
+    for M, N, K, variant, tile, _ in CASES + more:
+        kpm = _config(M, N, K, variant, tile)
+        info = compile_info(kpm.compileArgs(), num_stages=kpm.NUM_STAGES, kernel=kpm.KERNEL_VARIANT, edge_tiles=kpm.EDGE_TILES)
+        plan, slots = (ctypes.c_int * 7)(), (ctypes.c_int * 3)()
+        assert lib.kcg_internal_plan_split(ctypes.byref(info), 1, 1, plan) == 0
+        assert lib.kcg_internal_launch_slots(ctypes.byref(info), 1, 1, slots) == 0
+        if tile not in programs:
+            programs[tile] = str(tmp_path / "x".join(map(str, tile)))
+            subprocess.run(["g++", "-O1", "-std=c++17", "-I/usr/local/cuda/include", "-I" + kernels, "-o", programs[tile],
+                            os.path.join(tests, "slot_check.cpp")] + [f"-DSC_B{d}={v}" for d, v in zip("MNK", tile)], check=True)
+        r = subprocess.run([programs[tile]] + [str(v) for v in (M, N, K, plan[1], plan[2], plan[3], *slots)], capture_output=True, text=True)
+        assert r.returncode == 0, (M, N, K, tile, list(plan), list(slots), r.stdout + r.stderr)
+        wholes.append(int(r.stdout.split()[1]))
+        slots_plain = (ctypes.c_int * 3)()
+        assert lib.kcg_internal_launch_slots(ctypes.byref(info), 0, 1, slots_plain) == 0
+        assert slots_plain[2] == 0 and list(slots_plain[:2]) == list(slots[:2])
+    assert 0 in wholes or mode == "0"
+    assert max(wholes) > 148
