@@ -1505,8 +1505,8 @@ static int launch_impl(uint64_t function, const kcg_kernel_info* info, int devic
     if (factor > 1 || ws_epilogue || sk_per > 0 || h2) {
       const size_t partials = (slots.split + slots.whole) * info->bm * info->bn * sizeof(float);
       size_t need = partials;
-      // one counter per CTA half; before them the two words of the split fp32 kernel
-      const size_t tiles = static_cast<size_t>(T > first ? T - first : 1) * (pair ? 2 : 1) + (h2 ? 4 : 0);
+      // one counter per CTA half; before them the words of the split fp32 kernel
+      const size_t tiles = static_cast<size_t>(T > first ? T - first : 1) * (pair ? 2 : 1) + (h2 ? kcg::H2_WORDS : 0);
       if (h2) {
         parts = kcg::split_f32_layout(partials, M, N, K);
         need = parts.end;
@@ -1553,7 +1553,7 @@ static int launch_impl(uint64_t function, const kcg_kernel_info* info, int devic
       p.splitk_ws = reinterpret_cast<float*>(ws);
       if (h2) {
         unsigned int* words = p.tile_counters;
-        p.tile_counters += 4;
+        p.tile_counters += kcg::H2_WORDS;
         if (split_now) p.h2_words = words;
       }
     }
@@ -1577,12 +1577,23 @@ static int launch_impl(uint64_t function, const kcg_kernel_info* info, int devic
       p.columns = q.columns;
       p.scale_a = q.scale_a;
       p.scale_b = q.scale_b;
-      // the parts as one matrix of 64 halves a row, A's and then B's, up to the last row of B's: boxes past it read zeros
-      const uint64_t kb = blocks_of(K, kcg::H2_BK), row_b0 = (parts.parts_b - parts.parts_a) / 128;
-      p.parts_b_row = static_cast<int>(row_b0);
-      if (int e = encode_map(s, &p.tmWs, KCG_DTYPE_FLOAT16, ws + parts.parts_a, 64, row_b0 + blocks_of(N, 64) * kb * 128, 128,
-                             64, 128, 3))
-        return e;
+      q.far_a = reinterpret_cast<uint8_t*>(ws + parts.far_a);
+      q.far_b = reinterpret_cast<uint8_t*>(ws + parts.far_b);
+      q.far_scale_a = reinterpret_cast<float*>(ws + parts.far_scale_a);
+      q.far_scale_b = reinterpret_cast<float*>(ws + parts.far_scale_b);
+      p.far_scale_a = static_cast<int>((parts.far_scale_a - parts.scale_a) / 4);
+      p.far_scale_b = static_cast<int>((parts.far_scale_b - parts.scale_b) / 4);
+      p.far_zero_b = p.far_scale_b + parts.far_slots_b;
+      p.far_zero_a = p.far_zero_b + static_cast<int>((parts.scale_b - parts.scale_a) / 4);
+      q.far_slots_a = parts.far_slots_a;
+      q.far_slots_b = parts.far_slots_b;
+      // the parts as one matrix of 64 halves a row: A's, B's, the far ones; boxes past it read zeros
+      auto row_of = [&](size_t offset) { return static_cast<int>((offset - parts.parts_a) / 128); };
+      p.parts_b_row = row_of(parts.parts_b);
+      p.far_a_row = row_of(parts.far_a);
+      p.far_b_row = row_of(parts.far_b);
+      p.parts_rows = row_of(parts.scale_a);
+      if (int e = encode_map(s, &p.tmWs, KCG_DTYPE_FLOAT16, ws + parts.parts_a, 64, p.parts_rows, 128, 64, 128, 3)) return e;
       if (int e = encode_map(s, &p.tmC, KCG_DTYPE_FLOAT32, C, N, M, static_cast<uint64_t>(ldc) * 4, 32, 32, 3)) return e;
       if (int e = kcg_internal_split_f32(stream, &q, pdl_on() ? 1 : 0)) return e;
     }

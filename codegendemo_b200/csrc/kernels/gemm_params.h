@@ -87,8 +87,8 @@ struct alignas(64) KcgGemmParams {
   // this on.
   int whole_slot0;
   // KERNEL_VARIANT 6 (gemm_tcgen05_f32h2.cuh): the factors of the parts' products, [K block][rows of A] and [K block][64
-  // columns of B] with these pitches, those of the finished columns, and {not every value splits, CTAs done}; no words:
-  // 3xTF32 throughout. tmWs maps the parts, those of B from row parts_b_row on.
+  // columns of B] with these pitches, those of the finished columns, and the words (H2_WORDS below); no words: 3xTF32
+  // throughout. tmWs maps the parts, those of B from row parts_b_row on.
   const float* scale_a;
   const float* scale_b;
   const float* columns;
@@ -101,6 +101,9 @@ struct alignas(64) KcgGemmParams {
   // no flags between GPUs: the data is in place when every rank's kernel has completed).
   int n_peers;
   void* peerC[KCG_MAX_PEERS];
+  // KERNEL_VARIANT 6: rows of tmWs; far parts, in slots of a chunk each: their first rows there; their factors, [slot][128 rows of
+  // A] and [slot], as places from scale_a and from scale_b on, and the place of a zero from each.
+  int parts_rows, far_a_row, far_b_row, far_scale_a, far_scale_b, far_zero_a, far_zero_b;
 };
 
 namespace kcg {
@@ -274,6 +277,16 @@ constexpr int ck_smem_bytes(int BN, int BK, int stages, int pair = 0) { return c
 // fp32 through fp16 parts (gemm_tcgen05_f32h2.cuh): 256-row tiles on CTA pairs; the kernel it falls back to is the 3xTF32
 // pair kernel of the same tile with K blocks of 32 and h2_x3_stages stages.
 constexpr int H2_BK = 64;  // K block = chunk of one exponent
+// Words between the split and the product, zero between launches: what the split found (H2_UNSPLIT | H2_FAR) and, on the same line,
+// the CTAs of the product that are done; slots taken for far parts of A, of B; and H2_FLAGS flags that a value does not split, for
+// the CTAs of the split itself. These lie on lines of their own: a thousand CTAs that set one word while others asked for it
+// took 30 us.
+constexpr unsigned int H2_UNSPLIT = 1u, H2_FAR = 2u;
+constexpr int H2_LINE = 32, H2_FOUND = 0, H2_DONE = 1, H2_FAR_A = H2_LINE, H2_FAR_B = 2 * H2_LINE, H2_FLAG = 3 * H2_LINE, H2_FLAGS = 32;
+constexpr int H2_WORDS = H2_FLAG + H2_FLAGS * H2_LINE;
+// A factor is a power of two: those of a chunk of B and of the first row of a panel of A carry the chunk's slot of far parts
+// (from 1 on, 0: none) in the bits below.
+constexpr unsigned int H2_SLOT_BITS = 0x7fffffu;
 constexpr int h2_config_error(int BM, int BN, int BK) {
   if (BM != 256) return 2;
   if (BN != 128 && BN != 256) return 3;

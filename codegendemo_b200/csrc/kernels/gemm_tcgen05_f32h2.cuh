@@ -7,10 +7,15 @@
 // below 2^-24 of the product instead of 2^-20; and kind::f16 multiplies twice as many values a cycle as kind::tf32 and reads
 // half as many bytes for it. Error against 64 bits, uniform values: 1.4e-7 at K = 1024, 1.9e-7 at 4096, 2.6e-7 at 11008,
 // where 3xTF32 has 1.0e-6 (normwise; largest 2e-6 and 5e-6).
-// What does not split - an infinity, a NaN, values whose largest is outside 2^+-50, a value so far (about 2^-30) below
-// the largest one beside it that its parts would keep less than 21 bits - sets a word, and this kernel then multiplies the
-// fp32 operands as 3xTF32 (TcGemmF32x3, in the same launch): no input loses accuracy over that kernel. Values drawn from a
-// normal distribution set it about once in thirty products of 4096 x 4096 operands; the split stops early then.
+// A chunk with a value so far (about 2^-30) below the largest one beside it that its parts would keep less than 21 bits has far
+// parts: such values alone, under an exponent of their own, in one of a limited number of slots (kcg_f32split.cu). It is multiplied
+// once more for them. What does not split at all - an infinity, a NaN, values whose largest is outside 2^+-50, more chunks with far
+// parts than slots - sets a word, and this kernel then multiplies the fp32 operands as 3xTF32 (TcGemmF32x3, in the same launch):
+// no input loses accuracy over that kernel. Values drawn from a normal distribution need far parts about once in thirty products of
+// 4096 x 4096 operands. Times of a call with values that all split / with one far value / that fall back after the split (every
+// value of A exp(8 x normal)) / of 3xTF32 alone, us: 1024x7936x768 48 / 57 / 86 / 66, 1536x5632x1024 56 / 65 / 105 / 84, 512x11008x4096
+// 177 / 213 / 242 / 209, 2048x4096x4096 188 / 250 / 336 / 300, 4096^3 380 / 426 / 592 / 566, 2048x11008x11008 1350 / 1477 / 2073 / 2012 (calls in
+// a row; without far parts one such value took 82, 96, 239, 349, 609, 2115).
 //
 // Each 64 values of K (a chunk) are multiplied into a fresh accumulator in tensor memory, the two correction products
 // first; the first hi * hi product scales what they have summed by 2^-12 (scale-input-d). The accumulating warps add
@@ -82,46 +87,75 @@ struct TcGemmF32H2 {
     }
   }
 
-  // True: not every value splits, nothing was computed.
-  __device__ static __forceinline__ bool multiply(const KcgGemmParams& p) {
-    extern __shared__ __align__(1024) uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                               ~static_cast<uintptr_t>(1023));
-    Barriers* bars = reinterpret_cast<Barriers*>(smem + RING_BYTES + STORE_BYTES);
+  // The chunks that a unit of a product with far parts multiplies, in order, as runs: of every K block the parts (what = 0) and, where
+  // one of the tile's panels of A or chunks of B has far parts there, those of A with the parts of B (1), those of B with the parts
+  // of A (2), both (3), each a run of one; panels and chunks that have none stand in with zeros. Every role walks the same sequence.
+  // Without far parts a unit is one run: the roles' inner loops go over a run, by increments alone, and know nothing of all this.
+  // (With the walk inside the accumulating loop 2048x4096x4096 took 248 us instead of 188, with that loop compiled twice 196.)
+  struct Chunks {
+    const KcgGemmParams& p;
+    int m0, n0, kb, run, end;
+    uint32_t what, left;  // left: bit `what` of the runs of this K block that are still to come
+    int base;             // K blocks base .. base + 31: which of them have far parts of A, of B
+    uint32_t with_a, with_b;
+    __device__ __forceinline__ Chunks(const KcgGemmParams& p_, const Unit& w)
+        : p(p_), m0(w.m0), n0(w.n0), kb(w.kb0), run(0), end(w.kb0 + w.kbn), what(0u), left(0u), base(w.kb0 - 32), with_a(0u), with_b(0u) {}
+    // slots of far parts (0: none) of panel i of the tile's rows and of chunk i of its columns
+    __device__ __forceinline__ int slot_a(int k, int i) const {
+      if (m0 + i * 128 >= p.M) return 0;
+      return __float_as_uint(__ldcg(p.scale_a + static_cast<size_t>(k) * p.scale_lda + m0 + i * 128)) & H2_SLOT_BITS;
+    }
+    __device__ __forceinline__ int slot_b(int k, int i) const {
+      if (n0 + i * 64 >= p.N) return 0;
+      return __float_as_uint(__ldcg(p.scale_b + static_cast<size_t>(k) * p.scale_ldb + (n0 >> 6) + i)) & H2_SLOT_BITS;
+    }
+    __device__ __forceinline__ bool any_a(int k) const { return (slot_a(k, 0) | slot_a(k, 1)) != 0; }
+    __device__ __forceinline__ bool any_b(int k) const {
+      int any = 0;
+#pragma unroll
+      for (int i = 0; i < kBN / 64; ++i) any |= slot_b(k, i);
+      return any != 0;
+    }
+    // The next run; false: none. A whole warp looks up 32 K blocks together and walks those without far parts as one run; one
+    // thread takes them one by one.
+    template <bool kWarp>
+    __device__ __forceinline__ bool next() {
+      if (left == 0u) {
+        kb += run;
+        if (kb >= end) return false;
+        if (kWarp) {
+          if (kb >= base + 32) {
+            base = kb;
+            const int k = base + static_cast<int>(threadIdx.x & 31);
+            with_a = __ballot_sync(0xffffffffu, k < end && any_a(k));
+            with_b = __ballot_sync(0xffffffffu, k < end && any_b(k));
+          }
+        } else {
+          base = kb;
+          with_a = any_a(kb) ? 1u : 0u;
+          with_b = any_b(kb) ? 1u : 0u;
+        }
+        const uint32_t a = with_a >> (kb - base), b = with_b >> (kb - base);
+        const int clear = (a | b) != 0u ? __ffs(a | b) - 1 : 32;  // K blocks without far parts from here on
+        const int rest = (kWarp && end - base > 32 ? base + 32 : end) - kb;
+        run = !kWarp || clear == 0 ? 1 : clear < rest ? clear : rest;
+        left = 1u | (clear != 0 ? 0u : (a & 1u) << 1 | (b & 1u) << 2 | (a & b & 1u) << 3);
+      }
+      what = __ffs(left) - 1;
+      left &= left - 1u;
+      return true;
+    }
+    __device__ __forceinline__ bool far_a() const { return (what & 1u) != 0u; }
+    __device__ __forceinline__ bool far_b() const { return (what & 2u) != 0u; }
+  };
+
+  __device__ static __forceinline__ void roles(const KcgGemmParams& p, uint8_t* smem, Barriers* bars, uint32_t tmem_base, uint32_t rank,
+                                               bool far) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tiles_m = (p.M + kBM - 1) / kBM, tiles_n = (p.N + kBN - 1) / kBN;
     const int num_kb = (p.K + kBK - 1) / kBK;
-
-    if (threadIdx.x == 0) {
-      for (int s = 0; s < kStages; ++s) {
-        mbar_init(&bars->full[s], 1);
-        mbar_init(&bars->empty[s], 1);
-      }
-      for (int a = 0; a < 2; ++a) {
-        mbar_init(&bars->tmem_full[a], 1);
-        mbar_init(&bars->tmem_empty[a], 16);  // one arrival per accumulating warp of each CTA
-      }
-      bars->abort_flag = 0u;
-      bars->last_flag = 0u;
-      fence_mbar_init();
-      fence_proxy_async_smem();
-      tma_prefetch_desc(&p.tmWs);
-    }
-    if (warp == 1) tmem_alloc_pair(&bars->tmem_base, TMEM_COLS);
-    tc_fence_before_sync();
-    __syncthreads();
-    cluster_sync_all();  // the peer's barriers exist before anyone signals them
-    tc_fence_after_sync();
-    const uint32_t tmem_base = bars->tmem_base;
-    const uint32_t rank = cluster_cta_rank();  // 0 = leader
     const int unit0 = static_cast<int>(blockIdx.x >> 1), unit_stride = static_cast<int>(gridDim.x >> 1);
-
-    griddep_wait();  // the parts, their exponents and the word are written by the kernel before this one
-    const bool unsplit = *reinterpret_cast<volatile unsigned int*>(p.h2_words) != 0u;
-
-    if (unsplit) {
-      // (no role runs; the right to allocate tensor memory is kept for the other kernel)
-    } else if (warp < 4) {
+    if (warp < 4) {
       Fallback::template reg_dec<CTL_REGS>();
       if (warp == 1) tmem_relinquish_pair();
       if (warp == 0 && lane == 0) {
@@ -133,26 +167,54 @@ struct TcGemmF32H2 {
         while (ok && units.next(w)) {
           const int a_row0 = ((w.m0 >> 7) + static_cast<int>(rank)) * num_kb;
           const int b_chunk0 = (w.n0 + static_cast<int>(rank) * BNL) >> 6;
-          for (int kb = w.kb0; kb < w.kb0 + w.kbn; ++kb, ++it) {
-            const uint32_t s = it % kStages;
-            if (!mbar_wait(&bars->empty[s], ((it / kStages) & 1u) ^ 1u, &bars->abort_flag)) {
-              report(p, bars, KCG_ST_TIMEOUT_PRODUCER, it, s);
-              ok = false;
-              break;
+          int a_row, b_row[BNL / 64];
+          auto rows_of = [&](int kb) {
+            // (chunks of columns past the problem, and those without far parts, lie past the map or are read as something for
+            // results that are not stored, as are panels of rows past it)
+            a_row = (a_row0 + kb) * 256;
+#pragma unroll
+            for (int j = 0; j < BNL / 64; ++j) b_row[j] = p.parts_b_row + ((b_chunk0 + j) * num_kb + kb) * 128;
+          };
+          auto load = [&](int run) {
+            for (int i = 0; i < run; ++i, ++it) {
+              const uint32_t s = it % kStages;
+              if (!mbar_wait(&bars->empty[s], ((it / kStages) & 1u) ^ 1u, &bars->abort_flag)) {
+                report(p, bars, KCG_ST_TIMEOUT_PRODUCER, it, s);
+                ok = false;
+                break;
+              }
+              // completion bytes of both CTAs land on the leader's barrier
+              const uint32_t full_leader = map_to_cta(smem_u32(&bars->full[s]), 0u);
+              if (rank == 0u) mbar_expect_tx(&bars->full[s], static_cast<uint32_t>(2 * STAGE_BYTES));
+              uint8_t* sa = smem + s * STAGE_BYTES;
+#pragma unroll
+              for (int j = 0; j < 2; ++j) tma_load_2d_pair(sa + j * BOX_BYTES, &p.tmWs, full_leader, 0, a_row + j * 128);
+#pragma unroll
+              for (int j = 0; j < BNL / 64; ++j) tma_load_2d_pair(sa + A_BYTES + j * BOX_BYTES, &p.tmWs, full_leader, 0, b_row[j]);
+              a_row += 256;
+#pragma unroll
+              for (int j = 0; j < BNL / 64; ++j) b_row[j] += 128;
             }
-            // completion bytes of both CTAs land on the leader's barrier
-            const uint32_t full_leader = map_to_cta(smem_u32(&bars->full[s]), 0u);
-            if (rank == 0u) mbar_expect_tx(&bars->full[s], static_cast<uint32_t>(2 * STAGE_BYTES));
-            uint8_t* sa = smem + s * STAGE_BYTES;
-            // (chunks of columns past the problem lie past the map and read as zero; panels of rows past it read what lies
-            // behind, into rows of the result that are not stored)
+          };
+          if (!far) {
+            rows_of(w.kb0);
+            load(w.kbn);
+            continue;
+          }
+          for (Chunks ch(p, w); ok && ch.template next<false>();) {
+            rows_of(ch.kb);
+            if (ch.far_a()) {
+              const int slot = ch.slot_a(ch.kb, static_cast<int>(rank));
+              a_row = slot > 0 ? p.far_a_row + (slot - 1) * 256 : p.parts_rows;
+            }
+            if (ch.far_b()) {
 #pragma unroll
-            for (int j = 0; j < 2; ++j)
-              tma_load_2d_pair(sa + j * BOX_BYTES, &p.tmWs, full_leader, 0, (a_row0 + kb) * 256 + j * 128);
-#pragma unroll
-            for (int j = 0; j < BNL / 64; ++j)
-              tma_load_2d_pair(sa + A_BYTES + j * BOX_BYTES, &p.tmWs, full_leader, 0,
-                               p.parts_b_row + ((b_chunk0 + j) * num_kb + kb) * 128);
+              for (int j = 0; j < BNL / 64; ++j) {
+                const int slot = ch.slot_b(ch.kb, static_cast<int>(rank) * (BNL / 64) + j);
+                b_row[j] = slot > 0 ? p.far_b_row + (slot - 1) * 128 : p.parts_rows;
+              }
+            }
+            load(1);
           }
         }
         griddep_launch_dependents();  // every load is issued: the stream's next kernel may be brought in
@@ -166,33 +228,38 @@ struct TcGemmF32H2 {
         Iter units(p, unit0, unit_stride, tiles_m, tiles_n, num_kb);
         Unit w;
         while (ok && units.next(w)) {
-          for (int kb = 0; kb < w.kbn; ++kb, ++it) {
-            const uint32_t s = it % kStages, ab = it & 1u;
-            if (!mbar_wait_warp(&bars->tmem_empty[ab], ((it >> 1) & 1u) ^ 1u, &bars->abort_flag) ||
-                !mbar_wait_warp(&bars->full[s], (it / kStages) & 1u, &bars->abort_flag)) {
-              report(p, bars, KCG_ST_TIMEOUT_MMA, it, s);
-              ok = false;
-              break;
-            }
-            tc_fence_after_sync();
-            if (elect_one()) {
-              const uint64_t a_hi = ring_a + s * (STAGE_BYTES >> 4), a_lo = a_hi + (128 * 128 >> 4);
-              const uint64_t b_hi = ring_b + s * (STAGE_BYTES >> 4), b_lo = b_hi + (kBK * 128 >> 4);
-              const uint32_t d = tmem_base_u + ab * kBN;
-#pragma unroll
-              for (int ks = 0; ks < KSTEPS; ++ks) {  // 16 values of K: 32 bytes of a row of A, 16 rows of B
-                umma_ss_pair<false>(d, a_lo + ks * 2, b_hi + ks * 128, IDESC, ks > 0 ? 1u : 0u);
-                umma_ss_pair<false>(d, a_hi + ks * 2, b_lo + ks * 128, IDESC, 1u);
+          Chunks ch(p, w);
+          for (bool more = true; more && ok; more = far) {  // (one run without far parts)
+            if (far && !ch.template next<true>()) break;
+            const int run = far ? ch.run : w.kbn;
+            for (int i = 0; i < run; ++i, ++it) {
+              const uint32_t s = it % kStages, ab = it & 1u;
+              if (!mbar_wait_warp(&bars->tmem_empty[ab], ((it >> 1) & 1u) ^ 1u, &bars->abort_flag) ||
+                  !mbar_wait_warp(&bars->full[s], (it / kStages) & 1u, &bars->abort_flag)) {
+                report(p, bars, KCG_ST_TIMEOUT_MMA, it, s);
+                ok = false;
+                break;
               }
-              umma_ss_pair_f16_scaled_d<12>(d, a_hi, b_hi, IDESC);
+              tc_fence_after_sync();
+              if (elect_one()) {
+                const uint64_t a_hi = ring_a + s * (STAGE_BYTES >> 4), a_lo = a_hi + (128 * 128 >> 4);
+                const uint64_t b_hi = ring_b + s * (STAGE_BYTES >> 4), b_lo = b_hi + (kBK * 128 >> 4);
+                const uint32_t d = tmem_base_u + ab * kBN;
 #pragma unroll
-              for (int ks = 1; ks < KSTEPS; ++ks) umma_ss_pair<false>(d, a_hi + ks * 2, b_hi + ks * 128, IDESC, 1u);
-              umma_commit_pair(smem_u32(&bars->empty[s]));
-              umma_commit_pair(map_to_cta(smem_u32(&bars->empty[s]), 1u));
-              umma_commit_pair(smem_u32(&bars->tmem_full[ab]));
-              umma_commit_pair(map_to_cta(smem_u32(&bars->tmem_full[ab]), 1u));
+                for (int ks = 0; ks < KSTEPS; ++ks) {  // 16 values of K: 32 bytes of a row of A, 16 rows of B
+                  umma_ss_pair<false>(d, a_lo + ks * 2, b_hi + ks * 128, IDESC, ks > 0 ? 1u : 0u);
+                  umma_ss_pair<false>(d, a_hi + ks * 2, b_lo + ks * 128, IDESC, 1u);
+                }
+                umma_ss_pair_f16_scaled_d<12>(d, a_hi, b_hi, IDESC);
+#pragma unroll
+                for (int ks = 1; ks < KSTEPS; ++ks) umma_ss_pair<false>(d, a_hi + ks * 2, b_hi + ks * 128, IDESC, 1u);
+                umma_commit_pair(smem_u32(&bars->empty[s]));
+                umma_commit_pair(map_to_cta(smem_u32(&bars->empty[s]), 1u));
+                umma_commit_pair(smem_u32(&bars->tmem_full[ab]));
+                umma_commit_pair(map_to_cta(smem_u32(&bars->tmem_full[ab]), 1u));
+              }
+              __syncwarp();
             }
-            __syncwarp();
           }
         }
       }
@@ -213,56 +280,78 @@ struct TcGemmF32H2 {
         float acc[PIECES * 32];
 #pragma unroll
         for (int i = 0; i < PIECES * 32; ++i) acc[i] = 0.f;
-        const float* sa = p.scale_a + static_cast<size_t>(w.kb0) * p.scale_lda + w.m0 + rank * 128 + row_in_acc;
-        const float* sb = p.scale_b + static_cast<size_t>(w.kb0) * p.scale_ldb + ((w.n0 + col_half0) >> 6);
         // the factors of this warp's columns, PIECES of them in a lane (those past the edge are read, not used)
         float columns[PIECES];
 #pragma unroll
         for (int i = 0; i < PIECES; ++i) columns[i] = __ldcg(p.columns + w.n0 + col_half0 + lane * PIECES + i);
         float next_a = 0.f, next_b[CHUNKS];
-        auto fetch = [&]() {  // the factors of a chunk, one chunk ahead of its products
-          next_a = __ldcg(sa);
+        int at_a = 0, at_b[CHUNKS];  // where the factors of the next chunk lie
+        auto fetch = [&]() {     // them, one chunk ahead of its products, without the slots of far parts
+          auto power = [](float factor) { return __uint_as_float(__float_as_uint(factor) & ~H2_SLOT_BITS); };
+          next_a = power(__ldcg(p.scale_a + at_a));
+          at_a += p.scale_lda;
 #pragma unroll
-          for (int i = 0; i < CHUNKS; ++i) next_b[i] = __ldcg(sb + i);
-          sa += p.scale_lda;
-          sb += p.scale_ldb;
+          for (int i = 0; i < CHUNKS; ++i) {
+            next_b[i] = power(__ldcg(p.scale_b + at_b[i]));
+            at_b[i] += p.scale_ldb;
+          }
         };
-        if (w.kbn > 0) fetch();
-        for (int kb = 0; kb < w.kbn; ++kb, ++it) {
-          const uint32_t ab = it & 1u;
-          float f[CHUNKS];
+        Chunks ch(p, w);
+        for (bool more = w.kbn > 0; more; more = far) {
+          if (far && !ch.template next<true>()) break;
+          const int run = far ? ch.run : w.kbn;
+          const int kb0 = far ? ch.kb : w.kb0;
+          at_a = kb0 * p.scale_lda + w.m0 + static_cast<int>(rank) * 128 + row_in_acc;
 #pragma unroll
-          for (int i = 0; i < CHUNKS; ++i) f[i] = next_a * next_b[i];
-          if (kb + 1 < w.kbn) fetch();
-          // A warp whose wait ran out stops reading tensor memory but keeps walking the unit's chunks (their waits return
-          // at once under the abort flag), so that all eight reach the vote below together.
-          if (ok) {
-            const bool got = mbar_wait(&bars->tmem_full[ab], (it >> 1) & 1u, &bars->abort_flag);
-            if (!__all_sync(0xffffffffu, got)) {
-              if (lane == 0) report(p, bars, KCG_ST_TIMEOUT_EPILOGUE, it, ab);
-              ok = false;
+          for (int i = 0; i < CHUNKS; ++i) at_b[i] = kb0 * p.scale_ldb + ((w.n0 + col_half0) >> 6) + i;
+          if (ch.far_a()) {
+            const int slot = ch.slot_a(kb0, static_cast<int>(rank));
+            at_a = slot > 0 ? p.far_scale_a + (slot - 1) * 128 + row_in_acc : p.far_zero_a;
+          }
+          if (ch.far_b()) {
+#pragma unroll
+            for (int i = 0; i < CHUNKS; ++i) {
+              const int slot = ch.slot_b(kb0, (col_half0 >> 6) + i);
+              at_b[i] = slot > 0 ? p.far_scale_b + slot - 1 : p.far_zero_b;
             }
           }
-          if (!ok) continue;
-          tc_fence_after_sync();
-          const uint32_t tmem_acc = tmem_base + ab * kBN + col_half0 + (static_cast<uint32_t>(q * 32) << 16);
+          fetch();
+          for (int j = 0; j < run; ++j, ++it) {
+            const uint32_t ab = it & 1u;
+            float f[CHUNKS];
 #pragma unroll
-          for (int c = 0; c < PIECES; ++c) {
-            uint32_t r[32];
-            tmem_ld_32x32b_x32(tmem_acc + c * 32, r);
-            tmem_ld_wait();
-            const float2 f2 = make_float2(f[c / 2], f[c / 2]);
-#pragma unroll
-            for (int i = 0; i < 32; i += 2) {  // (the factor is a power of two: its product is exact)
-              float* x = acc + c * 32 + i;
-              const float2 y = __ffma2_rn(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), f2,
-                                          make_float2(x[0], x[1]));
-              x[0] = y.x, x[1] = y.y;
+            for (int i = 0; i < CHUNKS; ++i) f[i] = next_a * next_b[i];
+            if (j + 1 < run) fetch();
+            // A warp whose wait ran out stops reading tensor memory but keeps walking the unit's chunks (their waits return
+            // at once under the abort flag), so that all eight reach the vote below together.
+            if (ok) {
+              const bool got = mbar_wait(&bars->tmem_full[ab], (it >> 1) & 1u, &bars->abort_flag);
+              if (!__all_sync(0xffffffffu, got)) {
+                if (lane == 0) report(p, bars, KCG_ST_TIMEOUT_EPILOGUE, it, ab);
+                ok = false;
+              }
             }
+            if (!ok) continue;
+            tc_fence_after_sync();
+            const uint32_t tmem_acc = tmem_base + ab * kBN + col_half0 + (static_cast<uint32_t>(q * 32) << 16);
+#pragma unroll
+            for (int c = 0; c < PIECES; ++c) {
+              uint32_t r[32];
+              tmem_ld_32x32b_x32(tmem_acc + c * 32, r);
+              tmem_ld_wait();
+              const float2 f2 = make_float2(f[c / 2], f[c / 2]);
+#pragma unroll
+              for (int i = 0; i < 32; i += 2) {  // (the factor is a power of two: its product is exact)
+                float* x = acc + c * 32 + i;
+                const float2 y = __ffma2_rn(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), f2,
+                                            make_float2(x[0], x[1]));
+                x[0] = y.x, x[1] = y.y;
+              }
+            }
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster_cta(map_to_cta(smem_u32(&bars->tmem_empty[ab]), 0u));  // (the reads are complete)
           }
-          tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive_cluster_cta(map_to_cta(smem_u32(&bars->tmem_empty[ab]), 0u));  // (the reads are complete)
         }
         // The accumulating warps leave a unit as one: the store meets on a named barrier.
         ok = named_bar_all(2, NUM_EPI_THREADS, ok);
@@ -346,6 +435,48 @@ struct TcGemmF32H2 {
       if (lane == 0) tma_store_wait_read<0>();  // shared memory outlives the stores' reads
       __syncwarp();
     }
+  }
+
+  // What the split found; with H2_UNSPLIT nothing was computed.
+  __device__ static __forceinline__ uint32_t multiply(const KcgGemmParams& p) {
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                               ~static_cast<uintptr_t>(1023));
+    Barriers* bars = reinterpret_cast<Barriers*>(smem + RING_BYTES + STORE_BYTES);
+    const int warp = threadIdx.x >> 5;
+
+    if (threadIdx.x == 0) {
+      for (int s = 0; s < kStages; ++s) {
+        mbar_init(&bars->full[s], 1);
+        mbar_init(&bars->empty[s], 1);
+      }
+      for (int a = 0; a < 2; ++a) {
+        mbar_init(&bars->tmem_full[a], 1);
+        mbar_init(&bars->tmem_empty[a], 16);  // one arrival per accumulating warp of each CTA
+      }
+      bars->abort_flag = 0u;
+      bars->last_flag = 0u;
+      fence_mbar_init();
+      fence_proxy_async_smem();
+      tma_prefetch_desc(&p.tmWs);
+    }
+    if (warp == 1) tmem_alloc_pair(&bars->tmem_base, TMEM_COLS);
+    tc_fence_before_sync();
+    __syncthreads();
+    cluster_sync_all();  // the peer's barriers exist before anyone signals them
+    tc_fence_after_sync();
+    const uint32_t tmem_base = bars->tmem_base;
+    const uint32_t rank = cluster_cta_rank();  // 0 = leader
+
+    griddep_wait();  // the parts, their exponents and the words are written by the kernel before this one
+    const uint32_t found = __ldcg(p.h2_words + H2_FOUND);
+    const bool unsplit = (found & H2_UNSPLIT) != 0u;
+
+    if (unsplit) {
+      // (no role runs; the right to allocate tensor memory is kept for the other kernel)
+    } else {
+      roles(p, smem, bars, tmem_base, rank, (found & H2_FAR) != 0u);
+    }
 
     // ------------------------------------------------------------ common exit
     __syncwarp();
@@ -375,17 +506,21 @@ struct TcGemmF32H2 {
       }
       __syncthreads();
     }
-    return unsplit;
+    return found;
   }
 
   __device__ static void run(const KcgGemmParams& p) {
     // No words: the launch had no memory for the parts and no kernel before it has written any.
-    if (p.h2_words == nullptr || multiply(p)) Fallback::run(p);
-    // Every CTA has read the word: the last one clears it for the stream's next launch.
+    const uint32_t found = p.h2_words == nullptr ? H2_UNSPLIT : multiply(p);
+    if (found & H2_UNSPLIT) Fallback::run(p);
+    // Every CTA has read the word: the last one clears them all for the stream's next launch.
     if (p.h2_words != nullptr && threadIdx.x == 0) {
-      if (atomicAdd(p.h2_words + 1, 1u) == gridDim.x - 1) {
-        p.h2_words[1] = 0u;
-        p.h2_words[0] = 0u;
+      if (atomicAdd(p.h2_words + H2_DONE, 1u) == gridDim.x - 1) {
+        p.h2_words[H2_DONE] = 0u;
+        if (found != 0u) {
+          p.h2_words[H2_FOUND] = 0u;
+          for (int i = H2_LINE; i < H2_WORDS; i += H2_LINE) p.h2_words[i] = 0u;
+        }
       }
     }
   }

@@ -315,3 +315,106 @@ def test_parts_larger_than_any_workspace():
     kern.checkStatus()
     _as_tf32(M, N, K, 256).run(a, b, want)
     assert torch.equal(c, want)
+
+
+def _spread(kind, gen):
+    """Operands in which some values lie 2^-34 .. 2^-45 below the largest beside them (none is a power of two)."""
+    M, N, K = 1280, 832, 1092
+    a, b = [torch.rand(s, generator=gen) + 0.5 for s in ((M, K), (K, N))]
+    small = lambda n: (torch.rand(n, generator=gen) + 0.5) * torch.exp2(-torch.randint(35, 46, (n,), generator=gen).float())
+    if kind in ("a", "both"):  # of the first and the last panel of rows and chunk of K, many of one chunk
+        for row, k in ((0, 3), (129, 64), (1279, 1091), (700, 640)):
+            a[row, k] = small(1)[0]
+        a[300:340, 100:110] = small(400).view(40, 10)
+    if kind in ("b", "both"):
+        for k, col in ((1, 2), (64, 100), (1091, 831), (641, 300)):
+            b[k, col] = small(1)[0]
+        b[684:700, 450:470] = small(320).view(16, 20)
+    # a row and a column of small values alone but for one, which faces zeros
+    a[300] = torch.where(a[300] > 1e-6, 0.0, a[300])
+    b[:, 455] = torch.where(b[:, 455] > 1e-6, 0.0, b[:, 455])
+    a[300, 64], b[64], b[640, 455], a[:, 640] = 1.0, 0.0, 1.0, 0.0
+    return a.cuda(), b.cuda()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["a", "b", "both"])
+@pytest.mark.parametrize("bn,split", [(128, 1), (128, 3), (256, 1), (256, 2)])
+def test_far_parts(kind, bn, split):
+    """A few chunks with values far below the largest beside them: multiplied once more, not the whole product as 3xTF32; every
+    value as close as 3xTF32 guarantees, in every call and beside a fused epilogue, and the next call not affected."""
+    gen = torch.Generator().manual_seed(21)
+    a, b = _spread(kind, gen)
+    (M, K), N = a.shape, b.shape[1]
+    kern, other = _kernel(M, N, K, bn, split), _as_tf32(M, N, K, bn)
+    c, tf32 = [torch.empty((M, N), device="cuda") for _ in range(2)]
+    other.run(a, b, tf32)
+    ref = a.double() @ b.double()
+    bias = torch.rand(N, generator=gen).cuda()
+    first = None
+    for _ in range(3):
+        c.fill_(float("nan"))
+        kern.run(a, b, c)
+        kern.checkStatus()
+        assert ((c.double() - ref).abs() <= _bound(a, b)).all()
+        assert first is None or torch.equal(c, first)  # whichever slots the chunks got
+        first = c.clone()
+    err = [float((t.double() - ref).norm() / ref.norm()) for t in (first, tf32)]
+    assert err[0] < 0.6 * err[1], err  # (its own result, not 3xTF32's)
+    assert (first[300].abs().max() > 0) == (kind != "b") and (first[:, 455].abs().max() > 0) == (kind != "a")
+    kern.run(a, b, c, bias=bias, relu=True)
+    assert torch.equal(c, (first + bias).clamp(min=0))
+    plain = [t.clamp(min=0.25) for t in (a, b)]
+    kern.run(*plain, c)
+    kern.checkStatus()
+    ref = plain[0].double() @ plain[1].double()
+    assert ((c.double() - ref).abs() <= _bound(*plain)).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("operand", ["a", "b"])
+def test_more_far_values_than_slots(operand, monkeypatch):
+    """Far values in every chunk, or below far values: the whole product as 3xTF32, bit for bit, and the next call as ever."""
+    monkeypatch.setenv("KCG_TAIL_SPLIT", "0")  # (each kernel's own cuts into K ranges would sum in another order)
+    M, N, K = 1280, 832, 1024
+    gen = torch.Generator().manual_seed(22)
+    plain = [(torch.rand(s, generator=gen) + 0.5).cuda() for s in ((M, K), (K, N))]
+    kern, other = _kernel(M, N, K, 256), _as_tf32(M, N, K, 256)
+    c, before, want = [torch.empty((M, N), device="cuda") for _ in range(3)]
+    kern.run(*plain, before)
+    for every in (True, False):
+        a, b = [t.clone() for t in plain]
+        x = a if operand == "a" else b
+        if every:
+            x[::64, ::64] = 1.2345678 * 2.0 ** -40
+        elif operand == "a":
+            x[9, 70:72] = torch.tensor([1.2345678 * 2.0 ** -34, 1.2345678 * 2.0 ** -70]).cuda()
+        else:
+            x[70:72, 9] = torch.tensor([1.2345678 * 2.0 ** -34, 1.2345678 * 2.0 ** -70]).cuda()
+        other.run(a, b, want)
+        kern.run(a, b, c)
+        kern.checkStatus()
+        assert torch.equal(c, want)
+        kern.run(*plain, c)
+        assert torch.equal(c, before)
+
+
+@pytest.mark.gpu
+def test_far_parts_in_a_graph():
+    """Captured, with a remainder cut into ranges: chunks with far parts in one replay, none in the next, others after that."""
+    M, N, K = 2560, 2304, 1024
+    gen = torch.Generator(device="cuda").manual_seed(23)
+    a, b = [torch.rand(s, generator=gen, device="cuda") + 0.5 for s in ((M, K), (K, N))]
+    kern = _kernel(M, N, K, 256)
+    c, want = [torch.empty((M, N), device="cuda") for _ in range(2)]
+    kern.run(a, b, c)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        kern.run(a, b, c)
+    for row, col, value in ((9, 3, 1.2345678e-12), (9, 3, 0.5), (2559, 1023, 1.2345678e-13), (2559, 1023, float("nan")), (2559, 1023, 0.5)):
+        a[row, col] = b[col, row % N] = value
+        graph.replay()
+        kern.run(a, b, want)
+        assert torch.equal(c.nan_to_num(nan=123.0), want.nan_to_num(nan=123.0))
+        if value == value:
+            assert ((c.double() - a.double() @ b.double()).abs() <= _bound(a, b)).all()
